@@ -179,6 +179,9 @@ def rmsnorm_bwd(dy, x, rstd, w, dw_accum=None):
     if not dy.is_contiguous():
         _no_recording("making a gradient contiguous")
         dy = dy.contiguous()
+    if not x.is_contiguous():             # keys of the packed QKV buffer are rows of a wider buffer
+        _no_recording("making a norm input contiguous")
+        x = x.contiguous()
     rows, H = x.shape
     dx = torch.empty_like(x)
     acc = dw_accum is not None and dw_accum.dtype == torch.float32 and dw_accum.is_contiguous()

@@ -103,6 +103,22 @@ def test_rmsnorm(rows, H):
     assert _rel(dx, dxr) < 5e-3 and _rel(dw, dwr) < 5e-3
 
 
+@pytest.mark.parametrize("rows,H,width", [(257, 128, 640), (64, 1024, 1536)])
+def test_rmsnorm_of_rows_inside_a_wider_buffer(rows, H, width):
+    """Keys of a packed QKV buffer: rows of H elements whose stride is the packed width."""
+    KC = _K()
+    from kareus_b200.kernels import ref
+    x = torch.randn(rows, width, device="cuda").bfloat16()[:, 128:128 + H]
+    dy = torch.randn(rows, width, device="cuda").bfloat16()[:, :H]
+    w = (1 + 0.1 * torch.randn(H, device="cuda")).bfloat16()
+    y, rstd = KC.rmsnorm_fwd(x, w, 1e-6)
+    yr, rr = ref.rmsnorm_fwd(x.float(), w.float(), 1e-6)
+    assert _rel(y, yr) < 5e-3 and _rel(rstd, rr) < 1e-5
+    dx, dw = KC.rmsnorm_bwd(dy, x, rstd, w)
+    dxr, dwr = ref.rmsnorm_bwd(dy.float(), x.float(), rr, w.float())
+    assert _rel(dx, dxr) < 5e-3 and _rel(dw, dwr) < 5e-3
+
+
 def test_rope_strided_views_and_inverse():
     KC = _K()
     from kareus_b200.kernels import ref
