@@ -1,0 +1,333 @@
+// bf16 GEMM on pairs of SMs: one 256 x BN output tile per two-CTA cluster (tcgen05 cta_group::2).
+//
+// Both CTAs of a cluster work on one instruction stream: the leader (even rank) issues M = 256 MMAs
+// whose A rows 0..127 / 128..255 and B rows 0..BN/2-1 / BN/2..BN-1 come from the shared memory of
+// CTA 0 / CTA 1, and each CTA keeps its 128 rows of the accumulator in its own TMEM.  Per SM and
+// 64-deep K step that is 16 KB of A and at most 16 KB of B through L2 and shared memory for
+// 512 tensor clocks, half of the B traffic of a 128x256 tile on one SM, which leaves room in TMEM
+// for two accumulators (the epilogue of a tile runs under the main loop of the next) and in shared
+// memory for six stages.
+//
+//   warp 0      TMA producer of this CTA's halves (both CTAs count on the leader's `full` barriers)
+//   warp 1      MMA issuer (leader CTA only); allocates TMEM in both CTAs
+//   warps 2..9  epilogue: TMEM → registers → 4 KB of swizzled shared memory per warp → TMA store
+//               (bf16 / fp32 output) or TMA reduce-add (fp32 `C +=`: the addition happens in L2, so
+//               nobody waits for the old value and several K parts of a tile may add at once)
+//
+// BN is a run-time multiple of 64 (64..256): the launcher picks the width whose last wave is fullest.
+// Loads use no multicast: every CTA fetches its own halves.
+//
+// What bounds it: at 256 columns the tensor pipe (519 clocks per 64-deep step of 512 needed) and with it the
+// power limit; below that the 64 B per clock that reach an SM.  bf16, us before (one-SM 128x256 and 256x256
+// tiles) / now, one B200 in a loop: 16384 x 16384 x 3072 forward 1180 / 1023, input gradient 1282 / 1154,
+// weight gradient 1523 / 1093; weight gradients 5120 x 3072 488 / 344, 12288 x 2048 (7600 tokens) 502 / 263,
+// 128256 x 3072 (4096 tokens) 4479 / 2335; 640-wide QKV shard 117 / 68 forward.
+#include "sm100.cuh"
+#include "launch.h"
+#include "host_utils.h"
+#include "gemm_plan.h"
+
+namespace kb {
+
+constexpr int GP_BM = 256;                     // rows of a tile (128 per CTA)
+constexpr int GP_BK = 64;
+constexpr int GP_STAGES = 6;
+constexpr int GP_EPI_WARPS = 8;                // 4 TMEM lane quarters x 2 sets of column slabs
+constexpr int GP_THREADS = (2 + GP_EPI_WARPS) * 32;
+constexpr int GP_A_BYTES = 128 * GP_BK * 2;    // 16 KB: this CTA's rows of A
+constexpr int GP_B_BYTES = 128 * GP_BK * 2;    // 16 KB: room for this CTA's rows of B (BN / 2 of them)
+constexpr int GP_STAGE_BYTES = GP_A_BYTES + GP_B_BYTES;
+constexpr int GP_TILE_BYTES = GP_STAGE_BYTES * GP_STAGES;
+constexpr int GP_STG_BYTES = GP_EPI_WARPS * 4096;
+constexpr int GP_SMEM = GP_TILE_BYTES + GP_STG_BYTES + 256 + 1024;
+static_assert(GP_SMEM <= 227 * 1024, "shared memory per CTA");
+
+// Work unit u of a launch → tile and K range.  The first `whole` units are whole tiles; the remaining
+// tiles are cut into `ks` K parts each, part-major (all tiles of part 0, then part 1, ...), so that the
+// clusters that run side by side walk the same K range of neighbouring tiles and share operands in L2.
+struct PairWork {
+  int tiles_m, tiles_n, group_m, nk, whole, split_tiles, ks;
+  __device__ __forceinline__ int units() const { return whole + split_tiles * ks; }
+  __device__ __forceinline__ void decode(int u, int& tm, int& tn, int& kb0, int& kb1) const {
+    int t;
+    if (u < whole) {
+      t = u;
+      kb0 = 0;
+      kb1 = nk;
+    } else {
+      const int r = u - whole;
+      const int part = r / split_tiles;
+      t = whole + r - part * split_tiles;
+      kb0 = split_begin(nk, ks, part);
+      kb1 = split_begin(nk, ks, part + 1);
+    }
+    // m-tiles are taken in groups of `group_m`; inside a group the m index runs fastest, so the tiles in
+    // flight cover a near-square patch of C
+    const int per_group = group_m * tiles_n;
+    const int g = t / per_group;
+    const int first_m = g * group_m;
+    const int gsz = min(group_m, tiles_m - first_m);
+    const int r = t - g * per_group;
+    tm = first_m + r % gsz;
+    tn = r / gsz;
+  }
+};
+
+template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ CUtensorMap tmC, const PairWork w, const int M, const int N, const int bn,
+                 int* status) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + GP_TILE_BYTES + GP_STG_BYTES);   // used in the leader
+  uint64_t* empty = full + GP_STAGES;
+  uint64_t* tfull = empty + GP_STAGES;      // [2]
+  uint64_t* tempty = tfull + 2;             // [2] used in the leader
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = blockIdx.x & 1;          // rank in the cluster (clusters are consecutive pairs of CTAs)
+  const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
+  const int num_units = w.units();
+  const int half_n = bn >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < GP_STAGES; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&tfull[i], 1);
+      mbar_init(&tempty[i], 2 * GP_EPI_WARPS);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                       // the peer's barriers exist before anything arrives on them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ producer (each CTA: its own halves)
+    if (elect_one()) {
+      prefetch_tmap(&tmA);
+      prefetch_tmap(&tmB);
+      // bytes of both CTAs, counted on the leader's barrier; MN-major B comes in whole 64-wide chunks
+      const int b_chunks = (half_n + 63) >> 6;
+      const uint32_t b_bytes = B_MN ? b_chunks * 8192u : static_cast<uint32_t>(half_n) * GP_BK * 2u;
+      const uint32_t stage_tx = 2u * (GP_A_BYTES + b_bytes);
+      const uint32_t full0 = cluster_addr(full, 0);
+      int s = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      for (int u = first; u < num_units && ok; u += step) {
+        int tm, tn, kb0, kb1;
+        w.decode(u, tm, tn, kb0, kb1);
+        const int m0 = tm * GP_BM + rank * 128;
+        const int n0 = tn * bn + rank * half_n;
+        for (int kb_ = kb0; kb_ < kb1; ++kb_) {
+          if (!mbar_wait(&empty[s], ph, abort_flag, status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
+          uint8_t* a_dst = smem + s * GP_STAGE_BYTES;
+          uint8_t* b_dst = a_dst + GP_A_BYTES;
+          const uint32_t bar = full0 + s * 8;
+          if (rank == 0) mbar_expect_tx(&full[s], stage_tx);
+          const int k0 = kb_ * GP_BK;
+          if constexpr (!A_MN) {
+            tma_load_2d_pair(a_dst, &tmA, bar, k0, m0);
+          } else {
+            tma_load_2d_pair(a_dst, &tmA, bar, m0, k0);
+            tma_load_2d_pair(a_dst + 8192, &tmA, bar, m0 + 64, k0);
+          }
+          if constexpr (!B_MN) {
+            tma_load_2d_pair(b_dst, &tmB, bar, k0, n0);
+          } else {
+            tma_load_2d_pair(b_dst, &tmB, bar, n0, k0);
+            if (b_chunks > 1) tma_load_2d_pair(b_dst + 8192, &tmB, bar, n0 + 64, k0);
+          }
+          if (++s == GP_STAGES) { s = 0; ph ^= 1u; }
+        }
+      }
+      if (!ok) {
+        // leave no copy in flight: tile loads land within microseconds, give them 200 us
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 200000ull) {}
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer (leader)
+    // One thread chosen by elect.sync runs the whole role: with `lane == 0` in its place the four MMAs of
+    // a step took 605 clocks at every tile width (512 at 256 columns and 128 at 64 is what they need),
+    // because the compiler then cannot keep descriptors and addresses in uniform registers.
+    if (rank == 0 && elect_one()) {
+      const uint32_t idesc = make_idesc_bf16(GP_BM, bn, A_MN, B_MN);
+      const uint32_t smem0 = smem_u32(smem);
+      const uint64_t ad0 = A_MN ? make_smem_desc(smem0, 8192, 1024) : make_smem_desc(smem0, 16, 1024);
+      const uint64_t bd0 = B_MN ? make_smem_desc(smem0 + GP_A_BYTES, 8192, 1024)
+                                : make_smem_desc(smem0 + GP_A_BYTES, 16, 1024);
+      constexpr uint64_t ka = (A_MN ? 2048 : 32) >> 4, kb = (B_MN ? 2048 : 32) >> 4;   // descriptor step of 16 in K
+      uint32_t tile_i = 0;
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int u = first; u < num_units && ok; u += step, ++tile_i) {
+        int tm, tn, kb0, kb1;
+        w.decode(u, tm, tn, kb0, kb1);
+        const uint32_t buf = tile_i & 1u;
+        if (!mbar_wait(&tempty[buf], ((tile_i >> 1) & 1u) ^ 1u, abort_flag, status, ST_TIMEOUT_TMEM_EMPTY)) break;
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + buf * 256;
+        for (int kb_ = kb0; kb_ < kb1; ++kb_) {
+          if (!mbar_wait(&full[s], ph, abort_flag, status, ST_TIMEOUT_FULL)) { ok = false; break; }
+          tc_fence_after();
+          const uint64_t ad = ad0 + static_cast<uint64_t>(s * (GP_STAGE_BYTES >> 4));
+          const uint64_t bd = bd0 + static_cast<uint64_t>(s * (GP_STAGE_BYTES >> 4));
+#pragma unroll
+          for (int k = 0; k < GP_BK / 16; ++k)
+            umma_ss_pair(d_tmem, ad + k * ka, bd + k * kb, idesc, (kb_ > kb0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(&empty[s]);                              // both CTAs may refill the stage
+          if (kb_ == kb1 - 1) umma_commit_pair(&tfull[buf]);        // both CTAs' halves are complete
+          if (++s == GP_STAGES) { s = 0; ph ^= 1u; }
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ epilogue
+    const int q = warp & 3;                   // TMEM lane quarter
+    const int h = (warp - 2) >> 2;            // this warp takes the column slabs h, h + 2, ...
+    uint8_t* stg = smem + GP_TILE_BYTES + (warp - 2) * 4096;
+    constexpr int SLAB = OUT_F32 ? 32 : 64;   // output columns of one 128-byte wide slab
+    const int slabs = bn / SLAB;
+    const uint32_t stg_row = smem_u32(stg) + lane * 128;
+    uint32_t tile_i = 0;
+    for (int u = first; u < num_units; u += step, ++tile_i) {
+      int tm, tn, kb0, kb1;
+      w.decode(u, tm, tn, kb0, kb1);
+      const uint32_t buf = tile_i & 1u;
+      if (!mbar_wait(&tfull[buf], (tile_i >> 1) & 1u, abort_flag, status, ST_TIMEOUT_TMEM_FULL)) break;
+      tc_fence_after();
+      const int row0 = tm * GP_BM + rank * 128 + q * 32;
+      const uint32_t taddr = tmem_base + buf * 256 + (static_cast<uint32_t>(q * 32) << 16);
+#pragma unroll 1
+      for (int c = h; c < slabs; c += 2) {
+        uint32_t o[32];
+        if constexpr (OUT_F32) {
+          tmem_ld_32x32(taddr + c * 32, o);
+          tmem_ld_wait();
+        } else {
+          uint32_t v0[32], v1[32];
+          tmem_ld_32x32(taddr + c * 64, v0);
+          tmem_ld_32x32(taddr + c * 64 + 32, v1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            o[j] = pack_bf16x2(__uint_as_float(v0[2 * j]), __uint_as_float(v0[2 * j + 1]));
+            o[16 + j] = pack_bf16x2(__uint_as_float(v1[2 * j]), __uint_as_float(v1[2 * j + 1]));
+          }
+        }
+        if (c + 2 >= slabs) {
+          // this warp's last read of the accumulator: hand it back before the stores go out
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(cluster_addr(&tempty[buf], 0));
+        }
+        if (lane == 0) tma_store_wait_read<0>();      // the previous slab has left the staging buffer
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          st_shared_v4(stg_row + ((j ^ (lane & 7)) << 4), o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        const int col = tn * bn + c * SLAB;
+        if (lane == 0 && row0 < M && col < N) {       // the tensor map clips what crosses the edge
+          if constexpr (ACCUM) tma_reduce_add_2d(&tmC, stg, col, row0);
+          else tma_store_2d(&tmC, stg, col, row0);
+          tma_store_commit();
+        }
+      }
+      if (slabs <= h) {                               // no slab for this warp (narrow tile): release all the same
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(cluster_addr(&tempty[buf], 0));
+      }
+    }
+    if (lane == 0) tma_store_wait<0>();               // nothing in flight out of shared memory at exit
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                                 // the peer's MMAs and arrivals no longer touch this CTA
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, 512);
+  }
+}
+
+template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
+static int launch_pair(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
+                       const PairPlan& pl, int pairs, int* status, cudaStream_t stream) {
+  CUtensorMap tmA, tmB, tmC;
+  int rc;
+  if (!A_MN) rc = make_tmap_2d_bf16(&tmA, A, K, M, lda, GP_BK, 128);
+  else       rc = make_tmap_2d_bf16(&tmA, A, M, K, lda, 64, GP_BK);
+  if (rc) return rc;
+  if (!B_MN) rc = make_tmap_2d_bf16(&tmB, B, K, N, ldb, GP_BK, pl.bn / 2);
+  else       rc = make_tmap_2d_bf16(&tmB, B, N, K, ldb, 64, GP_BK);
+  if (rc) return rc;
+  {
+    const uint64_t dims[2] = {(uint64_t)N, (uint64_t)M};
+    const uint64_t str[1] = {(uint64_t)ldc * (OUT_F32 ? 4 : 2)};
+    const uint32_t box[2] = {OUT_F32 ? 32u : 64u, 32u};
+    rc = make_tmap(&tmC, C, OUT_F32 ? 4 : 2, 2, dims, str, box, 3);
+    if (rc) return rc;
+  }
+  auto kern = gemm_pair_kernel<A_MN, B_MN, OUT_F32, ACCUM>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM);
+    if (e != cudaSuccess) return 1000 + static_cast<int>(e);
+    configured = true;
+  }
+  PairWork w;
+  w.tiles_m = (M + GP_BM - 1) / GP_BM;
+  w.tiles_n = (N + pl.bn - 1) / pl.bn;
+  w.nk = (K + GP_BK - 1) / GP_BK;
+  w.ks = ACCUM ? pl.ks : 1;
+  const int tiles = w.tiles_m * w.tiles_n;
+  w.split_tiles = w.ks > 1 ? pl.split_tiles : 0;
+  w.whole = tiles - w.split_tiles;
+  // m-tiles per group: about 24 MB of A rows, at most 16 tiles
+  const long panel = (long)GP_BM * K * 2;
+  long gm = (24L << 20) / panel;
+  gm = gm < 8 ? 8 : gm > 16 ? 16 : gm;
+  w.group_m = gm < w.tiles_m ? (int)gm : w.tiles_m;
+  const int units = w.whole + w.split_tiles * w.ks;
+  const int grid = 2 * (units < pairs ? units : pairs);
+  KB_LAUNCH(kern, grid, GP_THREADS, GP_SMEM, stream, tmA, tmB, tmC, w, M, N, pl.bn, status);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 2000 + static_cast<int>(e);
+}
+
+int gemm_pair_dispatch(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda, int b_mn, int ldb,
+                       int ldc, int out_f32, int accumulate, const PairPlan& pl, int pairs, int* status,
+                       cudaStream_t stream) {
+#define GP_GO(AM, BM_)                                                                                         \
+  do {                                                                                                         \
+    if (out_f32 && accumulate) return launch_pair<AM, BM_, true, true>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, status, stream); \
+    if (out_f32) return launch_pair<AM, BM_, true, false>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, status, stream);              \
+    return launch_pair<AM, BM_, false, false>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, status, stream);                          \
+  } while (0)
+  if (!a_mn && !b_mn) GP_GO(false, false);
+  if (!a_mn && b_mn) GP_GO(false, true);
+  if (a_mn && !b_mn) GP_GO(true, false);
+  GP_GO(true, true);
+#undef GP_GO
+}
+
+}  // namespace kb

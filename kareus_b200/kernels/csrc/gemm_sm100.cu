@@ -14,12 +14,10 @@
 #include "sm100.cuh"
 #include "launch.h"
 #include "host_utils.h"
+#include "gemm_plan.h"
 #include <stdlib.h>
 
 namespace kb {
-
-int gemm256_dispatch(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda, int b_mn, int ldb,
-                     int ldc, int out_f32, int accumulate, int num_sms, int ks, int* status, cudaStream_t stream);
 
 constexpr int GEMM_BM = 128;
 constexpr int GEMM_BK = 64;
@@ -115,7 +113,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (elect_one()) {
       prefetch_tmap(&tmA);
       prefetch_tmap(&tmB);
       uint32_t it = 0;
@@ -160,6 +158,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint32_t it = 0;
     uint32_t tile_i = 0;
     bool ok = true;
+    if (elect_one())             // one thread runs the role, see elect_one()
     for (int u = blockIdx.x; u < num_units && ok; u += gridDim.x, ++tile_i) {
       const uint32_t buf = tile_i & 1u;
       const uint32_t bph = (tile_i >> 1) & 1u;
@@ -172,23 +171,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const uint32_t ph = (it / GEMM_STAGES) & 1u;
         if (!mbar_wait(&full[s], ph, abort_flag, status, ST_TIMEOUT_FULL)) { ok = false; break; }
         tc_fence_after();
-        if (lane == 0) {
-          const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
-          const uint32_t b_addr = a_addr + S::A_BYTES;
+        const uint32_t a_addr = smem_u32(smem + s * S::STAGE_BYTES);
+        const uint32_t b_addr = a_addr + S::A_BYTES;
 #pragma unroll
-          for (int k = 0; k < GEMM_BK / 16; ++k) {
-            const uint64_t ad = A_MN ? make_smem_desc(a_addr + k * 2048, 8192, 1024)
-                                     : make_smem_desc(a_addr + k * 32, 16, 1024);
-            const uint64_t bd = B_MN ? make_smem_desc(b_addr + k * 2048, 8192, 1024)
-                                     : make_smem_desc(b_addr + k * 32, 16, 1024);
-            umma_ss(d_tmem, ad, bd, idesc, (kb_ > kb0 || k > 0) ? 1u : 0u);
-          }
-          umma_commit(&empty[s]);                       // stage reusable once these MMAs retire
-          if (kb_ == kb1 - 1) umma_commit(&tfull[buf]); // accumulator complete
+        for (int k = 0; k < GEMM_BK / 16; ++k) {
+          const uint64_t ad = A_MN ? make_smem_desc(a_addr + k * 2048, 8192, 1024)
+                                   : make_smem_desc(a_addr + k * 32, 16, 1024);
+          const uint64_t bd = B_MN ? make_smem_desc(b_addr + k * 2048, 8192, 1024)
+                                   : make_smem_desc(b_addr + k * 32, 16, 1024);
+          umma_ss(d_tmem, ad, bd, idesc, (kb_ > kb0 || k > 0) ? 1u : 0u);
         }
-        __syncwarp();
+        umma_commit(&empty[s]);                       // stage reusable once these MMAs retire
+        if (kb_ == kb1 - 1) umma_commit(&tfull[buf]); // accumulator complete
       }
     }
+    __syncwarp();
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..5)
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
@@ -362,74 +359,65 @@ static int dispatch_out(const void* A, const void* B, void* C, int M, int N, int
   return launch_gemm<BN, A_MN, B_MN, false, false>(A, B, C, M, N, K, lda, ldb, ldc, num_sms, 1, status, stream, ep);
 }
 
-// ----------------------------------------------------------------------------- split-K choice
-// Modelled time of an accumulating GEMM in units of one 64-deep K step of a 128x256 tile (~0.4 us):
-// `waves` rounds of one unit each; a unit costs its K steps plus a fixed part (pipeline fill, epilogue,
-// and with ks > 1 the reductions that every part sends to C).  Constants fitted to a sweep over the
-// weight-gradient shapes of a 3B Llama layer at tensor-parallel sizes 1, 2 and 8 on a B200:
-//   step   1.0 (128x256), 0.6 (128x128), 1.85 (256x256: twice the FLOPs, a little less L2 traffic per
-//          FLOP)
-//   fixed  14 + 2 ks (128-row tiles), 26 + 3 ks (256x256)
-static inline double model_time(long tiles, int ks, int nk, int grid, double step, double fixed0, double fixed_ks) {
-  const long units = tiles * ks;
-  const long waves = (units + grid - 1) / grid;
-  return waves * (static_cast<double>((nk + ks - 1) / ks) * step + fixed0 + fixed_ks * ks);
+// ----------------------------------------------------------------------------- tile and split choice
+static int g_force_bn = 0, g_force_ks = 0, g_force_single = 0;   // measurement and test overrides, see below
+
+static bool split_allowed() {
+  static const bool allow = [] { const char* e = getenv("KB_GEMM_SPLITK"); return !(e && e[0] == '0'); }();
+  return allow;
 }
 
-struct SplitChoice {
-  int ks;
-  double time;
-};
-static SplitChoice choose_split(long tiles, int nk, int grid, double step, double fixed0, double fixed_ks) {
-  static const bool allow = [] { const char* e = getenv("KB_GEMM_SPLITK"); return !(e && e[0] == '0'); }();
-  SplitChoice best{1, model_time(tiles, 1, nk, grid, step, fixed0, fixed_ks)};
-  if (!allow) return best;
-  for (int ks = 2; ks <= 8; ++ks) {
-    if (nk / ks < 8) break;
-    const double t = model_time(tiles, ks, nk, grid, step, fixed0, fixed_ks);
-    if (t < best.time * 0.97) best = SplitChoice{ks, t};       // a split must pay for its extra traffic
+// Modelled time of the two-SM kernel at tile width `bn`, in 64-deep K steps of a 256 x 256 tile.
+static PairPlan plan_pair_width(int M, int N, int K, int pairs, int bn, bool accumulate) {
+  // Measured per step: a step moves 16 KB of A and bn / 256 x 16 KB of B into each SM, which takes about 64 B per
+  // clock whatever the width, so narrow tiles are bound by that and not by the tensor pipe (16384 x 16384 x 3072,
+  // us per step: 0.381 at 256 columns, 0.312 at 192, 0.266 at 128, 0.229 at 64).
+  static const double step_cost[5] = {0, 0.60, 0.70, 0.82, 1.0};
+  const int nk = (K + GEMM_BK - 1) / GEMM_BK;
+  const double step = step_cost[bn / 64], fixed = 3.0;
+  const long tiles = (long)((M + 255) / 256) * ((N + bn - 1) / bn);
+  const long full_waves = tiles / pairs, rest = tiles - full_waves * pairs;
+  const double base = full_waves * (nk * step + fixed);
+  PairPlan best{bn, 1, 0, base + (rest ? nk * step + fixed : 0.0) + 4.0};
+  if (accumulate && rest && split_allowed())
+    for (int ks = 2; ks <= 8 && nk / ks >= 8; ++ks) {
+      const long waves = (rest * ks + pairs - 1) / pairs;
+      const double t = base + waves * ((nk + ks - 1) / ks * step + fixed) + 4.0;
+      if (t < best.cost * 0.97) best = PairPlan{bn, ks, (int)rest, t};   // a split must pay for its extra additions
+    }
+  return best;
+}
+
+static PairPlan plan_pair(int M, int N, int K, int pairs, bool accumulate) {
+  PairPlan best = plan_pair_width(M, N, K, pairs, 256, accumulate);
+  for (int bn = 192; bn >= 64; bn -= 64) {
+    const PairPlan p = plan_pair_width(M, N, K, pairs, bn, accumulate);
+    if (p.cost < best.cost) best = p;
   }
   return best;
 }
 
-// Accumulating output (weight gradients: few tiles, long K): tile and K split by modelled time.
-struct AccumPlan {
-  bool tile256;
-  int ks;
-};
-static int g_force_tile = 0, g_force_ks = 0;   // measurement override, see kb_gemm_accum_force
-static AccumPlan plan_accumulate(int M, int N, int K, int num_sms, bool fits256) {
-  const int nk = (K + GEMM_BK - 1) / GEMM_BK;
-  if (g_force_ks > 0) {
-    const int ks = g_force_ks <= nk ? g_force_ks : nk;
-    return AccumPlan{g_force_tile == 256 && fits256, ks};
-  }
-  const bool narrow = (N <= 128) || (N % 256 != 0 && N % 256 <= 128);
-  const int bn = narrow ? 128 : 256;
-  const long tiles128 = (long)((M + GEMM_BM - 1) / GEMM_BM) * ((N + bn - 1) / bn);
-  const SplitChoice c128 = choose_split(tiles128, nk, num_sms, narrow ? 0.6 : 1.0, 14.0, 2.0);
-  if (fits256) {
-    const long tiles256 = (long)((M + 255) / 256) * ((N + 255) / 256);
-    const SplitChoice c256 = choose_split(tiles256, nk, num_sms, 1.85, 26.0, 3.0);
-    if (c256.time < c128.time) return AccumPlan{true, c256.ks};
-  }
-  return AccumPlan{false, c128.ks};
-}
-
 }  // namespace kb
 
-// Tile (128 or 256 rows) and K split that kb_gemm_bf16 uses for an accumulating fp32 output of this shape.
+// Tile rows (256: the two-SM kernel) and K split of the tiles after the last full wave that kb_gemm_bf16 uses for
+// an accumulating fp32 output of this shape.
 extern "C" void kb_gemm_accum_plan(int M, int N, int K, int num_sms, int* tile_rows, int* ks) {
-  const bool fits256 = M >= 512 && N >= 512 && K >= 2048 && (N % 256 == 0 || N >= 4096);
-  const kb::AccumPlan pl = kb::plan_accumulate(M, N, K, num_sms, fits256);
-  *tile_rows = pl.tile256 ? 256 : 128;
+  const kb::PairPlan pl = kb::plan_pair(M, N, K, num_sms / 2, true);
+  *tile_rows = 256;
   *ks = pl.ks;
 }
 
-// Measurement aid: force the tile (128 / 256) and K split of accumulating GEMMs; ks = 0 returns to the model.
+// Measurement aid: force the tile rows (128 / 256) and K split of accumulating GEMMs; ks = 0 returns to the model.
 extern "C" void kb_gemm_accum_force(int tile_rows, int ks) {
-  kb::g_force_tile = tile_rows;
+  kb::g_force_single = ks > 0 && tile_rows == 128 ? 256 : 0;
   kb::g_force_ks = ks;
+}
+
+// Measurement aid: force the tile width of the two-SM kernel (64..256), or with a negative width the one-SM
+// kernel (-128 / -256); 0 returns to the model.
+extern "C" void kb_gemm_force_width(int bn) {
+  kb::g_force_bn = bn > 0 ? bn : 0;
+  kb::g_force_single = bn < 0 ? -bn : 0;
 }
 
 // C[M,N] (+)= op(A) * op(B)^T.
@@ -451,26 +439,24 @@ extern "C" int kb_gemm_bias_act_bf16(const void* A, const void* B, void* C, int 
   if ((lda & 7) || (ldb & 7) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
     return ST_BAD_ARG;
   if (num_sms <= 0) num_sms = device_sm_count();
-  int ks = 1;
-  {
-    // large problems with a long K loop: 256x256 tile per SM (a third less L2 traffic per FLOP; its
-    // epilogue is not overlapped, which only pays off when the main loop is long), see gemm256_sm100.cu
-    static const bool allow256 = [] { const char* e = getenv("KB_GEMM256"); return !(e && e[0] == '0'); }();
-    const long tiles256 = (long)((M + 255) / 256) * ((N + 255) / 256);
-    const bool fits256 = plain && allow256 && M >= 512 && N >= 512 && K >= 2048 && (N % 256 == 0 || N >= 4096);
-    if (fits256 && !(out_f32 && accumulate) && tiles256 >= num_sms)
-      return gemm256_dispatch(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, num_sms, 1, status,
-                              stream);
-    if (out_f32 && accumulate) {
-      const AccumPlan pl = plan_accumulate(M, N, K, num_sms, fits256);
-      ks = pl.ks;
-      if (pl.tile256)
-        return gemm256_dispatch(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, num_sms, pl.ks,
-                                status, stream);
+  if (accumulate && !out_f32) return ST_BAD_ARG;
+  // The two-SM kernel stores through TMA: 16-byte aligned output rows.
+  const bool tma_out = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc & (out_f32 ? 3 : 7)) == 0;
+  if (plain && tma_out && num_sms >= 2 && !g_force_single) {
+    const int pairs = num_sms / 2;
+    PairPlan pl = g_force_bn ? plan_pair_width(M, N, K, pairs, g_force_bn, accumulate != 0)
+                             : plan_pair(M, N, K, pairs, accumulate != 0);
+    if (g_force_ks > 0 && accumulate) {
+      const int nk = (K + GEMM_BK - 1) / GEMM_BK;
+      pl.ks = g_force_ks <= nk ? g_force_ks : nk;
+      pl.split_tiles = ((M + 255) / 256) * ((N + pl.bn - 1) / pl.bn);
     }
+    return gemm_pair_dispatch(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, pl, pairs, status, stream);
   }
+  int ks = 1;
+  if (g_force_ks > 0 && accumulate) ks = g_force_ks <= (K + GEMM_BK - 1) / GEMM_BK ? g_force_ks : (K + GEMM_BK - 1) / GEMM_BK;
   // narrow outputs waste less of the last wave with the 128-wide tile
-  const bool narrow = (N <= 128) || (N % 256 != 0 && N % 256 <= 128);
+  const bool narrow = g_force_single ? g_force_single == 128 : (N <= 128) || (N % 256 != 0 && N % 256 <= 128);
 #define KB_GO(BN_)                                                                                         \
   do {                                                                                                     \
     if (!a_mn && !b_mn) return dispatch_out<BN_, false, false>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, accumulate, num_sms, ks, status, stream, ep); \

@@ -44,6 +44,37 @@ def test_gemm_layouts(M, N, K, ta, tb):
         assert _rel(acc, want2) < 2e-3
 
 
+@pytest.mark.parametrize("bn", [64, 128, 192, 256])
+@pytest.mark.parametrize("M,N,K", [(8, 8, 8), (136, 72, 64), (257, 264, 400), (600, 520, 136), (2000, 1096, 720)])
+@pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, False), (True, True)])
+def test_two_sm_gemm_tile_edges(bn, M, N, K, ta, tb):
+    """Every tile width of the two-SM kernel at the edges of its tiles (256 rows, bn columns, 64-deep steps, parts
+    of less than a tile included).  bf16 results are within one rounding of the fp32 product (2^-9 relative, as a
+    norm), fp32 sums within fp32 accumulation of exact bf16 products."""
+    import ctypes
+    KC = _K()
+    L = KC.lib()
+    L.kb_gemm_force_width.argtypes = [ctypes.c_int]
+    L.kb_gemm_force_width.restype = None
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N * 3 + K)
+    a = torch.randn((K, (M + 7) // 8 * 8) if ta else (M, K), device="cuda", generator=g).bfloat16()
+    a = a[:, :M] if ta else a
+    b = torch.randn((N, K) if tb else (K, N), device="cuda", generator=g).bfloat16()
+    want = (a.double().t() if ta else a.double()) @ (b.double().t() if tb else b.double())
+    acc = torch.randn(M, N, device="cuda", generator=g)
+    want_acc = acc.double() + want
+    try:
+        L.kb_gemm_force_width(bn)
+        c = KC.gemm(a, b, trans_a=ta, trans_b=tb)
+        f = KC.gemm(a, b, trans_a=ta, trans_b=tb, out_dtype=torch.float32)
+        KC.gemm(a, b, trans_a=ta, trans_b=tb, accumulate=acc)
+        KC.check_status()
+    finally:
+        L.kb_gemm_force_width(0)
+    assert _rel(c, want.float()) < 2 ** -8
+    assert _rel(f, want.float()) < 1e-5 and _rel(acc, want_acc.float()) < 1e-5
+
+
 @pytest.mark.parametrize("tile,ks", [(128, 2), (128, 3), (128, 7), (256, 2), (256, 5)])
 @pytest.mark.parametrize("n_out,n_in,tokens", [(640, 3072, 4096), (3072, 384, 2048), (1024, 1024, 8192),
                                                (520, 776, 4096)])
