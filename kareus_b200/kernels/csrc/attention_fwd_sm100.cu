@@ -1,18 +1,21 @@
 // Causal GQA flash-attention forward for sm_100a, head dim 128, bf16 in / bf16 out, fp32 softmax.
 //
-// One CTA owns a tile of 128 query rows of one (batch, head) and walks the visible key tiles:
-//   warp 0      TMA producer: Q once, then K and V tiles into a 2-stage ring (128B swizzle)
-//   warp 1      MMA issuer:   S = Q·Kᵀ (tcgen05, accumulator in TMEM, double buffered) and
-//                             O += P·V (P from shared memory, V as an MN-major operand)
-//   warps 2..17 softmax:      four threads per query row, 32 key columns each (warp = TMEM lane quarter
-//                             x column chunk): S from TMEM once, kept in registers → scale, mask, row
-//                             maximum exchanged among the four threads through spare TMEM columns and a
-//                             128-thread named barrier → P (bf16) into swizzled shared memory, partial
-//                             row sums per thread.  Sixteen warps, four per scheduler: with one thread
-//                             per row and one warp per scheduler the exponentials set the pace.
-// The S of tile j+1 is issued before the softmax of tile j finishes, so tensor cores and the
-// exponent units overlap.  O stays in TMEM for the whole row tile; it is rescaled only when the
-// running maximum moves by more than 2^8 ("lazy rescale"), which happens on the first tiles only.
+// One CTA owns two tiles of 128 query rows of one (batch, head) and walks the key tiles they see; one
+// K and V tile in shared memory serves both.  Three warpgroups:
+//   warps 0..3  softmax of the first query tile, warps 4..7 of the second: one thread per query row.  All 128
+//               scores of the row come from TMEM into registers, the row maximum needs no exchange, and
+//               P (bf16) goes back into the TMEM columns the scores came from
+//   warp 8      TMA producer: both Q tiles once, then K and V tiles through a ring of five 32 KB stages
+//   warp 9      MMA issuer (warps 10 and 11 fill its warpgroup): S = Q·Kᵀ (both operands from shared memory) and O += P·V (P from TMEM)
+// The two query tiles alternate: while one is in its softmax the tensor cores work on the other.
+// TMEM: S|P and O of both tiles, 4 x 128 columns.  S of the next key tile is issued behind the P·V that
+// read P, so its arrival also says that O may be touched; O is rescaled only when the running maximum
+// moves by more than 2^8 ("lazy rescale"), which happens on the first tiles only.
+//
+// Why this split: with P in shared memory and one query tile per CTA a key tile costs the shared memory
+// pipe 64 KB of loads in, 32 KB of P in and 128 KB of operands out for 1024 tensor clocks; here it is
+// 32 + 0 + 96 KB.  The pace is then set by the exponentials (16 a clock and SM: 1024 clocks per tile and
+// head, as many as the two products need) and by how well two warps per scheduler cover each other.
 //
 // Chunked keys (context parallelism without a gathered copy): the logical key sequence may be cut
 // into equal chunks that live in different buffers — each context-parallel rank's K/V shard inside
@@ -37,8 +40,10 @@ namespace kb {
 constexpr int FA_BM = 128;      // query rows per CTA
 constexpr int FA_BN = 128;      // keys per tile
 constexpr int FA_D = 128;       // head dim
-constexpr int FA_SOFTMAX_WARPS = 16;
-constexpr int FA_THREADS = (2 + FA_SOFTMAX_WARPS) * 32;
+constexpr int FA_THREADS = 12 * 32;   // three warpgroups: the register split below is by warpgroup
+constexpr int FA_REGS_SOFTMAX = 208, FA_REGS_AUX = 80;   // a row of scores lives in registers
+constexpr int FA_REGS_TOTAL = 256 * FA_REGS_SOFTMAX + 128 * FA_REGS_AUX;   // must not exceed registers at launch x threads
+constexpr int FA_STAGES = 5;    // K and V tiles alternate in one ring
 constexpr int FA_TILE_BYTES = FA_BN * FA_D * 2;   // 32 KB: two 64-wide swizzled chunks of 16 KB
 constexpr int FA_CHUNK = 16384;
 
@@ -65,38 +70,33 @@ struct FwdParams {
   int q_offset;         // absolute position of query row 0 relative to key 0
   float scale_log2;     // softmax scale * log2(e)
   int causal;
+  int tiles_per_cta;    // query tiles of a CTA: 2, or 1 where that leaves SMs idle
   int* status;
   ChunkGeom geom;       // chunk tables (all zero: one K/V buffer, one query chunk at q_offset)
 };
 
-constexpr int FA_KSTAGES = 2;   // K tiles are released as soon as their S MMA retires
-constexpr int FA_VSTAGES = 2;   // V tiles after their P·V MMA
-
 struct FaSmem {
-  static constexpr int Q_OFF = 0;
-  static constexpr int K_OFF = Q_OFF + FA_TILE_BYTES;
-  static constexpr int V_OFF = K_OFF + FA_KSTAGES * FA_TILE_BYTES;
-  static constexpr int P_OFF = V_OFF + FA_VSTAGES * FA_TILE_BYTES;
-  static constexpr int BAR_OFF = P_OFF + 2 * FA_TILE_BYTES;   // P is double buffered
+  static constexpr int Q_OFF = 0;                               // two query tiles; O leaves through them as well
+  static constexpr int KV_OFF = 2 * FA_TILE_BYTES;
+  static constexpr int BAR_OFF = KV_OFF + FA_STAGES * FA_TILE_BYTES;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+  static_assert(TOTAL <= 227 * 1024, "shared memory per CTA");
 };
 
 __global__ void __launch_bounds__(FA_THREADS, 1)
 flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ KvMaps kv,
-                      const FwdParams p) {
+                      const __grid_constant__ CUtensorMap tmO, const FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FaSmem::BAR_OFF);
-  uint64_t* q_full = bars + 0;
-  uint64_t* k_full = bars + 1;    // [FA_KSTAGES]
-  uint64_t* k_empty = bars + 4;   // [FA_KSTAGES]
-  uint64_t* v_full = bars + 7;    // [2]
-  uint64_t* v_empty = bars + 9;   // [2]
-  uint64_t* s_full = bars + 11;   // [2]
-  uint64_t* s_empty = bars + 13;  // [2]
-  uint64_t* p_full = bars + 15;   // [2]
-  uint64_t* pv_done = bars + 17;  // [2]  P·V of the tile that used P buffer b has retired
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+  uint64_t* q_full = bars + 0;     // [2] per query tile
+  uint64_t* full = bars + 2;       // [FA_STAGES] K(j) is in stage 2j, V(j) in stage 2j + 1 (modulo the ring)
+  uint64_t* empty = bars + 7;      // [FA_STAGES]
+  uint64_t* s_full = bars + 12;    // [2] scores are in TMEM (and the tile's previous P·V has retired)
+  uint64_t* p_most = bars + 14;    // [2] P of the first 96 keys is in TMEM (one arrival per warp)
+  uint64_t* p_rest = bars + 16;    // [2] P of the last 32 keys
+  uint64_t* o_full = bars + 18;    // [2] the tile's last P·V has retired
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -104,319 +104,294 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   // heavy (late) query tiles first
   const int n_qtiles = (p.sq + FA_BM - 1) / FA_BM;
-  const int qt = n_qtiles - 1 - static_cast<int>(blockIdx.x);
+  const int qt0 = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) * p.tiles_per_cta;
   const int head = blockIdx.y;
   const int batch = blockIdx.z;
   const int g = head / p.rep, r = head % p.rep;
-  const int q0 = qt * FA_BM;
-  // absolute position of local query row x of this tile is q_off + x
-  const int q_off = p.geom.q_offset_of(q0, p.q_offset);
-  // keys visible to this tile: [0, kv_end)
-  int kv_end = p.skv;
-  if (p.causal) {
-    const int last_q = q_off + min(q0 + FA_BM, p.sq) - 1;
-    kv_end = min(p.skv, last_q + 1);
-  }
-  const int n_kv = kv_end > 0 ? (kv_end + FA_BN - 1) / FA_BN : 0;
+  // query tile t of this CTA: first row, its absolute position minus the row, visible key tiles
+  auto tile_q0 = [&](int t) { return (qt0 + t) * FA_BM; };
+  auto tile_valid = [&](int t) { return t < p.tiles_per_cta && qt0 + t < n_qtiles; };
+  auto tile_nkv = [&](int t) {
+    if (!tile_valid(t)) return 0;
+    const int q0 = tile_q0(t);
+    int kv_end = p.skv;    // keys visible to the tile: [0, kv_end)
+    if (p.causal) kv_end = min(p.skv, p.geom.q_offset_of(q0, p.q_offset) + min(q0 + FA_BM, p.sq));
+    return kv_end > 0 ? (kv_end + FA_BN - 1) / FA_BN : 0;
+  };
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    for (int i = 0; i < FA_KSTAGES; ++i) {
-      mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 1);
+    for (int i = 0; i < FA_STAGES; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], 1);
+      mbar_init(&q_full[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&s_empty[i], FA_SOFTMAX_WARPS);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&p_full[i], FA_SOFTMAX_WARPS);
-      mbar_init(&pv_done[i], 1);
+      mbar_init(&p_most[i], 4);
+      mbar_init(&p_rest[i], 4);
+      mbar_init(&o_full[i], 1);
     }
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  if (warp == 9) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s = tmem_base;         // 2 x 128 columns
-  const uint32_t tmem_o = tmem_base + 256;   // 128 columns
-  const uint32_t tmem_x = tmem_base + 384;   // 12 columns: row maxima (2 x 4) and row sums (4) of the column chunks
+  const uint32_t tmem_base = *tmem_slot;     // S|P of tile t at 128 t, O of tile t at 256 + 128 t
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ producer
-    if (lane == 0 && n_kv > 0) {
-      prefetch_tmap(&tmQ);
-      prefetch_tmap(&kv.k[0]);
-      prefetch_tmap(&kv.v[0]);
-      mbar_expect_tx(q_full, FA_TILE_BYTES);
-      tma_load_5d(smem + FaSmem::Q_OFF, &tmQ, q_full, 0, r, g, batch, q0);
-      tma_load_5d(smem + FaSmem::Q_OFF + FA_CHUNK, &tmQ, q_full, 64, r, g, batch, q0);
-      bool okp = true;
-      auto load_k = [&](int j) {
-        const int s = j % FA_KSTAGES;
-        const uint32_t ph = (j / FA_KSTAGES) & 1u;
-        if (!mbar_wait(&k_empty[s], ph ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { okp = false; return; }
-        uint8_t* kd = smem + FaSmem::K_OFF + s * FA_TILE_BYTES;
-        mbar_expect_tx(&k_full[s], FA_TILE_BYTES);
-        int src, srow;
-        p.geom.locate(j * FA_BN, src, srow);
-        tma_load_4d(kd, &kv.k[src], &k_full[s], 0, g, batch, srow);
-        tma_load_4d(kd + FA_CHUNK, &kv.k[src], &k_full[s], 64, g, batch, srow);
-      };
-      load_k(0);
-      // K runs one tile ahead of V: K(j+1) is requested before V(j)
-      for (int j = 0; j < n_kv && okp; ++j) {
-        if (j + 1 < n_kv) load_k(j + 1);
-        if (!okp) break;
-        const int s = j % FA_VSTAGES;
-        const uint32_t ph = (j / FA_VSTAGES) & 1u;
-        if (!mbar_wait(&v_empty[s], ph ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
-        uint8_t* vd = smem + FaSmem::V_OFF + s * FA_TILE_BYTES;
-        mbar_expect_tx(&v_full[s], FA_TILE_BYTES);
-        int src, srow;
-        p.geom.locate(j * FA_BN, src, srow);
-        tma_load_4d(vd, &kv.v[src], &v_full[s], 0, g, batch, srow);
-        tma_load_4d(vd + FA_CHUNK, &kv.v[src], &v_full[s], 64, g, batch, srow);
-      }
-      if (*abort_flag) {
-        const uint64_t t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 200000ull) {}
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc_s = make_idesc_bf16(FA_BM, FA_BN, false, false);  // Q K-major, K K-major
-    constexpr uint32_t idesc_o = make_idesc_bf16(FA_BM, FA_D, false, true);    // P K-major, V MN-major
-    const uint32_t q_addr = smem_u32(smem + FaSmem::Q_OFF);
-    const uint32_t p_addr = smem_u32(smem + FaSmem::P_OFF);
-    bool ok = n_kv > 0;
-    auto issue_s = [&](int j) {
-      const int s = j & 1;
-      const int ks = j % FA_KSTAGES;
-      const uint32_t k_addr = smem_u32(smem + FaSmem::K_OFF + ks * FA_TILE_BYTES);
-      if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < FA_D / 16; ++k) {
-          const uint32_t off = (k >> 2) * FA_CHUNK + (k & 3) * 32;
-          umma_ss(tmem_s + s * FA_BN, make_smem_desc(q_addr + off, 16, 1024), make_smem_desc(k_addr + off, 16, 1024),
-                  idesc_s, k > 0 ? 1u : 0u);
+  if (warp >= 8) {
+    regs_dec<FA_REGS_AUX>();
+    if (warp == 8) {
+      // ------------------------------------------------------------------ producer
+      const int n0 = tile_nkv(0), n1 = tile_nkv(1), n = max(n0, n1);
+      if (n > 0 && elect_one()) {
+        prefetch_tmap(&tmQ);
+        prefetch_tmap(&kv.k[0]);
+        prefetch_tmap(&kv.v[0]);
+        bool okp = true;
+        int st = 0;
+        uint32_t ph = 1;
+        auto load = [&](const CUtensorMap* map, int srow) {
+          if (!mbar_wait(&empty[st], ph, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { okp = false; return; }
+          uint8_t* d = smem + FaSmem::KV_OFF + st * FA_TILE_BYTES;
+          mbar_expect_tx(&full[st], FA_TILE_BYTES);
+          tma_load_4d(d, map, &full[st], 0, g, batch, srow);
+          tma_load_4d(d + FA_CHUNK, map, &full[st], 64, g, batch, srow);
+          if (++st == FA_STAGES) { st = 0; ph ^= 1u; }
+        };
+        auto load_q = [&](int t) {
+          uint8_t* d = smem + FaSmem::Q_OFF + t * FA_TILE_BYTES;
+          mbar_expect_tx(&q_full[t], FA_TILE_BYTES);
+          tma_load_5d(d, &tmQ, &q_full[t], 0, r, g, batch, tile_q0(t));
+          tma_load_5d(d + FA_CHUNK, &tmQ, &q_full[t], 64, r, g, batch, tile_q0(t));
+        };
+        if (n0 > 0) load_q(0);
+        for (int j = 0; j < n && okp; ++j) {
+          int src, srow;
+          p.geom.locate(j * FA_BN, src, srow);
+          load(&kv.k[src], srow);
+          if (j == 0 && n1 > 0) load_q(1);
+          if (okp) load(&kv.v[src], srow);
         }
-        umma_commit(&k_empty[ks]);
-        umma_commit(&s_full[s]);
+        if (*abort_flag) {
+          const uint64_t t0 = globaltimer_ns();
+          while (globaltimer_ns() - t0 < 200000ull) {}
+        }
       }
       __syncwarp();
-    };
-    if (ok) ok = mbar_wait(q_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL);
-    if (ok) ok = mbar_wait(&k_full[0], 0, abort_flag, p.status, ST_TIMEOUT_FULL);
-    if (ok) {
-      tc_fence_after();
-      issue_s(0);
-    }
-    for (int j = 0; j < n_kv && ok; ++j) {
-      const int s = j & 1;
-      if (j + 1 < n_kv) {
-        const int s1 = (j + 1) & 1;
-        const uint32_t ph1 = ((j + 1) >> 1) & 1u;
-        if (!mbar_wait(&k_full[(j + 1) % FA_KSTAGES], ((j + 1) / FA_KSTAGES) & 1u, abort_flag, p.status,
-                       ST_TIMEOUT_FULL)) { ok = false; break; }
-        if (!mbar_wait(&s_empty[s1], ph1 ^ 1u, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
-        tc_fence_after();
-        issue_s(j + 1);
-      }
-      if (!mbar_wait(&p_full[s], (j >> 1) & 1u, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-      if (!mbar_wait(&v_full[s], (j >> 1) & 1u, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-      tc_fence_after();
-      if (lane == 0) {
-        const uint32_t v_addr = smem_u32(smem + FaSmem::V_OFF + s * FA_TILE_BYTES);
-#pragma unroll
-        for (int k = 0; k < FA_BN / 16; ++k) {
-          // A = P [128 rows][128 keys] K-major: two 64-key chunks; B = V [keys][d] MN-major
-          const uint32_t a_off = (k >> 2) * FA_CHUNK + (k & 3) * 32;
-          umma_ss(tmem_o, make_smem_desc(p_addr + s * FA_TILE_BYTES + a_off, 16, 1024),
-                  make_smem_desc(v_addr + k * 2048, FA_CHUNK, 1024), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+    } else if (warp == 9) {
+      // ------------------------------------------------------------------ MMA issuer
+      const int n0 = tile_nkv(0), n1 = tile_nkv(1), n = max(n0, n1);
+      if (n > 0 && elect_one()) {             // one thread runs the whole role, see elect_one()
+        constexpr uint32_t idesc_s = make_idesc_bf16(FA_BM, FA_BN, false, false);  // Q K-major, K K-major
+        constexpr uint32_t idesc_o = make_idesc_bf16(FA_BM, FA_D, false, true);    // P (TMEM), V MN-major
+        const uint32_t smem0 = smem_u32(smem);
+        const uint64_t qd0 = make_smem_desc(smem0 + FaSmem::Q_OFF, 16, 1024);
+        const uint64_t kd0 = make_smem_desc(smem0 + FaSmem::KV_OFF, 16, 1024);
+        const uint64_t vd0 = make_smem_desc(smem0 + FaSmem::KV_OFF, FA_CHUNK, 1024);
+        bool ok = true;
+        auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+          if (ok) ok = mbar_wait(bar, parity, abort_flag, p.status, code);
+          return ok;
+        };
+        auto issue_s = [&](int t, int ks) {
+          const uint64_t qd = qd0 + static_cast<uint64_t>(t * (FA_TILE_BYTES >> 4));
+          const uint64_t kd = kd0 + static_cast<uint64_t>(ks * (FA_TILE_BYTES >> 4));
+          const uint32_t d = tmem_base + t * 128;
+  #pragma unroll
+          for (int k = 0; k < FA_D / 16; ++k) {
+            const uint64_t off = ((k >> 2) * FA_CHUNK + (k & 3) * 32) >> 4;
+            umma_ss(d, qd + off, kd + off, idesc_s, k > 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[t]);
+        };
+        int ks = 0;                                // stage of K(j) / K(j+1), its phase
+        uint32_t kph = 0;
+        if (wait(&full[0], 0, ST_TIMEOUT_FULL)) {
+  #pragma unroll
+          for (int t = 0; t < 2; ++t)
+            if ((t ? n1 : n0) > 0 && wait(&q_full[t], 0, ST_TIMEOUT_FULL)) {
+              tc_fence_after();
+              issue_s(t, 0);
+            }
+          if (ok) umma_commit(&empty[0]);
         }
-        umma_commit(&v_empty[s]);
-        umma_commit(&pv_done[s]);
+        for (int j = 0; j < n && ok; ++j) {
+          int vs = ks + 1;
+          uint32_t vph = kph;
+          if (vs == FA_STAGES) { vs = 0; vph ^= 1u; }
+          ks = vs + 1;
+          kph = vph;
+          if (ks == FA_STAGES) { ks = 0; kph ^= 1u; }
+          if (!wait(&full[vs], vph, ST_TIMEOUT_FULL)) break;
+          const uint64_t vd = vd0 + static_cast<uint64_t>(vs * (FA_TILE_BYTES >> 4));
+  #pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            const int nt = t ? n1 : n0;
+            if (j >= nt || !ok) continue;
+            const uint32_t d = tmem_base + 256 + t * 128, a = tmem_base + t * 128;
+            if (!wait(&p_most[t], j & 1u, ST_TIMEOUT_TMEM_FULL)) continue;
+            tc_fence_after();
+  #pragma unroll
+            for (int k = 0; k < 6; ++k)            // 16 keys: 8 columns of P, 16 rows of V
+              umma_ts(d, a + k * 8, vd + k * (2048 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+            if (!wait(&p_rest[t], j & 1u, ST_TIMEOUT_TMEM_FULL)) continue;
+            tc_fence_after();
+  #pragma unroll
+            for (int k = 6; k < 8; ++k) umma_ts(d, a + k * 8, vd + k * (2048 >> 4), idesc_o, 1u);
+            if (j + 1 < nt) {
+              if (!wait(&full[ks], kph, ST_TIMEOUT_FULL)) continue;
+              tc_fence_after();
+              issue_s(t, ks);                      // overwrites P: the products before it read it in order
+            } else {
+              umma_commit(&o_full[t]);
+            }
+          }
+          if (!ok) break;
+          umma_commit(&empty[vs]);
+          if (j + 1 < n) umma_commit(&empty[ks]);
+        }
       }
       __syncwarp();
     }
   } else {
+    regs_inc<FA_REGS_SOFTMAX>();
     // ------------------------------------------------------------------ softmax + epilogue
-    const int quarter = warp & 3;
-    const int c = (warp - 2) >> 2;                 // chunk of 32 key columns, and of 32 output columns
-    const int row = quarter * 32 + lane;           // row inside the tile = TMEM lane
-    const int qpos = q_off + q0 + row;             // absolute position of this query
-    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    const int group_bar = 1 + quarter;             // named barrier of the four warps that share these rows
-    const uint32_t full = 0xffffffffu;
+    const int t = warp >> 2;                       // query tile
+    const int row = (warp & 3) * 32 + lane;        // row inside the tile = TMEM lane
+    const int n_kv = tile_nkv(t);
+    const int q0 = tile_q0(t);
+    const int qrow = q0 + row;
+    const int q_off = tile_valid(t) ? p.geom.q_offset_of(q0, p.q_offset) : 0;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t t_s = tmem_base + t * 128 + lane_addr, t_o = tmem_base + 256 + t * 128 + lane_addr;
+    const uint32_t all = 0xffffffffu;
     float m_ref = -INFINITY;   // reference maximum (scaled, log2 domain) used for the exponentials
-    float l_part = 0.f;        // sum of this thread's exponentials
-    bool ok = n_kv > 0;
-    bool group_ok = true;      // false once the group has left the loop together after a failed wait
+    float l_sum = 0.f;
+    bool ok = true;            // warp-uniform
     for (int j = 0; j < n_kv; ++j) {
-      const int s = j & 1;
-      // a thread whose wait failed keeps coming to the group barrier (with good = false), so that the
-      // four warps leave together and nobody is left waiting at it
-      const bool good = __all_sync(full, ok && mbar_wait(&s_full[s], (j >> 1) & 1u, abort_flag, p.status,
-                                                         ST_TIMEOUT_TMEM_FULL));
+      ok = __all_sync(all, mbar_wait(&s_full[t], j & 1u, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL));
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t v[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_s + c * 32, v[c]);
+      tmem_ld_wait();
       const int key0 = j * FA_BN;
       // warp-uniform: does any row of this tile need masking?
-      const bool tile_mask = (p.causal && key0 + FA_BN - 1 > q_off + q0) || (key0 + FA_BN > p.skv);
-      uint32_t v[32];
-      if (good) {
-        tc_fence_after();
-        tmem_ld_32x32(tmem_s + s * FA_BN + lane_addr + c * 32, v);
-        tmem_ld_wait();
-        if (tile_mask) {
+      if ((p.causal && key0 + FA_BN - 1 > q_off + q0) || (key0 + FA_BN > p.skv)) {
+        // keys at or above `lim` (relative to this tile) are hidden from this row
+        const int lim = min(p.causal ? q_off + qrow + 1 : p.skv, p.skv) - key0;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int key = key0 + c * 32 + i;
-            if ((p.causal && key > qpos) || key >= p.skv) v[i] = 0xff800000u;   // -inf
-          }
-        }
-        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int i = 0; i < 32; i += 8) {
-          mx4[0] = fmax3(mx4[0], __uint_as_float(v[i + 0]), __uint_as_float(v[i + 1]));
-          mx4[1] = fmax3(mx4[1], __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
-          mx4[2] = fmax3(mx4[2], __uint_as_float(v[i + 4]), __uint_as_float(v[i + 5]));
-          mx4[3] = fmax3(mx4[3], __uint_as_float(v[i + 6]), __uint_as_float(v[i + 7]));
-        }
-        const float mloc = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-        // slot j & 1: a thread can be one barrier ahead of the slowest reader of its group, never two
-        tmem_st_32x32_x1(tmem_x + lane_addr + (j & 1) * 4 + c, __float_as_uint(mloc));
-        tmem_st_wait();
-        tc_fence_before();
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i >= lim) v[c][i] = 0xff800000u;   // -inf
       }
-      if (!bar128_all(group_bar, good)) { ok = false; group_ok = false; break; }
-      tc_fence_after();
-      uint32_t m4[4];
-      tmem_ld_32x32_x4(tmem_x + lane_addr + (j & 1) * 4, m4);
-      tmem_ld_wait();
-      // S has been read: its buffer may take the scores of tile j+2
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&s_empty[s]);
-      const float mx = fmaxf(fmaxf(__uint_as_float(m4[0]), __uint_as_float(m4[1])),
-                             fmaxf(__uint_as_float(m4[2]), __uint_as_float(m4[3]))) * p.scale_log2;
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; i += 8)
+#pragma unroll
+          for (int h = 0; h < 4; ++h)
+            mx4[h] = fmax3(mx4[h], __uint_as_float(v[c][i + 2 * h]), __uint_as_float(v[c][i + 2 * h + 1]));
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
       float rescale = 1.f;
-      bool do_rescale = false;
       if (mx > m_ref + 8.f) {       // also true on the first tile (m_ref = -inf)
-        if (j > 0 && m_ref != -INFINITY) {
-          rescale = fast_exp2(m_ref - mx);
-          do_rescale = true;
-        }
+        rescale = m_ref == -INFINITY ? 1.f : fast_exp2(m_ref - mx);
         m_ref = mx;
       }
-      const float mref = (m_ref == -INFINITY) ? 0.f : m_ref;
-      // O may only be touched once the previous P·V has retired (rare path: the running maximum
-      // moved by more than 2^8); the decision is made warp-uniform for the .aligned TMEM accesses.
-      // This thread rescales its 32 columns of O.
-      if (__any_sync(full, do_rescale)) {
-        const bool got = __all_sync(full, mbar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1u, abort_flag, p.status,
-                                                    ST_TIMEOUT_TMEM_FULL));
-        if (got) {
-          tc_fence_after();
+      // s_full also covers the tile's previous P·V, so O is at rest here; made warp-uniform for the .aligned accesses
+      if (__any_sync(all, rescale != 1.f)) {
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
           uint32_t o[32];
-          tmem_ld_32x32(tmem_o + lane_addr + c * 32, o);
+          tmem_ld_32x32(t_o + c * 32, o);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * rescale);
-          tmem_st_32x32(tmem_o + lane_addr + c * 32, o);
-          tmem_st_wait();
-        } else {
-          ok = false;
+          tmem_st_32x32(t_o + c * 32, o);
         }
+        tmem_st_wait();
       }
-      // the P buffer of this parity was last read by the P·V of tile j-2
-      if (ok && j >= 2) {
-        if (!__all_sync(full, mbar_wait(&pv_done[s], ((j >> 1) & 1u) ^ 1u, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)))
-          ok = false;
-      }
-      if (!ok) continue;            // the group learns of it at its next barrier
-      // ---- P = exp2(S·scale − m), partial row sum, bf16 pack into the swizzled operand layout
-      // (16-byte unit u of row r goes to unit (u ^ (r & 7)) of that row inside its 64-key chunk)
-      uint8_t* p_row = smem + FaSmem::P_OFF + s * FA_TILE_BYTES + (c >> 1) * FA_CHUNK + row * 128;
+      const float mref = (m_ref == -INFINITY) ? 0.f : m_ref;
       const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
       const float2 nm2 = make_float2(-mref, -mref);
       float2 ps2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      // P = exp2(S·scale − m) of 32 keys: partial row sum, bf16 pairs into 16 columns of TMEM
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        uint32_t w[4];
+      for (int c = 0; c < 4; ++c) {
+        uint32_t w[16];
 #pragma unroll
-        for (int h2 = 0; h2 < 4; ++h2) {
-          const int i = 8 * u + 2 * h2;
-          float2 x = __ffma2_rn(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), sc2, nm2);
+        for (int i = 0; i < 16; ++i) {
+          float2 x = __ffma2_rn(make_float2(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), sc2, nm2);
           x.x = fast_exp2(x.x);
           x.y = fast_exp2(x.y);
-          ps2[h2 & 1] = __fadd2_rn(ps2[h2 & 1], x);
-          w[h2] = pack_bf16x2(x.x, x.y);
+          ps2[i & 1] = __fadd2_rn(ps2[i & 1], x);
+          w[i] = pack_bf16x2(x.x, x.y);
         }
-        const int unit = (c & 1) * 4 + u;              // 16-byte unit inside the 64-key chunk
-        *reinterpret_cast<uint4*>(p_row + ((unit ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-      l_part = l_part * rescale + (ps2[0].x + ps2[0].y) + (ps2[1].x + ps2[1].y);
-      tc_fence_before();
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[s]);
-    }
-    // ---- epilogue: O / l → global, LSE; this thread writes its 32 columns of the row
-    const int qrow = q0 + row;
-    if (n_kv > 0) {
-      if (group_ok) {
-        const bool good = __all_sync(full, ok && mbar_wait(&pv_done[(n_kv - 1) & 1], ((n_kv - 1) >> 1) & 1u, abort_flag,
-                                                           p.status, ST_TIMEOUT_TMEM_FULL));
-        if (good) {
-          tmem_st_32x32_x1(tmem_x + lane_addr + 8 + c, __float_as_uint(l_part));
+        tmem_st_32x32_x16(t_s + c * 16, w);
+        if (c >= 2) {
           tmem_st_wait();
           tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(c == 2 ? &p_most[t] : &p_rest[t]);
         }
-        if (bar128_all(group_bar, good)) {
+      }
+      l_sum = l_sum * rescale + ((ps2[0].x + ps2[0].y) + (ps2[1].x + ps2[1].y));
+    }
+    // ---- epilogue: O / l through this tile's Q buffer (the warp's 32 rows) and a TMA store; LSE
+    if (tile_valid(t)) {
+      float* lse = p.lse + (static_cast<size_t>(batch) * p.hq + head) * p.sq;
+      if (n_kv > 0) {
+        if (ok) ok = __all_sync(all, mbar_wait(&o_full[t], 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL));
+        if (ok) {
           tc_fence_after();
-          uint32_t l4[4];
-          tmem_ld_32x32_x4(tmem_x + lane_addr + 8, l4);
-          uint32_t o[32];
-          tmem_ld_32x32(tmem_o + lane_addr + c * 32, o);
-          tmem_ld_wait();
-          const float l_sum = (__uint_as_float(l4[0]) + __uint_as_float(l4[1])) +
-                              (__uint_as_float(l4[2]) + __uint_as_float(l4[3]));
           const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
-          if (qrow < p.sq) {
-            __nv_bfloat16* orow = p.out + ((static_cast<size_t>(qrow) * p.b + batch) * p.hq + head) * FA_D + c * 32;
+          // two 64-wide halves of 32 rows x 128 bytes, 16-byte units swizzled by row as the tensor map expects
+          uint8_t* stg = smem + FaSmem::Q_OFF + t * FA_TILE_BYTES + (warp & 3) * 8192;
+          const uint32_t stg_row = smem_u32(stg) + lane * 128;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t o[32];
+            tmem_ld_32x32(t_o + c * 32, o);
+            tmem_ld_wait();
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-              uint4 w;
-              w.x = pack_bf16x2(__uint_as_float(o[8 * u + 0]) * inv, __uint_as_float(o[8 * u + 1]) * inv);
-              w.y = pack_bf16x2(__uint_as_float(o[8 * u + 2]) * inv, __uint_as_float(o[8 * u + 3]) * inv);
-              w.z = pack_bf16x2(__uint_as_float(o[8 * u + 4]) * inv, __uint_as_float(o[8 * u + 5]) * inv);
-              w.w = pack_bf16x2(__uint_as_float(o[8 * u + 6]) * inv, __uint_as_float(o[8 * u + 7]) * inv);
-              reinterpret_cast<uint4*>(orow)[u] = w;
+              uint32_t w[4];
+#pragma unroll
+              for (int h = 0; h < 4; ++h)
+                w[h] = pack_bf16x2(__uint_as_float(o[8 * u + 2 * h]) * inv, __uint_as_float(o[8 * u + 2 * h + 1]) * inv);
+              const int unit = (c & 1) * 4 + u;
+              st_shared_v4(stg_row + (c >> 1) * 4096 + ((unit ^ (lane & 7)) << 4), w[0], w[1], w[2], w[3]);
             }
-            if (c == 0)
-              p.lse[(static_cast<size_t>(batch) * p.hq + head) * p.sq + qrow] =
-                  (l_sum > 0.f) ? (m_ref + log2f(l_sum)) * 0.6931471805599453f : -INFINITY;
           }
+          fence_proxy_async_smem();
+          __syncwarp();
+          const int row0 = q0 + (warp & 3) * 32;
+          if (lane == 0 && row0 < p.sq) {              // the tensor map clips rows past sq
+            tma_store_4d(&tmO, stg, 0, head, batch, row0);
+            tma_store_4d(&tmO, stg + 4096, 64, head, batch, row0);
+            tma_store_commit();
+          }
+          if (qrow < p.sq) lse[qrow] = (l_sum > 0.f) ? (m_ref + log2f(l_sum)) * 0.6931471805599453f : -INFINITY;
+          if (lane == 0) tma_store_wait<0>();          // nothing in flight out of shared memory at exit
         }
-      }
-    } else {
-      // no visible key at all (only possible with a negative q_offset): zero output
-      if (qrow < p.sq) {
-        __nv_bfloat16* orow = p.out + ((static_cast<size_t>(qrow) * p.b + batch) * p.hq + head) * FA_D + c * 32;
-        for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(orow)[i] = make_uint4(0, 0, 0, 0);
-        if (c == 0) p.lse[(static_cast<size_t>(batch) * p.hq + head) * p.sq + qrow] = -INFINITY;
+      } else if (qrow < p.sq) {
+        // no visible key at all (only possible with a negative q_offset): zero output
+        uint4* orow = reinterpret_cast<uint4*>(p.out + ((static_cast<size_t>(qrow) * p.b + batch) * p.hq + head) * FA_D);
+        for (int i = 0; i < FA_D / 8; ++i) orow[i] = make_uint4(0, 0, 0, 0);
+        lse[qrow] = -INFINITY;
       }
     }
+    __syncwarp();
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 9) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -456,15 +431,33 @@ static int launch_fwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
   p.causal = causal;
   p.status = status;
   p.geom = geom;
+  // Pairs of query tiles halve the K/V traffic and keep the tensor cores busy during a softmax; where single
+  // tiles already fit the chip in one wave, they halve the work of the longest CTA instead.
+  const int n_q = (sq + FA_BM - 1) / FA_BM;
+  p.tiles_per_cta = (long)n_q * g * rep * b <= device_sm_count() ? 1 : 2;
+  CUtensorMap tmO;
+  {
+    // [sq, b, hq, d]: boxes of 32 rows x 64 columns of one (batch, head)
+    const uint64_t hq = (uint64_t)g * rep;
+    uint64_t dims[4] = {FA_D, hq, (uint64_t)b, (uint64_t)sq};
+    uint64_t str[3] = {FA_D * 2, hq * FA_D * 2, (uint64_t)b * hq * FA_D * 2};
+    uint32_t box[4] = {64, 1, 1, 32};
+    const int rc = make_tmap(&tmO, out, 2, 4, dims, str, box, 3);
+    if (rc) return rc;
+  }
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(flash_attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          FaSmem::TOTAL);
     if (e != cudaSuccess) return 1000 + (int)e;
+    cudaFuncAttributes attr;
+    e = cudaFuncGetAttributes(&attr, flash_attn_fwd_kernel);
+    if (e != cudaSuccess) return 1000 + (int)e;
+    if (attr.numRegs * FA_THREADS < FA_REGS_TOTAL) return ST_BAD_ARG;   // the register split would wait forever
     configured = true;
   }
-  dim3 grid((sq + FA_BM - 1) / FA_BM, g * rep, b);
-  KB_LAUNCH(flash_attn_fwd_kernel, grid, FA_THREADS, FaSmem::TOTAL, stream, tmQ, kv, p);
+  dim3 grid((n_q + p.tiles_per_cta - 1) / p.tiles_per_cta, g * rep, b);
+  KB_LAUNCH(flash_attn_fwd_kernel, grid, FA_THREADS, FaSmem::TOTAL, stream, tmQ, kv, tmO, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + (int)e;
 }

@@ -329,6 +329,37 @@ def test_flash_attention_backward_offsets():
         assert dk[(cid + 1) * c:].abs().max().item() == 0
 
 
+# query tiles go in pairs once single tiles no longer fit the chip in one wave (148 SMs): an odd number of tiles, fewer
+# rows than a tile, one row, a last tile of one row, and pairs whose halves see different numbers of key tiles
+@pytest.mark.parametrize("sq,skv,b,g,rep,off,causal",
+                         [(1, 1, 3, 2, 2, 0, True), (1, 1, 50, 2, 2, 0, True), (127, 127, 40, 2, 2, 0, True),
+                          (129, 129, 20, 2, 3, 0, True), (641, 641, 9, 2, 3, 0, True), (1000, 1000, 4, 2, 3, 0, True),
+                          (385, 1025, 12, 1, 4, 640, True), (385, 300, 12, 1, 4, 640, True), (300, 200, 20, 1, 4, -150, True),
+                          (260, 131, 16, 2, 2, 0, False)])
+def test_flash_attention_tile_pairs(sq, skv, b, g, rep, off, causal):
+    KC = _K()
+    from kareus_b200.kernels import attention_cuda, ref
+    d = 128
+    q = torch.randn(sq, b, g, rep, d, device="cuda").bfloat16()
+    k = torch.randn(skv, b, g, d, device="cuda").bfloat16()
+    v = torch.randn(skv, b, g, d, device="cuda").bfloat16()
+    out, lse = attention_cuda.forward(q, k, v, d ** -0.5, causal, off, None)
+    do = torch.randn_like(out)
+    dq, dk, dv = attention_cuda.backward(do, q, k, v, out, lse, d ** -0.5, causal, off, None)
+    KC.check_status()
+    o_ref, lse_ref = ref.attention_fwd(q.float(), k.float(), v.float(), d ** -0.5, causal, off)
+    wq, wk, wv = ref.attention_bwd(do.float(), q.float(), k.float(), v.float(), o_ref,
+                                   lse_ref.masked_fill(lse_ref == float("-inf"), 0.0), d ** -0.5, causal, off)
+    torch.testing.assert_close(lse, lse_ref, rtol=1e-3, atol=1e-3)
+    # P and dS are rounded to bf16 (2^-9 each) and so are the results: below 1e-2 of the tensor.  One key leaves
+    # dS = P (dP - delta) = 0 up to rounding, so dq and dk are compared with the size of their terms there.
+    assert _rel(out, o_ref) < 1e-2 and _rel(dv, wv) < 1e-2
+    if skv > 1:
+        assert _rel(dq, wq) < 2e-2 and _rel(dk, wk) < 2e-2
+    else:
+        assert dq.abs().max() < 0.5 and dk.abs().max() < 2.0
+
+
 def test_gelu_geglu_kernels():
     from kareus_b200.engine.context import OpContext
     from kareus_b200.ops.activations import GegluOp, GeluOp, gelu_grad_ref, gelu_ref
