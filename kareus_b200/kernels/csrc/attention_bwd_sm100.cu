@@ -1,26 +1,22 @@
 // Causal GQA flash-attention backward for sm_100a (head dim 128, bf16, fp32 accumulation).
 //
-// One CTA owns 128 keys of one (batch, query head) and walks the query tiles that can see them:
-//   warp 0      TMA producer: K and V once, then per query tile Q (two buffers, one tile ahead) and dO
-//   warp 1      MMA issuer (tcgen05, accumulators in TMEM):
-//                 S  = Q·Kᵀ          dP = dO·Vᵀ                       (per query tile)
-//                 dV += Pᵀ·dO        dK += dSᵀ·Q        dQ = dS·K      (per query tile)
-//   warps 2..17 four threads per query row, 32 key columns each: P = exp2(S·c − lse) as soon as S is
-//               there (dO of the tile may still be on its way), then dS = P∘(dP − δ)·scale once dP is
-//               there; both as bf16 into swizzled shared memory.  Sixteen warps, four per scheduler: with
-//               one warp per scheduler this arithmetic, not the tensor pipe, set the pace of the walk
-//   warps 18..21 dQ from TMEM → shared memory (the dS buffer, free between the products of one tile and
-//               the dS pass of the next) → TMA reduce-add into the fp32 accumulator in global memory,
-//               32 columns at a time, while the next tile is worked on
-// The walk is a pipeline: S of tile i+1 is issued right behind the three products of tile i (its Q is
-// already in shared memory), the dO buffer is refilled as soon as those products retire, and dQ of
-// tile i is drained while P of tile i+1 is computed.
-// P and dS are stored once ([q][key], keys contiguous) and serve as K-major operands (dQ) and, read
-// through MN-major descriptors, as the transposed operands of dV and dK — no transposes anywhere.
-// TMEM: S + dP|dQ (shared) + dV + dK = 512 columns.  dK/dV stay in TMEM across the whole walk and
-// are added to fp32 accumulators at the end (query heads of one KV group run in different CTAs).
-// Shared memory: K, V, Q x 2, dO, P, dS = 7 tiles of 32 KB.
-// A second kernel converts the fp32 accumulators into the packed bf16 gradient of the QKV GEMM.
+// One CTA owns 128 keys of one (batch, query head) and walks the query tiles that can see them.  Scores are
+// kept transposed (rows = keys), so that P leaves the registers as the TMEM operand of dV:
+//   warps 0..15  four threads per key row, 32 query columns each: Pᵀ = exp2(Sᵀ·c − lse) as soon as Sᵀ is there,
+//                bf16 into the TMEM columns the scores came from; then dSᵀ = Pᵀ∘(dPᵀ − δ) once dPᵀ is there, bf16
+//                into swizzled shared memory.  lse and δ of a query tile are staged next to its Q
+//   warps 16..19 dQ from TMEM → 8 KB of shared memory per warp → TMA reduce-add into the fp32 accumulator in
+//                global memory, 32 rows x 32 columns at a time, no barrier between the warps
+//   warp 20      TMA producer: K and V once, then per query tile Q and its row statistics (two buffers) and dO
+//   warp 21      MMA issuer (tcgen05, accumulators in TMEM), per query tile i in this order:
+//                  dPᵀ = V·dOᵀ,  dV += Pᵀ·dO,  Sᵀ(i+1) = K·Qᵀ,  dQ = dS·K,  dK += dSᵀ·Q
+// The order is what makes it a pipeline: Pᵀ(i+1) is computed under dQ and dK of tile i, dSᵀ under dV and the next
+// scores, and dQ of tile i leaves TMEM under dK.  dSᵀ is stored once ([key][query], queries contiguous) and serves
+// as K-major operand (dK) and, through an MN-major descriptor, as transposed operand of dQ.  The softmax scale is
+// applied to dQ and dK once, where they leave, and not to every element of dS.
+// TMEM: Sᵀ|Pᵀ + dPᵀ|dQ + dV + dK = 512 columns.  dK/dV stay in TMEM across the whole walk and are added to fp32
+// accumulators at the end (query heads of one KV group run in different CTAs).
+// Shared memory: K, V, Q x 2, dO, dS, dQ staging = 7 tiles of 32 KB.
 //
 // Chunked keys and queries (context parallelism, see attention_chunks.h): K/V tiles may come from
 // several source buffers (other GPUs' shards through their peer mappings, plain TMA loads), query
@@ -40,13 +36,14 @@ namespace kb {
 constexpr int FB_T = 128;                      // tile edge (queries, keys) and head dim
 constexpr int FB_TILE = FB_T * FB_T * 2;       // 32 KB bf16 tile as two 64-wide swizzled chunks
 constexpr int FB_CHUNK = 16384;
-constexpr int FB_SOFTMAX_WARPS = 16;             // 4 TMEM lane quarters x 4 chunks of 32 key columns
-constexpr int FB_THREADS = (2 + FB_SOFTMAX_WARPS + 4) * 32;
+constexpr int FB_SOFTMAX_WARPS = 16;             // 4 TMEM lane quarters x 4 chunks of 32 query columns
+constexpr int FB_DQ_WARP = FB_SOFTMAX_WARPS;     // first of the four dQ warps
+constexpr int FB_TMA_WARP = FB_DQ_WARP + 4, FB_MMA_WARP = FB_DQ_WARP + 5;
+constexpr int FB_THREADS = (FB_SOFTMAX_WARPS + 6) * 32;
+constexpr int FB_STATS = 2 * FB_T;               // floats of row statistics per query tile: −lse·log2(e), then −δ
 
 struct BwdParams {
-  const float* lse;      // [b, hq, sq]  natural log
-  const float* delta;    // [b, hq, sq]  rowsum(dO ∘ O)
-  float* dq_acc;         // [sq, b, hq, d]
+  const float* stats;    // [b, hq, query tiles, 2, 128], see attn_stats_kernel
   float* dk_acc;         // [skv, b, g, d]
   float* dv_acc;         // [skv, b, g, d]
   int sq, skv, b, hq, rep, q_offset, causal;
@@ -64,9 +61,11 @@ __device__ __forceinline__ bool q_tile_sees(const BwdParams& p, int qt, int k0) 
 
 struct FbSmem {
   // Q_OFF: two consecutive tiles (buffer = iteration & 1)
-  static constexpr int K_OFF = 0, V_OFF = FB_TILE, Q_OFF = 2 * FB_TILE, DO_OFF = 4 * FB_TILE, P_OFF = 5 * FB_TILE,
-                       DS_OFF = 6 * FB_TILE, BAR_OFF = 7 * FB_TILE, TOTAL = BAR_OFF + 256 + 1024;
-  static_assert(TOTAL <= 227 * 1024, "shared memory per CTA");
+  static constexpr int K_OFF = 0, V_OFF = FB_TILE, Q_OFF = 2 * FB_TILE, DO_OFF = 4 * FB_TILE, DS_OFF = 5 * FB_TILE,
+                       STG_OFF = 6 * FB_TILE, STAT_OFF = 7 * FB_TILE, BAR_OFF = STAT_OFF + 2 * FB_STATS * 4;
+  // what is left of 227 KB aligns the tiles to 1024 bytes; the kernel checks that it suffices
+  static constexpr int USED = BAR_OFF + 256, TOTAL = 227 * 1024;
+  static_assert(USED <= TOTAL, "shared memory per CTA");
 };
 
 __device__ __forceinline__ float bwd_exp2(float x) {
@@ -78,38 +77,31 @@ __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, 
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// Named barrier 1 of the four dQ warps; the second form returns whether `ok` held on all 128 threads.
-__device__ __forceinline__ void drain_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-__device__ __forceinline__ bool drain_all(bool ok) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred P, Q;\n\tsetp.ne.u32 P, %1, 0;\n\tbar.red.and.pred Q, 1, 128, P;\n\tselp.u32 %0, 1, 0, Q;\n\t}"
-      : "=r"(r)
-      : "r"(static_cast<uint32_t>(ok))
-      : "memory");
-  return r != 0;
-}
-
 __global__ void __launch_bounds__(FB_THREADS, 1)
 flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ KvMaps kv,
                       const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmDQ,
                       const BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  if (smem - smem_raw + FbSmem::USED > FbSmem::TOTAL) {   // the same for all threads
+    if (threadIdx.x == 0) atomicCAS(p.status, 0, ST_BAD_ARG);
+    return;
+  }
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FbSmem::BAR_OFF);
   uint64_t* kv_full = bars + 0;
-  uint64_t* q_full = bars + 1;      // [2] Q of iteration i is in buffer i & 1
+  uint64_t* q_full = bars + 1;      // [2] Q and statistics of iteration i are in buffer i & 1
   uint64_t* q_empty = bars + 3;     // [2] the MMAs that read that buffer have retired
   uint64_t* do_full = bars + 5;
-  uint64_t* do_empty = bars + 6;    // the MMAs that read dO (and P, dS) of this iteration have retired
-  uint64_t* s_full = bars + 7;      // S is in TMEM
-  uint64_t* dp_full = bars + 8;     // dP is in TMEM
-  uint64_t* pds_full = bars + 9;    // P and dS are in shared memory, S and dP have been read (one arrival per warp)
-  uint64_t* dq_full = bars + 10;    // dQ (and this iteration's dV/dK updates) retired
-  uint64_t* dq_empty = bars + 11;   // dQ has been read out of TMEM
-  uint64_t* all_done = bars + 12;   // every MMA of the walk has retired
-  uint64_t* stage_free = bars + 13; // the dQ reductions have read their staging area (the dS buffer)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* do_empty = bars + 6;    // dPᵀ and dV of this iteration have retired
+  uint64_t* s_full = bars + 7;      // Sᵀ is in TMEM
+  uint64_t* p_full = bars + 8;      // Pᵀ is in TMEM, Sᵀ has been read (one arrival per warp)
+  uint64_t* dp_full = bars + 9;     // dPᵀ is in TMEM
+  uint64_t* ds_full = bars + 10;    // dSᵀ is in shared memory, dPᵀ has been read (one arrival per warp)
+  uint64_t* ds_empty = bars + 11;   // dQ and dK of this iteration have retired
+  uint64_t* dq_full = bars + 12;    // dQ is in TMEM
+  uint64_t* dq_empty = bars + 13;   // dQ has been read out of TMEM (one arrival per dQ warp)
+  uint64_t* all_done = bars + 14;   // every MMA of the walk has retired
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -122,46 +114,34 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   for (int qt = 0; qt < n_q; ++qt) n_it += q_tile_sees(p, qt, k0) ? 1 : 0;
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&q_full[i], 1);
-      mbar_init(&q_empty[i], 1);
-    }
-    mbar_init(do_full, 1);
-    mbar_init(do_empty, 1);
-    mbar_init(s_full, 1);
-    mbar_init(dp_full, 1);
-    mbar_init(pds_full, FB_SOFTMAX_WARPS);
-    mbar_init(dq_full, 1);
-    mbar_init(dq_empty, 1);
-    mbar_init(all_done, 1);
-    mbar_init(stage_free, 1);
+    for (int i = 0; i < 15; ++i)
+      mbar_init(&bars[i], &bars[i] == p_full || &bars[i] == ds_full ? FB_SOFTMAX_WARPS : &bars[i] == dq_empty ? 4 : 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  if (warp == FB_MMA_WARP) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // dQ of a tile goes where its dP was: dP has been read by then, and S of the next tile can be issued
-  // while dQ is drained
+  // Pᵀ of query chunk c goes into the first 16 of the 32 columns of its scores.  dQ of a tile goes where its dPᵀ
+  // was: that has been read by then.
   const uint32_t t_s = tmem_base, t_dp = tmem_base + 128, t_dv = tmem_base + 256, t_dk = tmem_base + 384;
   const uint32_t t_dq = t_dp;
 
-  if (warp == 0) {
-    if (lane == 0 && n_it > 0) {
+  if (warp == FB_TMA_WARP) {
+    if (n_it > 0 && elect_one()) {
       int src, srow;
       p.geom.locate(k0, src, srow);
       prefetch_tmap(&tmQ); prefetch_tmap(&kv.k[src]); prefetch_tmap(&kv.v[src]); prefetch_tmap(&tmDO);
+      const float* stats = p.stats + (static_cast<size_t>(batch) * p.hq + head) * n_q * FB_STATS;
       mbar_expect_tx(kv_full, 2 * FB_TILE);
       tma_load_4d(smem + FbSmem::K_OFF, &kv.k[src], kv_full, 0, g, batch, srow);
       tma_load_4d(smem + FbSmem::K_OFF + FB_CHUNK, &kv.k[src], kv_full, 64, g, batch, srow);
       tma_load_4d(smem + FbSmem::V_OFF, &kv.v[src], kv_full, 0, g, batch, srow);
       tma_load_4d(smem + FbSmem::V_OFF + FB_CHUNK, &kv.v[src], kv_full, 64, g, batch, srow);
-      // per visible tile: Q(it) into buffer it & 1, then dO(it).  The buffer of Q(it) was released by the
-      // products of tile it-2 and dO by those of tile it-1, so Q(it+1) goes out right behind dO(it): one
-      // tile ahead of the MMAs.
+      // per visible tile: Q(it) into buffer it & 1 (released by dK of tile it-2), then dO(it) (released by dV of
+      // tile it-1): Q(it+1) goes out right behind dO(it), one tile ahead of the MMAs
       int it = 0;
       for (int qt = 0; qt < n_q; ++qt) {
         if (!q_tile_sees(p, qt, k0)) continue;
@@ -169,9 +149,11 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const int q0 = qt * FB_T;
         if (!mbar_wait(&q_empty[qb], ((it >> 1) & 1u) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
         uint8_t* qdst = smem + FbSmem::Q_OFF + qb * FB_TILE;
-        mbar_expect_tx(&q_full[qb], FB_TILE);
+        mbar_expect_tx(&q_full[qb], FB_TILE + FB_STATS * 4);
         tma_load_5d(qdst, &tmQ, &q_full[qb], 0, r, g, batch, q0);
         tma_load_5d(qdst + FB_CHUNK, &tmQ, &q_full[qb], 64, r, g, batch, q0);
+        bulk_load(smem + FbSmem::STAT_OFF + qb * FB_STATS * 4, stats + static_cast<size_t>(qt) * FB_STATS, FB_STATS * 4,
+                  &q_full[qb]);
         if (!mbar_wait(do_empty, (it & 1u) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
         mbar_expect_tx(do_full, FB_TILE);
         tma_load_4d(smem + FbSmem::DO_OFF, &tmDO, do_full, 0, head, batch, q0);
@@ -183,257 +165,265 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         while (globaltimer_ns() - t0 < 200000ull) {}
       }
     }
-  } else if (warp == 1) {
-    constexpr uint32_t id_kk = make_idesc_bf16(FB_T, FB_T, false, false);   // A K-major, B K-major
-    constexpr uint32_t id_mm = make_idesc_bf16(FB_T, FB_T, true, true);     // A MN-major, B MN-major
-    constexpr uint32_t id_km = make_idesc_bf16(FB_T, FB_T, false, true);    // A K-major, B MN-major
-    const uint32_t a_k = smem_u32(smem + FbSmem::K_OFF), a_v = smem_u32(smem + FbSmem::V_OFF);
-    const uint32_t a_q0 = smem_u32(smem + FbSmem::Q_OFF), a_do = smem_u32(smem + FbSmem::DO_OFF);
-    const uint32_t a_p = smem_u32(smem + FbSmem::P_OFF), a_ds = smem_u32(smem + FbSmem::DS_OFF);
-    auto kmaj = [](uint32_t base, int k) { return make_smem_desc(base + (k >> 2) * FB_CHUNK + (k & 3) * 32, 16, 1024); };
-    auto mnmaj = [](uint32_t base, int k) { return make_smem_desc(base + k * 2048, FB_CHUNK, 1024); };
-    bool ok = n_it > 0;
-    if (ok) ok = mbar_wait(kv_full, 0, abort_flag, p.status, ST_TIMEOUT_FULL);
-    if (ok) ok = mbar_wait(&q_full[0], 0, abort_flag, p.status, ST_TIMEOUT_FULL);
-    if (ok) {
-      tc_fence_after();
-      if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) umma_ss(t_s, kmaj(a_q0, k), kmaj(a_k, k), id_kk, k > 0);
-        umma_commit(s_full);
-      }
-      __syncwarp();
-    }
-    for (int it = 0; it < n_it && ok; ++it) {
-      const uint32_t ph = it & 1u;
-      const uint32_t a_q = a_q0 + (it & 1) * FB_TILE;
-      // dP(it) overwrites the columns that held dQ(it-1)
-      if (!mbar_wait(do_full, ph, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-      if (!mbar_wait(dq_empty, ph ^ 1u, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
-      tc_fence_after();
-      if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) umma_ss(t_dp, kmaj(a_do, k), kmaj(a_v, k), id_kk, k > 0);
-        umma_commit(dp_full);
-      }
-      __syncwarp();
-      if (!mbar_wait(pds_full, ph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-      tc_fence_after();
-      if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) umma_ss(t_dv, mnmaj(a_p, k), mnmaj(a_do, k), id_mm, (it > 0 || k > 0));
-#pragma unroll
-        for (int k = 0; k < 8; ++k) umma_ss(t_dk, mnmaj(a_ds, k), mnmaj(a_q, k), id_mm, (it > 0 || k > 0));
-#pragma unroll
-        for (int k = 0; k < 8; ++k) umma_ss(t_dq, kmaj(a_ds, k), mnmaj(a_k, k), id_km, k > 0);
-        umma_commit(&q_empty[it & 1]);
-        umma_commit(do_empty);
-        umma_commit(dq_full);
-      }
-      __syncwarp();
-      if (it + 1 < n_it) {
-        // S of the next tile: its Q is already there, and S(it) has been read (pds_full above)
-        const int nb = (it + 1) & 1;
-        if (!mbar_wait(&q_full[nb], ((it + 1) >> 1) & 1u, abort_flag, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-        tc_fence_after();
-        if (lane == 0) {
-          const uint32_t a_qn = a_q0 + nb * FB_TILE;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) umma_ss(t_s, kmaj(a_qn, k), kmaj(a_k, k), id_kk, k > 0);
-          umma_commit(s_full);
-        }
-        __syncwarp();
-      }
-    }
-    if (ok && lane == 0) umma_commit(all_done);
     __syncwarp();
-  } else {
-    const int quarter = warp & 3;            // TMEM lanes this warp may read
-    const int row = quarter * 32 + lane;
-    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    const bool softmax_role = warp < 2 + FB_SOFTMAX_WARPS;
-    const int c = (warp - 2) >> 2;           // softmax warps: chunk of 32 key columns
-    bool ok = n_it > 0;
-    int it = -1;
-    if (softmax_role) {
-      const float lg2e = 1.4426950408889634f;
-      // 16-byte units of this thread inside its row of P / dS (two 64-wide swizzled chunks per row)
-      uint32_t unit_off[4];
+  } else if (warp == FB_MMA_WARP) {
+    if (n_it > 0 && elect_one()) {           // one thread runs the whole role, see elect_one()
+      constexpr uint32_t id_kk = make_idesc_bf16(FB_T, FB_T, false, false);   // A K-major, B K-major
+      constexpr uint32_t id_mm = make_idesc_bf16(FB_T, FB_T, true, true);     // A MN-major, B MN-major
+      constexpr uint32_t id_km = make_idesc_bf16(FB_T, FB_T, false, true);    // A K-major (or TMEM), B MN-major
+      const uint32_t base = smem_u32(smem);
+      // descriptors of an operand for 16-deep step k: K-major rows, or MN-major with 64-wide chunks
+      auto kmaj = [&](int off, int k) {
+        return make_smem_desc(base + off, 16, 1024) + static_cast<uint64_t>(((k >> 2) * FB_CHUNK + (k & 3) * 32) >> 4);
+      };
+      auto mnmaj = [&](int off, int k) {
+        return make_smem_desc(base + off, FB_CHUNK, 1024) + static_cast<uint64_t>((k * 2048) >> 4);
+      };
+      bool ok = true;
+      auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+        ok = mbar_wait(bar, parity, abort_flag, p.status, code);
+        if (ok) tc_fence_after();
+        return ok;
+      };
+      auto issue_s = [&](int i) {
+        const int q = FbSmem::Q_OFF + (i & 1) * FB_TILE;
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        unit_off[u] = (c >> 1) * FB_CHUNK + row * 128 + ((((c & 1) * 4 + u) ^ (row & 7)) << 4);
-      for (int qt = 0; qt < n_q && ok; ++qt) {
-        if (!q_tile_sees(p, qt, k0)) continue;
-        ++it;
+        for (int k = 0; k < 8; ++k) umma_ss(t_s, kmaj(FbSmem::K_OFF, k), kmaj(q, k), id_kk, k > 0);
+        umma_commit(s_full);
+      };
+      if (wait(kv_full, 0, ST_TIMEOUT_FULL) && wait(&q_full[0], 0, ST_TIMEOUT_FULL)) issue_s(0);
+      for (int it = 0; it < n_it && ok; ++it) {
         const uint32_t ph = it & 1u;
-        const int q0 = qt * FB_T;
-        const int q_off = p.geom.q_offset_of(q0, p.q_offset);
-        const int qrow = q0 + row;
-        const int qpos = q_off + qrow;
-        const bool valid = qrow < p.sq;
-        const size_t stat = (static_cast<size_t>(batch) * p.hq + head) * p.sq + (valid ? qrow : 0);
-        const float lse2 = valid ? p.lse[stat] * lg2e : 0.f;
-        const float dlt = valid ? p.delta[stat] : 0.f;
-        const bool tile_mask = (p.causal && k0 + FB_T - 1 > q_off + q0) || (k0 + FB_T > p.skv) || (q0 + FB_T > p.sq);
-        // S(it) ready: the products of tile it-1 were issued before it, so P and dS buffers are free
-        if (!mbar_wait(s_full, ph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-        tc_fence_after();
-        uint32_t pk[16];                       // this thread's 32 values of P as packed bf16, kept for dS
-        {
-          uint32_t sv[32];
-          tmem_ld_32x32(t_s + lane_addr + c * 32, sv);
-          tmem_ld_wait();
+        const int q = FbSmem::Q_OFF + (it & 1) * FB_TILE;
+        // dPᵀ(it) overwrites the columns that held dQ(it-1)
+        if (!wait(do_full, ph, ST_TIMEOUT_FULL) || !wait(dq_empty, ph ^ 1u, ST_TIMEOUT_TMEM_EMPTY)) break;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
+        for (int k = 0; k < 8; ++k) umma_ss(t_dp, kmaj(FbSmem::V_OFF, k), kmaj(FbSmem::DO_OFF, k), id_kk, k > 0);
+        umma_commit(dp_full);
+        if (!wait(p_full, ph, ST_TIMEOUT_TMEM_FULL)) break;
 #pragma unroll
-            for (int h2 = 0; h2 < 4; ++h2) {
-              const int i = 8 * u + 2 * h2;
-              float e0 = bwd_exp2(__uint_as_float(sv[i]) * p.scale_log2 - lse2);
-              float e1 = bwd_exp2(__uint_as_float(sv[i + 1]) * p.scale_log2 - lse2);
-              if (tile_mask) {
-                const int key = k0 + c * 32 + i;
-                if (!valid || (p.causal && key > qpos) || key >= p.skv) e0 = 0.f;
-                if (!valid || (p.causal && key + 1 > qpos) || key + 1 >= p.skv) e1 = 0.f;
-              }
-              pk[u * 4 + h2] = pack_bf16x2(e0, e1);
-            }
-            *reinterpret_cast<uint4*>(smem + FbSmem::P_OFF + unit_off[u]) =
-                make_uint4(pk[u * 4], pk[u * 4 + 1], pk[u * 4 + 2], pk[u * 4 + 3]);
-          }
+        for (int k = 0; k < 8; ++k)          // 16 queries: 8 columns of Pᵀ, 16 rows of dO
+          umma_ts(t_dv, t_s + (k >> 1) * 32 + (k & 1) * 8, mnmaj(FbSmem::DO_OFF, k), id_km, (it > 0 || k > 0));
+        umma_commit(do_empty);
+        if (it + 1 < n_it) {
+          // overwrites Pᵀ(it): the product before it reads it in order
+          if (!wait(&q_full[(it + 1) & 1], ((it + 1) >> 1) & 1u, ST_TIMEOUT_FULL)) break;
+          issue_s(it + 1);
         }
-        if (!mbar_wait(dp_full, ph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-        // the dS buffer doubled as staging area of the previous tile's dQ reductions
-        if (it > 0 && !mbar_wait(stage_free, (it - 1) & 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
-        tc_fence_after();
-        {
-          uint32_t dv[32];
-          tmem_ld_32x32(t_dp + lane_addr + c * 32, dv);
-          tmem_ld_wait();
+        if (!wait(ds_full, ph, ST_TIMEOUT_TMEM_FULL)) break;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint32_t wd[4];
+        for (int k = 0; k < 8; ++k) umma_ss(t_dq, mnmaj(FbSmem::DS_OFF, k), mnmaj(FbSmem::K_OFF, k), id_mm, k > 0);
+        umma_commit(dq_full);
 #pragma unroll
-            for (int h2 = 0; h2 < 4; ++h2) {
-              const int i = 8 * u + 2 * h2;
-              const float2 e = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[u * 4 + h2]));
-              const float d0 = e.x * (__uint_as_float(dv[i]) - dlt) * p.scale;
-              const float d1 = e.y * (__uint_as_float(dv[i + 1]) - dlt) * p.scale;
-              wd[h2] = pack_bf16x2(d0, d1);
-            }
-            *reinterpret_cast<uint4*>(smem + FbSmem::DS_OFF + unit_off[u]) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
-          }
-        }
-        tc_fence_before();
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(pds_full);
+        for (int k = 0; k < 8; ++k) umma_ss(t_dk, kmaj(FbSmem::DS_OFF, k), mnmaj(q, k), id_km, (it > 0 || k > 0));
+        umma_commit(&q_empty[it & 1]);
+        umma_commit(ds_empty);
       }
-    } else {
-      // dQ tile → fp32 reductions into the global accumulator, 32 columns (16 KB) at a time through the two
-      // halves of the dS buffer: 128-byte rows with their 16-byte units swizzled by row, as the tensor
-      // map of the accumulator expects
-      const bool leader = threadIdx.x == (2 + FB_SOFTMAX_WARPS) * 32;
-      uint8_t* stage = smem + FbSmem::DS_OFF;
-      for (int qt = 0; qt < n_q && ok; ++qt) {
-        if (!q_tile_sees(p, qt, k0)) continue;
-        ++it;
-        const uint32_t ph = it & 1u;
-        // one decision for the 128 threads (they meet at named barriers below); the leader comes here only
-        // after the previous tile's reductions have read the staging area
-        ok = drain_all(mbar_wait(dq_full, ph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL));
-        if (!ok) break;
-        tc_fence_after();
-#pragma unroll 1
-        for (int cc = 0; cc < 4; ++cc) {
-          uint8_t* buf = stage + (cc & 1) * 16384;
-          if (cc >= 2) {
-            if (leader) tma_store_wait_read<1>();      // the reduction of chunk cc-2 has read this half
-            drain_sync();
-          }
-          uint32_t v[32];
-          tmem_ld_32x32(t_dq + lane_addr + cc * 32, v);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<uint4*>(buf + row * 128 + ((j ^ (row & 7)) << 4)) =
-                make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          fence_proxy_async_smem();
-          if (cc == 3) tc_fence_before();
-          drain_sync();
-          if (leader) {
-            tma_reduce_add_4d(&tmDQ, buf, cc * 32, head, batch, qt * FB_T);   // rows past sq are clipped
-            tma_store_commit();
-          }
-        }
-        if (leader) {
-          mbar_arrive(dq_empty);                       // every thread's TMEM reads preceded the last barrier
-          tma_store_wait_read<0>();
-          mbar_arrive(stage_free);
-        }
-      }
-      if (leader) tma_store_wait<0>();                 // nothing in flight out of shared memory at exit
+      if (ok) umma_commit(all_done);
     }
-    // dV and dK of this key tile → fp32 accumulators (rows = keys); softmax warp (quarter, c) takes
-    // columns 32c..32c+31 of both
-    if (n_it > 0 && softmax_role) {
-      if (ok) ok = mbar_wait(all_done, 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
+    __syncwarp();
+  } else if (warp < FB_SOFTMAX_WARPS) {
+    const int row = (warp & 3) * 32 + lane;        // key row of the tile = TMEM lane
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const int c = warp >> 2;                       // chunk of 32 query columns
+    const int key = k0 + row;
+    // 16-byte units of this thread inside its row of dSᵀ (two 64-wide swizzled chunks per row)
+    const uint32_t ds_row = smem_u32(smem) + FbSmem::DS_OFF + (c >> 1) * FB_CHUNK + row * 128;
+    const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
+    bool ok = true;
+    int it = -1;
+    for (int qt = 0; qt < n_q && ok; ++qt) {
+      if (!q_tile_sees(p, qt, k0)) continue;
+      ++it;
+      const uint32_t ph = it & 1u;
+      const int q0 = qt * FB_T;
+      const int q_off = p.geom.q_offset_of(q0, p.q_offset);
+      const float4* stat = reinterpret_cast<const float4*>(smem + FbSmem::STAT_OFF + (it & 1) * FB_STATS * 4) + c * 8;
+      const bool tile_mask = (p.causal && k0 + FB_T - 1 > q_off + q0) || (k0 + FB_T > p.skv);
+      // the scores were issued behind the arrival of Q and its statistics; this wait makes the latter visible here
+      ok = __all_sync(0xffffffffu,
+                      mbar_wait(&q_full[it & 1], (it >> 1) & 1u, abort_flag, p.status, ST_TIMEOUT_FULL) &&
+                          mbar_wait(s_full, ph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL));
+      if (!ok) break;
       tc_fence_after();
-      const int key = k0 + row;
+      uint32_t pk[16];                             // 32 values of Pᵀ as packed bf16, kept for dSᵀ
+      {
+        uint32_t sv[32];
+        tmem_ld_32x32(t_s + lane_addr + c * 32, sv);
+        tmem_ld_wait();
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const float4 nl = stat[u];               // rows past sq carry −inf: Pᵀ = 0
+          float2 a = __ffma2_rn(make_float2(__uint_as_float(sv[4 * u]), __uint_as_float(sv[4 * u + 1])), sc2,
+                                make_float2(nl.x, nl.y));
+          float2 b = __ffma2_rn(make_float2(__uint_as_float(sv[4 * u + 2]), __uint_as_float(sv[4 * u + 3])), sc2,
+                                make_float2(nl.z, nl.w));
+          pk[2 * u] = pack_bf16x2(bwd_exp2(a.x), bwd_exp2(a.y));
+          pk[2 * u + 1] = pack_bf16x2(bwd_exp2(b.x), bwd_exp2(b.y));
+        }
+      }
+      if (tile_mask) {
+        // query column x of the chunk sees this key from `first` on
+        const int first = key >= p.skv ? 32 : p.causal ? key - (q_off + q0 + c * 32) : 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if (2 * i < first) pk[i] &= 0xffff0000u;
+          if (2 * i + 1 < first) pk[i] &= 0x0000ffffu;
+        }
+      }
+      tmem_st_32x32_x16(t_s + lane_addr + c * 32, pk);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+      // ds_empty: the products of the previous tile have read the dS buffer
+      ok = __all_sync(0xffffffffu, mbar_wait(ds_empty, ph ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY) &&
+                                       mbar_wait(dp_full, ph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL));
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t dv[32];
+      tmem_ld_32x32(t_dp + lane_addr + c * 32, dv);
+      tmem_ld_wait();
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        uint32_t wd[4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float4 nd = stat[FB_T / 4 + 2 * u + h];
+          const int i = 8 * u + 4 * h;
+          const float2 e0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[i / 2]));
+          const float2 e1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[i / 2 + 1]));
+          const float2 d0 = __fmul2_rn(e0, __fadd2_rn(make_float2(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])),
+                                                      make_float2(nd.x, nd.y)));
+          const float2 d1 = __fmul2_rn(e1, __fadd2_rn(make_float2(__uint_as_float(dv[i + 2]), __uint_as_float(dv[i + 3])),
+                                                      make_float2(nd.z, nd.w)));
+          wd[2 * h] = pack_bf16x2(d0.x, d0.y);
+          wd[2 * h + 1] = pack_bf16x2(d1.x, d1.y);
+        }
+        st_shared_v4(ds_row + ((((c & 1) * 4 + u) ^ (row & 7)) << 4), wd[0], wd[1], wd[2], wd[3]);
+      }
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ds_full);
+    }
+    // dV and dK of this key tile → fp32 accumulators (rows = keys); this warp takes columns 32c..32c+31 of both
+    if (n_it > 0) {
+      if (ok) ok = mbar_wait(all_done, 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
+      __syncwarp();
+      tc_fence_after();
       const bool kvalid = ok && key < p.skv;
       const size_t base = ((static_cast<size_t>(kvalid ? key : 0) * p.b + batch) * (p.hq / p.rep) + g) * FB_T;
 #pragma unroll 1
       for (int which = 0; which < 2; ++which) {
         float* dst = (which == 0 ? p.dv_acc : p.dk_acc) + base + c * 32;
+        const float f = which == 0 ? 1.f : p.scale;
         uint32_t v[32];
         tmem_ld_32x32((which == 0 ? t_dv : t_dk) + lane_addr + c * 32, v);
         tmem_ld_wait();
         if (kvalid) {
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            red_add_v4(dst + 4 * j, __uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                       __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+            red_add_v4(dst + 4 * j, __uint_as_float(v[4 * j]) * f, __uint_as_float(v[4 * j + 1]) * f,
+                       __uint_as_float(v[4 * j + 2]) * f, __uint_as_float(v[4 * j + 3]) * f);
         }
       }
     }
+  } else if (warp < FB_TMA_WARP) {
+    // dQ tile → fp32 reductions into the global accumulator.  The warp's 32 rows go out 32 columns (4 KB) at a time
+    // through two buffers: 128-byte rows with their 16-byte units swizzled by row, as the tensor map expects.
+    // The second half of the columns is read before the buffers are free again, so that TMEM is handed back early.
+    const int quarter = warp & 3;
+    const uint32_t t_mine = t_dq + (static_cast<uint32_t>(quarter * 32) << 16);
+    uint8_t* stg = smem + FbSmem::STG_OFF + quarter * 8192;
+    const uint32_t stg_row = smem_u32(stg) + lane * 128;
+    auto put = [&](int buf, const uint32_t (&v)[32]) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        st_shared_v4(stg_row + buf * 4096 + ((j ^ (lane & 7)) << 4), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    };
+    int it = -1;
+    for (int qt = 0; qt < n_q; ++qt) {
+      if (!q_tile_sees(p, qt, k0)) continue;
+      ++it;
+      if (!__all_sync(0xffffffffu, mbar_wait(dq_full, it & 1u, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL))) break;
+      tc_fence_after();
+      const int row0 = qt * FB_T + quarter * 32;
+      uint32_t v0[32], v1[32];
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        tmem_ld_32x32(t_mine + half * 64, v0);
+        tmem_ld_32x32(t_mine + half * 64 + 32, v1);
+        tmem_ld_wait();
+        if (half == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(dq_empty);
+        }
+        if (lane == 0) tma_store_wait_read<0>();      // the reductions before these have read both buffers
+        __syncwarp();
+        put(0, v0);
+        put(1, v1);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && row0 < p.sq) {               // the tensor map clips rows past sq
+          tma_reduce_add_4d(&tmDQ, stg, half * 64, head, batch, row0);
+          tma_reduce_add_4d(&tmDQ, stg + 4096, half * 64 + 32, head, batch, row0);
+          tma_store_commit();
+        }
+      }
+    }
+    if (lane == 0) tma_store_wait<0>();               // nothing in flight out of shared memory at exit
+    __syncwarp();
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == FB_MMA_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
 }
 
-// delta[b, h, s] = Σ_d dO[s,b,h,d] · O[s,b,h,d]   (both [s,b,h,d] contiguous), one warp per row
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
-                                  float* __restrict__ delta, int S, int B, int H) {
-  const long rows = static_cast<long>(S) * B * H;
-  const int lane = threadIdx.x & 31;
-  for (long w = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w < rows;
-       w += (static_cast<long>(gridDim.x) * blockDim.x) >> 5) {
-    const uint2 a = reinterpret_cast<const uint2*>(dO + w * FB_T)[lane];
-    const uint2 b = reinterpret_cast<const uint2*>(O + w * FB_T)[lane];
-    const float2 a0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.x));
-    const float2 a1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.y));
-    const float2 b0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b.x));
-    const float2 b1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b.y));
-    float s = a0.x * b0.x + a0.y * b0.y + a1.x * b1.x + a1.y * b1.y;
+// Row statistics for the kernel above, one 1 KB block per query tile of one (batch, head): 128 x −lse·log2(e), then
+// 128 x −δ with δ = Σ_d dO·O (both [s,b,h,d] contiguous).  Rows past S get −inf and 0.  Half a warp per row.
+__global__ void __launch_bounds__(256)
+attn_stats_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
+                  const float* __restrict__ lse, float* __restrict__ stats, int S, int S_pad, int B, int H) {
+  const long rows = static_cast<long>(S_pad) * B * H;
+  const int l = threadIdx.x & 15;
+  const long step = (static_cast<long>(gridDim.x) * blockDim.x) >> 4;
+  for (long w0 = (static_cast<long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31)) >> 4; w0 < rows; w0 += step) {
+    const long w = w0 + ((threadIdx.x >> 4) & 1);
+    const int h = static_cast<int>(w % H);
+    const long sb = w / H;
+    const int bb = static_cast<int>(sb % B), ss = static_cast<int>(sb / B);
+    float s = 0.f;
+    if (ss < S && w < rows) {
+      const uint4 a = reinterpret_cast<const uint4*>(dO + w * FB_T)[l];
+      const uint4 b = reinterpret_cast<const uint4*>(O + w * FB_T)[l];
+      const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
+      const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) {
-      const int h = static_cast<int>(w % H);
-      const long sb = w / H;
-      const int bb = static_cast<int>(sb % B);
-      const long ss = sb / B;
-      delta[(static_cast<long>(bb) * H + h) * S + ss] = s;
+      for (int i = 0; i < 4; ++i) {
+        const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(b2[i]);
+        s += x.x * y.x + x.y * y.y;
+      }
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (l == 0 && w < rows) {
+      const long bh = static_cast<long>(bb) * H + h;
+      float* t = stats + (bh * (S_pad / FB_T) + ss / FB_T) * FB_STATS + ss % FB_T;
+      t[0] = ss < S ? lse[bh * S + ss] * -1.4426950408889634f : -INFINITY;
+      t[FB_T] = -s;
     }
   }
 }
 
-// fp32 accumulator [rows(s,b), heads, d] → bf16 strided view (strides in elements per s, b, head)
+// fp32 accumulator [rows(s,b), heads, d] times `scale` → bf16 strided view (strides in elements per s, b, head)
 __global__ void attn_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ out, long n_vec, int B,
-                                    int G, int R, long st_s, long st_b, long st_g, long st_r) {
+                                    int G, int R, long st_s, long st_b, long st_g, long st_r, float scale) {
   // one thread per 4 elements of d
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_vec;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
@@ -446,8 +436,8 @@ __global__ void attn_convert_kernel(const float* __restrict__ acc, __nv_bfloat16
     const float4 v = reinterpret_cast<const float4*>(acc)[i];
     __nv_bfloat16* o = out + ss * st_s + bb * st_b + gg * st_g + rr * st_r + dv * 4;
     uint2 w;
-    *reinterpret_cast<__nv_bfloat162*>(&w.x) = __floats2bfloat162_rn(v.x, v.y);
-    *reinterpret_cast<__nv_bfloat162*>(&w.y) = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<__nv_bfloat162*>(&w.x) = __floats2bfloat162_rn(v.x * scale, v.y * scale);
+    *reinterpret_cast<__nv_bfloat162*>(&w.y) = __floats2bfloat162_rn(v.z * scale, v.w * scale);
     *reinterpret_cast<uint2*>(o) = w;
   }
 }
@@ -472,9 +462,9 @@ static int make_qkv_map(CUtensorMap* m, const void* ptr, int d, int inner_heads,
 
 using namespace kb;
 
-// Scratch: `work` must hold (sq*b*hq*d + 2*skv*b*g*d + b*hq*sq) floats; it is zeroed here.
+// Scratch: `work` (16-byte aligned) must hold the fp32 accumulators of dQ, dK and dV, zeroed here, and the row statistics.
 extern "C" long kb_flash_attn_bwd_scratch_floats(int sq, int skv, int b, int g, int rep, int d) {
-  return (long)sq * b * g * rep * d + 2L * skv * b * g * d + (long)b * g * rep * sq;
+  return (long)sq * b * g * rep * d + 2L * skv * b * g * d + (long)b * g * rep * ((sq + FB_T - 1) / FB_T) * FB_STATS;
 }
 
 namespace kb {
@@ -523,20 +513,22 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
   float* dq_acc = work;
   float* dk_acc = dq_acc + n_dq;
   float* dv_acc = dk_acc + n_dkv;
-  float* delta = dv_acc + n_dkv;
+  float* stats = dv_acc + n_dkv;
   cudaError_t e = kb::memset_async(work, 0, sizeof(float) * (n_dq + 2 * n_dkv), stream);
   if (e != cudaSuccess) return 1000 + (int)e;
   {
-    const long rows = (long)sq * b * hq;
-    long blocks = (rows * 32 + 255) / 256;
+    const int s_pad = (sq + FB_T - 1) / FB_T * FB_T;
+    const long rows = (long)s_pad * b * hq;
+    long blocks = (rows * 16 + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    KB_LAUNCH(attn_delta_kernel, (int)blocks, 256, 0, stream, (const __nv_bfloat16*)dO, (const __nv_bfloat16*)o, delta, sq, b, hq);
+    KB_LAUNCH(attn_stats_kernel, (int)blocks, 256, 0, stream, (const __nv_bfloat16*)dO, (const __nv_bfloat16*)o, lse, stats,
+              sq, s_pad, b, hq);
   }
   CUtensorMap tmDO;
   int rc = make_qkv_map(&tmDO, dO, d, 1, hq, b, sq, 0, d, (long)hq * d, (long)b * hq * d, 0);
   if (rc) return rc;
   BwdParams p;
-  p.lse = lse; p.delta = delta; p.dq_acc = dq_acc; p.dk_acc = dk_acc; p.dv_acc = dv_acc;
+  p.stats = stats; p.dk_acc = dk_acc; p.dv_acc = dv_acc;
   p.sq = sq; p.skv = skv; p.b = b; p.hq = hq; p.rep = rep; p.q_offset = q_offset; p.causal = causal;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   p.geom = geom;
@@ -548,10 +540,10 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
   }
   CUtensorMap tmDQ;
   {
-    // fp32 accumulator [sq, b, hq, d]: boxes of 128 rows x 32 columns (128 bytes, swizzled) of one (b, head)
+    // fp32 accumulator [sq, b, hq, d]: boxes of 32 rows x 32 columns (128 bytes, swizzled) of one (b, head)
     uint64_t dims[4] = {(uint64_t)d, (uint64_t)hq, (uint64_t)b, (uint64_t)sq};
     uint64_t str[3] = {(uint64_t)d * 4, (uint64_t)hq * d * 4, (uint64_t)b * hq * d * 4};
-    uint32_t box[4] = {32, 1, 1, FB_T};
+    uint32_t box[4] = {32, 1, 1, 32};
     rc = make_tmap(&tmDQ, dq_acc, 4, 4, dims, str, box, 3);
     if (rc) return rc;
   }
@@ -569,7 +561,7 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     long blocks = (nvec + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
     KB_LAUNCH(attn_convert_kernel, (int)blocks, 256, 0, stream, (const float*)dq_acc, (__nv_bfloat16*)out.dq, nvec, b, g, rep,
-              out.dqs_s, out.dqs_b, out.dqs_g, out.dqs_r);
+              out.dqs_s, out.dqs_b, out.dqs_g, out.dqs_r, scale);
     nvec = n_dkv / 4;
     blocks = (nvec + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
