@@ -2,9 +2,11 @@
 //
 // One CTA owns 128 keys of one (batch, query head) and walks the query tiles that can see them.  Scores are
 // kept transposed (rows = keys), so that P leaves the registers as the TMEM operand of dV:
-//   warps 0..15  four threads per key row, 32 query columns each: Pᵀ = exp2(Sᵀ·c − lse) as soon as Sᵀ is there,
+//   warps 0..15  32 keys x 32 query columns each, as matrix fragments (a thread meets 8 columns on 4 rows): Pᵀ = exp2(Sᵀ·c − lse) as soon as Sᵀ is there,
 //                bf16 into the TMEM columns the scores came from; then dSᵀ = Pᵀ∘(dPᵀ − δ) once dPᵀ is there, bf16
-//                into swizzled shared memory.  lse and δ of a query tile are staged next to its Q
+//                into swizzled shared memory.  lse and δ of a query tile are staged next to its Q; with a key row
+//                per thread every thread would read all of its columns' statistics, which cost the shared-memory
+//                pipe more than the operands of two products
 //   warps 16..19 dQ from TMEM → 8 KB of shared memory per warp → TMA reduce-add into the fp32 accumulator in
 //                global memory, 32 rows x 32 columns at a time, no barrier between the warps
 //   warp 20      TMA producer: K and V once, then per query tile Q and its row statistics (two buffers) and dO
@@ -223,12 +225,12 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
     __syncwarp();
   } else if (warp < FB_SOFTMAX_WARPS) {
-    const int row = (warp & 3) * 32 + lane;        // key row of the tile = TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int c = warp >> 2;                       // chunk of 32 query columns
-    const int key = k0 + row;
-    // 16-byte units of this thread inside its row of dSᵀ (two 64-wide swizzled chunks per row)
-    const uint32_t ds_row = smem_u32(smem) + FbSmem::DS_OFF + (c >> 1) * FB_CHUNK + row * 128;
+    // this thread's fragment: key rows frag_row + 8 x (0..3), query columns frag_col + 8 n + (0, 1) of the chunk
+    const int frag_row = (warp & 3) * 32 + (lane >> 2), frag_col = 2 * (lane & 3);
+    // its rows of dSᵀ (two 64-wide swizzled chunks per row; frag_row & 7 is the row inside the swizzle atom)
+    const uint32_t ds_base = smem_u32(smem) + FbSmem::DS_OFF + (c >> 1) * FB_CHUNK + frag_row * 128 + (lane & 3) * 4;
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
     bool ok = true;
     int it = -1;
@@ -238,7 +240,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       const uint32_t ph = it & 1u;
       const int q0 = qt * FB_T;
       const int q_off = p.geom.q_offset_of(q0, p.q_offset);
-      const float4* stat = reinterpret_cast<const float4*>(smem + FbSmem::STAT_OFF + (it & 1) * FB_STATS * 4) + c * 8;
+      const float* stat = reinterpret_cast<const float*>(smem + FbSmem::STAT_OFF + (it & 1) * FB_STATS * 4) + c * 32 + frag_col;
       const bool tile_mask = (p.causal && k0 + FB_T - 1 > q_off + q0) || (k0 + FB_T > p.skv);
       // the scores were issued behind the arrival of Q and its statistics; this wait makes the latter visible here
       ok = __all_sync(0xffffffffu,
@@ -246,32 +248,38 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                           mbar_wait(s_full, ph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL));
       if (!ok) break;
       tc_fence_after();
-      uint32_t pk[16];                             // 32 values of Pᵀ as packed bf16, kept for dSᵀ
+      uint32_t pk[2][8];                           // Pᵀ of the fragment as packed bf16, kept for dSᵀ
       {
-        uint32_t sv[32];
-        tmem_ld_32x32(t_s + lane_addr + c * 32, sv);
+        uint32_t sv[2][16];
+        tmem_ld_16x256b_x4(t_s + lane_addr + c * 32, sv[0]);
+        tmem_ld_16x256b_x4(t_s + lane_addr + (16u << 16) + c * 32, sv[1]);
         tmem_ld_wait();
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const float4 nl = stat[u];               // rows past sq carry −inf: Pᵀ = 0
-          float2 a = __ffma2_rn(make_float2(__uint_as_float(sv[4 * u]), __uint_as_float(sv[4 * u + 1])), sc2,
-                                make_float2(nl.x, nl.y));
-          float2 b = __ffma2_rn(make_float2(__uint_as_float(sv[4 * u + 2]), __uint_as_float(sv[4 * u + 3])), sc2,
-                                make_float2(nl.z, nl.w));
-          pk[2 * u] = pack_bf16x2(bwd_exp2(a.x), bwd_exp2(a.y));
-          pk[2 * u + 1] = pack_bf16x2(bwd_exp2(b.x), bwd_exp2(b.y));
+        for (int n = 0; n < 4; ++n) {
+          const float2 nl = *reinterpret_cast<const float2*>(stat + 8 * n);   // rows past sq carry −inf: Pᵀ = 0
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            const float2 x = __ffma2_rn(make_float2(__uint_as_float(sv[h >> 1][4 * n + 2 * (h & 1)]),
+                                                    __uint_as_float(sv[h >> 1][4 * n + 2 * (h & 1) + 1])), sc2, nl);
+            pk[h >> 1][2 * n + (h & 1)] = pack_bf16x2(bwd_exp2(x.x), bwd_exp2(x.y));
+          }
         }
       }
       if (tile_mask) {
-        // query column x of the chunk sees this key from `first` on
-        const int first = key >= p.skv ? 32 : p.causal ? key - (q_off + q0 + c * 32) : 0;
+        // fragment column x sees its key from `first` on
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          if (2 * i < first) pk[i] &= 0xffff0000u;
-          if (2 * i + 1 < first) pk[i] &= 0x0000ffffu;
+        for (int h = 0; h < 4; ++h) {
+          const int key = k0 + frag_row + 8 * h;
+          const int first = key >= p.skv ? 32 : p.causal ? key - (q_off + q0 + c * 32 + frag_col) : 0;
+#pragma unroll
+          for (int n = 0; n < 4; ++n) {
+            if (8 * n < first) pk[h >> 1][2 * n + (h & 1)] &= 0xffff0000u;
+            if (8 * n + 1 < first) pk[h >> 1][2 * n + (h & 1)] &= 0x0000ffffu;
+          }
         }
       }
-      tmem_st_32x32_x16(t_s + lane_addr + c * 32, pk);
+      tmem_st_16x128b_x4(t_s + lane_addr + c * 32, pk[0]);
+      tmem_st_16x128b_x4(t_s + lane_addr + (16u << 16) + c * 32, pk[1]);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -281,26 +289,21 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                                        mbar_wait(dp_full, ph, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL));
       if (!ok) break;
       tc_fence_after();
-      uint32_t dv[32];
-      tmem_ld_32x32(t_dp + lane_addr + c * 32, dv);
+      uint32_t dv[2][16];
+      tmem_ld_16x256b_x4(t_dp + lane_addr + c * 32, dv[0]);
+      tmem_ld_16x256b_x4(t_dp + lane_addr + (16u << 16) + c * 32, dv[1]);
       tmem_ld_wait();
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        uint32_t wd[4];
+      for (int n = 0; n < 4; ++n) {
+        const float2 nd = *reinterpret_cast<const float2*>(stat + FB_T + 8 * n);
+        const uint32_t unit = ds_base + ((((c & 1) * 4 + n) ^ (frag_row & 7)) << 4);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float4 nd = stat[FB_T / 4 + 2 * u + h];
-          const int i = 8 * u + 4 * h;
-          const float2 e0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[i / 2]));
-          const float2 e1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[i / 2 + 1]));
-          const float2 d0 = __fmul2_rn(e0, __fadd2_rn(make_float2(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])),
-                                                      make_float2(nd.x, nd.y)));
-          const float2 d1 = __fmul2_rn(e1, __fadd2_rn(make_float2(__uint_as_float(dv[i + 2]), __uint_as_float(dv[i + 3])),
-                                                      make_float2(nd.z, nd.w)));
-          wd[2 * h] = pack_bf16x2(d0.x, d0.y);
-          wd[2 * h + 1] = pack_bf16x2(d1.x, d1.y);
+        for (int h = 0; h < 4; ++h) {
+          const float2 e = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[h >> 1][2 * n + (h & 1)]));
+          const float2 d = __fmul2_rn(e, __fadd2_rn(make_float2(__uint_as_float(dv[h >> 1][4 * n + 2 * (h & 1)]),
+                                                                __uint_as_float(dv[h >> 1][4 * n + 2 * (h & 1) + 1])), nd));
+          st_shared_u32(unit + h * 1024, pack_bf16x2(d.x, d.y));
         }
-        st_shared_v4(ds_row + ((((c & 1) * 4 + u) ^ (row & 7)) << 4), wd[0], wd[1], wd[2], wd[3]);
       }
       tc_fence_before();
       fence_proxy_async_smem();
@@ -312,6 +315,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (ok) ok = mbar_wait(all_done, 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
       __syncwarp();
       tc_fence_after();
+      const int key = k0 + (warp & 3) * 32 + lane;
       const bool kvalid = ok && key < p.skv;
       const size_t base = ((static_cast<size_t>(kvalid ? key : 0) * p.b + batch) * (p.hq / p.rep) + g) * FB_T;
 #pragma unroll 1
