@@ -21,6 +21,8 @@ def _lib():
         L.kb_flash_attn_bwd.restype = c_int
         L.kb_flash_attn_bwd_scratch_floats.argtypes = [I] * 6
         L.kb_flash_attn_bwd_scratch_floats.restype = c_long
+        L.kb_flash_attn_bwd_launches.argtypes = [I] * 5
+        L.kb_flash_attn_bwd_launches.restype = c_int
         _DECLARED = True
     return L
 
@@ -74,7 +76,7 @@ def backward(do, q, k, v, o, lse, scale, causal=True, q_offset=0, kv_len=None, o
                              sq, skv, b, g, rep, d, float(scale), 1 if causal else 0, int(q_offset), st.data_ptr(),
                              KC._stream())
     KC._check(rc, "flash_attn_bwd")
-    KC._count(6)
+    KC._count(L.kb_flash_attn_bwd_launches(sq, skv, b, g, rep))
     if out is not None:
         return out
     return dq.reshape(q.shape), dk, dv
@@ -116,5 +118,5 @@ def backward_chunked(do, q, sources, table, chunk_rows, q_positions, o, lse, sca
         _int_array(dv_row_base), work.data_ptr(), sq, b, g, rep, d, float(scale), 1 if causal else 0, st.data_ptr(),
         KC._stream())
     KC._check(rc, "flash_attn_bwd_chunked")
-    KC._count(6)
+    KC._count(L.kb_flash_attn_bwd_launches(sq, skv, b, g, rep))
     return dq, dkv

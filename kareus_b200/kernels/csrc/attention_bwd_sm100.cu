@@ -1,6 +1,6 @@
 // Causal GQA flash-attention backward for sm_100a (head dim 128, bf16, fp32 accumulation).
 //
-// One CTA owns 128 keys of one (batch, query head) and walks the query tiles that can see them.  Scores are
+// One CTA owns 128 keys of one (batch, KV group) and walks the query tiles that can see them.  Scores are
 // kept transposed (rows = keys), so that P leaves the registers as the TMEM operand of dV:
 //   warps 0..15  32 keys x 32 query columns each, as matrix fragments (a thread meets 8 columns on 4 rows): Pᵀ = exp2(Sᵀ·c − lse) as soon as Sᵀ is there,
 //                bf16 into the TMEM columns the scores came from; then dSᵀ = Pᵀ∘(dPᵀ − δ) once dPᵀ is there, bf16
@@ -16,8 +16,10 @@
 // scores, and dQ of tile i leaves TMEM under dK.  dSᵀ is stored once ([key][query], queries contiguous) and serves
 // as K-major operand (dK) and, through an MN-major descriptor, as transposed operand of dQ.  The softmax scale is
 // applied to dQ and dK once, where they leave, and not to every element of dS.
-// TMEM: Sᵀ|Pᵀ + dPᵀ|dQ + dV + dK = 512 columns.  dK/dV stay in TMEM across the whole walk and are added to fp32
-// accumulators at the end (query heads of one KV group run in different CTAs).
+// TMEM: Sᵀ|Pᵀ + dPᵀ|dQ + dV + dK = 512 columns.  dK/dV stay in TMEM across the whole walk.
+// A CTA walks all query heads of its KV group one after the other and writes dK and dV itself.  Where that leaves
+// SMs idle (merge_heads), every query head gets its own CTA and dK/dV are added up in fp32 accumulators.  Starting
+// and ending a CTA costs about as much as three query tiles, and accumulators have to be zeroed and converted.
 // Shared memory: K, V, Q x 2, dO, dS, dQ staging = 7 tiles of 32 KB.
 //
 // Chunked keys and queries (context parallelism, see attention_chunks.h): K/V tiles may come from
@@ -44,10 +46,29 @@ constexpr int FB_TMA_WARP = FB_DQ_WARP + 4, FB_MMA_WARP = FB_DQ_WARP + 5;
 constexpr int FB_THREADS = (FB_SOFTMAX_WARPS + 6) * 32;
 constexpr int FB_STATS = 2 * FB_T;               // floats of row statistics per query tile: −lse·log2(e), then −δ
 
+// Destinations, strides in elements.
+struct RowMap {
+  int chunk_rows;                    // 0: rows map to themselves
+  int base[MAX_KV_CHUNKS];
+  __device__ __forceinline__ long at(long row) const {
+    if (chunk_rows == 0) return row;
+    const int c = static_cast<int>(row / chunk_rows);
+    return base[c] + (row - static_cast<long>(c) * chunk_rows);
+  }
+};
+struct BwdOut {
+  void* dq; long dqs_s, dqs_b, dqs_g, dqs_r;
+  void* dk; long dks_s, dks_b, dks_g;
+  void* dv; long dvs_s, dvs_b, dvs_g;
+  RowMap dk_rows, dv_rows;
+};
+
 struct BwdParams {
   const float* stats;    // [b, hq, query tiles, 2, 128], see attn_stats_kernel
-  float* dk_acc;         // [skv, b, g, d]
+  float* dk_acc;         // [skv, b, g, d]  (one query head per CTA)
   float* dv_acc;         // [skv, b, g, d]
+  int heads;             // query heads of a CTA: rep (the CTA writes dK and dV) or 1
+  BwdOut out;
   int sq, skv, b, hq, rep, q_offset, causal;
   float scale, scale_log2;
   int* status;
@@ -60,6 +81,21 @@ __device__ __forceinline__ bool q_tile_sees(const BwdParams& p, int qt, int k0) 
   const int q0 = qt * FB_T;
   return p.geom.q_offset_of(q0, p.q_offset) + q0 + FB_T - 1 >= k0;
 }
+
+// The query tiles of heads head0, head0 + 1, ... that see a key tile, in order.
+struct QTiles {
+  int n_q, qt, head;
+  __device__ __forceinline__ QTiles(int n, int head0) : n_q(n), qt(-1), head(head0) {}
+  __device__ __forceinline__ bool next(const BwdParams& p, int k0, int head1) {
+    for (;;) {
+      if (++qt == n_q) {
+        qt = 0;
+        if (++head >= head1) return false;
+      }
+      if (q_tile_sees(p, qt, k0)) return true;
+    }
+  }
+};
 
 struct FbSmem {
   // Q_OFF: two consecutive tiles (buffer = iteration & 1)
@@ -108,12 +144,13 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kt = blockIdx.x;                 // key tile; tile 0 is seen by the most queries → first
-  const int head = blockIdx.y, batch = blockIdx.z;
-  const int g = head / p.rep, r = head % p.rep;
+  const int head0 = blockIdx.y * p.heads, head1 = head0 + p.heads, batch = blockIdx.z;
+  const int g = head0 / p.rep;
   const int k0 = kt * FB_T;
   const int n_q = (p.sq + FB_T - 1) / FB_T;
-  int n_it = 0;                              // query tiles that see this key tile
+  int n_it = 0;                              // query tiles that see this key tile, over all heads
   for (int qt = 0; qt < n_q; ++qt) n_it += q_tile_sees(p, qt, k0) ? 1 : 0;
+  n_it *= p.heads;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 15; ++i)
@@ -136,7 +173,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       int src, srow;
       p.geom.locate(k0, src, srow);
       prefetch_tmap(&tmQ); prefetch_tmap(&kv.k[src]); prefetch_tmap(&kv.v[src]); prefetch_tmap(&tmDO);
-      const float* stats = p.stats + (static_cast<size_t>(batch) * p.hq + head) * n_q * FB_STATS;
+      const float* stats = p.stats + static_cast<size_t>(batch) * p.hq * n_q * FB_STATS;
       mbar_expect_tx(kv_full, 2 * FB_TILE);
       tma_load_4d(smem + FbSmem::K_OFF, &kv.k[src], kv_full, 0, g, batch, srow);
       tma_load_4d(smem + FbSmem::K_OFF + FB_CHUNK, &kv.k[src], kv_full, 64, g, batch, srow);
@@ -145,8 +182,9 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // per visible tile: Q(it) into buffer it & 1 (released by dK of tile it-2), then dO(it) (released by dV of
       // tile it-1): Q(it+1) goes out right behind dO(it), one tile ahead of the MMAs
       int it = 0;
-      for (int qt = 0; qt < n_q; ++qt) {
-        if (!q_tile_sees(p, qt, k0)) continue;
+      QTiles tiles(n_q, head0);
+      while (tiles.next(p, k0, head1)) {
+        const int qt = tiles.qt, head = tiles.head, r = head - g * p.rep;
         const int qb = it & 1;
         const int q0 = qt * FB_T;
         if (!mbar_wait(&q_empty[qb], ((it >> 1) & 1u) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
@@ -154,8 +192,8 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         mbar_expect_tx(&q_full[qb], FB_TILE + FB_STATS * 4);
         tma_load_5d(qdst, &tmQ, &q_full[qb], 0, r, g, batch, q0);
         tma_load_5d(qdst + FB_CHUNK, &tmQ, &q_full[qb], 64, r, g, batch, q0);
-        bulk_load(smem + FbSmem::STAT_OFF + qb * FB_STATS * 4, stats + static_cast<size_t>(qt) * FB_STATS, FB_STATS * 4,
-                  &q_full[qb]);
+        bulk_load(smem + FbSmem::STAT_OFF + qb * FB_STATS * 4, stats + (static_cast<size_t>(head) * n_q + qt) * FB_STATS,
+                  FB_STATS * 4, &q_full[qb]);
         if (!mbar_wait(do_empty, (it & 1u) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
         mbar_expect_tx(do_full, FB_TILE);
         tma_load_4d(smem + FbSmem::DO_OFF, &tmDO, do_full, 0, head, batch, q0);
@@ -234,11 +272,11 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
     bool ok = true;
     int it = -1;
-    for (int qt = 0; qt < n_q && ok; ++qt) {
-      if (!q_tile_sees(p, qt, k0)) continue;
+    QTiles tiles(n_q, head0);
+    while (ok && tiles.next(p, k0, head1)) {
       ++it;
       const uint32_t ph = it & 1u;
-      const int q0 = qt * FB_T;
+      const int q0 = tiles.qt * FB_T;
       const int q_off = p.geom.q_offset_of(q0, p.q_offset);
       const float* stat = reinterpret_cast<const float*>(smem + FbSmem::STAT_OFF + (it & 1) * FB_STATS * 4) + c * 32 + frag_col;
       const bool tile_mask = (p.causal && k0 + FB_T - 1 > q_off + q0) || (k0 + FB_T > p.skv);
@@ -310,16 +348,20 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_full);
     }
-    // dV and dK of this key tile → fp32 accumulators (rows = keys); this warp takes columns 32c..32c+31 of both
+    // dV and dK of this key tile (rows = keys); this warp has columns 32c..32c+31 of both
+    const int row = (warp & 3) * 32 + lane;
     if (n_it > 0) {
       if (ok) ok = mbar_wait(all_done, 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
       __syncwarp();
       tc_fence_after();
-      const int key = k0 + (warp & 3) * 32 + lane;
-      const bool kvalid = ok && key < p.skv;
+    }
+    if (p.heads < p.rep) {
+      // one query head of several: into the fp32 accumulators
+      const int key = k0 + row;
+      const bool kvalid = ok && n_it > 0 && key < p.skv;
       const size_t base = ((static_cast<size_t>(kvalid ? key : 0) * p.b + batch) * (p.hq / p.rep) + g) * FB_T;
 #pragma unroll 1
-      for (int which = 0; which < 2; ++which) {
+      for (int which = 0; which < 2 && n_it > 0; ++which) {
         float* dst = (which == 0 ? p.dv_acc : p.dk_acc) + base + c * 32;
         const float f = which == 0 ? 1.f : p.scale;
         uint32_t v[32];
@@ -332,11 +374,49 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                        __uint_as_float(v[4 * j + 2]) * f, __uint_as_float(v[4 * j + 3]) * f);
         }
       }
+    } else {
+      // bf16 through shared memory (the query buffers, read to the end by now), then whole rows; keys that no
+      // query sees get zeros
+      constexpr int PITCH = FB_T * 2 + 16;
+      static_assert(FbSmem::Q_OFF + 2 * FB_T * PITCH <= FbSmem::DS_OFF, "staging of dV and dK");
+      uint8_t* stg = smem + FbSmem::Q_OFF;
+#pragma unroll 1
+      for (int which = 0; which < 2; ++which) {
+        const float f = which == 0 ? 1.f : p.scale;
+        uint32_t v[32];
+        if (n_it > 0) {
+          tmem_ld_32x32((which == 0 ? t_dv : t_dk) + lane_addr + c * 32, v);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = 0u;
+        }
+        const uint32_t dst = smem_u32(stg) + which * FB_T * PITCH + row * PITCH + c * 64;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          st_shared_v4(dst + j * 16, pack_bf16x2(__uint_as_float(v[8 * j]) * f, __uint_as_float(v[8 * j + 1]) * f),
+                       pack_bf16x2(__uint_as_float(v[8 * j + 2]) * f, __uint_as_float(v[8 * j + 3]) * f),
+                       pack_bf16x2(__uint_as_float(v[8 * j + 4]) * f, __uint_as_float(v[8 * j + 5]) * f),
+                       pack_bf16x2(__uint_as_float(v[8 * j + 6]) * f, __uint_as_float(v[8 * j + 7]) * f));
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(FB_SOFTMAX_WARPS * 32) : "memory");
+      if (ok) {
+        const BwdOut& o = p.out;
+#pragma unroll 1
+        for (int x = warp; x < 2 * FB_T; x += FB_SOFTMAX_WARPS) {
+          const int which = x >> 7, key = k0 + (x & 127);
+          if (key >= p.skv) continue;
+          const uint2 w = *reinterpret_cast<const uint2*>(stg + which * FB_T * PITCH + (x & 127) * PITCH + lane * 8);
+          __nv_bfloat16* dst =
+              which == 0 ? reinterpret_cast<__nv_bfloat16*>(o.dv) + o.dv_rows.at(key) * o.dvs_s + batch * o.dvs_b + g * o.dvs_g
+                         : reinterpret_cast<__nv_bfloat16*>(o.dk) + o.dk_rows.at(key) * o.dks_s + batch * o.dks_b + g * o.dks_g;
+          reinterpret_cast<uint2*>(dst)[lane] = w;
+        }
+      }
     }
   } else if (warp < FB_TMA_WARP) {
     // dQ tile → fp32 reductions into the global accumulator.  The warp's 32 rows go out 32 columns (4 KB) at a time
     // through two buffers: 128-byte rows with their 16-byte units swizzled by row, as the tensor map expects.
-    // The second half of the columns is read before the buffers are free again, so that TMEM is handed back early.
     const int quarter = warp & 3;
     const uint32_t t_mine = t_dq + (static_cast<uint32_t>(quarter * 32) << 16);
     uint8_t* stg = smem + FbSmem::STG_OFF + quarter * 8192;
@@ -347,35 +427,45 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         st_shared_v4(stg_row + buf * 4096 + ((j ^ (lane & 7)) << 4), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     };
     int it = -1;
-    for (int qt = 0; qt < n_q; ++qt) {
-      if (!q_tile_sees(p, qt, k0)) continue;
+    QTiles tiles(n_q, head0);
+    while (tiles.next(p, k0, head1)) {
       ++it;
+      const int qt = tiles.qt, head = tiles.head;
       if (!__all_sync(0xffffffffu, mbar_wait(dq_full, it & 1u, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL))) break;
       tc_fence_after();
       const int row0 = qt * FB_T + quarter * 32;
-      uint32_t v0[32], v1[32];
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        tmem_ld_32x32(t_mine + half * 64, v0);
-        tmem_ld_32x32(t_mine + half * 64 + 32, v1);
-        tmem_ld_wait();
-        if (half == 1) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(dq_empty);
-        }
-        if (lane == 0) tma_store_wait_read<0>();      // the reductions before these have read both buffers
-        __syncwarp();
-        put(0, v0);
-        put(1, v1);
+      auto send = [&](int col) {                      // both buffers: 64 columns from `col` on
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && row0 < p.sq) {               // the tensor map clips rows past sq
-          tma_reduce_add_4d(&tmDQ, stg, half * 64, head, batch, row0);
-          tma_reduce_add_4d(&tmDQ, stg + 4096, half * 64 + 32, head, batch, row0);
+          tma_reduce_add_4d(&tmDQ, stg, col, head, batch, row0);
+          tma_reduce_add_4d(&tmDQ, stg + 4096, col + 32, head, batch, row0);
           tma_store_commit();
         }
-      }
+      };
+      auto buffers_free = [&] {                       // the reductions before this one have read both buffers
+        if (lane == 0) tma_store_wait_read<0>();
+        __syncwarp();
+      };
+      uint32_t v0[32], v1[32];
+      tmem_ld_32x32(t_mine, v0);
+      tmem_ld_32x32(t_mine + 32, v1);
+      tmem_ld_wait();
+      buffers_free();
+      // dPᵀ of the next tile waits for these columns: read all of them before anything is sent
+      put(0, v0);
+      tmem_ld_32x32(t_mine + 64, v0);
+      put(1, v1);
+      tmem_ld_32x32(t_mine + 96, v1);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(dq_empty);
+      send(0);
+      buffers_free();
+      put(0, v0);
+      put(1, v1);
+      send(64);
     }
     if (lane == 0) tma_store_wait<0>();               // nothing in flight out of shared memory at exit
     __syncwarp();
@@ -466,17 +556,30 @@ static int make_qkv_map(CUtensorMap* m, const void* ptr, int d, int inner_heads,
 
 using namespace kb;
 
-// Scratch: `work` (16-byte aligned) must hold the fp32 accumulators of dQ, dK and dV, zeroed here, and the row statistics.
+namespace kb {
+
+// Does a CTA walk all query heads of its KV group?  Rounds of CTAs over the SMs, plus half a round for the uneven end,
+// times the length of a CTA in query tiles, of which three pay for its start and end.
+static bool merge_heads(int sq, int skv, int b, int g, int rep) {
+  if (rep == 1) return true;
+  const double n_q = (sq + FB_T - 1) / FB_T, ctas = (double)((skv + FB_T - 1) / FB_T) * b * g, sms = device_sm_count();
+  return (ctas / sms + 0.5) * (n_q * rep + 3) < (ctas * rep / sms + 0.5) * (n_q + 3);
+}
+static long stats_floats(int sq, int b, int hq) { return (long)b * hq * ((sq + FB_T - 1) / FB_T) * FB_STATS; }
+
+}  // namespace kb
+
+// Scratch: `work` (16-byte aligned) must hold the fp32 accumulators, zeroed here, and the row statistics.
 extern "C" long kb_flash_attn_bwd_scratch_floats(int sq, int skv, int b, int g, int rep, int d) {
-  return (long)sq * b * g * rep * d + 2L * skv * b * g * d + (long)b * g * rep * ((sq + FB_T - 1) / FB_T) * FB_STATS;
+  return (long)sq * b * g * rep * d + stats_floats(sq, b, g * rep) +
+         (merge_heads(sq, skv, b, g, rep) ? 0 : 2L * skv * b * g * d);
+}
+// Kernels and memsets of one backward call.
+extern "C" int kb_flash_attn_bwd_launches(int sq, int skv, int b, int g, int rep) {
+  return merge_heads(sq, skv, b, g, rep) ? 4 : 7;
 }
 
 namespace kb {
-
-struct RowMap {
-  int chunk_rows;                    // 0: rows map to themselves
-  int base[MAX_KV_CHUNKS];
-};
 
 // fp32 accumulator [logical rows, b, g, d] → bf16 rows of a strided destination where logical chunk c
 // starts at destination row map.base[c] (dK/dV straight into the layout a reduce-scatter expects)
@@ -488,11 +591,7 @@ __global__ void attn_convert_chunked_kernel(const float* __restrict__ acc, __nv_
     long rest = i / (FB_T / 4);
     const int gg = static_cast<int>(rest % G); rest /= G;
     const int bb = static_cast<int>(rest % B);
-    long ss = rest / B;
-    if (map.chunk_rows > 0) {
-      const int c = static_cast<int>(ss / map.chunk_rows);
-      ss = map.base[c] + (ss - static_cast<long>(c) * map.chunk_rows);
-    }
+    const long ss = map.at(rest / B);
     const float4 v = reinterpret_cast<const float4*>(acc)[i];
     __nv_bfloat16* o = out + ss * st_s + bb * st_b + gg * st_g + dv * 4;
     uint2 w;
@@ -502,23 +601,18 @@ __global__ void attn_convert_chunked_kernel(const float* __restrict__ acc, __nv_
   }
 }
 
-struct BwdOut {
-  void* dq; long dqs_s, dqs_b, dqs_g, dqs_r;
-  void* dk; long dks_s, dks_b, dks_g;
-  void* dv; long dvs_s, dvs_b, dvs_g;
-  RowMap dk_rows, dv_rows;
-};
-
 static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom& geom, const void* o, const void* dO,
                       const float* lse, const BwdOut& out, float* work, int sq, int skv, int b, int g, int rep, int d,
                       float scale, int causal, int q_offset, int last_key, int* status, cudaStream_t stream) {
   const int hq = g * rep;
   const long n_dq = (long)sq * b * hq * d, n_dkv = (long)skv * b * g * d;
+  const bool merged = merge_heads(sq, skv, b, g, rep);
   float* dq_acc = work;
-  float* dk_acc = dq_acc + n_dq;
-  float* dv_acc = dk_acc + n_dkv;
-  float* stats = dv_acc + n_dkv;
-  cudaError_t e = kb::memset_async(work, 0, sizeof(float) * (n_dq + 2 * n_dkv), stream);
+  float* stats = dq_acc + n_dq;
+  float* dk_acc = merged ? nullptr : stats + stats_floats(sq, b, hq);
+  float* dv_acc = merged ? nullptr : dk_acc + n_dkv;
+  cudaError_t e = kb::memset_async(dq_acc, 0, sizeof(float) * n_dq, stream);
+  if (e == cudaSuccess && !merged) e = kb::memset_async(dk_acc, 0, sizeof(float) * 2 * n_dkv, stream);
   if (e != cudaSuccess) return 1000 + (int)e;
   {
     const int s_pad = (sq + FB_T - 1) / FB_T * FB_T;
@@ -532,7 +626,7 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
   int rc = make_qkv_map(&tmDO, dO, d, 1, hq, b, sq, 0, d, (long)hq * d, (long)b * hq * d, 0);
   if (rc) return rc;
   BwdParams p;
-  p.stats = stats; p.dk_acc = dk_acc; p.dv_acc = dv_acc;
+  p.stats = stats; p.dk_acc = dk_acc; p.dv_acc = dv_acc; p.heads = merged ? rep : 1; p.out = out;
   p.sq = sq; p.skv = skv; p.b = b; p.hq = hq; p.rep = rep; p.q_offset = q_offset; p.causal = causal;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   p.geom = geom;
@@ -552,12 +646,12 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     if (rc) return rc;
   }
   int n_kv = (skv + FB_T - 1) / FB_T;
-  if (causal) {
+  if (causal && !merged) {
     const int lim = (last_key + FB_T - 1) / FB_T;      // keys >= last_key are seen by no query
     if (lim < n_kv) n_kv = lim > 0 ? lim : 0;
   }
   if (n_kv > 0) {
-    dim3 grid(n_kv, hq, b);
+    dim3 grid(n_kv, hq / p.heads, b);
     KB_LAUNCH(flash_attn_bwd_kernel, grid, FB_THREADS, FbSmem::TOTAL, stream, tmQ, kv, tmDO, tmDQ, p);
   }
   {
@@ -566,13 +660,15 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     if (blocks > 148 * 16) blocks = 148 * 16;
     KB_LAUNCH(attn_convert_kernel, (int)blocks, 256, 0, stream, (const float*)dq_acc, (__nv_bfloat16*)out.dq, nvec, b, g, rep,
               out.dqs_s, out.dqs_b, out.dqs_g, out.dqs_r, scale);
-    nvec = n_dkv / 4;
-    blocks = (nvec + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    KB_LAUNCH(attn_convert_chunked_kernel, (int)blocks, 256, 0, stream, (const float*)dk_acc, (__nv_bfloat16*)out.dk, nvec, b,
-              g, out.dks_s, out.dks_b, out.dks_g, out.dk_rows);
-    KB_LAUNCH(attn_convert_chunked_kernel, (int)blocks, 256, 0, stream, (const float*)dv_acc, (__nv_bfloat16*)out.dv, nvec, b,
-              g, out.dvs_s, out.dvs_b, out.dvs_g, out.dv_rows);
+    if (!merged) {
+      nvec = n_dkv / 4;
+      blocks = (nvec + 255) / 256;
+      if (blocks > 148 * 16) blocks = 148 * 16;
+      KB_LAUNCH(attn_convert_chunked_kernel, (int)blocks, 256, 0, stream, (const float*)dk_acc, (__nv_bfloat16*)out.dk, nvec,
+                b, g, out.dks_s, out.dks_b, out.dks_g, out.dk_rows);
+      KB_LAUNCH(attn_convert_chunked_kernel, (int)blocks, 256, 0, stream, (const float*)dv_acc, (__nv_bfloat16*)out.dv, nvec,
+                b, g, out.dvs_s, out.dvs_b, out.dvs_g, out.dv_rows);
+    }
   }
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + (int)e;

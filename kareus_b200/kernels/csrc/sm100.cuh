@@ -80,20 +80,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait.  `abort_flag` lives in shared memory and is shared by all roles of the CTA.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
+  // the timer is read only now and then: a read takes longer than most waits
+  uint64_t t0 = 0;
   uint32_t spins = 0;
-  while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
+  while (!mbar_try_wait(bar, parity)) {
     if ((++spins & 63u) == 0u) {
       if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > KB_WAIT_NS) {
+      const uint64_t t = globaltimer_ns();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > KB_WAIT_NS) {
         *abort_flag = 1;
         if (status) atomicCAS(status, 0, code);
         return false;
       }
     }
   }
+  return true;
 }
 
 // ----------------------------------------------------------------------------- fences

@@ -404,14 +404,14 @@ def test_layernorm_and_bias_kernels():
 
 
 @pytest.mark.parametrize("cp,c", [(2, 128), (2, 256), (4, 128)])
-def test_chunked_attention_matches_reference(cp, c):
+def test_chunked_attention_matches_reference(cp, c, b=2):
     """Context-parallel attention in one launch: K/V chunks in several buffers (here: local tensors that
     stand for the ranks' shards), two query chunks with their own positions, dK/dV scattered per chunk
     into a rank-ordered buffer.  Every rank's view is checked against the fp32 statement of the math."""
     from kareus_b200.kernels import attention_bwd_native, attention_native, ref
     from kareus_b200.parallel.ring_attention import chunk_owner, chunk_table
     KC = _K()
-    b, g, rep, d = 2, 2, 3, 128
+    g, rep, d = 2, 3, 128
     gen = torch.Generator(device="cuda").manual_seed(11 * cp + c)
     packed = [torch.randn(2 * c, b, g, (rep + 2) * d, device="cuda", generator=gen).bfloat16() for _ in range(cp)]
     qs = [p[..., : rep * d].unflatten(-1, (rep, d)) for p in packed]
@@ -444,6 +444,13 @@ def test_chunked_attention_matches_reference(cp, c):
                 wv[j * c:(j + 1) * c].abs().max() == 0, ("dv", rank, j)
             if wk[j * c:(j + 1) * c].abs().max() == 0:      # chunk no local query can see: exact zeros
                 assert dkv[dk_base[j]:dk_base[j] + c].abs().max() == 0
+
+
+# enough (batch, group) pairs that the backward gives all query heads of a group to one CTA, which writes dK/dV itself
+def test_attention_backward_merged_heads():
+    test_chunked_attention_matches_reference(2, 128, b=10)
+    test_flash_attention_backward(640, 8, 4, 3)
+    test_flash_attention_backward(300, 20, 3, 1)
 
 
 @pytest.mark.parametrize("M,N,K", [(256, 384, 512), (1000, 328, 200), (4096, 4096, 2048)])
