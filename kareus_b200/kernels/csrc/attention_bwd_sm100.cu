@@ -43,7 +43,10 @@ constexpr int FB_CHUNK = 16384;
 constexpr int FB_SOFTMAX_WARPS = 16;             // 4 TMEM lane quarters x 4 chunks of 32 query columns
 constexpr int FB_DQ_WARP = FB_SOFTMAX_WARPS;     // first of the four dQ warps
 constexpr int FB_TMA_WARP = FB_DQ_WARP + 4, FB_MMA_WARP = FB_DQ_WARP + 5;
-constexpr int FB_THREADS = (FB_SOFTMAX_WARPS + 6) * 32;
+constexpr int FB_THREADS = (FB_SOFTMAX_WARPS + 8) * 32;   // six warpgroups; the last two warps only fill theirs
+// Registers a thread: what the block is launched with, and after the dQ warps have taken some from the last warpgroup
+constexpr int FB_REGS = 80, FB_REGS_DQ = 120, FB_REGS_AUX = 40;
+static_assert(FB_REGS_DQ + FB_REGS_AUX <= 2 * FB_REGS, "the shares must not exceed the registers at launch");
 constexpr int FB_STATS = 2 * FB_T;               // floats of row statistics per query tile: −lse·log2(e), then −δ
 
 // Destinations, strides in elements.
@@ -84,15 +87,27 @@ __device__ __forceinline__ bool q_tile_sees(const BwdParams& p, int qt, int k0) 
 
 // The query tiles of heads head0, head0 + 1, ... that see a key tile, in order.
 struct QTiles {
-  int n_q, qt, head;
-  __device__ __forceinline__ QTiles(int n, int head0) : n_q(n), qt(-1), head(head0) {}
+  int n_q, first, qt, head;
+  // first query tile worth looking at: exact for one query chunk, where visible tiles are a suffix
+  static __device__ __forceinline__ int first_tile(const BwdParams& p, int n_q, int k0) {
+    return p.causal && p.geom.q_chunk_rows == 0 ? min(n_q, max(0, k0 - p.q_offset) / FB_T) : 0;
+  }
+  static __device__ __forceinline__ int count(const BwdParams& p, int n_q, int k0) {
+    const int f = first_tile(p, n_q, k0);
+    if (!p.causal || p.geom.q_chunk_rows == 0) return n_q - f;
+    int n = 0;
+    for (int qt = f; qt < n_q; ++qt) n += q_tile_sees(p, qt, k0) ? 1 : 0;
+    return n;
+  }
+  __device__ __forceinline__ QTiles(const BwdParams& p, int n, int k0, int head0)
+      : n_q(n), first(first_tile(p, n, k0)), qt(first - 1), head(head0) {}
   __device__ __forceinline__ bool next(const BwdParams& p, int k0, int head1) {
     for (;;) {
-      if (++qt == n_q) {
-        qt = 0;
-        if (++head >= head1) return false;
+      if (++qt >= n_q) {
+        qt = first;
+        if (++head >= head1 || first >= n_q) return false;
       }
-      if (q_tile_sees(p, qt, k0)) return true;
+      if (p.geom.q_chunk_rows == 0 || q_tile_sees(p, qt, k0)) return true;
     }
   }
 };
@@ -143,14 +158,15 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt = blockIdx.x;                 // key tile; tile 0 is seen by the most queries → first
-  const int head0 = blockIdx.y * p.heads, head1 = head0 + p.heads, batch = blockIdx.z;
+  // key tile 0 is seen by the most queries: its CTAs go first, over all heads and batches, so that the short ones fill
+  // the end.  The CTAs of neighbouring key tiles of a head walk the same queries at the same time, which keeps L2 useful.
+  const int kt = blockIdx.y;
+  const int units = p.hq / p.heads, batch = blockIdx.x / units;
+  const int head0 = (blockIdx.x - batch * units) * p.heads, head1 = head0 + p.heads;
   const int g = head0 / p.rep;
   const int k0 = kt * FB_T;
   const int n_q = (p.sq + FB_T - 1) / FB_T;
-  int n_it = 0;                              // query tiles that see this key tile, over all heads
-  for (int qt = 0; qt < n_q; ++qt) n_it += q_tile_sees(p, qt, k0) ? 1 : 0;
-  n_it *= p.heads;
+  const int n_it = QTiles::count(p, n_q, k0) * p.heads;   // query tiles that see this key tile, over all heads
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 15; ++i)
@@ -168,111 +184,115 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const uint32_t t_s = tmem_base, t_dp = tmem_base + 128, t_dv = tmem_base + 256, t_dk = tmem_base + 384;
   const uint32_t t_dq = t_dp;
 
-  if (warp == FB_TMA_WARP) {
-    if (n_it > 0 && elect_one()) {
-      int src, srow;
-      p.geom.locate(k0, src, srow);
-      prefetch_tmap(&tmQ); prefetch_tmap(&kv.k[src]); prefetch_tmap(&kv.v[src]); prefetch_tmap(&tmDO);
-      const float* stats = p.stats + static_cast<size_t>(batch) * p.hq * n_q * FB_STATS;
-      mbar_expect_tx(kv_full, 2 * FB_TILE);
-      tma_load_4d(smem + FbSmem::K_OFF, &kv.k[src], kv_full, 0, g, batch, srow);
-      tma_load_4d(smem + FbSmem::K_OFF + FB_CHUNK, &kv.k[src], kv_full, 64, g, batch, srow);
-      tma_load_4d(smem + FbSmem::V_OFF, &kv.v[src], kv_full, 0, g, batch, srow);
-      tma_load_4d(smem + FbSmem::V_OFF + FB_CHUNK, &kv.v[src], kv_full, 64, g, batch, srow);
-      // per visible tile: Q(it) into buffer it & 1 (released by dK of tile it-2), then dO(it) (released by dV of
-      // tile it-1): Q(it+1) goes out right behind dO(it), one tile ahead of the MMAs
-      int it = 0;
-      QTiles tiles(n_q, head0);
-      while (tiles.next(p, k0, head1)) {
-        const int qt = tiles.qt, head = tiles.head, r = head - g * p.rep;
-        const int qb = it & 1;
-        const int q0 = qt * FB_T;
-        if (!mbar_wait(&q_empty[qb], ((it >> 1) & 1u) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
-        uint8_t* qdst = smem + FbSmem::Q_OFF + qb * FB_TILE;
-        mbar_expect_tx(&q_full[qb], FB_TILE + FB_STATS * 4);
-        tma_load_5d(qdst, &tmQ, &q_full[qb], 0, r, g, batch, q0);
-        tma_load_5d(qdst + FB_CHUNK, &tmQ, &q_full[qb], 64, r, g, batch, q0);
-        bulk_load(smem + FbSmem::STAT_OFF + qb * FB_STATS * 4, stats + (static_cast<size_t>(head) * n_q + qt) * FB_STATS,
-                  FB_STATS * 4, &q_full[qb]);
-        if (!mbar_wait(do_empty, (it & 1u) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
-        mbar_expect_tx(do_full, FB_TILE);
-        tma_load_4d(smem + FbSmem::DO_OFF, &tmDO, do_full, 0, head, batch, q0);
-        tma_load_4d(smem + FbSmem::DO_OFF + FB_CHUNK, &tmDO, do_full, 64, head, batch, q0);
-        ++it;
-      }
-      if (*abort_flag) {
-        const uint64_t t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 200000ull) {}
-      }
-    }
-    __syncwarp();
-  } else if (warp == FB_MMA_WARP) {
-    if (n_it > 0 && elect_one()) {           // one thread runs the whole role, see elect_one()
-      constexpr uint32_t id_kk = make_idesc_bf16(FB_T, FB_T, false, false);   // A K-major, B K-major
-      constexpr uint32_t id_mm = make_idesc_bf16(FB_T, FB_T, true, true);     // A MN-major, B MN-major
-      constexpr uint32_t id_km = make_idesc_bf16(FB_T, FB_T, false, true);    // A K-major (or TMEM), B MN-major
-      const uint32_t base = smem_u32(smem);
-      // descriptors of an operand for 16-deep step k: K-major rows, or MN-major with 64-wide chunks
-      auto kmaj = [&](int off, int k) {
-        return make_smem_desc(base + off, 16, 1024) + static_cast<uint64_t>(((k >> 2) * FB_CHUNK + (k & 3) * 32) >> 4);
-      };
-      auto mnmaj = [&](int off, int k) {
-        return make_smem_desc(base + off, FB_CHUNK, 1024) + static_cast<uint64_t>((k * 2048) >> 4);
-      };
-      bool ok = true;
-      auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
-        ok = mbar_wait(bar, parity, abort_flag, p.status, code);
-        if (ok) tc_fence_after();
-        return ok;
-      };
-      auto issue_s = [&](int i) {
-        const int q = FbSmem::Q_OFF + (i & 1) * FB_TILE;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) umma_ss(t_s, kmaj(FbSmem::K_OFF, k), kmaj(q, k), id_kk, k > 0);
-        umma_commit(s_full);
-      };
-      if (wait(kv_full, 0, ST_TIMEOUT_FULL) && wait(&q_full[0], 0, ST_TIMEOUT_FULL)) issue_s(0);
-      for (int it = 0; it < n_it && ok; ++it) {
-        const uint32_t ph = it & 1u;
-        const int q = FbSmem::Q_OFF + (it & 1) * FB_TILE;
-        // dPᵀ(it) overwrites the columns that held dQ(it-1)
-        if (!wait(do_full, ph, ST_TIMEOUT_FULL) || !wait(dq_empty, ph ^ 1u, ST_TIMEOUT_TMEM_EMPTY)) break;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) umma_ss(t_dp, kmaj(FbSmem::V_OFF, k), kmaj(FbSmem::DO_OFF, k), id_kk, k > 0);
-        umma_commit(dp_full);
-        if (!wait(p_full, ph, ST_TIMEOUT_TMEM_FULL)) break;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)          // 16 queries: 8 columns of Pᵀ, 16 rows of dO
-          umma_ts(t_dv, t_s + (k >> 1) * 32 + (k & 1) * 8, mnmaj(FbSmem::DO_OFF, k), id_km, (it > 0 || k > 0));
-        umma_commit(do_empty);
-        if (it + 1 < n_it) {
-          // overwrites Pᵀ(it): the product before it reads it in order
-          if (!wait(&q_full[(it + 1) & 1], ((it + 1) >> 1) & 1u, ST_TIMEOUT_FULL)) break;
-          issue_s(it + 1);
+  if (warp >= FB_TMA_WARP) {
+    regs_dec<FB_REGS_AUX>();
+    if (warp == FB_TMA_WARP) {
+      if (n_it > 0 && elect_one()) {
+        int src, srow;
+        p.geom.locate(k0, src, srow);
+        prefetch_tmap(&tmQ); prefetch_tmap(&kv.k[src]); prefetch_tmap(&kv.v[src]); prefetch_tmap(&tmDO);
+        const float* stats = p.stats + static_cast<size_t>(batch) * p.hq * n_q * FB_STATS;
+        mbar_expect_tx(kv_full, 2 * FB_TILE);
+        tma_load_4d(smem + FbSmem::K_OFF, &kv.k[src], kv_full, 0, g, batch, srow);
+        tma_load_4d(smem + FbSmem::K_OFF + FB_CHUNK, &kv.k[src], kv_full, 64, g, batch, srow);
+        tma_load_4d(smem + FbSmem::V_OFF, &kv.v[src], kv_full, 0, g, batch, srow);
+        tma_load_4d(smem + FbSmem::V_OFF + FB_CHUNK, &kv.v[src], kv_full, 64, g, batch, srow);
+        // per visible tile: Q(it) into buffer it & 1 (released by dK of tile it-2), then dO(it) (released by dV of
+        // tile it-1): Q(it+1) goes out right behind dO(it), one tile ahead of the MMAs
+        int it = 0;
+        QTiles tiles(p, n_q, k0, head0);
+        while (tiles.next(p, k0, head1)) {
+          const int qt = tiles.qt, head = tiles.head, r = head - g * p.rep;
+          const int qb = it & 1;
+          const int q0 = qt * FB_T;
+          if (!mbar_wait(&q_empty[qb], ((it >> 1) & 1u) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+          uint8_t* qdst = smem + FbSmem::Q_OFF + qb * FB_TILE;
+          mbar_expect_tx(&q_full[qb], FB_TILE + FB_STATS * 4);
+          tma_load_5d(qdst, &tmQ, &q_full[qb], 0, r, g, batch, q0);
+          tma_load_5d(qdst + FB_CHUNK, &tmQ, &q_full[qb], 64, r, g, batch, q0);
+          bulk_load(smem + FbSmem::STAT_OFF + qb * FB_STATS * 4, stats + (static_cast<size_t>(head) * n_q + qt) * FB_STATS,
+                    FB_STATS * 4, &q_full[qb]);
+          if (!mbar_wait(do_empty, (it & 1u) ^ 1u, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+          mbar_expect_tx(do_full, FB_TILE);
+          tma_load_4d(smem + FbSmem::DO_OFF, &tmDO, do_full, 0, head, batch, q0);
+          tma_load_4d(smem + FbSmem::DO_OFF + FB_CHUNK, &tmDO, do_full, 64, head, batch, q0);
+          ++it;
         }
-        if (!wait(ds_full, ph, ST_TIMEOUT_TMEM_FULL)) break;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) umma_ss(t_dq, mnmaj(FbSmem::DS_OFF, k), mnmaj(FbSmem::K_OFF, k), id_mm, k > 0);
-        umma_commit(dq_full);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) umma_ss(t_dk, kmaj(FbSmem::DS_OFF, k), mnmaj(q, k), id_km, (it > 0 || k > 0));
-        umma_commit(&q_empty[it & 1]);
-        umma_commit(ds_empty);
+        if (*abort_flag) {
+          const uint64_t t0 = globaltimer_ns();
+          while (globaltimer_ns() - t0 < 200000ull) {}
+        }
       }
-      if (ok) umma_commit(all_done);
+      __syncwarp();
+    } else if (warp == FB_MMA_WARP) {
+      if (n_it > 0 && elect_one()) {           // one thread runs the whole role, see elect_one()
+        constexpr uint32_t id_kk = make_idesc_bf16(FB_T, FB_T, false, false);   // A K-major, B K-major
+        constexpr uint32_t id_mm = make_idesc_bf16(FB_T, FB_T, true, true);     // A MN-major, B MN-major
+        constexpr uint32_t id_km = make_idesc_bf16(FB_T, FB_T, false, true);    // A K-major (or TMEM), B MN-major
+          // Descriptors of an operand for 16-deep step k: K-major rows, or MN-major with 64-wide chunks.  Only the low
+        // word depends on the address; `lo` is made opaque once per tile, or the compiler would keep all 40 of them
+        // in registers.
+        uint32_t lo = (smem_u32(smem) & 0x3FFFFu) >> 4;
+        constexpr uint64_t DESC_HI = make_smem_desc(0, 0, 1024);
+        auto desc = [&](uint32_t lbo, int off) { return DESC_HI | (lo + ((lbo >> 4) << 16) + static_cast<uint32_t>(off >> 4)); };
+        auto kmaj = [&](int off, int k) { return desc(16, off + (k >> 2) * FB_CHUNK + (k & 3) * 32); };
+        auto mnmaj = [&](int off, int k) { return desc(FB_CHUNK, off + k * 2048); };
+        bool ok = true;
+        auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+          ok = mbar_wait(bar, parity, abort_flag, p.status, code);
+          if (ok) tc_fence_after();
+          return ok;
+        };
+        auto issue_s = [&](int i) {
+          const int q = FbSmem::Q_OFF + (i & 1) * FB_TILE;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) umma_ss(t_s, kmaj(FbSmem::K_OFF, k), kmaj(q, k), id_kk, k > 0);
+          umma_commit(s_full);
+        };
+        if (wait(kv_full, 0, ST_TIMEOUT_FULL) && wait(&q_full[0], 0, ST_TIMEOUT_FULL)) issue_s(0);
+        for (int it = 0; it < n_it && ok; ++it) {
+          const uint32_t ph = it & 1u;
+          const int q = FbSmem::Q_OFF + (it & 1) * FB_TILE;
+          asm volatile("" : "+r"(lo));
+          // dPᵀ(it) overwrites the columns that held dQ(it-1)
+          if (!wait(do_full, ph, ST_TIMEOUT_FULL) || !wait(dq_empty, ph ^ 1u, ST_TIMEOUT_TMEM_EMPTY)) break;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) umma_ss(t_dp, kmaj(FbSmem::V_OFF, k), kmaj(FbSmem::DO_OFF, k), id_kk, k > 0);
+          umma_commit(dp_full);
+          if (!wait(p_full, ph, ST_TIMEOUT_TMEM_FULL)) break;
+#pragma unroll
+          for (int k = 0; k < 8; ++k)          // 16 queries: 8 columns of Pᵀ, 16 rows of dO
+            umma_ts(t_dv, t_s + (k >> 1) * 32 + (k & 1) * 8, mnmaj(FbSmem::DO_OFF, k), id_km, (it > 0 || k > 0));
+          umma_commit(do_empty);
+          if (it + 1 < n_it) {
+            // overwrites Pᵀ(it): the product before it reads it in order
+            if (!wait(&q_full[(it + 1) & 1], ((it + 1) >> 1) & 1u, ST_TIMEOUT_FULL)) break;
+            issue_s(it + 1);
+          }
+          if (!wait(ds_full, ph, ST_TIMEOUT_TMEM_FULL)) break;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) umma_ss(t_dq, mnmaj(FbSmem::DS_OFF, k), mnmaj(FbSmem::K_OFF, k), id_mm, k > 0);
+          umma_commit(dq_full);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) umma_ss(t_dk, kmaj(FbSmem::DS_OFF, k), mnmaj(q, k), id_km, (it > 0 || k > 0));
+          umma_commit(&q_empty[it & 1]);
+          umma_commit(ds_empty);
+        }
+        if (ok) umma_commit(all_done);
+      }
+      __syncwarp();
     }
-    __syncwarp();
   } else if (warp < FB_SOFTMAX_WARPS) {
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int c = warp >> 2;                       // chunk of 32 query columns
     // this thread's fragment: key rows frag_row + 8 x (0..3), query columns frag_col + 8 n + (0, 1) of the chunk
     const int frag_row = (warp & 3) * 32 + (lane >> 2), frag_col = 2 * (lane & 3);
-    // its rows of dSᵀ (two 64-wide swizzled chunks per row; frag_row & 7 is the row inside the swizzle atom)
-    const uint32_t ds_base = smem_u32(smem) + FbSmem::DS_OFF + (c >> 1) * FB_CHUNK + frag_row * 128 + (lane & 3) * 4;
+    // the row of dSᵀ whose address this thread gives to the matrix stores (two 64-wide swizzled chunks per row)
+    const uint32_t ds_row = smem_u32(smem) + FbSmem::DS_OFF + (c >> 1) * FB_CHUNK + ((warp & 3) * 32 + lane) * 128;
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
     bool ok = true;
     int it = -1;
-    QTiles tiles(n_q, head0);
+    QTiles tiles(p, n_q, k0, head0);
     while (ok && tiles.next(p, k0, head1)) {
       ++it;
       const uint32_t ph = it & 1u;
@@ -334,14 +354,15 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
         const float2 nd = *reinterpret_cast<const float2*>(stat + FB_T + 8 * n);
-        const uint32_t unit = ds_base + ((((c & 1) * 4 + n) ^ (frag_row & 7)) << 4);
+        uint32_t w[4];
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
           const float2 e = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[h >> 1][2 * n + (h & 1)]));
           const float2 d = __fmul2_rn(e, __fadd2_rn(make_float2(__uint_as_float(dv[h >> 1][4 * n + 2 * (h & 1)]),
                                                                 __uint_as_float(dv[h >> 1][4 * n + 2 * (h & 1) + 1])), nd));
-          st_shared_u32(unit + h * 1024, pack_bf16x2(d.x, d.y));
+          w[h] = pack_bf16x2(d.x, d.y);
         }
+        stmatrix_x4(ds_row + ((((c & 1) * 4 + n) ^ (lane & 7)) << 4), w);
       }
       tc_fence_before();
       fence_proxy_async_smem();
@@ -403,20 +424,23 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (ok) {
         const BwdOut& o = p.out;
 #pragma unroll 1
-        for (int x = warp; x < 2 * FB_T; x += FB_SOFTMAX_WARPS) {
-          const int which = x >> 7, key = k0 + (x & 127);
-          if (key >= p.skv) continue;
-          const uint2 w = *reinterpret_cast<const uint2*>(stg + which * FB_T * PITCH + (x & 127) * PITCH + lane * 8);
-          __nv_bfloat16* dst =
-              which == 0 ? reinterpret_cast<__nv_bfloat16*>(o.dv) + o.dv_rows.at(key) * o.dvs_s + batch * o.dvs_b + g * o.dvs_g
-                         : reinterpret_cast<__nv_bfloat16*>(o.dk) + o.dk_rows.at(key) * o.dks_s + batch * o.dks_b + g * o.dks_g;
-          reinterpret_cast<uint2*>(dst)[lane] = w;
+        for (int which = 0; which < 2; ++which) {
+          const long st_s = which == 0 ? o.dvs_s : o.dks_s;
+          __nv_bfloat16* dst = which == 0 ? reinterpret_cast<__nv_bfloat16*>(o.dv) + batch * o.dvs_b + g * o.dvs_g
+                                          : reinterpret_cast<__nv_bfloat16*>(o.dk) + batch * o.dks_b + g * o.dks_g;
+          // a key tile never crosses a chunk of the row map
+          dst += (which == 0 ? o.dv_rows.at(k0) : o.dk_rows.at(k0)) * st_s + lane * 4;
+          const uint8_t* src = stg + which * FB_T * PITCH + lane * 8;
+#pragma unroll
+          for (int x = warp; x < FB_T; x += FB_SOFTMAX_WARPS)
+            if (k0 + x < p.skv) *reinterpret_cast<uint2*>(dst + x * st_s) = *reinterpret_cast<const uint2*>(src + x * PITCH);
         }
       }
     }
-  } else if (warp < FB_TMA_WARP) {
+  } else {
     // dQ tile → fp32 reductions into the global accumulator.  The warp's 32 rows go out 32 columns (4 KB) at a time
     // through two buffers: 128-byte rows with their 16-byte units swizzled by row, as the tensor map expects.
+    regs_inc<FB_REGS_DQ>();
     const int quarter = warp & 3;
     const uint32_t t_mine = t_dq + (static_cast<uint32_t>(quarter * 32) << 16);
     uint8_t* stg = smem + FbSmem::STG_OFF + quarter * 8192;
@@ -427,7 +451,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         st_shared_v4(stg_row + buf * 4096 + ((j ^ (lane & 7)) << 4), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     };
     int it = -1;
-    QTiles tiles(n_q, head0);
+    QTiles tiles(p, n_q, k0, head0);
     while (tiles.next(p, k0, head1)) {
       ++it;
       const int qt = tiles.qt, head = tiles.head;
@@ -447,24 +471,24 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (lane == 0) tma_store_wait_read<0>();
         __syncwarp();
       };
-      uint32_t v0[32], v1[32];
+      uint32_t v0[32], v1[32], v2[32];
       tmem_ld_32x32(t_mine, v0);
       tmem_ld_32x32(t_mine + 32, v1);
+      tmem_ld_32x32(t_mine + 64, v2);
       tmem_ld_wait();
       buffers_free();
       // dPᵀ of the next tile waits for these columns: read all of them before anything is sent
       put(0, v0);
-      tmem_ld_32x32(t_mine + 64, v0);
-      put(1, v1);
-      tmem_ld_32x32(t_mine + 96, v1);
+      tmem_ld_32x32(t_mine + 96, v0);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(dq_empty);
+      put(1, v1);
       send(0);
       buffers_free();
-      put(0, v0);
-      put(1, v1);
+      put(0, v2);
+      put(1, v0);
       send(64);
     }
     if (lane == 0) tma_store_wait<0>();               // nothing in flight out of shared memory at exit
@@ -634,6 +658,10 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
   if (!configured) {
     e = cudaFuncSetAttribute(flash_attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FbSmem::TOTAL);
     if (e != cudaSuccess) return 1000 + (int)e;
+    cudaFuncAttributes attr;
+    e = cudaFuncGetAttributes(&attr, flash_attn_bwd_kernel);
+    if (e != cudaSuccess) return 1000 + (int)e;
+    if (attr.numRegs < FB_REGS) return ST_BAD_ARG;   // the register split would wait forever
     configured = true;
   }
   CUtensorMap tmDQ;
@@ -651,7 +679,7 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     if (lim < n_kv) n_kv = lim > 0 ? lim : 0;
   }
   if (n_kv > 0) {
-    dim3 grid(n_kv, hq / p.heads, b);
+    dim3 grid(hq / p.heads * b, n_kv);
     KB_LAUNCH(flash_attn_bwd_kernel, grid, FB_THREADS, FbSmem::TOTAL, stream, tmQ, kv, tmDO, tmDQ, p);
   }
   {

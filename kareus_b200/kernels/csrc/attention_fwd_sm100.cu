@@ -199,7 +199,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           const uint64_t qd = qd0 + static_cast<uint64_t>(t * (FA_TILE_BYTES >> 4));
           const uint64_t kd = kd0 + static_cast<uint64_t>(ks * (FA_TILE_BYTES >> 4));
           const uint32_t d = tmem_base + t * 128;
-  #pragma unroll
+#pragma unroll
           for (int k = 0; k < FA_D / 16; ++k) {
             const uint64_t off = ((k >> 2) * FA_CHUNK + (k & 3) * 32) >> 4;
             umma_ss(d, qd + off, kd + off, idesc_s, k > 0 ? 1u : 0u);
@@ -209,7 +209,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         int ks = 0;                                // stage of K(j) / K(j+1), its phase
         uint32_t kph = 0;
         if (wait(&full[0], 0, ST_TIMEOUT_FULL)) {
-  #pragma unroll
+#pragma unroll
           for (int t = 0; t < 2; ++t)
             if ((t ? n1 : n0) > 0 && wait(&q_full[t], 0, ST_TIMEOUT_FULL)) {
               tc_fence_after();
@@ -226,19 +226,19 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           if (ks == FA_STAGES) { ks = 0; kph ^= 1u; }
           if (!wait(&full[vs], vph, ST_TIMEOUT_FULL)) break;
           const uint64_t vd = vd0 + static_cast<uint64_t>(vs * (FA_TILE_BYTES >> 4));
-  #pragma unroll
+#pragma unroll
           for (int t = 0; t < 2; ++t) {
             const int nt = t ? n1 : n0;
             if (j >= nt || !ok) continue;
             const uint32_t d = tmem_base + 256 + t * 128, a = tmem_base + t * 128;
             if (!wait(&p_most[t], j & 1u, ST_TIMEOUT_TMEM_FULL)) continue;
             tc_fence_after();
-  #pragma unroll
+#pragma unroll
             for (int k = 0; k < 6; ++k)            // 16 keys: 8 columns of P, 16 rows of V
               umma_ts(d, a + k * 8, vd + k * (2048 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
             if (!wait(&p_rest[t], j & 1u, ST_TIMEOUT_TMEM_FULL)) continue;
             tc_fence_after();
-  #pragma unroll
+#pragma unroll
             for (int k = 6; k < 8; ++k) umma_ts(d, a + k * 8, vd + k * (2048 >> 4), idesc_o, 1u);
             if (j + 1 < nt) {
               if (!wait(&full[ks], kph, ST_TIMEOUT_FULL)) continue;
