@@ -66,6 +66,19 @@ def rmsnorm_bwd(dy, x, rstd, w, dw_accum=None):
     return dx, dw
 
 
+def rmsnorm_fwd_heads(x, w, eps):
+    """RMSNorm over the last dimension of a ``[..., H]`` view; returns ``(y contiguous, rstd [rows])``."""
+    if is_cuda(x):
+        return _cuda().rmsnorm_fwd_heads(x, w, eps)
+    y, rstd = ref.rmsnorm_fwd(x.reshape(-1, x.shape[-1]), w, eps)
+    return y.view(x.shape), rstd
+
+
+def scale(x, s):
+    """``x * s.to(x.dtype)`` for a scalar tensor ``s``."""
+    return _cuda().scale(x, s) if is_cuda(x) else x * s.to(x.dtype)
+
+
 # ----------------------------------------------------------------------------- rope
 def rope_inplace(q, k, freqs, inverse=False):
     """Rotate ``q`` and ``k`` (views are fine) in place."""

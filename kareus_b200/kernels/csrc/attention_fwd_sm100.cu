@@ -102,11 +102,10 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  // heavy (late) query tiles first
+  // late query tiles see the most keys: they go first, over all heads and batches, so that the short ones fill the end
   const int n_qtiles = (p.sq + FA_BM - 1) / FA_BM;
-  const int qt0 = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) * p.tiles_per_cta;
-  const int head = blockIdx.y;
-  const int batch = blockIdx.z;
+  const int qt0 = (static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y)) * p.tiles_per_cta;
+  const int batch = blockIdx.x / p.hq, head = blockIdx.x - batch * p.hq;
   const int g = head / p.rep, r = head % p.rep;
   // query tile t of this CTA: first row, its absolute position minus the row, visible key tiles
   auto tile_q0 = [&](int t) { return (qt0 + t) * FA_BM; };
@@ -456,7 +455,7 @@ static int launch_fwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     if (attr.numRegs * FA_THREADS < FA_REGS_TOTAL) return ST_BAD_ARG;   // the register split would wait forever
     configured = true;
   }
-  dim3 grid((n_q + p.tiles_per_cta - 1) / p.tiles_per_cta, g * rep, b);
+  dim3 grid(g * rep * b, (n_q + p.tiles_per_cta - 1) / p.tiles_per_cta);
   KB_LAUNCH(flash_attn_fwd_kernel, grid, FA_THREADS, FaSmem::TOTAL, stream, tmQ, kv, tmO, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + (int)e;

@@ -167,7 +167,78 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   }
 }
 
-// Narrow rows (per-head q/k norm, H <= 256): one warp per row.
+// Many rows of up to 256 VPL elements: one warp per row, VPL 16-byte vectors a lane, all requested before the first
+// is used and no barrier between rows.  Bound by memory: 16384 x 3072 takes 48 us in a power-limited training step (62
+// with a CTA per row and its barrier).
+template <int VPL>
+__global__ void __launch_bounds__(256)
+rmsnorm_fwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                        __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int rows, int H, float eps) {
+  const int lane = threadIdx.x & 31, nvec = H >> 3;
+  const uint4* wr = reinterpret_cast<const uint4*>(w);
+  for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += gridDim.x * 8) {
+    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * H);
+    uint4 xv[VPL];
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) xv[i] = lane + 32 * i < nvec ? __ldcs(xr + lane + 32 * i) : make_uint4(0, 0, 0, 0);
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      float f[8];
+      unpack8(xv[i], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    }
+    const float r = rsqrtf(warp_sum(ss) / static_cast<float>(H) + eps);
+    if (lane == 0) rstd[row] = r;
+    uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * H);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      if (lane + 32 * i >= nvec) continue;
+      float f[8], g[8];
+      unpack8(xv[i], f);
+      unpack8(wr[lane + 32 * i], g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * r * g[j];
+      yr[lane + 32 * i] = pack8(f);
+    }
+  }
+}
+
+// Head vectors (per-head q/k norm): H / 8 lanes per row (a power of two up to 32), 16 bytes a lane.  Row n is
+// x + (n / inner) * st_outer + (n % inner) * st_inner, so that q and k are read where the QKV projection left them;
+// y is contiguous.  Rows are 16-byte aligned.
+__global__ void __launch_bounds__(256)
+rmsnorm_fwd_heads_kernel(const __nv_bfloat16* __restrict__ x, unsigned inner, long st_outer, long st_inner,
+                         const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, float* __restrict__ rstd,
+                         unsigned rows, int H, float eps) {
+  const unsigned lanes = H >> 3, per_warp = 32 / lanes, lane = threadIdx.x & 31;
+  const unsigned sub = lane / lanes, l = lane - sub * lanes;
+  const unsigned step = gridDim.x * 8 * per_warp;
+  float g[8];
+  unpack8(reinterpret_cast<const uint4*>(w)[l], g);
+#pragma unroll 2
+  for (unsigned r0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * per_warp; r0 < rows; r0 += step) {
+    const unsigned row = r0 + sub;
+    const bool valid = row < rows;
+    const unsigned o = row / inner;
+    float f[8];
+    unpack8(valid ? reinterpret_cast<const uint4*>(x + o * st_outer + (row - o * inner) * st_inner)[l] : make_uint4(0, 0, 0, 0),
+            f);
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    for (unsigned d = lanes >> 1; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+    const float r = rsqrtf(ss / static_cast<float>(H) + eps);
+    if (!valid) continue;
+    if (l == 0) rstd[row] = r;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = f[j] * r * g[j];
+    reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * H)[l] = pack8(f);
+  }
+}
+
+// Narrow rows that the kernel above does not take: one warp per row.
 __global__ void rmsnorm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                         __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int rows, int H,
                                         float eps) {
@@ -281,14 +352,24 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   }
 }
 
-// `accumulate`: add the column sums to dw (the fp32 main gradient of the weight) instead of storing them.
-__global__ void rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int nparts,
-                                         int H, int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= H) return;
+// Column sums of the partial rows.  32 columns per CTA, a column of threads for each of 32 interleaved sets of rows:
+// a thread per column walked all (up to 1200) rows alone and took 31 us for 2048 columns, this takes 5.
+// `accumulate`: add the sums to dw (the fp32 main gradient of the weight) instead of storing them.
+__global__ void __launch_bounds__(1024)
+rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int nparts, int H, int accumulate) {
+  __shared__ float sum[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + tx;
   float s = 0.f;
-  for (int p = 0; p < nparts; ++p) s += partial[static_cast<size_t>(p) * H + c];
-  dw[c] = accumulate ? dw[c] + s : s;
+  if (c < H) {
+#pragma unroll 4
+    for (int p = ty; p < nparts; p += 32) s += partial[static_cast<size_t>(p) * H + c];
+  }
+  sum[ty][tx] = s;
+  __syncthreads();
+  const int col = blockIdx.x * 32 + ty;             // one warp per column
+  const float t = warp_sum(sum[tx][ty]);
+  if (tx == 0 && col < H) dw[col] = accumulate ? dw[col] + t : t;
 }
 
 // General (slow) backward for narrow rows: one warp per row, dw via atomics.
@@ -408,45 +489,46 @@ rope_vec_kernel(__nv_bfloat16* __restrict__ q, long qs_s, long qs_b, long qs_g, 
 }
 
 // ----------------------------------------------------------------------------- SwiGLU
-// x [rows, 2F] = [gate | up]; y [rows, F]
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long rows, int F) {
-  const int fv = F >> 3;
-  const long total = rows * fv;
-  for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long r = i / fv;
-    const int c = static_cast<int>(i % fv);
-    const uint4* xr = reinterpret_cast<const uint4*>(x + r * 2 * F);
+// x [rows, 2F] = [gate | up]; y [rows, F].  `Index` is unsigned while rows * F / 8 fits: a 64-bit division per vector
+// cost more instructions than the rest (16384 x 8192, in a power-limited step: forward 219 → 192 us,
+// backward 288 → 252).
+template <typename Index>
+__global__ void __launch_bounds__(256)
+swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, Index total, Index fv) {
+  const uint4* xv = reinterpret_cast<const uint4*>(x);
+  for (Index i = static_cast<Index>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+       i += static_cast<Index>(gridDim.x) * blockDim.x) {
+    const Index r = i / fv;
+    const size_t g = static_cast<size_t>(i) + static_cast<size_t>(r) * fv;     // gate vector; its up vector is fv further
     float a[8], b[8];
-    unpack8(xr[c], a);
-    unpack8(xr[fv + c], b);
+    unpack8(xv[g], a);
+    unpack8(xv[g + fv], b);
 #pragma unroll
     for (int j = 0; j < 8; ++j) a[j] = a[j] / (1.f + __expf(-a[j])) * b[j];
-    reinterpret_cast<uint4*>(y + r * F)[c] = pack8(a);
+    reinterpret_cast<uint4*>(y)[i] = pack8(a);
   }
 }
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                                  __nv_bfloat16* __restrict__ dx, long rows, int F) {
-  const int fv = F >> 3;
-  const long total = rows * fv;
-  for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long r = i / fv;
-    const int c = static_cast<int>(i % fv);
-    const uint4* xr = reinterpret_cast<const uint4*>(x + r * 2 * F);
+template <typename Index>
+__global__ void __launch_bounds__(256)
+swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                  __nv_bfloat16* __restrict__ dx, Index total, Index fv) {
+  const uint4* xv = reinterpret_cast<const uint4*>(x);
+  for (Index i = static_cast<Index>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+       i += static_cast<Index>(gridDim.x) * blockDim.x) {
+    const Index r = i / fv;
+    const size_t o = static_cast<size_t>(i) + static_cast<size_t>(r) * fv;
     float a[8], b[8], g[8], da[8], db[8];
-    unpack8(xr[c], a);
-    unpack8(xr[fv + c], b);
-    unpack8(reinterpret_cast<const uint4*>(dy + r * F)[c], g);
+    unpack8(xv[o], a);
+    unpack8(xv[o + fv], b);
+    unpack8(reinterpret_cast<const uint4*>(dy)[i], g);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float s = 1.f / (1.f + __expf(-a[j]));
       da[j] = g[j] * b[j] * s * (1.f + a[j] * (1.f - s));
       db[j] = g[j] * a[j] * s;
     }
-    uint4* dr = reinterpret_cast<uint4*>(dx + r * 2 * F);
-    dr[c] = pack8(da);
-    dr[fv + c] = pack8(db);
+    reinterpret_cast<uint4*>(dx)[o] = pack8(da);
+    reinterpret_cast<uint4*>(dx)[o + fv] = pack8(db);
   }
 }
 
@@ -517,20 +599,48 @@ __global__ void embedding_fwd_kernel(const long* __restrict__ tokens, const __nv
     for (int c = threadIdx.x; c < hv; c += blockDim.x) dst[c] = inside ? src[c] : make_uint4(0, 0, 0, 0);
   }
 }
-__global__ void embedding_bwd_kernel(const long* __restrict__ tokens, const __nv_bfloat16* __restrict__ dout,
-                                     float* __restrict__ gw, long ntok, int H, long vocab_start, long vlocal) {
+// Scatter-add of token gradients into the fp32 weight gradient: 16-byte reductions, four elements a thread (H is a
+// multiple of 4 and rows are 16-byte aligned; `wide` false: single elements).
+__global__ void __launch_bounds__(256)
+embedding_bwd_kernel(const long* __restrict__ tokens, const __nv_bfloat16* __restrict__ dout, float* __restrict__ gw,
+                     long ntok, int H, long vocab_start, long vlocal, bool wide) {
   for (long t = blockIdx.x; t < ntok; t += gridDim.x) {
     const long id = tokens[t] - vocab_start;
     if (id < 0 || id >= vlocal) continue;
     float* dst = gw + id * H;
     const __nv_bfloat16* src = dout + t * H;
-    for (int c = threadIdx.x; c < H; c += blockDim.x) atomicAdd(dst + c, __bfloat162float(src[c]));
+    if (wide) {
+      for (int c = threadIdx.x * 4; c < H; c += blockDim.x * 4) {
+        const uint2 u = *reinterpret_cast<const uint2*>(src + c);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+        asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + c), "f"(a.x), "f"(a.y), "f"(b.x),
+                     "f"(b.y)
+                     : "memory");
+      }
+    } else {
+      for (int c = threadIdx.x; c < H; c += blockDim.x) atomicAdd(dst + c, __bfloat162float(src[c]));
+    }
   }
 }
 
 // ----------------------------------------------------------------------------- cross entropy
 // Pass 1: per row (max, sum exp(x-max), target logit) over this rank's vocabulary shard.
+// What bounds both passes is arithmetic as much as memory: the exponentials alone take 117 us for 4096 x 128256 at 1.9 GHz,
+// reading the logits once 158 us.  Hence maxima on bf16 pairs and paired fp32 operations around the exponential.
 constexpr int CE_THREADS = 512;
+constexpr int CE_UNROLL = 2;        // vectors a thread requests at once
+// exp(x - base) of the eight elements of a vector, in pairs
+__device__ __forceinline__ void exp_pairs(const uint4& u, float base, float2 (&e)[4]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+  const float2 nb = make_float2(-base, -base), l2e = make_float2(1.4426950408889634f, 1.4426950408889634f);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    e[i] = __fmul2_rn(__fadd2_rn(__bfloat1622float2(h[i]), nb), l2e);
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e[i].x) : "f"(e[i].x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e[i].y) : "f"(e[i].y));
+  }
+}
 __global__ void __launch_bounds__(CE_THREADS)
 ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restrict__ targets, float* __restrict__ omax,
                 float* __restrict__ osum, float* __restrict__ otgt, long rows, int V, long vocab_start) {
@@ -540,23 +650,36 @@ ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restrict
     const __nv_bfloat16* lr = logits + row * V;
     const uint4* l4 = reinterpret_cast<const uint4*>(lr);
     float m = -INFINITY, s = 0.f;
-    for (int c = threadIdx.x; c < vv; c += CE_THREADS) {
-      float f[8];
-      unpack8(l4[c], f);
-      float lm = f[0];
+    for (int c0 = threadIdx.x; c0 < vv; c0 += CE_UNROLL * CE_THREADS) {
+      uint4 u[CE_UNROLL];
 #pragma unroll
-      for (int j = 1; j < 8; ++j) lm = fmaxf(lm, f[j]);
-      const float nm = fmaxf(m, lm);
-      float acc = 0.f;
+      for (int k = 0; k < CE_UNROLL; ++k)
+        u[k] = c0 + k * CE_THREADS < vv ? l4[c0 + k * CE_THREADS]
+                                        : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf
+      // the maximum of the pairs as they are (exact)
+      __nv_bfloat162 m2 = __floats2bfloat162_rn(m, m);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc += __expf(f[j] - nm);
-      s = s * __expf(m - nm) + acc;
+      for (int k = 0; k < CE_UNROLL; ++k) {
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u[k]);
+        m2 = __hmax2(m2, __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
+      }
+      const float nm = fmaxf(__low2float(m2), __high2float(m2));
+      const float base = nm == -INFINITY ? 0.f : nm;
+      float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < CE_UNROLL; ++k) {
+        float2 e[4];
+        exp_pairs(u[k], base, e);
+        acc = __fadd2_rn(acc, __fadd2_rn(__fadd2_rn(e[0], e[1]), __fadd2_rn(e[2], e[3])));
+      }
+      s = s * __expf(m - base) + (acc.x + acc.y);
       m = nm;
     }
     for (int c = (vv << 3) + threadIdx.x; c < V; c += CE_THREADS) {
       const float f = __bfloat162float(lr[c]);
       const float nm = fmaxf(m, f);
-      s = s * __expf(m - nm) + __expf(f - nm);
+      const float ref = nm == -INFINITY ? 0.f : nm;
+      s = s * __expf(m - ref) + __expf(f - ref);
       m = nm;
     }
     const float gm = block_max<CE_THREADS>(m, red);
@@ -580,16 +703,36 @@ ce_grad_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ targ
     uint4* l4 = reinterpret_cast<uint4*>(lr);
     const float m = gmax[row], inv = 1.f / gsum[row], sc = scale[row];
     const long t = targets[row] - vocab_start;
-    for (int c = threadIdx.x; c < vv; c += CE_THREADS) {
-      float f[8];
-      unpack8(l4[c], f);
+    const int tv = t >= 0 && t < V ? static_cast<int>(t >> 3) : -1;      // vector that holds the target
+    for (int c0 = threadIdx.x; c0 < vv; c0 += 2 * CE_THREADS) {
+      const bool two = c0 + CE_THREADS < vv;
+      uint4 u[2];
+      u[0] = l4[c0];
+      if (two) u[1] = l4[c0 + CE_THREADS];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float p = __expf(f[j] - m) * inv;
-        if (static_cast<long>(c) * 8 + j == t) p -= 1.f;
-        f[j] = p * sc;
+      for (int k = 0; k < 2; ++k) {
+        if (k == 1 && !two) break;
+        const int c = c0 + k * CE_THREADS;
+        float2 e[4];
+        exp_pairs(u[k], m, e);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) e[j] = __fmul2_rn(e[j], make_float2(inv, inv));
+        if (c == tv) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (2 * j == static_cast<int>(t & 7)) e[j].x -= 1.f;
+            if (2 * j + 1 == static_cast<int>(t & 7)) e[j].y -= 1.f;
+          }
+        }
+        float f[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          e[j] = __fmul2_rn(e[j], make_float2(sc, sc));
+          f[2 * j] = e[j].x;
+          f[2 * j + 1] = e[j].y;
+        }
+        l4[c] = pack8(f);
       }
-      l4[c] = pack8(f);
     }
     for (int c = (vv << 3) + threadIdx.x; c < V; c += CE_THREADS) {
       float p = __expf(__bfloat162float(lr[c]) - m) * inv;
@@ -649,9 +792,17 @@ __global__ void sumsq_f32_kernel(const float* __restrict__ x, long n, float* __r
   __shared__ float red[32];
   float s = 0.f;
   const long n4 = n >> 2;
-  for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const float4 t = reinterpret_cast<const float4*>(x)[i];
+  const long step = static_cast<long>(gridDim.x) * blockDim.x;
+  long i4 = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (; i4 + 3 * step < n4; i4 += 4 * step) {        // four vectors in flight a thread
+    float4 t[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) t[k] = reinterpret_cast<const float4*>(x)[i4 + k * step];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s += t[k].x * t[k].x + t[k].y * t[k].y + t[k].z * t[k].z + t[k].w * t[k].w;
+  }
+  for (; i4 < n4; i4 += step) {
+    const float4 t = reinterpret_cast<const float4*>(x)[i4];
     s += t.x * t.x + t.y * t.y + t.z * t.z + t.w * t.w;
   }
   for (long i = (n4 << 2) + static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
@@ -724,6 +875,13 @@ static int norm_fwd_ctas(int H) {
   return cached[nv.id];
 }
 
+// A thread per item, for kernels that stream many arrays: CTAs that take neighbouring pieces in launch order run closer to
+// the memory rate than a resident set that strides over all of them (AdamW, eight streams, 201 M elements: 914 us against
+// 951, 6.6 and 6.35 TB/s).  With two or three streams it is the other way round (residual add 8.2 against 7.8 us).
+static inline int grid_once(long work, int threads) {
+  const long b = (work + threads - 1) / threads;
+  return static_cast<int>(b < 1 ? 1 : b > (1L << 30) ? (1L << 30) : b);
+}
 static inline int grid_for(long work, int threads, int max_blocks) {
   long b = (work + threads - 1) / threads;
   if (b < 1) b = 1;
@@ -738,7 +896,20 @@ using namespace kb;
 
 extern "C" int kb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int rows, int H, float eps,
                               cudaStream_t st) {
-  if (H % 8 == 0 && H >= 512) {
+  if (H % 8 == 0 && H >= 512 && H <= 4096 && rows >= 148 * 40) {
+    // a warp per row pays once most warp slots have a row (8997 x 2048: 14 us, 16.5 with a CTA per row; 3800 x 2048: 10.7
+    // and 9.1)
+    const int grid = grid_for(rows, 8, 148 * 8);
+    const int vpl = (H / 8 + 31) / 32;
+#define KB_ROWS(V_)                                                                                               \
+    KB_LAUNCH((rmsnorm_fwd_rows_kernel<V_>), grid, 256, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,    \
+              (__nv_bfloat16*)y, rstd, rows, H, eps)
+    if (vpl <= 4) KB_ROWS(4);
+    else if (vpl <= 8) KB_ROWS(8);
+    else if (vpl <= 12) KB_ROWS(12);
+    else KB_ROWS(16);
+#undef KB_ROWS
+  } else if (H % 8 == 0 && H >= 512) {
     const NormVariant nv = norm_variant(H);
     const int grid = grid_for(rows, 1, norm_fwd_ctas(H));          // one resident wave: rows are dealt evenly
 #define KB_FWD(T_, V_)                                                                                            \
@@ -750,6 +921,42 @@ extern "C" int kb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd
     KB_LAUNCH(rmsnorm_fwd_warp_kernel, grid_for(rows, 8, 148 * 8), 256, 0, st, 
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rstd, rows, H, eps);
   }
+  KB_CHECK_LAUNCH();
+}
+
+// Rows of H elements at x + (n / inner) * st_outer + (n % inner) * st_inner (strides in elements); y contiguous.
+// Takes H = 8 * 2^k up to 256 and 16-byte aligned rows; returns 7 otherwise.
+extern "C" int kb_rmsnorm_fwd_heads(const void* x, long outer, int inner, long st_outer, long st_inner, const void* w, void* y,
+                                    float* rstd, int H, float eps, cudaStream_t st) {
+  const int lanes = H / 8;
+  const long rows = outer * inner;
+  if (H % 8 || lanes < 1 || lanes > 32 || (lanes & (lanes - 1)) || inner < 1 || outer < 1 || rows >= (1L << 31)) return 7;
+  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) ||
+      ((st_outer | st_inner) & 7))
+    return 7;
+  KB_LAUNCH(rmsnorm_fwd_heads_kernel, grid_for(rows * lanes, 256, 148 * 8), 256, 0, st, (const __nv_bfloat16*)x, inner,
+            st_outer, st_inner, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rstd, (unsigned)rows, H, eps);
+  KB_CHECK_LAUNCH();
+}
+
+// y = x * s with the scalar rounded to bf16 first, as a bf16 tensor times a bf16 scalar; s is read on the device.
+namespace kb {
+__global__ void __launch_bounds__(256)
+scale_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ s, __nv_bfloat16* __restrict__ y, long nvec) {
+  const float f = __bfloat162float(__float2bfloat16(*s));
+  for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec;
+       i += static_cast<long>(gridDim.x) * blockDim.x) {
+    float a[8];
+    unpack8(reinterpret_cast<const uint4*>(x)[i], a);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] *= f;
+    reinterpret_cast<uint4*>(y)[i] = pack8(a);
+  }
+}
+}  // namespace kb
+extern "C" int kb_scale(const void* x, const float* s, void* y, long n, cudaStream_t st) {
+  if (n % 8) return 7;
+  KB_LAUNCH(scale_kernel, grid_for(n / 8, 256, 148 * 16), 256, 0, st, (const __nv_bfloat16*)x, s, (__nv_bfloat16*)y, n / 8);
   KB_CHECK_LAUNCH();
 }
 
@@ -772,7 +979,7 @@ extern "C" int kb_rmsnorm_bwd_acc(const void* dy, const void* x, const float* rs
               (const __nv_bfloat16*)w, (__nv_bfloat16*)dx, scratch, rows, H)
     KB_NORM_DISPATCH(nv, KB_BWD)
 #undef KB_BWD
-    KB_LAUNCH(rmsnorm_dw_reduce_kernel, (H + 255) / 256, 256, 0, st, scratch, dw, grid, H, accumulate);
+    KB_LAUNCH(rmsnorm_dw_reduce_kernel, (H + 31) / 32, 1024, 0, st, scratch, dw, grid, H, accumulate);
   } else {
     if (!accumulate) kb::memset_async(dw, 0, sizeof(float) * H, st);    // the kernel adds with atomics
     KB_LAUNCH(rmsnorm_bwd_warp_kernel, grid_for(rows, 8, 148 * 4), 256, sizeof(float) * H, st, 
@@ -812,14 +1019,20 @@ extern "C" int kb_rope(void* q, long qs_s, long qs_b, long qs_g, long qs_r, int 
 
 extern "C" int kb_swiglu_fwd(const void* x, void* y, long rows, int F, cudaStream_t st) {
   if (F % 8) return 7;
-  KB_LAUNCH(swiglu_fwd_kernel, grid_for(rows * (F / 8), 256, 148 * 16), 256, 0, st, (const __nv_bfloat16*)x,
-                                                                              (__nv_bfloat16*)y, rows, F);
+  const long total = rows * (F / 8);
+  const int grid = grid_for(total, 256, 148 * 16);
+  const __nv_bfloat16* xb = (const __nv_bfloat16*)x;
+  if (total < (1L << 31)) KB_LAUNCH(swiglu_fwd_kernel<unsigned>, grid, 256, 0, st, xb, (__nv_bfloat16*)y, (unsigned)total, F / 8);
+  else KB_LAUNCH(swiglu_fwd_kernel<long>, grid, 256, 0, st, xb, (__nv_bfloat16*)y, total, F / 8);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_swiglu_bwd(const void* dy, const void* x, void* dx, long rows, int F, cudaStream_t st) {
   if (F % 8) return 7;
-  KB_LAUNCH(swiglu_bwd_kernel, grid_for(rows * (F / 8), 256, 148 * 16), 256, 0, st, 
-      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (__nv_bfloat16*)dx, rows, F);
+  const long total = rows * (F / 8);
+  const int grid = grid_for(total, 256, 148 * 16);
+  const __nv_bfloat16 *g = (const __nv_bfloat16*)dy, *xb = (const __nv_bfloat16*)x;
+  if (total < (1L << 31)) KB_LAUNCH(swiglu_bwd_kernel<unsigned>, grid, 256, 0, st, g, xb, (__nv_bfloat16*)dx, (unsigned)total, F / 8);
+  else KB_LAUNCH(swiglu_bwd_kernel<long>, grid, 256, 0, st, g, xb, (__nv_bfloat16*)dx, total, F / 8);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_dropout_add_fwd(const void* x, const void* res, void* y, long n, float p, unsigned seed,
@@ -850,8 +1063,9 @@ extern "C" int kb_embedding_fwd(const long* tokens, const void* w, void* out, lo
 }
 extern "C" int kb_embedding_bwd(const long* tokens, const void* dout, float* gw, long ntok, int H, long vocab_start,
                                 long vlocal, cudaStream_t st) {
+  const bool wide = H % 4 == 0 && (reinterpret_cast<uintptr_t>(gw) & 15) == 0 && (reinterpret_cast<uintptr_t>(dout) & 7) == 0;
   KB_LAUNCH(embedding_bwd_kernel, grid_for(ntok, 1, 148 * 16), 256, 0, st, tokens, (const __nv_bfloat16*)dout, gw, ntok, H,
-                                                                     vocab_start, vlocal);
+                                                                     vocab_start, vlocal, wide);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_ce_stats(const void* logits, const long* targets, float* omax, float* osum, float* otgt, long rows,
@@ -869,7 +1083,7 @@ extern "C" int kb_ce_grad(void* logits, const long* targets, const float* gmax, 
 extern "C" int kb_adamw(void* p, const float* g, float* m, float* v, float* master, long n, float lr, float b1,
                         float b2, float eps, float wd, float bc1, float bc2, const float* grad_scale_ptr,
                         float grad_scale, cudaStream_t st) {
-  KB_LAUNCH(adamw_kernel, grid_for(n / 4 + 1, 256, 148 * 16), 256, 0, st, (__nv_bfloat16*)p, g, m, v, master, n, lr, b1, b2,
+  KB_LAUNCH(adamw_kernel, grid_once(n / 4 + 1, 256), 256, 0, st, (__nv_bfloat16*)p, g, m, v, master, n, lr, b1, b2,
                                                                     eps, wd, bc1, bc2, grad_scale_ptr, grad_scale);
   KB_CHECK_LAUNCH();
 }
@@ -906,6 +1120,6 @@ extern "C" int kb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const float
   const int grid = rows < NOALLOC_MAX_CTAS ? rows : NOALLOC_MAX_CTAS;
   KB_LAUNCH((rmsnorm_bwd_kernel<256, 4>), grid, 256, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, rstd,
                                                     (const __nv_bfloat16*)w, (__nv_bfloat16*)dx, partial, rows, H);
-  KB_LAUNCH(rmsnorm_dw_reduce_kernel, (H + 255) / 256, 256, 0, st, partial, dw, grid, H, 0);
+  KB_LAUNCH(rmsnorm_dw_reduce_kernel, (H + 31) / 32, 1024, 0, st, partial, dw, grid, H, 0);
   KB_CHECK_LAUNCH();
 }

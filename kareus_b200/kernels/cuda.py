@@ -53,6 +53,8 @@ def _declare(L) -> None:
         "kb_gemm_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P],
         "kb_gemm_bias_act_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, I, P, P],
         "kb_rmsnorm_fwd": [P, P, P, P, I, I, F, P],
+        "kb_rmsnorm_fwd_heads": [P, LNG, I, LNG, LNG, P, P, P, I, F, P],
+        "kb_scale": [P, P, P, LNG, P],
         "kb_rmsnorm_bwd": [P, P, P, P, P, P, P, I, I, P],
         "kb_rmsnorm_bwd_acc": [P, P, P, P, P, P, P, I, I, I, P],
         "kb_rope": [P, LNG, LNG, LNG, LNG, I, I, P, LNG, LNG, LNG, I, P, P, I, I, I, I, P],
@@ -165,6 +167,44 @@ def rmsnorm_fwd(x, w, eps):
                                 _stream()), "rmsnorm_fwd")
     _count()
     return y, rstd
+
+
+def rmsnorm_fwd_heads(x, w, eps):
+    """RMSNorm over the last dimension of a strided ``[..., H]`` view (q or k inside the packed QKV buffer), read where
+    it lies.  Returns a contiguous tensor of ``x``'s shape and ``rstd`` (one value per row)."""
+    H = x.shape[-1]
+    if _bf16(x) and x.dim() >= 2 and x.stride(-1) == 1 and x.numel() and x.data_ptr() % 16 == 0:
+        # leading dimensions as (outer rows of one stride) x (inner rows of one stride)
+        dims = [(n, st) for n, st in zip(x.shape[:-1], x.stride()[:-1]) if n > 1] or [(1, H)]
+        inner, st_in = dims.pop()
+        while dims and dims[-1][1] == inner * st_in:
+            inner *= dims.pop()[0]
+        outer, st_out = dims.pop() if dims else (1, 0)
+        while dims and dims[-1][1] == outer * st_out:
+            outer *= dims.pop()[0]
+        wb = w if _bf16(w) else w.to(torch.bfloat16)
+        lanes = H // 8
+        if (not dims and H % 8 == 0 and lanes <= 32 and lanes & (lanes - 1) == 0 and st_in % 8 == 0 and st_out % 8 == 0
+                and wb.is_contiguous() and wb.data_ptr() % 16 == 0 and outer * inner < 1 << 31):
+            y = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+            rstd = torch.empty(outer * inner, dtype=torch.float32, device=x.device)
+            _check(lib().kb_rmsnorm_fwd_heads(x.data_ptr(), outer, inner, st_out, st_in, wb.data_ptr(), y.data_ptr(),
+                                              rstd.data_ptr(), H, float(eps), _stream()), "rmsnorm_fwd_heads")
+            _count()
+            return y, rstd
+    y, rstd = rmsnorm_fwd(x.reshape(-1, H), w, eps)
+    return y.view(x.shape), rstd
+
+
+def scale(x, s):
+    """``x * s.to(x.dtype)`` for a scalar tensor ``s``."""
+    if not (_bf16(x) and x.is_contiguous() and x.numel() and x.numel() % 8 == 0 and x.data_ptr() % 16 == 0 and s.numel() == 1
+            and s.dtype == torch.float32 and s.device == x.device):
+        return x * s.to(x.dtype)
+    y = torch.empty_like(x)
+    _check(lib().kb_scale(x.data_ptr(), s.data_ptr(), y.data_ptr(), x.numel(), _stream()), "scale")
+    _count()
+    return y
 
 
 def rmsnorm_bwd(dy, x, rstd, w, dw_accum=None):

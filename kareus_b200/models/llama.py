@@ -214,7 +214,7 @@ class _HeadLossFn(torch.autograd.Function):
         module = ctx.module
         # dloss is a scalar (1/num_microbatches scaling etc.); weights got the unscaled gradient,
         # so the caller must keep dloss == 1 or rescale main_grad — enforced by GPTModel.
-        dx = dx * dloss.to(dx.dtype)
+        dx = K.scale(dx, dloss)
         dx = dx.reshape(ctx.shape)
         if module.tp > 1 and not module.sp:
             dist.all_reduce(dx, group=module.group)

@@ -59,22 +59,20 @@ class QKVPostOp(nn.Module, GraphOperator):
         return q, k, v
 
     def forward(self, ctx, x):
-        s, b, _ = x.shape
         q, k, v = self.split(x)
         if self.qk_norm:
-            qc = q.reshape(-1, self.d)
-            kc = k.reshape(-1, self.d)
-            qn, q_rstd = K.rmsnorm_fwd(qc, self.q_norm_weight, self.eps)
-            kn, k_rstd = K.rmsnorm_fwd(kc, self.k_norm_weight, self.eps)
+            qn, q_rstd = K.rmsnorm_fwd_heads(q, self.q_norm_weight, self.eps)
+            kn, k_rstd = K.rmsnorm_fwd_heads(k, self.k_norm_weight, self.eps)
             if ctx.requires_grad:
-                ctx.save_for_backward(qc, q_rstd, kc, k_rstd)
-            return qn.view(s, b, self.g, self.rep, self.d), kn.view(s, b, self.g, self.d), v
+                ctx.save_for_backward(q, q_rstd, k, k_rstd)
+            return qn, kn, v
         return q, k, v
 
     def backward(self, ctx, dq, dk, dv):
         packed = getattr(dq, "_packed_base", None)
         if self.qk_norm:
-            qc, q_rstd, kc, k_rstd = ctx.saved_tensors
+            q, q_rstd, k, k_rstd = ctx.saved_tensors
+            qc, kc = q.reshape(-1, self.d), k.reshape(-1, self.d)
             dqc, dwq = K.rmsnorm_bwd(dq.reshape(-1, self.d), qc, q_rstd, self.q_norm_weight)
             dkc, dwk = K.rmsnorm_bwd(dk.reshape(-1, self.d), kc, k_rstd, self.k_norm_weight)
             accumulate_grad(self.q_norm_weight, dwq)

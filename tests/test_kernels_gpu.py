@@ -469,3 +469,62 @@ def test_gemm_bias_activation_epilogue(M, N, K, activation):
     assert _rel(got, want) < 1e-2
     only_act = KC.gemm(a, w, activation=activation)
     assert _rel(only_act, ref.bias_act(a.float() @ w.float().t(), None, activation)) < 1e-2
+
+
+# a warp per row from 148 * 40 rows on; 4, 8, 12 or 16 vectors a lane, last vectors of a row missing in some lanes
+@pytest.mark.parametrize("rows,H", [(5919, 1032), (5920, 512), (5923, 1032), (5950, 2056), (5921, 3072), (5927, 4088), (5920, 4096),
+                                    (5920, 4104)])
+def test_rmsnorm_forward_rows(rows, H):
+    KC = _K()
+    from kareus_b200.kernels import ref
+    x, w = torch.randn(rows, H, device="cuda").bfloat16(), torch.randn(H, device="cuda").bfloat16()
+    y, rstd = KC.rmsnorm_fwd(x, w, 1e-5)
+    want, rstd_w = ref.rmsnorm_fwd(x.double(), w.double(), 1e-5)
+    assert _rel(y, want) < 3e-3 and _rel(rstd, rstd_w) < 1e-5            # bf16 rounding of the result: 2^-9
+
+
+@pytest.mark.parametrize("s,b,g,rep,d", [(1, 1, 1, 1, 128), (37, 3, 2, 3, 128), (5, 2, 8, 2, 64), (9, 1, 3, 1, 256), (7, 2, 2, 2, 8),
+                                         (6, 2, 2, 2, 96)])
+def test_rmsnorm_heads_views(s, b, g, rep, d):
+    KC = _K()
+    from kareus_b200.kernels import ref
+    packed = torch.randn(s, b, g, (rep + 2) * d, device="cuda").bfloat16()
+    q = packed[..., : rep * d].unflatten(-1, (rep, d))
+    w = torch.randn(d, device="cuda").bfloat16()
+    for x in (q, packed[..., rep * d:(rep + 1) * d], q.permute(1, 0, 3, 2, 4), q.contiguous(), packed[..., d:2 * d].expand(s, b, g, d)):
+        y, rstd = KC.rmsnorm_fwd_heads(x, w, 1e-6)
+        want, rstd_w = ref.rmsnorm_fwd(x.reshape(-1, d).double(), w.double(), 1e-6)
+        assert y.shape == x.shape and y.is_contiguous()
+        assert _rel(y.reshape(-1, d), want) < 3e-3 and _rel(rstd, rstd_w) < 1e-5
+
+
+@pytest.mark.parametrize("rows,V", [(3, 8), (5, 16376), (2, 16384), (4, 16392), (3, 50264), (2, 4096)])
+def test_cross_entropy_vector_groups(rows, V):
+    """Rows around multiples of the two vectors a thread takes at once, with hidden logits."""
+    KC = _K()
+    logits = (4 * torch.randn(rows, V, device="cuda")).bfloat16()
+    logits[0, : V // 2] = float("-inf")
+    tgt = torch.randint(0, V, (rows,), device="cuda")
+    tgt[0], tgt[-1] = V - 1, V - 2
+    m, se, tl = KC.cross_entropy_local_stats(logits, tgt, 0)
+    x = logits.double()
+    assert torch.equal(m.double(), x.max(-1).values)
+    assert _rel(m.double() + se.double().log() - tl.double(), x.logsumexp(-1) - x.gather(1, tgt[:, None])[:, 0]) < 1e-5
+    sc = torch.rand(rows, device="cuda")
+    want = (x.softmax(-1) - torch.nn.functional.one_hot(tgt, V)) * sc.double()[:, None]
+    KC.cross_entropy_finish(logits, tgt, 0, m, se, sc)
+    assert _rel(logits, want) < 4e-3
+
+
+@pytest.mark.parametrize("H", [8, 1032, 3072])
+def test_embedding_backward_vectors(H):
+    KC = _K()
+    tok = torch.randint(0, 50, (3, 41), device="cuda")
+    dout = torch.randn(3, 41, H, device="cuda").bfloat16()
+    for gw in (torch.zeros(30, H, device="cuda"), torch.zeros(30 * H + 1, device="cuda")[1:].view(30, H)):
+        KC.embedding_bwd(dout, tok, gw, 10)
+        keep = (tok >= 10) & (tok < 40)
+        want = torch.zeros(30, H, device="cuda", dtype=torch.float64).index_add_(0, tok[keep] - 10, dout[keep].double())
+        assert _rel(gw, want) < 1e-6
+    x, s = torch.randn(5, H, device="cuda").bfloat16(), torch.tensor(0.3333, device="cuda")
+    assert torch.equal(KC.scale(x, s), x * s.to(x.dtype))
