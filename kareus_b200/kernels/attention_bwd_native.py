@@ -21,8 +21,6 @@ def _lib():
         L.kb_flash_attn_bwd.restype = c_int
         L.kb_flash_attn_bwd_scratch_floats.argtypes = [I] * 6
         L.kb_flash_attn_bwd_scratch_floats.restype = c_long
-        L.kb_flash_attn_bwd_launches.argtypes = [I] * 5
-        L.kb_flash_attn_bwd_launches.restype = c_int
         _DECLARED = True
     return L
 
@@ -31,7 +29,7 @@ def _geom5(t, kg):
     """(s, b, g, rep, d, strides(s, b, g, r)) of a query-like view."""
     if t.dim() == 5:
         s, b, g, rep, d = t.shape
-        return s, b, g, rep, d, (t.stride(0), t.stride(1), t.stride(2), t.stride(3))
+        return s, b, g, rep, d, t.stride()[:4]
     s, b, h, d = t.shape
     rep = h // kg
     return s, b, kg, rep, d, (t.stride(0), t.stride(1), t.stride(2) * rep, t.stride(2))
@@ -69,14 +67,13 @@ def backward(do, q, k, v, o, lse, scale, causal=True, q_offset=0, kv_len=None, o
     L = _lib()
     work = torch.empty(L.kb_flash_attn_bwd_scratch_floats(sq, skv, b, g, rep, d), dtype=torch.float32, device=q.device)
     st = KC.status_word(q.device)
-    rc = L.kb_flash_attn_bwd(q.data_ptr(), *qs, k.data_ptr(), k.stride(0), k.stride(1), k.stride(2),
-                             v.data_ptr(), v.stride(0), v.stride(1), v.stride(2), o4.data_ptr(), do4.data_ptr(),
-                             lse.data_ptr(), dq.data_ptr(), *dqs, dk.data_ptr(), dk.stride(0), dk.stride(1),
-                             dk.stride(2), dv.data_ptr(), dv.stride(0), dv.stride(1), dv.stride(2), work.data_ptr(),
+    rc = L.kb_flash_attn_bwd(q.data_ptr(), *qs, k.data_ptr(), *k.stride()[:3], v.data_ptr(), *v.stride()[:3], o4.data_ptr(),
+                             do4.data_ptr(), lse.data_ptr(), dq.data_ptr(), *dqs, dk.data_ptr(), *dk.stride()[:3],
+                             dv.data_ptr(), *dv.stride()[:3], work.data_ptr(),
                              sq, skv, b, g, rep, d, float(scale), 1 if causal else 0, int(q_offset), st.data_ptr(),
                              KC._stream())
     KC._check(rc, "flash_attn_bwd")
-    KC._count(L.kb_flash_attn_bwd_launches(sq, skv, b, g, rep))
+    KC._count(3)
     if out is not None:
         return out
     return dq.reshape(q.shape), dk, dv
@@ -118,5 +115,5 @@ def backward_chunked(do, q, sources, table, chunk_rows, q_positions, o, lse, sca
         _int_array(dv_row_base), work.data_ptr(), sq, b, g, rep, d, float(scale), 1 if causal else 0, st.data_ptr(),
         KC._stream())
     KC._check(rc, "flash_attn_bwd_chunked")
-    KC._count(L.kb_flash_attn_bwd_launches(sq, skv, b, g, rep))
+    KC._count(3)
     return dq, dkv

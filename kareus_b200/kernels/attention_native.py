@@ -35,13 +35,19 @@ def _lib():
 def _q_geometry(q):
     if q.dim() == 5:
         s, b, g, rep, d = q.shape
-        return s, b, g, rep, d, (q.stride(0), q.stride(1), q.stride(2), q.stride(3))
+        return s, b, g, rep, d, q.stride()[:4]
     s, b, h, d = q.shape
     return s, b, 1, h, d, (q.stride(0), q.stride(1), 0, q.stride(2))
 
 
 def _usable(t) -> bool:
-    return t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all(st % 8 == 0 for st in t.stride()[:-1])
+    st = t.stride()
+    if st[-1] != 1 or t.data_ptr() % 16:
+        return False
+    low = 0
+    for x in st[:-1]:
+        low |= x
+    return low % 8 == 0
 
 
 def unsupported_reason(d, g, kg, *tensors):
@@ -50,8 +56,9 @@ def unsupported_reason(d, g, kg, *tensors):
         return f"head dim {d} (the kernels are specialised for 128)"
     if g != kg:
         return f"query groups {g} do not match key groups {kg}"
-    if not all(_usable(t) for t in tensors):
-        return "an operand's head dim is not contiguous or a stride/base is not 16-byte aligned"
+    for t in tensors:
+        if not _usable(t):
+            return "an operand's head dim is not contiguous or a stride/base is not 16-byte aligned"
     return None
 
 
@@ -71,8 +78,8 @@ def forward(q, k, v, scale, causal=True, q_offset=0, kv_len=None, strict=False):
     out = torch.empty(sq, b, g * rep, d, dtype=q.dtype, device=q.device)
     lse = torch.empty(b, g * rep, sq, dtype=torch.float32, device=q.device)
     st = KC.status_word(q.device)
-    rc = _lib().kb_flash_attn_fwd(q.data_ptr(), *qs, k.data_ptr(), k.stride(0), k.stride(1), k.stride(2),
-                                  v.data_ptr(), v.stride(0), v.stride(1), v.stride(2), out.data_ptr(),
+    rc = _lib().kb_flash_attn_fwd(q.data_ptr(), *qs, k.data_ptr(), *k.stride()[:3], v.data_ptr(), *v.stride()[:3],
+                                  out.data_ptr(),
                                   lse.data_ptr(), sq, skv, b, g, rep, d, float(scale), 1 if causal else 0,
                                   int(q_offset), st.data_ptr(), KC._stream())
     KC._check(rc, "flash_attn_fwd")

@@ -504,10 +504,16 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 }
 
 // Row statistics for the kernel above, one 1 KB block per query tile of one (batch, head): 128 x −lse·log2(e), then
-// 128 x −δ with δ = Σ_d dO·O (both [s,b,h,d] contiguous).  Rows past S get −inf and 0.  Half a warp per row.
+// 128 x −δ with δ = Σ_d dO·O (both [s,b,h,d] contiguous).  Rows past S get −inf and 0.  Half a warp per row, which also
+// zeroes its row of the dQ accumulator; `zero` (n_zero vectors) are the accumulators of dK and dV, if there are any.
 __global__ void __launch_bounds__(256)
 attn_stats_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
-                  const float* __restrict__ lse, float* __restrict__ stats, unsigned S, unsigned S_pad, unsigned B, unsigned H) {
+                  const float* __restrict__ lse, float* __restrict__ stats, float4* __restrict__ dq_acc,
+                  float4* __restrict__ zero, long n_zero, unsigned S, unsigned S_pad, unsigned B, unsigned H) {
+  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_zero;
+       i += static_cast<long>(gridDim.x) * blockDim.x)
+    zero[i] = z;
   const unsigned rows = static_cast<unsigned>(S_pad) * B * H;
   const int l = threadIdx.x & 15;
   const unsigned step = (gridDim.x * blockDim.x) >> 4;
@@ -517,6 +523,9 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __r
     const unsigned sb = w / H, h = w - sb * H, ss = sb / B, bb = sb - ss * B;
     float s = 0.f;
     if (ss < S && w < rows) {
+      float4* acc = dq_acc + static_cast<size_t>(w) * (FB_T / 4) + l;
+      acc[0] = z;
+      acc[16] = z;
       const uint4 a = reinterpret_cast<const uint4*>(dO + static_cast<size_t>(w) * FB_T)[l];
       const uint4 b = reinterpret_cast<const uint4*>(O + static_cast<size_t>(w) * FB_T)[l];
       const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
@@ -539,31 +548,45 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __r
 }
 
 // fp32 accumulator [rows(s,b), heads, d] times `scale` → bf16 strided view (strides in elements per s, b, group, head
-// of the group).  Half a warp per head vector, 8 elements a thread: 16-byte stores, or two of 8 bytes where the view is
-// not aligned to 16 (`wide` false).  Bound by memory: 201 MB in and 101 MB out take 50 us (72 with 4 elements a thread
-// and 64-bit divisions).
+// of the group); `rows_of` moves chunks of s (dK/dV straight into the layout a reduce-scatter expects).
+struct Convert {
+  const float* acc;
+  __nv_bfloat16* out;
+  unsigned rows, G, R;
+  long st_s, st_b, st_g, st_r;
+  float scale;
+  bool wide;                  // the view is aligned to 16 bytes
+  RowMap rows_of;
+};
+// All accumulators of a call in one launch.  Half a warp per head vector, 8 elements a thread: 16-byte stores, or two of
+// 8 bytes where the view is not aligned to 16.  Bound by memory: 201 MB in and 101 MB out take 51 us (72 with 4 elements
+// a thread and 64-bit divisions).
 __global__ void __launch_bounds__(256)
-attn_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ out, unsigned rows, unsigned B, unsigned G,
-                    unsigned R, long st_s, long st_b, long st_g, long st_r, float scale, bool wide) {
+attn_convert_kernel(const __grid_constant__ Convert dq, const __grid_constant__ Convert dk, const __grid_constant__ Convert dv,
+                    unsigned B) {
   const int l = threadIdx.x & 15;
-  const unsigned step = (gridDim.x * blockDim.x) >> 4;
-#pragma unroll 2
-  for (unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; w < rows; w += step) {
-    const float4* src = reinterpret_cast<const float4*>(acc + static_cast<size_t>(w) * FB_T) + l * 2;
+  const unsigned step = (gridDim.x * blockDim.x) >> 4, total = dq.rows + dk.rows + dv.rows;
+  auto convert = [&](const Convert& c, unsigned w) {
+    const float4* src = reinterpret_cast<const float4*>(c.acc + static_cast<size_t>(w) * FB_T) + l * 2;
     const float4 a = __ldcs(src), b = __ldcs(src + 1);
-    const unsigned t = w / R, rr = w - t * R, u = t / G, gg = t - u * G, ss = u / B, bb = u - ss * B;
-    __nv_bfloat16* o = out + ss * st_s + bb * st_b + gg * st_g + rr * st_r + l * 8;
+    const unsigned t = w / c.R, rr = w - t * c.R, u = t / c.G, gg = t - u * c.G, ss = u / B, bb = u - ss * B;
+    __nv_bfloat16* o = c.out + c.rows_of.at(ss) * c.st_s + bb * c.st_b + gg * c.st_g + rr * c.st_r + l * 8;
     uint4 v;
-    v.x = pack_bf16x2(a.x * scale, a.y * scale);
-    v.y = pack_bf16x2(a.z * scale, a.w * scale);
-    v.z = pack_bf16x2(b.x * scale, b.y * scale);
-    v.w = pack_bf16x2(b.z * scale, b.w * scale);
-    if (wide) {
+    v.x = pack_bf16x2(a.x * c.scale, a.y * c.scale);
+    v.y = pack_bf16x2(a.z * c.scale, a.w * c.scale);
+    v.z = pack_bf16x2(b.x * c.scale, b.y * c.scale);
+    v.w = pack_bf16x2(b.z * c.scale, b.w * c.scale);
+    if (c.wide) {
       *reinterpret_cast<uint4*>(o) = v;
     } else {
       reinterpret_cast<uint2*>(o)[0] = make_uint2(v.x, v.y);
       reinterpret_cast<uint2*>(o)[1] = make_uint2(v.z, v.w);
     }
+  };
+  for (unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; w < total; w += step) {
+    if (w < dq.rows) convert(dq, w);
+    else if (w < dq.rows + dk.rows) convert(dk, w - dq.rows);
+    else convert(dv, w - dq.rows - dk.rows);
   }
 }
 
@@ -600,37 +623,12 @@ static long stats_floats(int sq, int b, int hq) { return (long)b * hq * ((sq + F
 
 }  // namespace kb
 
-// Scratch: `work` (16-byte aligned) must hold the fp32 accumulators, zeroed here, and the row statistics.
+// Scratch: `work` (16-byte aligned) must hold the fp32 accumulators, zeroed by the call, and the row statistics.
 extern "C" long kb_flash_attn_bwd_scratch_floats(int sq, int skv, int b, int g, int rep, int d) {
   return (long)sq * b * g * rep * d + stats_floats(sq, b, g * rep) +
          (merge_heads(sq, skv, b, g, rep) ? 0 : 2L * skv * b * g * d);
 }
-// Kernels and memsets of one backward call.
-extern "C" int kb_flash_attn_bwd_launches(int sq, int skv, int b, int g, int rep) {
-  return merge_heads(sq, skv, b, g, rep) ? 4 : 7;
-}
-
 namespace kb {
-
-// fp32 accumulator [logical rows, b, g, d] → bf16 rows of a strided destination where logical chunk c
-// starts at destination row map.base[c] (dK/dV straight into the layout a reduce-scatter expects)
-__global__ void attn_convert_chunked_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ out, long n_vec,
-                                            int B, int G, long st_s, long st_b, long st_g, RowMap map) {
-  for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_vec;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const int dv = static_cast<int>(i % (FB_T / 4));
-    long rest = i / (FB_T / 4);
-    const int gg = static_cast<int>(rest % G); rest /= G;
-    const int bb = static_cast<int>(rest % B);
-    const long ss = map.at(rest / B);
-    const float4 v = reinterpret_cast<const float4*>(acc)[i];
-    __nv_bfloat16* o = out + ss * st_s + bb * st_b + gg * st_g + dv * 4;
-    uint2 w;
-    *reinterpret_cast<__nv_bfloat162*>(&w.x) = __floats2bfloat162_rn(v.x, v.y);
-    *reinterpret_cast<__nv_bfloat162*>(&w.y) = __floats2bfloat162_rn(v.z, v.w);
-    *reinterpret_cast<uint2*>(o) = w;
-  }
-}
 
 static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom& geom, const void* o, const void* dO,
                       const float* lse, const BwdOut& out, float* work, int sq, int skv, int b, int g, int rep, int d,
@@ -642,16 +640,14 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
   float* stats = dq_acc + n_dq;
   float* dk_acc = merged ? nullptr : stats + stats_floats(sq, b, hq);
   float* dv_acc = merged ? nullptr : dk_acc + n_dkv;
-  cudaError_t e = kb::memset_async(dq_acc, 0, sizeof(float) * n_dq, stream);
-  if (e == cudaSuccess && !merged) e = kb::memset_async(dk_acc, 0, sizeof(float) * 2 * n_dkv, stream);
-  if (e != cudaSuccess) return 1000 + (int)e;
+  cudaError_t e;
   {
     const int s_pad = (sq + FB_T - 1) / FB_T * FB_T;
     const long rows = (long)s_pad * b * hq;
     long blocks = (rows * 16 + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
     KB_LAUNCH(attn_stats_kernel, (int)blocks, 256, 0, stream, (const __nv_bfloat16*)dO, (const __nv_bfloat16*)o, lse, stats,
-              sq, s_pad, b, hq);
+              reinterpret_cast<float4*>(dq_acc), reinterpret_cast<float4*>(dk_acc), merged ? 0L : 2 * n_dkv / 4, sq, s_pad, b, hq);
   }
   CUtensorMap tmDO;
   int rc = make_qkv_map(&tmDO, dO, d, 1, hq, b, sq, 0, d, (long)hq * d, (long)b * hq * d, 0);
@@ -690,20 +686,19 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     KB_LAUNCH(flash_attn_bwd_kernel, grid, FB_THREADS, FbSmem::TOTAL, stream, tmQ, kv, tmDO, tmDQ, p);
   }
   {
-    const long rows = (long)sq * b * hq;
-    long blocks = (rows * 16 + 255) / 256;
-    const bool wide = ((reinterpret_cast<uintptr_t>(out.dq) | ((out.dqs_s | out.dqs_b | out.dqs_g | out.dqs_r) * 2)) & 15) == 0;
-    KB_LAUNCH(attn_convert_kernel, (int)blocks, 256, 0, stream, (const float*)dq_acc, (__nv_bfloat16*)out.dq, (unsigned)rows,
-              b, g, rep, out.dqs_s, out.dqs_b, out.dqs_g, out.dqs_r, scale, wide);
-    if (!merged) {
-      const long nvec = n_dkv / 4;
-      blocks = (nvec + 255) / 256;
-      if (blocks > 148 * 16) blocks = 148 * 16;
-      KB_LAUNCH(attn_convert_chunked_kernel, (int)blocks, 256, 0, stream, (const float*)dk_acc, (__nv_bfloat16*)out.dk, nvec,
-                b, g, out.dks_s, out.dks_b, out.dks_g, out.dk_rows);
-      KB_LAUNCH(attn_convert_chunked_kernel, (int)blocks, 256, 0, stream, (const float*)dv_acc, (__nv_bfloat16*)out.dv, nvec,
-                b, g, out.dvs_s, out.dvs_b, out.dvs_g, out.dv_rows);
-    }
+    auto segment = [&](const float* acc, void* dst, long rows, int r, long st_s, long st_b, long st_g, long st_r, float f,
+                       const RowMap& map) {
+      const bool wide = ((reinterpret_cast<uintptr_t>(dst) | ((st_s | st_b | st_g | st_r) * 2)) & 15) == 0;
+      return Convert{acc, (__nv_bfloat16*)dst, (unsigned)rows, (unsigned)g, (unsigned)r, st_s, st_b, st_g, st_r, f, wide, map};
+    };
+    const long kv_rows = merged ? 0 : (long)skv * b * g;
+    RowMap plain;
+    plain.chunk_rows = 0;
+    const Convert cq = segment(dq_acc, out.dq, (long)sq * b * hq, rep, out.dqs_s, out.dqs_b, out.dqs_g, out.dqs_r, scale, plain);
+    const Convert ck = segment(dk_acc, out.dk, kv_rows, 1, out.dks_s, out.dks_b, out.dks_g, 0, 1.f, out.dk_rows);
+    const Convert cv = segment(dv_acc, out.dv, kv_rows, 1, out.dvs_s, out.dvs_b, out.dvs_g, 0, 1.f, out.dv_rows);
+    const long blocks = (((long)sq * b * hq + 2 * kv_rows) * 16 + 255) / 256;
+    KB_LAUNCH(attn_convert_kernel, (int)blocks, 256, 0, stream, cq, ck, cv, (unsigned)b);
   }
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + (int)e;
