@@ -12,7 +12,11 @@
 //   kb_rec_stream_wait(stream, ev)      note "stream waits for ev"   (likewise).
 //   kb_rec_next_epoch(&counter)         the next recorded launch that declares an epoch location takes
 //                                       its epoch from this host counter (incremented on every replay).
-//   kb_replay(list, compute_stream)     enqueue the whole list.
+//   kb_replay(list, compute_stream)     enqueue the whole list.  A list that stays on the compute stream and patches no
+//                                       epochs becomes a CUDA graph on its first replay: one launch instead of one per
+//                                       kernel (3.4 us each, which is what a step of a small model consisted of).
+//                                       Lists with side streams keep explicit stream order: kernels that wait on peer
+//                                       GPUs must start in the same order on every rank.
 //   kb_rec_launches(list)               kernels in the list (for launch accounting).
 //   kb_rec_free(list)
 #include "launch.h"
@@ -61,6 +65,8 @@ struct LaunchList {
   std::vector<cudaEvent_t> events;
   long launches = 0;
   bool finished = false;
+  cudaGraphExec_t graph = nullptr;
+  bool graph_tried = false;
 
   int stream_index(cudaStream_t s, cudaStream_t compute) {
     if (s == compute) return 0;
@@ -69,7 +75,57 @@ struct LaunchList {
     streams.push_back(s);
     return static_cast<int>(streams.size() - 1);
   }
+  // The operations in order as a chain of graph nodes; leaves `graph` null where that is not possible.
+  void build_graph() {
+    graph_tried = true;
+    if (streams.size() != 1) return;
+    for (const Op& op : ops)
+      if (op.epoch_counter) return;
+    cudaGraph_t g;
+    if (cudaGraphCreate(&g, 0) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    cudaGraphNode_t last = nullptr;
+    bool ok = true;
+    for (const Op& op : ops) {
+      cudaGraphNode_t node = nullptr;
+      const cudaGraphNode_t* deps = last ? &last : nullptr;
+      const size_t ndeps = last ? 1 : 0;
+      cudaError_t e = cudaSuccess;
+      if (op.kind == OP_LAUNCH) {
+        cudaKernelNodeParams p{};
+        p.func = const_cast<void*>(op.func);
+        p.gridDim = op.grid;
+        p.blockDim = op.block;
+        p.sharedMemBytes = static_cast<unsigned>(op.smem);
+        p.kernelParams = argptrs.data() + op.args_off;
+        e = cudaGraphAddKernelNode(&node, g, deps, ndeps, &p);
+      } else if (op.kind == OP_MEMCPY) {
+        e = cudaGraphAddMemcpyNode1D(&node, g, deps, ndeps, op.dst, op.src, op.bytes, cudaMemcpyDeviceToDevice);
+      } else if (op.kind == OP_MEMSET) {
+        cudaMemsetParams p{};
+        p.dst = op.dst;
+        p.value = static_cast<unsigned>(op.value) & 0xffu;
+        p.elementSize = 1;
+        p.width = op.bytes;
+        p.height = 1;
+        e = cudaGraphAddMemsetNode(&node, g, deps, ndeps, &p);
+      } else {
+        continue;                       // events of one stream with itself
+      }
+      if (e != cudaSuccess) {
+        ok = false;
+        break;
+      }
+      last = node;
+    }
+    if (ok && cudaGraphInstantiate(&graph, g, 0) != cudaSuccess) graph = nullptr;
+    cudaGraphDestroy(g);
+    cudaGetLastError();
+  }
   ~LaunchList() {
+    if (graph) cudaGraphExecDestroy(graph);
     for (cudaEvent_t e : events) cudaEventDestroy(e);
   }
 };
@@ -226,6 +282,16 @@ extern "C" int kb_replay(int list, cudaStream_t compute_stream) {
   if (list < 1 || list > static_cast<int>(g_lists.size())) return 7;
   LaunchList* L = g_lists[list - 1].get();
   if (!L || !L->finished || g_recording) return 7;
+  // inside a capture of the caller's the operations themselves are captured
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (L->streams.size() == 1 && cudaStreamIsCapturing(compute_stream, &cap) == cudaSuccess &&
+      cap == cudaStreamCaptureStatusNone) {
+    if (!L->graph_tried) L->build_graph();
+    if (L->graph) {
+      const cudaError_t ge = cudaGraphLaunch(L->graph, compute_stream);
+      return ge == cudaSuccess ? 0 : 2000 + static_cast<int>(ge);
+    }
+  }
   L->streams[0] = compute_stream;
   cudaError_t e = cudaSuccess;
   for (const Op& op : L->ops) {
