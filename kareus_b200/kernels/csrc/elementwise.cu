@@ -1093,6 +1093,21 @@ extern "C" int kb_sumsq(const void* x, long n, int is_f32, float* out, cudaStrea
   KB_CHECK_LAUNCH();
 }
 
+// Gradient norm from the sum of squares and the factor that clips it to `clip`, for the optimizer's own launch to read:
+// out[0] = sqrt(sumsq), out[1] = min(1, clip / (norm + 1e-6)).
+namespace kb {
+__global__ void clip_scale_kernel(const float* __restrict__ sumsq, float clip, float* __restrict__ out) {
+  const float norm = sqrtf(*sumsq);
+  const float f = clip / (norm + 1e-6f);
+  out[0] = norm;
+  out[1] = f > 1.f ? 1.f : f;       // a NaN norm stays visible in the update
+}
+}  // namespace kb
+extern "C" int kb_clip_scale(const float* sumsq, float clip, float* out, cudaStream_t st) {
+  KB_LAUNCH(clip_scale_kernel, 1, 1, 0, st, sumsq, clip, out);
+  KB_CHECK_LAUNCH();
+}
+
 // ----------------------------------------------------------------------------- allocation-free RMSNorm backward
 // Declared in kareus_b200_noalloc.h.  Same kernels as kb_rmsnorm_bwd; the per-CTA partial sums of
 // the weight gradient live in a fixed device array instead of caller-provided scratch.

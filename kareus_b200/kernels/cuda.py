@@ -69,6 +69,7 @@ def _declare(L) -> None:
         "kb_ce_grad": [P, P, P, P, P, LNG, I, LNG, P],
         "kb_adamw": [P, P, P, P, P, LNG, F, F, F, F, F, F, F, P, F, P],
         "kb_sumsq": [P, LNG, I, P, P],
+        "kb_clip_scale": [P, F, P, P],
     }
     for name, args in sig.items():
         fn = getattr(L, name)
@@ -349,8 +350,17 @@ def add(a, b):
 
 # ----------------------------------------------------------------------------- GEMM
 def _rowmajor_ok(t: torch.Tensor) -> bool:
-    return t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 \
-        and t.stride(0) >= t.shape[1]
+    st = t.stride()
+    return len(st) == 2 and st[1] == 1 and st[0] % 8 == 0 and t.data_ptr() % 16 == 0 and st[0] >= t.shape[1]
+
+
+def _aligned_rows(t: torch.Tensor) -> torch.Tensor:
+    """A contiguous copy of a GEMM operand whose rows cannot be read where they lie."""
+    _no_recording("making a GEMM operand contiguous")
+    c = t.contiguous()
+    if not _rowmajor_ok(c):
+        raise KernelError(f"gemm operands need 16-byte aligned rows: {tuple(t.shape)}")
+    return c
 
 
 ACTIVATIONS = {None: 0, "none": 0, "gelu": 1}
@@ -377,15 +387,15 @@ def gemm(a, b, trans_a=False, trans_b=True, out_dtype=None, accumulate=None, out
             return out
         return r
     if not _rowmajor_ok(a):
-        _no_recording("making a GEMM operand contiguous")
-        a = a.contiguous()
+        a = _aligned_rows(a)
     if not _rowmajor_ok(b):
-        _no_recording("making a GEMM operand contiguous")
-        b = b.contiguous()
-    if not (_rowmajor_ok(a) and _rowmajor_ok(b)):
-        raise KernelError(f"gemm operands need 16-byte aligned rows: a{tuple(a.shape)} b{tuple(b.shape)}")
-    M, K = (a.shape[1], a.shape[0]) if trans_a else (a.shape[0], a.shape[1])
-    N, Kb = (b.shape[0], b.shape[1]) if trans_b else (b.shape[1], b.shape[0])
+        b = _aligned_rows(b)
+    M, K = a.shape
+    if trans_a:
+        M, K = K, M
+    N, Kb = b.shape
+    if not trans_b:
+        N, Kb = Kb, N
     if K != Kb:
         raise ValueError(f"gemm shape mismatch: K={K} vs {Kb}")
     if accumulate is not None:
@@ -620,3 +630,11 @@ def sumsq(t):
            "sumsq")
     _count()
     return out[0]
+
+
+def clip_scale(total, clip):
+    """Gradient norm (0-dim) and clipping factor (``[1]``) from the fp32 sum of squares ``total``, in one launch."""
+    out = torch.empty(2, dtype=torch.float32, device=total.device)
+    _check(lib().kb_clip_scale(total.data_ptr(), float(clip), out.data_ptr(), _stream()), "clip_scale")
+    _count()
+    return out[0], out[1:]

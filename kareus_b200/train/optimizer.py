@@ -105,8 +105,8 @@ class DistributedAdamW:
             self.grad_shard.copy_(self.grad_flat[self.lo:self.hi])
         return self.grad_shard
 
-    def _grad_norm(self, g: torch.Tensor) -> torch.Tensor:
-        """Global L2 norm: every element counted once across tp × pp × dp-shards."""
+    def _grad_sumsq(self, g: torch.Tensor) -> torch.Tensor:
+        """Sum of squares of this rank's share: every element counted once across tp × pp × dp-shards."""
         total = K.sumsq(g)
         if self.tp_rank != 0:
             a, b = max(self.replicated_start, self.lo), self.hi
@@ -116,7 +116,11 @@ class DistributedAdamW:
             a, b = max(a0, self.lo), min(b0, self.hi)
             if b > a:
                 total = total - K.sumsq(g[a - self.lo:b - self.lo] if self.dp > 1 else self.grad_flat[a:b])
-        total = total.reshape(1).clone()
+        return total
+
+    def _grad_norm(self, g: torch.Tensor) -> torch.Tensor:
+        """Global L2 norm."""
+        total = self._grad_sumsq(g).reshape(1).clone()
         if self.dp > 1:
             dist.all_reduce(total, group=self.dp_group)
         if self.mp_group is not None:
@@ -127,10 +131,16 @@ class DistributedAdamW:
         """Reduce, clip, update.  Returns the gradient norm as a device scalar (no host sync)."""
         cfg = self.cfg
         g = self._reduce_grads()
-        norm = self._grad_norm(g)
-        self.last_grad_norm = norm
         scale_t = None
-        if cfg.grad_clip and cfg.grad_clip > 0:
+        clip = bool(cfg.grad_clip and cfg.grad_clip > 0)
+        fused = clip and g.is_cuda and g.dtype == torch.float32 and self.dp == 1 and self.mp_group is None
+        if fused:          # no other rank's share: norm and clipping factor in one launch
+            from ..kernels import cuda as KC
+            norm, scale_t = KC.clip_scale(self._grad_sumsq(g), cfg.grad_clip)
+        else:
+            norm = self._grad_norm(g)
+        self.last_grad_norm = norm
+        if clip and not fused:
             scale_t = torch.clamp(cfg.grad_clip / (norm + 1e-6), max=1.0).to(torch.float32).reshape(1)
         self.step_count += 1
         lr = cosine_lr(self.step_count - 1, cfg) if lr is None else lr
