@@ -6,7 +6,7 @@
 // 64-deep K step that is 16 KB of A and at most 16 KB of B through L2 and shared memory for
 // 512 tensor clocks, half of the B traffic of a 128x256 tile on one SM, which leaves room in TMEM
 // for two accumulators (the epilogue of a tile runs under the main loop of the next) and in shared
-// memory for six stages.
+// memory for six stages, up to nine at narrower tiles.
 //
 //   warp 0      TMA producer of this CTA's halves (both CTAs count on the leader's `full` barriers)
 //   warp 1      MMA issuer (leader CTA only); allocates TMEM in both CTAs
@@ -31,13 +31,15 @@ namespace kb {
 
 constexpr int GP_BM = 256;                     // rows of a tile (128 per CTA)
 constexpr int GP_BK = 64;
-constexpr int GP_STAGES = 6;
+constexpr int GP_MAX_STAGES = 9;
 constexpr int GP_EPI_WARPS = 8;                // 4 TMEM lane quarters x 2 sets of column slabs
 constexpr int GP_THREADS = (2 + GP_EPI_WARPS) * 32;
 constexpr int GP_A_BYTES = 128 * GP_BK * 2;    // 16 KB: this CTA's rows of A
-constexpr int GP_B_BYTES = 128 * GP_BK * 2;    // 16 KB: room for this CTA's rows of B (BN / 2 of them)
-constexpr int GP_STAGE_BYTES = GP_A_BYTES + GP_B_BYTES;
-constexpr int GP_TILE_BYTES = GP_STAGE_BYTES * GP_STAGES;
+constexpr int GP_TILE_BYTES = 6 * (GP_A_BYTES + 128 * GP_BK * 2);   // ring: six stages at BN = 256, more at narrower tiles
+// This CTA's rows of B (BN / 2 of them); MN-major B comes in whole 64-wide chunks.
+__host__ __device__ constexpr int gp_b_bytes(int bn, bool b_mn) {
+  return b_mn ? ((bn / 2 + 63) / 64) * 64 * GP_BK * 2 : bn / 2 * GP_BK * 2;
+}
 constexpr int GP_STG_BYTES = GP_EPI_WARPS * 4096;
 constexpr int GP_SMEM = GP_TILE_BYTES + GP_STG_BYTES + 256 + 1024;
 static_assert(GP_SMEM <= 227 * 1024, "shared memory per CTA");
@@ -81,8 +83,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + GP_TILE_BYTES + GP_STG_BYTES);   // used in the leader
-  uint64_t* empty = full + GP_STAGES;
-  uint64_t* tfull = empty + GP_STAGES;      // [2]
+  uint64_t* empty = full + GP_MAX_STAGES;
+  uint64_t* tfull = empty + GP_MAX_STAGES;  // [2]
   uint64_t* tempty = tfull + 2;             // [2] used in the leader
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -92,9 +94,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
   const int num_units = w.units();
   const int half_n = bn >> 1;
+  // What a narrow tile waits for is latency times bytes in flight, so it gets all the stages that fit
+  const int b_bytes = gp_b_bytes(bn, B_MN), stage_bytes = GP_A_BYTES + b_bytes;
+  const int stages = min(GP_MAX_STAGES, GP_TILE_BYTES / stage_bytes);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < GP_STAGES; ++i) {
+    for (int i = 0; i < GP_MAX_STAGES; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
@@ -117,10 +122,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (elect_one()) {
       prefetch_tmap(&tmA);
       prefetch_tmap(&tmB);
-      // bytes of both CTAs, counted on the leader's barrier; MN-major B comes in whole 64-wide chunks
       const int b_chunks = (half_n + 63) >> 6;
-      const uint32_t b_bytes = B_MN ? b_chunks * 8192u : static_cast<uint32_t>(half_n) * GP_BK * 2u;
-      const uint32_t stage_tx = 2u * (GP_A_BYTES + b_bytes);
+      const uint32_t stage_tx = 2u * stage_bytes;     // bytes of both CTAs, counted on the leader's barrier
       const uint32_t full0 = cluster_addr(full, 0);
       int s = 0;
       uint32_t ph = 1;
@@ -132,7 +135,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int n0 = tn * bn + rank * half_n;
         for (int kb_ = kb0; kb_ < kb1; ++kb_) {
           if (!mbar_wait(&empty[s], ph, abort_flag, status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
-          uint8_t* a_dst = smem + s * GP_STAGE_BYTES;
+          uint8_t* a_dst = smem + s * stage_bytes;
           uint8_t* b_dst = a_dst + GP_A_BYTES;
           const uint32_t bar = full0 + s * 8;
           if (rank == 0) mbar_expect_tx(&full[s], stage_tx);
@@ -149,7 +152,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             tma_load_2d_pair(b_dst, &tmB, bar, n0, k0);
             if (b_chunks > 1) tma_load_2d_pair(b_dst + 8192, &tmB, bar, n0 + 64, k0);
           }
-          if (++s == GP_STAGES) { s = 0; ph ^= 1u; }
+          if (++s == stages) { s = 0; ph ^= 1u; }
         }
       }
       if (!ok) {
@@ -185,14 +188,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int kb_ = kb0; kb_ < kb1; ++kb_) {
           if (!mbar_wait(&full[s], ph, abort_flag, status, ST_TIMEOUT_FULL)) { ok = false; break; }
           tc_fence_after();
-          const uint64_t ad = ad0 + static_cast<uint64_t>(s * (GP_STAGE_BYTES >> 4));
-          const uint64_t bd = bd0 + static_cast<uint64_t>(s * (GP_STAGE_BYTES >> 4));
+          const uint64_t ad = ad0 + static_cast<uint64_t>(s * (stage_bytes >> 4));
+          const uint64_t bd = bd0 + static_cast<uint64_t>(s * (stage_bytes >> 4));
 #pragma unroll
           for (int k = 0; k < GP_BK / 16; ++k)
             umma_ss_pair(d_tmem, ad + k * ka, bd + k * kb, idesc, (kb_ > kb0 || k > 0) ? 1u : 0u);
           umma_commit_pair(&empty[s]);                              // both CTAs may refill the stage
           if (kb_ == kb1 - 1) umma_commit_pair(&tfull[buf]);        // both CTAs' halves are complete
-          if (++s == GP_STAGES) { s = 0; ph ^= 1u; }
+          if (++s == stages) { s = 0; ph ^= 1u; }
         }
       }
     }

@@ -369,10 +369,10 @@ static bool split_allowed() {
 
 // Modelled time of the two-SM kernel at tile width `bn`, in 64-deep K steps of a 256 x 256 tile.
 static PairPlan plan_pair_width(int M, int N, int K, int pairs, int bn, bool accumulate) {
-  // Measured per step: a step moves 16 KB of A and bn / 256 x 16 KB of B into each SM, which takes about 64 B per
-  // clock whatever the width, so narrow tiles are bound by that and not by the tensor pipe (16384 x 16384 x 3072,
-  // us per step: 0.381 at 256 columns, 0.312 at 192, 0.266 at 128, 0.229 at 64).
-  static const double step_cost[5] = {0, 0.60, 0.70, 0.82, 1.0};
+  // Measured per step: a step moves 16 KB of A and bn / 256 x 16 KB of B into each SM, so narrow tiles are bound by the
+  // bytes in flight and not by the tensor pipe (16384 x 6144 x 3072, us per step: 0.41 at 256 columns, 0.30 at 192, 0.23 at
+  // 128, 0.17 at 64; with six stages at every width 0.32, 0.24 and 0.175).
+  static const double step_cost[5] = {0, 0.45, 0.57, 0.75, 1.0};
   const int nk = (K + GEMM_BK - 1) / GEMM_BK;
   const double step = step_cost[bn / 64], fixed = 3.0;
   const long tiles = (long)((M + 255) / 256) * ((N + bn - 1) / bn);
