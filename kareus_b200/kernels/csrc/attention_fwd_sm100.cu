@@ -15,7 +15,8 @@
 // Why this split: with P in shared memory and one query tile per CTA a key tile costs the shared memory
 // pipe 64 KB of loads in, 32 KB of P in and 128 KB of operands out for 1024 tensor clocks; here it is
 // 32 + 0 + 96 KB.  The pace is then set by the exponentials (16 a clock and SM: 1024 clocks per tile and
-// head, as many as the two products need) and by how well two warps per scheduler cover each other.
+// head, as many as the two products need) and by how well two warps per scheduler cover each other.  One B200, 4 x 4096
+// tokens, 24 / 8 heads: 590 → 373 us (0.70 → 1.10 PFLOP/s); 4096 queries against 16 k keys, 6 heads: 300 → 222 us.
 //
 // Chunked keys (context parallelism without a gathered copy): the logical key sequence may be cut
 // into equal chunks that live in different buffers — each context-parallel rank's K/V shard inside
@@ -104,8 +105,9 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   // late query tiles see the most keys: they go first, over all heads and batches, so that the short ones fill the end
   const int n_qtiles = (p.sq + FA_BM - 1) / FA_BM;
-  const int qt0 = (static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y)) * p.tiles_per_cta;
-  const int batch = blockIdx.x / p.hq, head = blockIdx.x - batch * p.hq;
+  const int bh = static_cast<int>(blockIdx.x) % (p.hq * p.b), from_last = static_cast<int>(blockIdx.x) / (p.hq * p.b);
+  const int qt0 = ((n_qtiles - 1) / p.tiles_per_cta - from_last) * p.tiles_per_cta;
+  const int batch = bh / p.hq, head = bh - batch * p.hq;
   const int g = head / p.rep, r = head % p.rep;
   // query tile t of this CTA: first row, its absolute position minus the row, visible key tiles
   auto tile_q0 = [&](int t) { return (qt0 + t) * FA_BM; };
@@ -455,7 +457,7 @@ static int launch_fwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     if (attr.numRegs * FA_THREADS < FA_REGS_TOTAL) return ST_BAD_ARG;   // the register split would wait forever
     configured = true;
   }
-  dim3 grid(g * rep * b, (n_q + p.tiles_per_cta - 1) / p.tiles_per_cta);
+  const dim3 grid((unsigned)(g * rep * b) * ((n_q + p.tiles_per_cta - 1) / p.tiles_per_cta));
   KB_LAUNCH(flash_attn_fwd_kernel, grid, FA_THREADS, FaSmem::TOTAL, stream, tmQ, kv, tmO, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + (int)e;
