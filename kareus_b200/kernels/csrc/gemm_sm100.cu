@@ -67,10 +67,11 @@ __device__ __forceinline__ void apply_epilogue(uint32_t (&v)[32], const Epilogue
   }
 }
 
+// `vec_out`: base and rows of C are 16-byte aligned, so that the epilogue may use 16-byte accesses.
 template <int BN, bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 void* __restrict__ Cout, int M, int N, int K, int ldc, int group_m, int ks, int* status,
+                 void* __restrict__ Cout, int M, int N, int K, int ldc, bool vec_out, int group_m, int ks, int* status,
                  Epilogue ep) {
   using S = GemmSmem<BN>;
   extern __shared__ uint8_t smem_raw[];
@@ -206,7 +207,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         // bf16 output with 16-byte aligned rows: go through this warp's 4 KB of shared memory (32 rows
         // x 128 B, 16-byte units XOR-swizzled by row) so every store instruction writes four full
         // 128-byte row segments instead of 32 scattered 16-byte pieces
-        if ((ldc & 7) == 0 && (N & 7) == 0) {
+        if (vec_out && (N & 7) == 0) {
           uint8_t* stg = smem + S::TILE_BYTES + S::BAR_BYTES + q * 4096;
           __nv_bfloat16* cbase = reinterpret_cast<__nv_bfloat16*>(Cout) + static_cast<size_t>(m0 + q * 32) * ldc;
 #pragma unroll 1
@@ -256,7 +257,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (row < M && col < N) {
           if constexpr (OUT_F32) {
             float* crow = reinterpret_cast<float*>(Cout) + static_cast<size_t>(row) * ldc + col;
-            if (col + 32 <= N && (ldc & 3) == 0) {
+            if (col + 32 <= N && vec_out) {
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 float4 o = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
@@ -281,7 +282,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
           } else {
             __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + static_cast<size_t>(row) * ldc + col;
-            if (col + 32 <= N && (ldc & 7) == 0) {
+            if (col + 32 <= N && vec_out) {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 uint4 o;
@@ -312,6 +313,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 // ----------------------------------------------------------------------------- host side
+// Base and rows of an output that are 16-byte aligned.
+static bool aligned_rows(const void* C, int ldc, int out_f32) {
+  return (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc & (out_f32 ? 3 : 7)) == 0;
+}
+
 template <int BN, bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
 static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                        int num_sms, int ks, int* status, cudaStream_t stream, Epilogue ep) {
@@ -342,7 +348,8 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   int group_m = (int)((40L << 20) / (panel > 0 ? panel : 1));
   if (group_m < 4) group_m = 4;
   if (group_m > tiles_m) group_m = tiles_m;
-  KB_LAUNCH(kern, grid, GEMM_THREADS, smem, stream, tmA, tmB, C, M, N, K, ldc, group_m, ks, status, ep);
+  KB_LAUNCH(kern, grid, GEMM_THREADS, smem, stream, tmA, tmB, C, M, N, K, ldc, aligned_rows(C, ldc, OUT_F32), group_m, ks,
+            status, ep);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + static_cast<int>(e);
 }
@@ -441,8 +448,7 @@ extern "C" int kb_gemm_bias_act_bf16(const void* A, const void* B, void* C, int 
   if (num_sms <= 0) num_sms = device_sm_count();
   if (accumulate && !out_f32) return ST_BAD_ARG;
   // The two-SM kernel stores through TMA: 16-byte aligned output rows.
-  const bool tma_out = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldc & (out_f32 ? 3 : 7)) == 0;
-  if (plain && tma_out && num_sms >= 2 && !g_force_single) {
+  if (plain && aligned_rows(C, ldc, out_f32) && num_sms >= 2 && !g_force_single) {
     const int pairs = num_sms / 2;
     PairPlan pl = g_force_bn ? plan_pair_width(M, N, K, pairs, g_force_bn, accumulate != 0)
                              : plan_pair(M, N, K, pairs, accumulate != 0);

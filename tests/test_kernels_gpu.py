@@ -119,6 +119,37 @@ def test_gemm_sm_limit_and_views():
     assert _rel(got, view.float() @ w.float().t()) < 1e-2
 
 
+# rows whose length allows 16-byte stores and rows whose length does not, from an aligned base and from 1, 2 or 4 elements on
+@pytest.mark.parametrize("off", [0, 1, 2, 4])
+@pytest.mark.parametrize("M,N,K", [(130, 256, 200), (300, 328, 136), (129, 250, 72), (257, 33, 64)])
+def test_gemm_output_base_alignment(off, M, N, K):
+    KC = _K()
+    from kareus_b200.kernels import ref
+    g = torch.Generator(device="cuda").manual_seed(M + N + off)
+    a = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    w = torch.randn(N, K, device="cuda", generator=g).bfloat16()
+    bias = torch.randn(N, device="cuda", generator=g).bfloat16()
+    want = a.double() @ w.double().t()
+
+    def place(dtype):
+        buf = torch.full((M * N + off + 8,), 3.0, device="cuda", dtype=dtype)
+        return buf, buf[off:off + M * N].view(M, N)
+
+    # bf16 results within one rounding (2^-9 relative, as a norm), fp32 sums within fp32 accumulation of exact products
+    for dtype, tol in ((torch.bfloat16, 2 ** -8), (torch.float32, 1e-5)):
+        for kw, expect in (({}, want), ({"bias": bias, "activation": "gelu"}, ref.bias_act(want, bias.double(), "gelu"))):
+            buf, out = place(dtype)
+            KC.gemm(a, w, out=out, **kw)
+            KC.check_status()
+            assert _rel(out, expect.float()) < tol
+            assert (buf[:off] == 3).all() and (buf[off + M * N:] == 3).all()
+    buf, acc = place(torch.float32)
+    KC.gemm(a, w, accumulate=acc)
+    KC.check_status()
+    assert _rel(acc, (want + 3).float()) < 1e-5
+    assert (buf[:off] == 3).all() and (buf[off + M * N:] == 3).all()
+
+
 @pytest.mark.parametrize("rows,H", [(64, 3072), (1000, 512), (33, 8192), (257, 128), (16, 4096)])
 def test_rmsnorm(rows, H):
     KC = _K()
