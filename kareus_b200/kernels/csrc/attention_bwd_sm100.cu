@@ -510,10 +510,11 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 // Row statistics for the kernel above, one 1 KB block per query tile of one (batch, head): 128 x −lse·log2(e), then
 // 128 x −δ with δ = Σ_d dO·O (both [s,b,h,d] contiguous).  Rows past S get −inf and 0.  Half a warp per row, which also
 // zeroes its row of the dQ accumulator; `zero` (n_zero vectors) are the accumulators of dK and dV, if there are any.
+// dO is 16-byte aligned (TMA reads it too); O need not be (`wide` false: 8 bytes).
 __global__ void __launch_bounds__(256)
 attn_stats_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
                   const float* __restrict__ lse, float* __restrict__ stats, float4* __restrict__ dq_acc,
-                  float4* __restrict__ zero, long n_zero, unsigned S, unsigned S_pad, unsigned B, unsigned H) {
+                  float4* __restrict__ zero, long n_zero, unsigned S, unsigned S_pad, unsigned B, unsigned H, bool wide) {
   const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_zero;
        i += static_cast<long>(gridDim.x) * blockDim.x)
@@ -531,7 +532,14 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __r
       acc[0] = z;
       acc[16] = z;
       const uint4 a = reinterpret_cast<const uint4*>(dO + static_cast<size_t>(w) * FB_T)[l];
-      const uint4 b = reinterpret_cast<const uint4*>(O + static_cast<size_t>(w) * FB_T)[l];
+      const __nv_bfloat16* o = O + static_cast<size_t>(w) * FB_T + l * 8;
+      uint4 b;
+      if (wide) {
+        b = *reinterpret_cast<const uint4*>(o);
+      } else {
+        const uint2 b0 = reinterpret_cast<const uint2*>(o)[0], b1 = reinterpret_cast<const uint2*>(o)[1];
+        b = make_uint4(b0.x, b0.y, b1.x, b1.y);
+      }
       const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
       const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
 #pragma unroll
@@ -645,17 +653,20 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
   float* dk_acc = merged ? nullptr : stats + stats_floats(sq, b, hq);
   float* dv_acc = merged ? nullptr : dk_acc + n_dkv;
   cudaError_t e;
+  // refused before anything is launched: the statistics kernel reads dO 16 bytes at a time
+  CUtensorMap tmDO;
+  int rc = make_qkv_map(&tmDO, dO, d, 1, hq, b, sq, 0, d, (long)hq * d, (long)b * hq * d, 0);
+  if (rc) return rc;
+  if (reinterpret_cast<uintptr_t>(o) & 7) return ST_BAD_ARG;
   {
     const int s_pad = (sq + FB_T - 1) / FB_T * FB_T;
     const long rows = (long)s_pad * b * hq;
     long blocks = (rows * 16 + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
     KB_LAUNCH(attn_stats_kernel, (int)blocks, 256, 0, stream, (const __nv_bfloat16*)dO, (const __nv_bfloat16*)o, lse, stats,
-              reinterpret_cast<float4*>(dq_acc), reinterpret_cast<float4*>(dk_acc), merged ? 0L : 2 * n_dkv / 4, sq, s_pad, b, hq);
+              reinterpret_cast<float4*>(dq_acc), reinterpret_cast<float4*>(dk_acc), merged ? 0L : 2 * n_dkv / 4, sq, s_pad, b, hq,
+              (reinterpret_cast<uintptr_t>(o) & 15) == 0);
   }
-  CUtensorMap tmDO;
-  int rc = make_qkv_map(&tmDO, dO, d, 1, hq, b, sq, 0, d, (long)hq * d, (long)b * hq * d, 0);
-  if (rc) return rc;
   BwdParams p;
   p.stats = stats; p.dk_acc = dk_acc; p.dv_acc = dv_acc; p.heads = merged ? rep : 1; p.out = out;
   p.sq = sq; p.skv = skv; p.b = b; p.hq = hq; p.rep = rep; p.q_offset = q_offset; p.causal = causal;

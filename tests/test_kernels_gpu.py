@@ -391,6 +391,29 @@ def test_flash_attention_tile_pairs(sq, skv, b, g, rep, off, causal):
         assert dq.abs().max() < 0.5 and dk.abs().max() < 2.0
 
 
+def test_flash_attention_backward_output_alignment():
+    """The forward output may start on any 8-byte boundary; a gradient that TMA cannot read is refused."""
+    KC = _K()
+    from kareus_b200.kernels import attention_cuda
+    s, b, g, rep, d = 200, 2, 2, 2, 128
+    q = torch.randn(s, b, g, rep, d, device="cuda").bfloat16()
+    k, v = torch.randn(2, s, b, g, d, device="cuda").bfloat16()
+    out, lse = attention_cuda.forward(q, k, v, d ** -0.5)
+    do = torch.randn_like(out)
+    want = attention_cuda.backward(do, q, k, v, out, lse, d ** -0.5)
+    moved = torch.empty(out.numel() + 4, device="cuda", dtype=out.dtype)[4:].view(out.shape).copy_(out)
+    assert moved.data_ptr() % 16 == 8
+    got = attention_cuda.backward(do, q, k, v, moved, lse, d ** -0.5)
+    KC.check_status()
+    # the same operands; dQ, dK and dV are summed in fp32 in an order that may differ, then rounded once (2^-9)
+    for a, w in zip(got, want):
+        assert _rel(a, w) < 2 ** -8
+    do_moved = torch.empty(out.numel() + 4, device="cuda", dtype=out.dtype)[4:].view(out.shape).copy_(do)
+    with pytest.raises(KC.KernelError):
+        attention_cuda.backward(do_moved, q, k, v, out, lse, d ** -0.5)
+    assert torch.ones(4, device="cuda").sum().item() == 4
+
+
 def test_gelu_geglu_kernels():
     from kareus_b200.engine.context import OpContext
     from kareus_b200.ops.activations import GegluOp, GeluOp, gelu_grad_ref, gelu_ref
