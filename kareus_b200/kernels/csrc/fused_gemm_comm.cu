@@ -381,7 +381,7 @@ fused_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       int tm, tn;
       coords(t, tm, tn);
       const int m0 = tm * FG_BM, n0 = tn * BN;
-      if (!mbar_wait(&tfull[buf], bph, abort_flag, status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (!mbar_wait_warp(&tfull[buf], bph, abort_flag, status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + buf * BN + (static_cast<uint32_t>(q * 32) << 16);
       __nv_bfloat16* cbase;        // row 0 of this warp's 32 rows in the destination
@@ -389,7 +389,8 @@ fused_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       bool own_mc = false;         // ... in the multicast variant (summed fetch after the local store)
       if (p.mode == MODE_RS) {
         if (!go_seen) {
-          if (!wait_u32_ge(p.go, p.epoch, false, status, ST_TIMEOUT_PEER, abort_flag, c.wait_ns)) { ok = false; break; }
+          const bool go = wait_u32_ge(p.go, p.epoch, false, status, ST_TIMEOUT_PEER, abort_flag, c.wait_ns);
+          if (!__all_sync(0xffffffffu, go)) { ok = false; break; }
           go_seen = true;
         }
         const int owner = tm / tiles_per_rank;

@@ -213,7 +213,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int tm, tn, kb0, kb1;
       w.decode(u, tm, tn, kb0, kb1);
       const uint32_t buf = tile_i & 1u;
-      if (!mbar_wait(&tfull[buf], (tile_i >> 1) & 1u, abort_flag, status, ST_TIMEOUT_TMEM_FULL)) break;
+      if (!mbar_wait_warp(&tfull[buf], (tile_i >> 1) & 1u, abort_flag, status, ST_TIMEOUT_TMEM_FULL)) break;
       tc_fence_after();
       const int row0 = tm * GP_BM + rank * 128 + q * 32;
       const uint32_t taddr = tmem_base + buf * 256 + (static_cast<uint32_t>(q * 32) << 16);
