@@ -14,8 +14,9 @@
 //                  dPᵀ = V·dOᵀ,  dV += Pᵀ·dO,  Sᵀ(i+1) = K·Qᵀ,  dQ = dS·K,  dK += dSᵀ·Q
 // The order is what makes it a pipeline: Pᵀ(i+1) is computed under dQ and dK of tile i, dSᵀ under dV and the next
 // scores, and dQ of tile i leaves TMEM under dK.  dSᵀ is stored once ([key][query], queries contiguous) and serves
-// as K-major operand (dK) and, through an MN-major descriptor, as transposed operand of dQ.  The softmax scale is
-// applied to dQ and dK once, where they leave, and not to every element of dS.
+// as K-major operand (dK) and, through an MN-major descriptor, as transposed operand of dQ.  The softmax scale goes into dS
+// before its rounding to bf16 (δ comes scaled, the scale of dPᵀ rides on the subtraction): it is not a power of two, so that
+// rounding first and scaling dQ and dK where they leave would round other values (0.3 % of the gradients as a norm).
 // TMEM: Sᵀ|Pᵀ + dPᵀ|dQ + dV + dK = 512 columns.  dK/dV stay in TMEM across the whole walk.
 // A CTA walks all query heads of its KV group one after the other and writes dK and dV itself.  Where that leaves
 // SMs idle (merge_heads), every query head gets its own CTA and dK/dV are added up in fp32 accumulators.  Starting
@@ -50,7 +51,7 @@ constexpr int FB_THREADS = (FB_SOFTMAX_WARPS + 8) * 32;   // six warpgroups; the
 // Registers a thread: what the block is launched with, and after the dQ warps have taken some from the last warpgroup
 constexpr int FB_REGS = 80, FB_REGS_DQ = 120, FB_REGS_AUX = 40;
 static_assert(FB_REGS_DQ + FB_REGS_AUX <= 2 * FB_REGS, "the shares must not exceed the registers at launch");
-constexpr int FB_STATS = 2 * FB_T;               // floats of row statistics per query tile: −lse·log2(e), then −δ
+constexpr int FB_STATS = 2 * FB_T;               // floats of row statistics per query tile: −lse·log2(e), then −δ·scale
 
 // Destinations, strides in elements.
 struct RowMap {
@@ -293,7 +294,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const int frag_row = (warp & 3) * 32 + (lane >> 2), frag_col = 2 * (lane & 3);
     // the row of dSᵀ whose address this thread gives to the matrix stores (two 64-wide swizzled chunks per row)
     const uint32_t ds_row = smem_u32(smem) + FbSmem::DS_OFF + (c >> 1) * FB_CHUNK + ((warp & 3) * 32 + lane) * 128;
-    const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
+    const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), scale2 = make_float2(p.scale, p.scale);
     bool ok = true;
     int it = -1;
     QTiles tiles(p, n_q, k0, head0);
@@ -362,8 +363,8 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
           const float2 e = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[h >> 1][2 * n + (h & 1)]));
-          const float2 d = __fmul2_rn(e, __fadd2_rn(make_float2(__uint_as_float(dv[h >> 1][4 * n + 2 * (h & 1)]),
-                                                                __uint_as_float(dv[h >> 1][4 * n + 2 * (h & 1) + 1])), nd));
+          const float2 d = __fmul2_rn(e, __ffma2_rn(make_float2(__uint_as_float(dv[h >> 1][4 * n + 2 * (h & 1)]),
+                                                                __uint_as_float(dv[h >> 1][4 * n + 2 * (h & 1) + 1])), scale2, nd));
           w[h] = pack_bf16x2(d.x, d.y);
         }
         stmatrix_x4(ds_row + ((((c & 1) * 4 + n) ^ (lane & 7)) << 4), w);
@@ -388,15 +389,14 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll 1
       for (int which = 0; which < 2 && n_it > 0; ++which) {
         float* dst = (which == 0 ? p.dv_acc : p.dk_acc) + base + c * 32;
-        const float f = which == 0 ? 1.f : p.scale;
         uint32_t v[32];
         tmem_ld_32x32((which == 0 ? t_dv : t_dk) + lane_addr + c * 32, v);
         tmem_ld_wait();
         if (kvalid) {
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            red_add_v4(dst + 4 * j, __uint_as_float(v[4 * j]) * f, __uint_as_float(v[4 * j + 1]) * f,
-                       __uint_as_float(v[4 * j + 2]) * f, __uint_as_float(v[4 * j + 3]) * f);
+            red_add_v4(dst + 4 * j, __uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]),
+                       __uint_as_float(v[4 * j + 3]));
         }
       }
     } else {
@@ -407,7 +407,6 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       uint8_t* stg = smem + FbSmem::Q_OFF;
 #pragma unroll 1
       for (int which = 0; which < 2; ++which) {
-        const float f = which == 0 ? 1.f : p.scale;
         uint32_t v[32];
         if (n_it > 0) {
           tmem_ld_32x32((which == 0 ? t_dv : t_dk) + lane_addr + c * 32, v);
@@ -419,10 +418,10 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const uint32_t dst = smem_u32(stg) + which * FB_T * PITCH + row * PITCH + c * 64;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          st_shared_v4(dst + j * 16, pack_bf16x2(__uint_as_float(v[8 * j]) * f, __uint_as_float(v[8 * j + 1]) * f),
-                       pack_bf16x2(__uint_as_float(v[8 * j + 2]) * f, __uint_as_float(v[8 * j + 3]) * f),
-                       pack_bf16x2(__uint_as_float(v[8 * j + 4]) * f, __uint_as_float(v[8 * j + 5]) * f),
-                       pack_bf16x2(__uint_as_float(v[8 * j + 6]) * f, __uint_as_float(v[8 * j + 7]) * f));
+          st_shared_v4(dst + j * 16, pack_bf16x2(__uint_as_float(v[8 * j]), __uint_as_float(v[8 * j + 1])),
+                       pack_bf16x2(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3])),
+                       pack_bf16x2(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5])),
+                       pack_bf16x2(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7])));
       }
       asm volatile("bar.sync 1, %0;" ::"n"(FB_SOFTMAX_WARPS * 32) : "memory");
       if (ok) {
@@ -508,13 +507,14 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 }
 
 // Row statistics for the kernel above, one 1 KB block per query tile of one (batch, head): 128 x −lse·log2(e), then
-// 128 x −δ with δ = Σ_d dO·O (both [s,b,h,d] contiguous).  Rows past S get −inf and 0.  Half a warp per row, which also
+// 128 x −δ·scale with δ = Σ_d dO·O (both [s,b,h,d] contiguous).  Rows past S get −inf and 0.  Half a warp per row, which also
 // zeroes its row of the dQ accumulator; `zero` (n_zero vectors) are the accumulators of dK and dV, if there are any.
 // dO is 16-byte aligned (TMA reads it too); O need not be (`wide` false: 8 bytes).
 __global__ void __launch_bounds__(256)
 attn_stats_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
                   const float* __restrict__ lse, float* __restrict__ stats, float4* __restrict__ dq_acc,
-                  float4* __restrict__ zero, long n_zero, unsigned S, unsigned S_pad, unsigned B, unsigned H, bool wide) {
+                  float4* __restrict__ zero, long n_zero, unsigned S, unsigned S_pad, unsigned B, unsigned H, float scale,
+                  bool wide) {
   const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_zero;
        i += static_cast<long>(gridDim.x) * blockDim.x)
@@ -554,19 +554,18 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __r
       const long bh = static_cast<long>(bb) * H + h;
       float* t = stats + (bh * (S_pad / FB_T) + ss / FB_T) * FB_STATS + ss % FB_T;
       t[0] = ss < S ? lse[bh * S + ss] * -1.4426950408889634f : -INFINITY;
-      t[FB_T] = -s;
+      t[FB_T] = -s * scale;
     }
   }
 }
 
-// fp32 accumulator [rows(s,b), heads, d] times `scale` → bf16 strided view (strides in elements per s, b, group, head
+// fp32 accumulator [rows(s,b), heads, d] → bf16 strided view (strides in elements per s, b, group, head
 // of the group); `rows_of` moves chunks of s (dK/dV straight into the layout a reduce-scatter expects).
 struct Convert {
   const float* acc;
   __nv_bfloat16* out;
   unsigned rows, G, R;
   long st_s, st_b, st_g, st_r;
-  float scale;
   bool wide;                  // the view is aligned to 16 bytes
   RowMap rows_of;
 };
@@ -584,10 +583,10 @@ attn_convert_kernel(const __grid_constant__ Convert dq, const __grid_constant__ 
     const unsigned t = w / c.R, rr = w - t * c.R, u = t / c.G, gg = t - u * c.G, ss = u / B, bb = u - ss * B;
     __nv_bfloat16* o = c.out + c.rows_of.at(ss) * c.st_s + bb * c.st_b + gg * c.st_g + rr * c.st_r + l * 8;
     uint4 v;
-    v.x = pack_bf16x2(a.x * c.scale, a.y * c.scale);
-    v.y = pack_bf16x2(a.z * c.scale, a.w * c.scale);
-    v.z = pack_bf16x2(b.x * c.scale, b.y * c.scale);
-    v.w = pack_bf16x2(b.z * c.scale, b.w * c.scale);
+    v.x = pack_bf16x2(a.x, a.y);
+    v.y = pack_bf16x2(a.z, a.w);
+    v.z = pack_bf16x2(b.x, b.y);
+    v.w = pack_bf16x2(b.z, b.w);
     if (c.wide) {
       *reinterpret_cast<uint4*>(o) = v;
     } else {
@@ -664,7 +663,7 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     long blocks = (rows * 16 + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
     KB_LAUNCH(attn_stats_kernel, (int)blocks, 256, 0, stream, (const __nv_bfloat16*)dO, (const __nv_bfloat16*)o, lse, stats,
-              reinterpret_cast<float4*>(dq_acc), reinterpret_cast<float4*>(dk_acc), merged ? 0L : 2 * n_dkv / 4, sq, s_pad, b, hq,
+              reinterpret_cast<float4*>(dq_acc), reinterpret_cast<float4*>(dk_acc), merged ? 0L : 2 * n_dkv / 4, sq, s_pad, b, hq, scale,
               (reinterpret_cast<uintptr_t>(o) & 15) == 0);
   }
   BwdParams p;
@@ -701,17 +700,17 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     KB_LAUNCH(flash_attn_bwd_kernel, grid, FB_THREADS, FbSmem::TOTAL, stream, tmQ, kv, tmDO, tmDQ, p);
   }
   {
-    auto segment = [&](const float* acc, void* dst, long rows, int r, long st_s, long st_b, long st_g, long st_r, float f,
+    auto segment = [&](const float* acc, void* dst, long rows, int r, long st_s, long st_b, long st_g, long st_r,
                        const RowMap& map) {
       const bool wide = ((reinterpret_cast<uintptr_t>(dst) | ((st_s | st_b | st_g | st_r) * 2)) & 15) == 0;
-      return Convert{acc, (__nv_bfloat16*)dst, (unsigned)rows, (unsigned)g, (unsigned)r, st_s, st_b, st_g, st_r, f, wide, map};
+      return Convert{acc, (__nv_bfloat16*)dst, (unsigned)rows, (unsigned)g, (unsigned)r, st_s, st_b, st_g, st_r, wide, map};
     };
     const long kv_rows = merged ? 0 : (long)skv * b * g;
     RowMap plain;
     plain.chunk_rows = 0;
-    const Convert cq = segment(dq_acc, out.dq, (long)sq * b * hq, rep, out.dqs_s, out.dqs_b, out.dqs_g, out.dqs_r, scale, plain);
-    const Convert ck = segment(dk_acc, out.dk, kv_rows, 1, out.dks_s, out.dks_b, out.dks_g, 0, 1.f, out.dk_rows);
-    const Convert cv = segment(dv_acc, out.dv, kv_rows, 1, out.dvs_s, out.dvs_b, out.dvs_g, 0, 1.f, out.dv_rows);
+    const Convert cq = segment(dq_acc, out.dq, (long)sq * b * hq, rep, out.dqs_s, out.dqs_b, out.dqs_g, out.dqs_r, plain);
+    const Convert ck = segment(dk_acc, out.dk, kv_rows, 1, out.dks_s, out.dks_b, out.dks_g, 0, out.dk_rows);
+    const Convert cv = segment(dv_acc, out.dv, kv_rows, 1, out.dvs_s, out.dvs_b, out.dvs_g, 0, out.dv_rows);
     const long blocks = (((long)sq * b * hq + 2 * kv_rows) * 16 + 255) / 256;
     KB_LAUNCH(attn_convert_kernel, (int)blocks, 256, 0, stream, cq, ck, cv, (unsigned)b);
   }

@@ -391,6 +391,32 @@ def test_flash_attention_tile_pairs(sq, skv, b, g, rep, off, causal):
         assert dq.abs().max() < 0.5 and dk.abs().max() < 2.0
 
 
+@pytest.mark.parametrize("s,b,g,rep", [(459, 2, 2, 2), (640, 8, 4, 3)])
+def test_flash_attention_backward_rounds_scaled_ds(s, b, g, rep):
+    """dS carries the softmax scale (not a power of two) when it is rounded to bf16.  The same roundings in fp64: what is left
+    is P and dS that fall on the other side of a rounding because of fp32 (1e-6 of the exponent, so about one in 2000) and the
+    final rounding of sums that differ by that (one in 40, 2^-8 each): 6e-4 as a norm.  Rounding dS before the scale is 3e-3 away."""
+    KC = _K()
+    from kareus_b200.kernels import attention_cuda
+    d = 128
+    scale = d ** -0.5
+    gen = torch.Generator(device="cuda").manual_seed(s)
+    rnd = lambda *sh: torch.randn(*sh, device="cuda", generator=gen).bfloat16()
+    q, k, v, do = rnd(s, b, g, rep, d), rnd(s, b, g, d), rnd(s, b, g, d), rnd(s, b, g * rep, d)
+    out, lse = attention_cuda.forward(q, k, v, scale)
+    dq, dk, dv = attention_cuda.backward(do, q, k, v, out, lse, scale)
+    KC.check_status()
+    q6, k6, v6, do6, o6 = (t.double() for t in (q, k, v, do.view(q.shape), out.view(q.shape)))
+    hidden = torch.ones(s, s, device="cuda", dtype=torch.bool).triu(1)
+    p = (torch.einsum("sbgrd,tbgd->bgrst", q6, k6) * scale - lse.double().view(b, g, rep, s, 1)).exp().masked_fill(hidden, 0)
+    p = p.bfloat16().double()
+    ds = p * (torch.einsum("sbgrd,tbgd->bgrst", do6, v6) - torch.einsum("sbgrd,sbgrd->bgrs", do6, o6)[..., None]) * scale
+    ds = ds.bfloat16().double()
+    assert _rel(dq, torch.einsum("bgrst,tbgd->sbgrd", ds, k6).bfloat16()) < 1.2e-3
+    assert _rel(dk, torch.einsum("bgrst,sbgrd->tbgd", ds, q6).bfloat16()) < 1.2e-3
+    assert _rel(dv, torch.einsum("bgrst,sbgrd->tbgd", p, do6).bfloat16()) < 1.2e-3
+
+
 def test_flash_attention_backward_output_alignment():
     """The forward output may start on any 8-byte boundary; a gradient that TMA cannot read is refused."""
     KC = _K()
