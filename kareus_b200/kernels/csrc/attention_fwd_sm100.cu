@@ -8,6 +8,8 @@
 //   warp 8      TMA producer: both Q tiles once, then K and V tiles through a ring of five 32 KB stages
 //   warp 9      MMA issuer (warps 10 and 11 fill its warpgroup): S = Q·Kᵀ (both operands from shared memory) and O += P·V (P from TMEM)
 // The two query tiles alternate: while one is in its softmax the tensor cores work on the other.
+// Where single query tiles already fit the chip in one wave, a CTA has one (its share is half as long) and the two softmax
+// warpgroups take its even and odd key tiles, each with its own scores, O, maximum and sum; they meet in the epilogue.
 // TMEM: S|P and O of both tiles, 4 x 128 columns.  S of the next key tile is issued behind the P·V that
 // read P, so its arrival also says that O may be touched; O is rescaled only when the running maximum
 // moves by more than 2^8 ("lazy rescale"), which happens on the first tiles only.
@@ -45,6 +47,7 @@ constexpr int FA_THREADS = 12 * 32;   // three warpgroups: the register split be
 constexpr int FA_REGS_SOFTMAX = 208, FA_REGS_AUX = 80;   // a row of scores lives in registers
 constexpr int FA_REGS_TOTAL = 256 * FA_REGS_SOFTMAX + 128 * FA_REGS_AUX;   // must not exceed registers at launch x threads
 constexpr int FA_STAGES = 5;    // K and V tiles alternate in one ring
+constexpr int FA_STAGES_SINGLE = 6;   // with one query tile: the place of the second is one more stage
 constexpr int FA_TILE_BYTES = FA_BN * FA_D * 2;   // 32 KB: two 64-wide swizzled chunks of 16 KB
 constexpr int FA_CHUNK = 16384;
 
@@ -71,7 +74,6 @@ struct FwdParams {
   int q_offset;         // absolute position of query row 0 relative to key 0
   float scale_log2;     // softmax scale * log2(e)
   int causal;
-  int tiles_per_cta;    // query tiles of a CTA: 2, or 1 where that leaves SMs idle
   int* status;
   ChunkGeom geom;       // chunk tables (all zero: one K/V buffer, one query chunk at q_offset)
 };
@@ -84,6 +86,8 @@ struct FaSmem {
   static_assert(TOTAL <= 227 * 1024, "shared memory per CTA");
 };
 
+// `single`: a CTA has one query tile and warpgroup t takes its key tiles t, t + 2, ...; else warpgroup t has query tile t.
+template <bool single>
 __global__ void __launch_bounds__(FA_THREADS, 1)
 flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ KvMaps kv,
                       const __grid_constant__ CUtensorMap tmO, const FwdParams p) {
@@ -91,13 +95,13 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FaSmem::BAR_OFF);
   uint64_t* q_full = bars + 0;     // [2] per query tile
-  uint64_t* full = bars + 2;       // [FA_STAGES] K(j) is in stage 2j, V(j) in stage 2j + 1 (modulo the ring)
-  uint64_t* empty = bars + 7;      // [FA_STAGES]
-  uint64_t* s_full = bars + 12;    // [2] scores are in TMEM (and the tile's previous P·V has retired)
-  uint64_t* p_most = bars + 14;    // [2] P of the first 96 keys is in TMEM (one arrival per warp)
-  uint64_t* p_rest = bars + 16;    // [2] P of the last 32 keys
-  uint64_t* o_full = bars + 18;    // [2] the tile's last P·V has retired
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+  uint64_t* full = bars + 2;       // [stages] K(j) is in stage 2j, V(j) in stage 2j + 1 (modulo the ring)
+  uint64_t* empty = bars + 8;      // [stages]
+  uint64_t* s_full = bars + 14;    // [2] scores are in TMEM (and the tile's previous P·V has retired)
+  uint64_t* p_most = bars + 16;    // [2] P of the first 96 keys is in TMEM (one arrival per warp)
+  uint64_t* p_rest = bars + 18;    // [2] P of the last 32 keys
+  uint64_t* o_full = bars + 20;    // [2] the tile's last P·V has retired
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -106,22 +110,26 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   // late query tiles see the most keys: they go first, over all heads and batches, so that the short ones fill the end
   const int n_qtiles = (p.sq + FA_BM - 1) / FA_BM;
   const int bh = static_cast<int>(blockIdx.x) % (p.hq * p.b), from_last = static_cast<int>(blockIdx.x) / (p.hq * p.b);
-  const int qt0 = ((n_qtiles - 1) / p.tiles_per_cta - from_last) * p.tiles_per_cta;
+  constexpr int tiles_per_cta = single ? 1 : 2;
+  const int qt0 = ((n_qtiles - 1) / tiles_per_cta - from_last) * tiles_per_cta;
   const int batch = bh / p.hq, head = bh - batch * p.hq;
   const int g = head / p.rep, r = head % p.rep;
-  // query tile t of this CTA: first row, its absolute position minus the row, visible key tiles
-  auto tile_q0 = [&](int t) { return (qt0 + t) * FA_BM; };
-  auto tile_valid = [&](int t) { return t < p.tiles_per_cta && qt0 + t < n_qtiles; };
+  constexpr int stages = single ? FA_STAGES_SINGLE : FA_STAGES;
+  constexpr int kv_off = single ? FaSmem::KV_OFF - FA_TILE_BYTES : FaSmem::KV_OFF;
+  // warpgroup t: first query row, are there such rows, key tiles that it walks
+  auto tile_q0 = [&](int t) { return (single ? qt0 : qt0 + t) * FA_BM; };
+  auto tile_valid = [&](int t) { return single || qt0 + t < n_qtiles; };
   auto tile_nkv = [&](int t) {
     if (!tile_valid(t)) return 0;
     const int q0 = tile_q0(t);
     int kv_end = p.skv;    // keys visible to the tile: [0, kv_end)
     if (p.causal) kv_end = min(p.skv, p.geom.q_offset_of(q0, p.q_offset) + min(q0 + FA_BM, p.sq));
-    return kv_end > 0 ? (kv_end + FA_BN - 1) / FA_BN : 0;
+    const int n = kv_end > 0 ? (kv_end + FA_BN - 1) / FA_BN : 0;
+    return single ? (n + 1 - t) >> 1 : n;
   };
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < FA_STAGES; ++i) {
+    for (int i = 0; i < FA_STAGES_SINGLE; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
@@ -145,7 +153,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     regs_dec<FA_REGS_AUX>();
     if (warp == 8) {
       // ------------------------------------------------------------------ producer
-      const int n0 = tile_nkv(0), n1 = tile_nkv(1), n = max(n0, n1);
+      const int n0 = tile_nkv(0), n1 = tile_nkv(1), n = single ? n0 + n1 : max(n0, n1);
       if (n > 0 && elect_one()) {
         prefetch_tmap(&tmQ);
         prefetch_tmap(&kv.k[0]);
@@ -155,11 +163,11 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         uint32_t ph = 1;
         auto load = [&](const CUtensorMap* map, int srow) {
           if (!mbar_wait(&empty[st], ph, abort_flag, p.status, ST_TIMEOUT_EMPTY)) { okp = false; return; }
-          uint8_t* d = smem + FaSmem::KV_OFF + st * FA_TILE_BYTES;
+          uint8_t* d = smem + kv_off + st * FA_TILE_BYTES;
           mbar_expect_tx(&full[st], FA_TILE_BYTES);
           tma_load_4d(d, map, &full[st], 0, g, batch, srow);
           tma_load_4d(d + FA_CHUNK, map, &full[st], 64, g, batch, srow);
-          if (++st == FA_STAGES) { st = 0; ph ^= 1u; }
+          if (++st == stages) { st = 0; ph ^= 1u; }
         };
         auto load_q = [&](int t) {
           uint8_t* d = smem + FaSmem::Q_OFF + t * FA_TILE_BYTES;
@@ -172,7 +180,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           int src, srow;
           p.geom.locate(j * FA_BN, src, srow);
           load(&kv.k[src], srow);
-          if (j == 0 && n1 > 0) load_q(1);
+          if (j == 0 && n1 > 0 && !single) load_q(1);
           if (okp) load(&kv.v[src], srow);
         }
         if (*abort_flag) {
@@ -183,21 +191,22 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       __syncwarp();
     } else if (warp == 9) {
       // ------------------------------------------------------------------ MMA issuer
-      const int n0 = tile_nkv(0), n1 = tile_nkv(1), n = max(n0, n1);
+      const int n0 = tile_nkv(0), n1 = tile_nkv(1), n = single ? n0 + n1 : max(n0, n1);
       if (n > 0 && elect_one()) {             // one thread runs the whole role, see elect_one()
         constexpr uint32_t idesc_s = make_idesc_bf16(FA_BM, FA_BN, false, false);  // Q K-major, K K-major
         constexpr uint32_t idesc_o = make_idesc_bf16(FA_BM, FA_D, false, true);    // P (TMEM), V MN-major
         const uint32_t smem0 = smem_u32(smem);
         const uint64_t qd0 = make_smem_desc(smem0 + FaSmem::Q_OFF, 16, 1024);
-        const uint64_t kd0 = make_smem_desc(smem0 + FaSmem::KV_OFF, 16, 1024);
-        const uint64_t vd0 = make_smem_desc(smem0 + FaSmem::KV_OFF, FA_CHUNK, 1024);
+        const uint64_t kd0 = make_smem_desc(smem0 + kv_off, 16, 1024);
+        const uint64_t vd0 = make_smem_desc(smem0 + kv_off, FA_CHUNK, 1024);
         bool ok = true;
         auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
           if (ok) ok = mbar_wait(bar, parity, abort_flag, p.status, code);
           return ok;
         };
-        auto issue_s = [&](int t, int ks) {
-          const uint64_t qd = qd0 + static_cast<uint64_t>(t * (FA_TILE_BYTES >> 4));
+        // scores of warpgroup t from query tile `qt` and the K in stage ks
+        auto issue_s = [&](int t, int qt, int ks) {
+          const uint64_t qd = qd0 + static_cast<uint64_t>(qt * (FA_TILE_BYTES >> 4));
           const uint64_t kd = kd0 + static_cast<uint64_t>(ks * (FA_TILE_BYTES >> 4));
           const uint32_t d = tmem_base + t * 128;
 #pragma unroll
@@ -207,51 +216,80 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
           umma_commit(&s_full[t]);
         };
-        int ks = 0;                                // stage of K(j) / K(j+1), its phase
-        uint32_t kph = 0;
-        if (wait(&full[0], 0, ST_TIMEOUT_FULL)) {
-#pragma unroll
-          for (int t = 0; t < 2; ++t)
-            if ((t ? n1 : n0) > 0 && wait(&q_full[t], 0, ST_TIMEOUT_FULL)) {
-              tc_fence_after();
-              issue_s(t, 0);
-            }
-          if (ok) umma_commit(&empty[0]);
-        }
-        for (int j = 0; j < n && ok; ++j) {
-          int vs = ks + 1;
-          uint32_t vph = kph;
-          if (vs == FA_STAGES) { vs = 0; vph ^= 1u; }
-          ks = vs + 1;
-          kph = vph;
-          if (ks == FA_STAGES) { ks = 0; kph ^= 1u; }
-          if (!wait(&full[vs], vph, ST_TIMEOUT_FULL)) break;
+        // O of warpgroup t += P · (V in stage vs), for its i-th key tile
+        auto issue_pv = [&](int t, int vs, int i) {
           const uint64_t vd = vd0 + static_cast<uint64_t>(vs * (FA_TILE_BYTES >> 4));
+          const uint32_t d = tmem_base + 256 + t * 128, a = tmem_base + t * 128;
+          if (!wait(&p_most[t], i & 1u, ST_TIMEOUT_TMEM_FULL)) return;
+          tc_fence_after();
 #pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const int nt = t ? n1 : n0;
-            if (j >= nt || !ok) continue;
-            const uint32_t d = tmem_base + 256 + t * 128, a = tmem_base + t * 128;
-            if (!wait(&p_most[t], j & 1u, ST_TIMEOUT_TMEM_FULL)) continue;
+          for (int k = 0; k < 6; ++k)            // 16 keys: 8 columns of P, 16 rows of V
+            umma_ts(d, a + k * 8, vd + k * (2048 >> 4), idesc_o, (i > 0 || k > 0) ? 1u : 0u);
+          if (!wait(&p_rest[t], i & 1u, ST_TIMEOUT_TMEM_FULL)) return;
+          tc_fence_after();
+#pragma unroll
+          for (int k = 6; k < 8; ++k) umma_ts(d, a + k * 8, vd + k * (2048 >> 4), idesc_o, 1u);
+        };
+        if constexpr (single) {
+          // scores of key tile j; they overwrite P of tile j - 2: the products before them read it in order
+          auto scores = [&](int j) {
+            const int x = 2 * j, st = x % FA_STAGES_SINGLE;
+            if (!wait(&full[st], (x / FA_STAGES_SINGLE) & 1u, ST_TIMEOUT_FULL)) return;
             tc_fence_after();
-#pragma unroll
-            for (int k = 0; k < 6; ++k)            // 16 keys: 8 columns of P, 16 rows of V
-              umma_ts(d, a + k * 8, vd + k * (2048 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-            if (!wait(&p_rest[t], j & 1u, ST_TIMEOUT_TMEM_FULL)) continue;
-            tc_fence_after();
-#pragma unroll
-            for (int k = 6; k < 8; ++k) umma_ts(d, a + k * 8, vd + k * (2048 >> 4), idesc_o, 1u);
-            if (j + 1 < nt) {
-              if (!wait(&full[ks], kph, ST_TIMEOUT_FULL)) continue;
-              tc_fence_after();
-              issue_s(t, ks);                      // overwrites P: the products before it read it in order
-            } else {
-              umma_commit(&o_full[t]);
-            }
+            issue_s(j & 1, 0, st);
+            umma_commit(&empty[st]);
+          };
+          if (wait(&q_full[0], 0, ST_TIMEOUT_FULL)) {
+            scores(0);
+            if (n > 1) scores(1);
           }
-          if (!ok) break;
-          umma_commit(&empty[vs]);
-          if (j + 1 < n) umma_commit(&empty[ks]);
+          for (int j = 0; j < n && ok; ++j) {
+            const int x = 2 * j + 1, st = x % FA_STAGES_SINGLE;
+            if (!wait(&full[st], (x / FA_STAGES_SINGLE) & 1u, ST_TIMEOUT_FULL)) break;
+            issue_pv(j & 1, st, j >> 1);
+            if (!ok) break;
+            umma_commit(&empty[st]);
+            if (j + 2 < n) scores(j + 2);
+            else umma_commit(&o_full[j & 1]);
+          }
+        } else {
+          int ks = 0;                                // stage of K(j) / K(j+1), its phase
+          uint32_t kph = 0;
+          if (wait(&full[0], 0, ST_TIMEOUT_FULL)) {
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+              if ((t ? n1 : n0) > 0 && wait(&q_full[t], 0, ST_TIMEOUT_FULL)) {
+                tc_fence_after();
+                issue_s(t, t, 0);
+              }
+            if (ok) umma_commit(&empty[0]);
+          }
+          for (int j = 0; j < n && ok; ++j) {
+            int vs = ks + 1;
+            uint32_t vph = kph;
+            if (vs == FA_STAGES) { vs = 0; vph ^= 1u; }
+            ks = vs + 1;
+            kph = vph;
+            if (ks == FA_STAGES) { ks = 0; kph ^= 1u; }
+            if (!wait(&full[vs], vph, ST_TIMEOUT_FULL)) break;
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+              const int nt = t ? n1 : n0;
+              if (j >= nt || !ok) continue;
+              issue_pv(t, vs, j);
+              if (!ok) continue;
+              if (j + 1 < nt) {
+                if (!wait(&full[ks], kph, ST_TIMEOUT_FULL)) continue;
+                tc_fence_after();
+                issue_s(t, t, ks);                   // overwrites P: the products before it read it in order
+              } else {
+                umma_commit(&o_full[t]);
+              }
+            }
+            if (!ok) break;
+            umma_commit(&empty[vs]);
+            if (j + 1 < n) umma_commit(&empty[ks]);
+          }
         }
       }
       __syncwarp();
@@ -259,7 +297,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   } else {
     regs_inc<FA_REGS_SOFTMAX>();
     // ------------------------------------------------------------------ softmax + epilogue
-    const int t = warp >> 2;                       // query tile
+    const int t = warp >> 2;                       // query tile, or share of the key tiles of the one
     const int row = (warp & 3) * 32 + lane;        // row inside the tile = TMEM lane
     const int n_kv = tile_nkv(t);
     const int q0 = tile_q0(t);
@@ -270,16 +308,17 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const uint32_t all = 0xffffffffu;
     float m_ref = -INFINITY;   // reference maximum (scaled, log2 domain) used for the exponentials
     float l_sum = 0.f;
+    const int key_first = single ? t * FA_BN : 0, key_step = single ? 2 * FA_BN : FA_BN;
     bool ok = true;            // warp-uniform
     for (int j = 0; j < n_kv; ++j) {
-      ok = __all_sync(all, mbar_wait(&s_full[t], j & 1u, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL));
+      ok = mbar_wait_warp(&s_full[t], j & 1u, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
       if (!ok) break;
       tc_fence_after();
       uint32_t v[4][32];
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_s + c * 32, v[c]);
       tmem_ld_wait();
-      const int key0 = j * FA_BN;
+      const int key0 = key_first + j * key_step;
       // warp-uniform: does any row of this tile need masking?
       if ((p.causal && key0 + FA_BN - 1 > q_off + q0) || (key0 + FA_BN > p.skv)) {
         // keys at or above `lim` (relative to this tile) are hidden from this row
@@ -343,48 +382,94 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
       l_sum = l_sum * rescale + ((ps2[0].x + ps2[0].y) + (ps2[1].x + ps2[1].y));
     }
-    // ---- epilogue: O / l through this tile's Q buffer (the warp's 32 rows) and a TMA store; LSE
-    if (tile_valid(t)) {
-      float* lse = p.lse + (static_cast<size_t>(batch) * p.hq + head) * p.sq;
-      if (n_kv > 0) {
-        if (ok) ok = __all_sync(all, mbar_wait(&o_full[t], 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL));
-        if (ok) {
-          tc_fence_after();
-          const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
-          // two 64-wide halves of 32 rows x 128 bytes, 16-byte units swizzled by row as the tensor map expects
-          uint8_t* stg = smem + FaSmem::Q_OFF + t * FA_TILE_BYTES + (warp & 3) * 8192;
-          const uint32_t stg_row = smem_u32(stg) + lane * 128;
+    // ---- epilogue: O / l through the query tile's Q buffer (the warp's 32 rows) and a TMA store; LSE
+    float* lse = p.lse + (static_cast<size_t>(batch) * p.hq + head) * p.sq;
+    // two 64-wide halves of 32 rows x 128 bytes, 16-byte units swizzled by row as the tensor map expects
+    uint8_t* stg = smem + FaSmem::Q_OFF + (single ? 0 : t) * FA_TILE_BYTES + (warp & 3) * 8192;
+    const int row0 = q0 + (warp & 3) * 32;
+    auto stage32 = [&](int c, const uint32_t (&o)[32], float f) {     // columns 32c.. of this thread's row, times f
+      const uint32_t stg_row = smem_u32(stg) + lane * 128;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t o[32];
-            tmem_ld_32x32(t_o + c * 32, o);
-            tmem_ld_wait();
+      for (int u = 0; u < 4; ++u) {
+        uint32_t w[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              uint32_t w[4];
-#pragma unroll
-              for (int h = 0; h < 4; ++h)
-                w[h] = pack_bf16x2(__uint_as_float(o[8 * u + 2 * h]) * inv, __uint_as_float(o[8 * u + 2 * h + 1]) * inv);
-              const int unit = (c & 1) * 4 + u;
-              st_shared_v4(stg_row + (c >> 1) * 4096 + ((unit ^ (lane & 7)) << 4), w[0], w[1], w[2], w[3]);
-            }
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          const int row0 = q0 + (warp & 3) * 32;
-          if (lane == 0 && row0 < p.sq) {              // the tensor map clips rows past sq
-            tma_store_4d(&tmO, stg, 0, head, batch, row0);
-            tma_store_4d(&tmO, stg + 4096, 64, head, batch, row0);
-            tma_store_commit();
-          }
-          if (qrow < p.sq) lse[qrow] = (l_sum > 0.f) ? (m_ref + log2f(l_sum)) * 0.6931471805599453f : -INFINITY;
-          if (lane == 0) tma_store_wait<0>();          // nothing in flight out of shared memory at exit
-        }
-      } else if (qrow < p.sq) {
-        // no visible key at all (only possible with a negative q_offset): zero output
+        for (int h = 0; h < 4; ++h)
+          w[h] = pack_bf16x2(__uint_as_float(o[8 * u + 2 * h]) * f, __uint_as_float(o[8 * u + 2 * h + 1]) * f);
+        const int unit = (c & 1) * 4 + u;
+        st_shared_v4(stg_row + (c >> 1) * 4096 + ((unit ^ (lane & 7)) << 4), w[0], w[1], w[2], w[3]);
+      }
+    };
+    auto put_lse = [&](float m, float l) {
+      if (qrow < p.sq) lse[qrow] = (l > 0.f) ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
+    };
+    if (tile_valid(t) && (single ? tile_nkv(0) : n_kv) == 0) {
+      // no visible key at all (only possible with a negative q_offset): zero output
+      if (qrow < p.sq && !(single && t)) {
         uint4* orow = reinterpret_cast<uint4*>(p.out + ((static_cast<size_t>(qrow) * p.b + batch) * p.hq + head) * FA_D);
         for (int i = 0; i < FA_D / 8; ++i) orow[i] = make_uint4(0, 0, 0, 0);
         lse[qrow] = -INFINITY;
+      }
+    } else if constexpr (single) {
+      // Both warpgroups put their maximum and sum where the key tiles were (all products have retired) and each writes
+      // half of the columns of O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / l.  A warp whose waits failed comes to the
+      // barrier as well; the abort flag, set by then, keeps all of them from storing.
+      for (int h = 0; h < 2; ++h)
+        if (ok && tile_nkv(h) > 0) ok = mbar_wait_warp(&o_full[h], 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
+      tc_fence_after();
+      float2* stat = reinterpret_cast<float2*>(smem + kv_off);           // [2][128]
+      stat[t * FA_BM + row] = make_float2(m_ref, l_sum);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      ok = __all_sync(all, ok && *abort_flag == 0);
+      if (ok) {
+        const float2 s0 = stat[row], s1 = stat[FA_BM + row];
+        const float m = fmaxf(s0.x, s1.x);
+        // a share without visible keys has l = 0 and an O that was never written; a NaN sum stays visible
+        const bool use0 = s0.y != 0.f, use1 = s1.y != 0.f;
+        const float f0 = s0.x == m ? 1.f : fast_exp2(s0.x - m), f1 = s1.x == m ? 1.f : fast_exp2(s1.x - m);
+        const float l = (use0 ? s0.y * f0 : 0.f) + (use1 ? s1.y * f1 : 0.f);
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+#pragma unroll 1
+        for (int c2 = 0; c2 < 2; ++c2) {
+          const int c = 2 * t + c2;
+          uint32_t o0[32], o1[32];
+          tmem_ld_32x32(tmem_base + 256 + lane_addr + c * 32, o0);
+          tmem_ld_32x32(tmem_base + 384 + lane_addr + c * 32, o1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            o0[i] = __float_as_uint((use0 ? __uint_as_float(o0[i]) * f0 : 0.f) + (use1 ? __uint_as_float(o1[i]) * f1 : 0.f));
+          stage32(c, o0, inv);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && row0 < p.sq) {                // the tensor map clips rows past sq
+          tma_store_4d(&tmO, stg + t * 4096, 64 * t, head, batch, row0);
+          tma_store_commit();
+        }
+        if (t == 0) put_lse(m, l);
+        if (lane == 0) tma_store_wait<0>();            // nothing in flight out of shared memory at exit
+      }
+    } else if (n_kv > 0) {
+      if (ok) ok = mbar_wait_warp(&o_full[t], 0, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL);
+      if (ok) {
+        tc_fence_after();
+        const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t o[32];
+          tmem_ld_32x32(t_o + c * 32, o);
+          tmem_ld_wait();
+          stage32(c, o, inv);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && row0 < p.sq) {                // the tensor map clips rows past sq
+          tma_store_4d(&tmO, stg, 0, head, batch, row0);
+          tma_store_4d(&tmO, stg + 4096, 64, head, batch, row0);
+          tma_store_commit();
+        }
+        put_lse(m_ref, l_sum);
+        if (lane == 0) tma_store_wait<0>();            // nothing in flight out of shared memory at exit
       }
     }
     __syncwarp();
@@ -420,6 +505,25 @@ static int make_kv_map(CUtensorMap* m, const void* ptr, int d, int g, int b, int
   return make_tmap(m, ptr, 2, 4, dims, str, box, 3);
 }
 
+template <bool single>
+static int launch_variant(const CUtensorMap& tmQ, const KvMaps& kv, const CUtensorMap& tmO, const FwdParams& p, int ctas,
+                          cudaStream_t stream) {
+  auto kern = flash_attn_fwd_kernel<single>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FaSmem::TOTAL);
+    if (e != cudaSuccess) return 1000 + (int)e;
+    cudaFuncAttributes attr;
+    e = cudaFuncGetAttributes(&attr, kern);
+    if (e != cudaSuccess) return 1000 + (int)e;
+    if (attr.numRegs * FA_THREADS < FA_REGS_TOTAL) return ST_BAD_ARG;   // the register split would wait forever
+    configured = true;
+  }
+  KB_LAUNCH(kern, (unsigned)ctas, FA_THREADS, FaSmem::TOTAL, stream, tmQ, kv, tmO, p);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 2000 + (int)e;
+}
+
 static int launch_fwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom& geom, void* out, float* lse, int sq,
                       int skv, int b, int g, int rep, float scale, int causal, int q_offset, int* status,
                       cudaStream_t stream) {
@@ -432,10 +536,6 @@ static int launch_fwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
   p.causal = causal;
   p.status = status;
   p.geom = geom;
-  // Pairs of query tiles halve the K/V traffic and keep the tensor cores busy during a softmax; where single
-  // tiles already fit the chip in one wave, they halve the work of the longest CTA instead.
-  const int n_q = (sq + FA_BM - 1) / FA_BM;
-  p.tiles_per_cta = (long)n_q * g * rep * b <= device_sm_count() ? 1 : 2;
   CUtensorMap tmO;
   {
     // [sq, b, hq, d]: boxes of 32 rows x 64 columns of one (batch, head)
@@ -446,21 +546,11 @@ static int launch_fwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     const int rc = make_tmap(&tmO, out, 2, 4, dims, str, box, 3);
     if (rc) return rc;
   }
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(flash_attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         FaSmem::TOTAL);
-    if (e != cudaSuccess) return 1000 + (int)e;
-    cudaFuncAttributes attr;
-    e = cudaFuncGetAttributes(&attr, flash_attn_fwd_kernel);
-    if (e != cudaSuccess) return 1000 + (int)e;
-    if (attr.numRegs * FA_THREADS < FA_REGS_TOTAL) return ST_BAD_ARG;   // the register split would wait forever
-    configured = true;
-  }
-  const dim3 grid((unsigned)(g * rep * b) * ((n_q + p.tiles_per_cta - 1) / p.tiles_per_cta));
-  KB_LAUNCH(flash_attn_fwd_kernel, grid, FA_THREADS, FaSmem::TOTAL, stream, tmQ, kv, tmO, p);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : 2000 + (int)e;
+  // Pairs of query tiles halve the K/V traffic; where single tiles already fit the chip in one wave, they halve the
+  // work of the longest CTA instead.
+  const int n_q = (sq + FA_BM - 1) / FA_BM, bh = g * rep * b;
+  if ((long)n_q * bh <= device_sm_count()) return launch_variant<true>(tmQ, kv, tmO, p, bh * n_q, stream);
+  return launch_variant<false>(tmQ, kv, tmO, p, bh * ((n_q + 1) / 2), stream);
 }
 
 }  // namespace kb

@@ -440,6 +440,34 @@ def test_flash_attention_backward_output_alignment():
     assert torch.ones(4, device="cuda").sum().item() == 4
 
 
+# one query tile per CTA, whose even and odd key tiles go to different warps: one, two, three and many key tiles, shares of
+# unequal length, a share whose keys are all hidden from some rows, query tiles that see nothing, no causal mask
+@pytest.mark.parametrize("sq,skv,b,g,rep,off,causal",
+                         [(1, 1, 1, 1, 1, 0, True), (128, 128, 2, 1, 2, 0, True), (129, 129, 1, 2, 3, 0, True),
+                          (77, 260, 2, 1, 1, 183, True), (130, 384, 1, 1, 2, 254, True), (256, 512, 1, 2, 2, 127, True),
+                          (200, 1500, 1, 1, 4, 1300, True), (384, 300, 1, 1, 2, -200, True), (100, 385, 3, 1, 2, 0, False),
+                          (1111, 1111, 1, 2, 2, 0, True)])
+def test_flash_attention_shared_query_tile(sq, skv, b, g, rep, off, causal):
+    assert (sq + 127) // 128 * b * g * rep <= _K().sm_count()
+    test_flash_attention_tile_pairs(sq, skv, b, g, rep, off, causal)
+
+
+def test_flash_attention_shared_query_tile_keeps_nan():
+    """A NaN score reaches its row's output whichever share of the keys it lies in, and no other row."""
+    KC = _K()
+    from kareus_b200.kernels import attention_cuda
+    s, d = 300, 128
+    q, v = torch.randn(s, 1, 1, 1, d, device="cuda").bfloat16(), torch.randn(s, 1, 1, d, device="cuda").bfloat16()
+    k = torch.randn(s, 1, 1, d, device="cuda").bfloat16()
+    for row in (0, 130, 299):
+        bad = q.clone()
+        bad[row, ..., 5] = float("nan")
+        out, _ = attention_cuda.forward(bad, k, v, d ** -0.5)
+        KC.check_status()
+        nan = out.isnan().all(-1).flatten()
+        assert nan[row] and nan.sum() == 1 and out.isnan().sum() == d
+
+
 def test_gelu_geglu_kernels():
     from kareus_b200.engine.context import OpContext
     from kareus_b200.ops.activations import GegluOp, GeluOp, gelu_grad_ref, gelu_ref
