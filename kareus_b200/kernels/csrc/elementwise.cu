@@ -629,7 +629,6 @@ embedding_bwd_kernel(const long* __restrict__ tokens, const __nv_bfloat16* __res
 // What bounds both passes is arithmetic as much as memory: the exponentials alone take 117 us for 4096 x 128256 at 1.9 GHz,
 // reading the logits once 158 us.  Hence maxima on bf16 pairs and paired fp32 operations around the exponential.
 constexpr int CE_THREADS = 512;
-constexpr int CE_UNROLL = 2;        // vectors a thread requests at once
 // exp(x - base) of the eight elements of a vector, in pairs
 __device__ __forceinline__ void exp_pairs(const uint4& u, float base, float2 (&e)[4]) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
@@ -650,16 +649,16 @@ ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restrict
     const __nv_bfloat16* lr = logits + row * V;
     const uint4* l4 = reinterpret_cast<const uint4*>(lr);
     float m = -INFINITY, s = 0.f;
-    for (int c0 = threadIdx.x; c0 < vv; c0 += CE_UNROLL * CE_THREADS) {
-      uint4 u[CE_UNROLL];
-#pragma unroll
-      for (int k = 0; k < CE_UNROLL; ++k)
-        u[k] = c0 + k * CE_THREADS < vv ? l4[c0 + k * CE_THREADS]
-                                        : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf
+    for (int c0 = threadIdx.x; c0 < vv; c0 += 2 * CE_THREADS) {
+      const bool two = c0 + CE_THREADS < vv;
+      uint4 u[2];
+      u[0] = l4[c0];
+      if (two) u[1] = l4[c0 + CE_THREADS];
       // the maximum of the pairs as they are (exact)
       __nv_bfloat162 m2 = __floats2bfloat162_rn(m, m);
 #pragma unroll
-      for (int k = 0; k < CE_UNROLL; ++k) {
+      for (int k = 0; k < 2; ++k) {
+        if (k == 1 && !two) break;
         const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u[k]);
         m2 = __hmax2(m2, __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
       }
@@ -667,7 +666,8 @@ ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restrict
       const float base = nm == -INFINITY ? 0.f : nm;
       float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int k = 0; k < CE_UNROLL; ++k) {
+      for (int k = 0; k < 2; ++k) {
+        if (k == 1 && !two) break;       // rows of up to 4096 elements have no second vector: its exponentials cost 17 %
         float2 e[4];
         exp_pairs(u[k], base, e);
         acc = __fadd2_rn(acc, __fadd2_rn(__fadd2_rn(e[0], e[1]), __fadd2_rn(e[2], e[3])));
