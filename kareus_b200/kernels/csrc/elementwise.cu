@@ -896,9 +896,9 @@ using namespace kb;
 
 extern "C" int kb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int rows, int H, float eps,
                               cudaStream_t st) {
-  if (H % 8 == 0 && H >= 512 && H <= 4096 && rows >= 148 * 40) {
+  if (H % 8 == 0 && H >= 512 && H <= 3072 && rows >= 148 * 40) {
     // a warp per row pays once most warp slots have a row (8997 x 2048: 14 us, 16.5 with a CTA per row; 3800 x 2048: 10.7
-    // and 9.1)
+    // and 9.1), and while two CTAs fit an SM: 16 vectors a lane take 151 registers (16384 x 4096: 68 us, 44 with a CTA per row)
     const int grid = grid_for(rows, 8, 148 * 8);
     const int vpl = (H / 8 + 31) / 32;
 #define KB_ROWS(V_)                                                                                               \
@@ -906,8 +906,7 @@ extern "C" int kb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd
               (__nv_bfloat16*)y, rstd, rows, H, eps)
     if (vpl <= 4) KB_ROWS(4);
     else if (vpl <= 8) KB_ROWS(8);
-    else if (vpl <= 12) KB_ROWS(12);
-    else KB_ROWS(16);
+    else KB_ROWS(12);
 #undef KB_ROWS
   } else if (H % 8 == 0 && H >= 512) {
     const NormVariant nv = norm_variant(H);
