@@ -644,9 +644,10 @@ __global__ void __launch_bounds__(CE_THREADS)
 ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restrict__ targets, float* __restrict__ omax,
                 float* __restrict__ osum, float* __restrict__ otgt, long rows, int V, long vocab_start) {
   __shared__ float red[32];
-  const int vv = V >> 3;
   for (long row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* lr = logits + row * V;
+    // rows of a vocabulary that is no multiple of 8 start on any boundary: those off 16 bytes go element by element
+    const int vv = reinterpret_cast<uintptr_t>(lr) & 15 ? 0 : V >> 3;
     const uint4* l4 = reinterpret_cast<const uint4*>(lr);
     float m = -INFINITY, s = 0.f;
     for (int c0 = threadIdx.x; c0 < vv; c0 += 2 * CE_THREADS) {
@@ -697,9 +698,9 @@ ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restrict
 __global__ void __launch_bounds__(CE_THREADS)
 ce_grad_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ targets, const float* __restrict__ gmax,
                const float* __restrict__ gsum, const float* __restrict__ scale, long rows, int V, long vocab_start) {
-  const int vv = V >> 3;
   for (long row = blockIdx.x; row < rows; row += gridDim.x) {
     __nv_bfloat16* lr = logits + row * V;
+    const int vv = reinterpret_cast<uintptr_t>(lr) & 15 ? 0 : V >> 3;
     uint4* l4 = reinterpret_cast<uint4*>(lr);
     const float m = gmax[row], inv = 1.f / gsum[row], sc = scale[row];
     const long t = targets[row] - vocab_start;

@@ -606,7 +606,8 @@ def test_rmsnorm_heads_views(s, b, g, rep, d):
         assert _rel(y.reshape(-1, d), want) < 3e-3 and _rel(rstd, rstd_w) < 1e-5
 
 
-@pytest.mark.parametrize("rows,V", [(3, 8), (5, 16376), (2, 16384), (4, 16392), (3, 50264), (2, 4096), (3, 4000), (2, 4104)])
+@pytest.mark.parametrize("rows,V", [(3, 8), (5, 16376), (2, 16384), (4, 16392), (3, 50264), (2, 4096), (3, 4000), (2, 4104),
+                                    (9, 50257), (9, 1003), (3, 5)])
 def test_cross_entropy_vector_groups(rows, V):
     """Rows around multiples of the two vectors a thread takes at once, with hidden logits."""
     KC = _K()
