@@ -90,7 +90,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int num_tiles = tiles_m * tiles_n;
   const int nk = (K + GEMM_BK - 1) / GEMM_BK;
   // split-K (accumulating outputs only): unit u = (tile u / ks, K part u % ks); every part adds its
-  // partial sum to C with vector reductions, so parts of one tile may run on different SMs at once
+  // partial sum to C with reductions, so parts of one tile may run on different SMs at once
   const int num_units = num_tiles * ks;
   constexpr uint32_t TMEM_COLS = (2 * BN <= 32) ? 32 : 2 * BN;
 
@@ -199,6 +199,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tile_coords(u / ks, tiles_m, tiles_n, group_m, tm, tn);
       const int m0 = tm * GEMM_BM;
       const int n0 = tn * BN;
+      uint8_t* stg = smem + S::TILE_BYTES + S::BAR_BYTES + q * 4096;     // this warp's staging
       if (!mbar_wait_warp(&tfull[buf], bph, abort_flag, status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const int row = m0 + q * 32 + lane;
@@ -208,7 +209,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         // x 128 B, 16-byte units XOR-swizzled by row) so every store instruction writes four full
         // 128-byte row segments instead of 32 scattered 16-byte pieces
         if (vec_out && (N & 7) == 0) {
-          uint8_t* stg = smem + S::TILE_BYTES + S::BAR_BYTES + q * 4096;
           __nv_bfloat16* cbase = reinterpret_cast<__nv_bfloat16*>(Cout) + static_cast<size_t>(m0 + q * 32) * ldc;
 #pragma unroll 1
           for (int cp = 0; cp < BN / 64; ++cp) {
@@ -254,31 +254,50 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tmem_ld_wait();
         const int col = n0 + c * 32;
         if constexpr (!ACCUM) apply_epilogue(v, ep, col, N);
-        if (row < M && col < N) {
+        if (OUT_F32 && !(col + 32 <= N && vec_out)) {
+          // rows that are not 16-byte aligned, or the edge: through the staging buffer (columns XOR-swizzled by row), so
+          // that an access takes 32 neighbouring columns of a row and not one column of 32 rows (4096 x 50257 x 3072: fp32
+          // 2.03 -> 1.23 ms, with accumulation 5.46 -> 1.54 ms)
+          float* st = reinterpret_cast<float*>(stg);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) st[lane * 32 + (j ^ lane)] = __uint_as_float(v[j]);
+          __syncwarp();
+          const int rows = min(32, M - (m0 + q * 32));
+          if (col + lane < N) {
+            float* cc = reinterpret_cast<float*>(Cout) + static_cast<size_t>(m0 + q * 32) * ldc + col + lane;
+#pragma unroll 1
+            for (int r0 = 0; r0 < rows; r0 += 8, cc += 8L * ldc) {
+              float old[8];
+              if (ACCUM && ks == 1) {
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                  if (r0 + r < rows) old[r] = cc[static_cast<long>(r) * ldc];
+              }
+#pragma unroll
+              for (int r = 0; r < 8; ++r) {
+                if (r0 + r >= rows) break;
+                const float o = st[(r0 + r) * 32 + (lane ^ (r0 + r))];
+                float* p = cc + static_cast<long>(r) * ldc;
+                if (ACCUM && ks > 1) atomicAdd(p, o);
+                else *p = ACCUM ? old[r] + o : o;
+              }
+            }
+          }
+          __syncwarp();
+        } else if (row < M && col < N) {
           if constexpr (OUT_F32) {
             float* crow = reinterpret_cast<float*>(Cout) + static_cast<size_t>(row) * ldc + col;
-            if (col + 32 <= N && vec_out) {
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                float4 o = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                                       __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
-                float4* p = reinterpret_cast<float4*>(crow) + j;
-                if constexpr (ACCUM) {
-                  if (ks > 1) { red_add_f32x4(p, o); continue; }
-                  float4 old = *p;
-                  o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-                }
-                *p = o;
+            for (int j = 0; j < 8; ++j) {
+              float4 o = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                     __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+              float4* p = reinterpret_cast<float4*>(crow) + j;
+              if constexpr (ACCUM) {
+                if (ks > 1) { red_add_f32x4(p, o); continue; }
+                float4 old = *p;
+                o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
               }
-            } else {
-              for (int j = 0; j < 32 && col + j < N; ++j) {
-                float o = __uint_as_float(v[j]);
-                if constexpr (ACCUM) {
-                  if (ks > 1) { atomicAdd(crow + j, o); continue; }
-                  o += crow[j];
-                }
-                crow[j] = o;
-              }
+              *p = o;
             }
           } else {
             __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + static_cast<size_t>(row) * ldc + col;
@@ -395,6 +414,26 @@ static PairPlan plan_pair_width(int M, int N, int K, int pairs, int bn, bool acc
   return best;
 }
 
+// K split of the one-SM kernel, which accumulating outputs take whose rows TMA cannot store: modelled time in 64-deep K
+// steps of a 128 x 256 tile (0.6 of it at 128 columns), with 14 + 2 ks steps of fill and epilogue a unit (weight gradients
+// of a 3B layer at tensor-parallel sizes 1, 2 and 8).  1000 x 1001 over 8192 tokens: 165 us in one part, 34 in the picked
+// number; 640 x 3070 over 16384: 217 and 64.
+static int split_single(int M, int N, int K, int num_sms, bool narrow) {
+  const int nk = (K + GEMM_BK - 1) / GEMM_BK, bn = narrow ? 128 : 256;
+  const long tiles = (long)((M + GEMM_BM - 1) / GEMM_BM) * ((N + bn - 1) / bn);
+  auto time = [&](int ks) {
+    return (tiles * ks + num_sms - 1) / num_sms * ((nk + ks - 1) / ks * (narrow ? 0.6 : 1.0) + 14.0 + 2.0 * ks);
+  };
+  int best = 1;
+  if (split_allowed())
+    for (int ks = 2; ks <= 8 && nk / ks >= 8; ++ks)
+      if (time(ks) < 0.97 * time(best)) best = ks;
+  return best;
+}
+
+// Narrow outputs waste less of the last wave with the 128-wide tile of the one-SM kernel.
+static bool narrow_single(int N) { return N <= 128 || (N % 256 != 0 && N % 256 <= 128); }
+
 static PairPlan plan_pair(int M, int N, int K, int pairs, bool accumulate) {
   PairPlan best = plan_pair_width(M, N, K, pairs, 256, accumulate);
   for (int bn = 192; bn >= 64; bn -= 64) {
@@ -459,10 +498,9 @@ extern "C" int kb_gemm_bias_act_bf16(const void* A, const void* B, void* C, int 
     }
     return gemm_pair_dispatch(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, pl, pairs, status, stream);
   }
-  int ks = 1;
+  const bool narrow = g_force_single ? g_force_single == 128 : narrow_single(N);
+  int ks = accumulate ? split_single(M, N, K, num_sms, narrow) : 1;
   if (g_force_ks > 0 && accumulate) ks = g_force_ks <= (K + GEMM_BK - 1) / GEMM_BK ? g_force_ks : (K + GEMM_BK - 1) / GEMM_BK;
-  // narrow outputs waste less of the last wave with the 128-wide tile
-  const bool narrow = g_force_single ? g_force_single == 128 : (N <= 128) || (N % 256 != 0 && N % 256 <= 128);
 #define KB_GO(BN_)                                                                                         \
   do {                                                                                                     \
     if (!a_mn && !b_mn) return dispatch_out<BN_, false, false>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, accumulate, num_sms, ks, status, stream, ep); \

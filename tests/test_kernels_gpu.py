@@ -105,6 +105,24 @@ def test_weight_gradient_split_k(tile, ks, n_out, n_in, tokens):
     assert _rel(acc, want) < 2e-3
 
 
+@pytest.mark.parametrize("n_out,n_in,tokens", [(640, 1026, 4096), (1000, 1001, 2048), (136, 33, 3000), (264, 130, 520), (2000, 4099, 700)])
+def test_weight_gradient_odd_rows(n_out, n_in, tokens):
+    """Gradients whose rows TMA cannot store, at the edges of 32-column groups and 128-row tiles, with and without a K split."""
+    KC = _K()
+    g = torch.Generator(device="cuda").manual_seed(n_in)
+    dy = torch.randn(tokens, n_out, device="cuda", generator=g).bfloat16()
+    x = torch.randn(tokens, (n_in + 7) // 8 * 8, device="cuda", generator=g).bfloat16()[:, :n_in]
+    want = dy.double().t() @ x.double()
+    buf = torch.full((n_out * n_in + 64,), 2.0, device="cuda")
+    acc = buf[:n_out * n_in].view(n_out, n_in)
+    KC.gemm(dy, x, trans_a=True, trans_b=False, accumulate=acc)
+    f = KC.gemm(dy, x, trans_a=True, trans_b=False, out_dtype=torch.float32)
+    KC.check_status()
+    # fp32 sums of exact bf16 products
+    assert _rel(acc, (want + 2).float()) < 1e-5 and _rel(f, want.float()) < 1e-5
+    assert (buf[n_out * n_in:] == 2).all()
+
+
 def test_gemm_sm_limit_and_views():
     KC = _K()
     a = torch.randn(512, 1024, device="cuda").bfloat16()
