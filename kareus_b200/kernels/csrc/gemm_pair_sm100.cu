@@ -12,7 +12,11 @@
 //   warp 1      MMA issuer (leader CTA only); allocates TMEM in both CTAs
 //   warps 2..9  epilogue: TMEM → registers → 4 KB of swizzled shared memory per warp → TMA store
 //               (bf16 / fp32 output) or TMA reduce-add (fp32 `C +=`: the addition happens in L2, so
-//               nobody waits for the old value and several K parts of a tile may add at once)
+//               nobody waits for the old value)
+//
+// K parts of a tile (`C +=` only).  Ordered: the first part adds to C, the others store their sums to a workspace, which a
+// second small kernel adds part by part, so that every run gives the same bits.  Not ordered: all parts add in L2 as they
+// come; this is for outputs of few tiles, where the second launch would cost a third of the time (see gemm_sm100.cu).
 //
 // BN is a run-time multiple of 64 (64..256): the launcher picks the width whose last wave is fullest.
 // Loads use no multicast: every CTA fetches its own halves.
@@ -49,7 +53,10 @@ static_assert(GP_SMEM <= 227 * 1024, "shared memory per CTA");
 // clusters that run side by side walk the same K range of neighbouring tiles and share operands in L2.
 struct PairWork {
   int tiles_m, tiles_n, group_m, nk, whole, split_tiles, ks;
+  bool ordered;
   __device__ __forceinline__ int units() const { return whole + split_tiles * ks; }
+  // slab of the workspace (256 x bn floats) that unit u stores to, negative if it goes to C
+  __device__ __forceinline__ int slab(int u) const { return ordered ? u - whole - split_tiles : -1; }
   __device__ __forceinline__ void decode(int u, int& tm, int& tn, int& kb0, int& kb1) const {
     int t;
     if (u < whole) {
@@ -63,6 +70,9 @@ struct PairWork {
       kb0 = split_begin(nk, ks, part);
       kb1 = split_begin(nk, ks, part + 1);
     }
+    coords(t, tm, tn);
+  }
+  __device__ __forceinline__ void coords(int t, int& tm, int& tn) const {
     // m-tiles are taken in groups of `group_m`; inside a group the m index runs fastest, so the tiles in
     // flight cover a near-square patch of C
     const int per_group = group_m * tiles_n;
@@ -78,8 +88,8 @@ struct PairWork {
 template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmC, const PairWork w, const int M, const int N, const int bn,
-                 int* status) {
+                 const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmW, const PairWork w,
+                 const int M, const int N, const int bn, int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + GP_TILE_BYTES + GP_STG_BYTES);   // used in the leader
@@ -249,7 +259,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         __syncwarp();
         const int col = tn * bn + c * SLAB;
         if (lane == 0 && row0 < M && col < N) {       // the tensor map clips what crosses the edge
-          if constexpr (ACCUM) tma_reduce_add_2d(&tmC, stg, col, row0);
+          if (ACCUM && w.slab(u) >= 0) tma_store_2d(&tmW, stg, c * SLAB, w.slab(u) * GP_BM + rank * 128 + q * 32);
+          else if constexpr (ACCUM) tma_reduce_add_2d(&tmC, stg, col, row0);
           else tma_store_2d(&tmC, stg, col, row0);
           tma_store_commit();
         }
@@ -272,10 +283,40 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
+// C += the sums that K parts 1 .. ks - 1 of the split tiles left in the workspace, part by part: four columns a thread.
+__global__ void __launch_bounds__(256)
+gemm_add_parts_kernel(float* __restrict__ C, int ldc, int M, int N, const float* __restrict__ work, const PairWork w, int bn) {
+  const int vecs = bn >> 2, per_tile = GP_BM * vecs, total = w.split_tiles * per_tile;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int tile = i / per_tile, rest = i - tile * per_tile, r = rest / vecs, c = (rest - r * vecs) * 4;
+    int tm, tn;
+    w.coords(w.whole + tile, tm, tn);
+    const int row = tm * GP_BM + r, col = tn * bn + c;
+    if (row >= M || col >= N) continue;
+    float* dst = C + static_cast<size_t>(row) * ldc + col;
+    const float* src = work + (static_cast<size_t>(tile) * GP_BM + r) * bn + c;
+    const size_t part = static_cast<size_t>(w.split_tiles) * GP_BM * bn;
+    if (col + 4 <= N) {
+      float4 v = *reinterpret_cast<const float4*>(dst);
+      for (int p = 1; p < w.ks; ++p, src += part) {
+        const float4 a = *reinterpret_cast<const float4*>(src);
+        v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+      }
+      *reinterpret_cast<float4*>(dst) = v;
+    } else {
+      for (int j = 0; col + j < N; ++j) {
+        float v = dst[j];
+        for (int p = 1; p < w.ks; ++p) v += src[(p - 1) * part + j];
+        dst[j] = v;
+      }
+    }
+  }
+}
+
 template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
 static int launch_pair(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
-                       const PairPlan& pl, int pairs, int* status, cudaStream_t stream) {
-  CUtensorMap tmA, tmB, tmC;
+                       const PairPlan& pl, int pairs, float* work, int* status, cudaStream_t stream) {
+  CUtensorMap tmA, tmB, tmC, tmW;
   int rc;
   if (!A_MN) rc = make_tmap_2d_bf16(&tmA, A, K, M, lda, GP_BK, 128);
   else       rc = make_tmap_2d_bf16(&tmA, A, M, K, lda, 64, GP_BK);
@@ -290,6 +331,15 @@ static int launch_pair(const void* A, const void* B, void* C, int M, int N, int 
     rc = make_tmap(&tmC, C, OUT_F32 ? 4 : 2, 2, dims, str, box, 3);
     if (rc) return rc;
   }
+  const bool split = ACCUM && pl.ks > 1 && pl.split_tiles > 0, ordered = split && pl.ordered;
+  tmW = tmC;
+  if (ordered) {
+    const uint64_t dims[2] = {(uint64_t)pl.bn, (uint64_t)pl.split_tiles * (pl.ks - 1) * GP_BM};
+    const uint64_t str[1] = {(uint64_t)pl.bn * 4};
+    const uint32_t box[2] = {32u, 32u};
+    rc = make_tmap(&tmW, work, 4, 2, dims, str, box, 3);
+    if (rc) return rc;
+  }
   auto kern = gemm_pair_kernel<A_MN, B_MN, OUT_F32, ACCUM>;
   static bool configured = false;
   if (!configured) {
@@ -301,9 +351,10 @@ static int launch_pair(const void* A, const void* B, void* C, int M, int N, int 
   w.tiles_m = (M + GP_BM - 1) / GP_BM;
   w.tiles_n = (N + pl.bn - 1) / pl.bn;
   w.nk = (K + GP_BK - 1) / GP_BK;
-  w.ks = ACCUM ? pl.ks : 1;
+  w.ks = split ? pl.ks : 1;
+  w.ordered = ordered;
   const int tiles = w.tiles_m * w.tiles_n;
-  w.split_tiles = w.ks > 1 ? pl.split_tiles : 0;
+  w.split_tiles = split ? pl.split_tiles : 0;
   w.whole = tiles - w.split_tiles;
   // m-tiles per group: about 24 MB of A rows, at most 16 tiles
   const long panel = (long)GP_BM * K * 2;
@@ -312,19 +363,23 @@ static int launch_pair(const void* A, const void* B, void* C, int M, int N, int 
   w.group_m = gm < w.tiles_m ? (int)gm : w.tiles_m;
   const int units = w.whole + w.split_tiles * w.ks;
   const int grid = 2 * (units < pairs ? units : pairs);
-  KB_LAUNCH(kern, grid, GP_THREADS, GP_SMEM, stream, tmA, tmB, tmC, w, M, N, pl.bn, status);
+  KB_LAUNCH(kern, grid, GP_THREADS, GP_SMEM, stream, tmA, tmB, tmC, tmW, w, M, N, pl.bn, status);
+  if (ordered) {
+    const int blocks = w.split_tiles * (GP_BM * pl.bn / 4 / 256);
+    KB_LAUNCH(gemm_add_parts_kernel, blocks, 256, 0, stream, static_cast<float*>(C), ldc, M, N, (const float*)work, w, pl.bn);
+  }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + static_cast<int>(e);
 }
 
 int gemm_pair_dispatch(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda, int b_mn, int ldb,
-                       int ldc, int out_f32, int accumulate, const PairPlan& pl, int pairs, int* status,
+                       int ldc, int out_f32, int accumulate, const PairPlan& pl, int pairs, float* work, int* status,
                        cudaStream_t stream) {
 #define GP_GO(AM, BM_)                                                                                         \
   do {                                                                                                         \
-    if (out_f32 && accumulate) return launch_pair<AM, BM_, true, true>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, status, stream); \
-    if (out_f32) return launch_pair<AM, BM_, true, false>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, status, stream);              \
-    return launch_pair<AM, BM_, false, false>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, status, stream);                          \
+    if (out_f32 && accumulate) return launch_pair<AM, BM_, true, true>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, work, status, stream);\
+    if (out_f32) return launch_pair<AM, BM_, true, false>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, work, status, stream);             \
+    return launch_pair<AM, BM_, false, false>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, work, status, stream);                         \
   } while (0)
   if (!a_mn && !b_mn) GP_GO(false, false);
   if (!a_mn && b_mn) GP_GO(false, true);

@@ -394,7 +394,7 @@ static bool split_allowed() {
 }
 
 // Modelled time of the two-SM kernel at tile width `bn`, in 64-deep K steps of a 256 x 256 tile.
-static PairPlan plan_pair_width(int M, int N, int K, int pairs, int bn, bool accumulate) {
+static PairPlan plan_pair_width(int M, int N, int K, int pairs, int bn, bool may_split) {
   // Measured per step: a step moves 16 KB of A and bn / 256 x 16 KB of B into each SM, so narrow tiles are bound by the
   // bytes in flight and not by the tensor pipe (16384 x 6144 x 3072, us per step: 0.41 at 256 columns, 0.30 at 192, 0.23 at
   // 128, 0.17 at 64; with six stages at every width 0.32, 0.24 and 0.175).
@@ -404,12 +404,34 @@ static PairPlan plan_pair_width(int M, int N, int K, int pairs, int bn, bool acc
   const long tiles = (long)((M + 255) / 256) * ((N + bn - 1) / bn);
   const long full_waves = tiles / pairs, rest = tiles - full_waves * pairs;
   const double base = full_waves * (nk * step + fixed);
-  PairPlan best{bn, 1, 0, base + (rest ? nk * step + fixed : 0.0) + 4.0};
-  if (accumulate && rest && split_allowed())
+  PairPlan best{bn, 1, 0, base + (rest ? nk * step + fixed : 0.0) + 4.0, false};
+  if (may_split && rest)
     for (int ks = 2; ks <= 8 && nk / ks >= 8; ++ks) {
       const long waves = (rest * ks + pairs - 1) / pairs;
       const double t = base + waves * ((nk + ks - 1) / ks * step + fixed) + 4.0;
-      if (t < best.cost * 0.97) best = PairPlan{bn, ks, (int)rest, t};   // a split must pay for its extra additions
+      if (t < best.cost * 0.97) best = PairPlan{bn, ks, (int)rest, t, false};   // a split must pay for its extra additions
+    }
+  return best;
+}
+
+// The same for `C +=` with parts added in order, in us.  Fitted to 73 weight gradients of 144..16384 x 184..8192, 560 to
+// 19152 tokens (within 10 %; the plans it picks take 0.2 % longer than the best width and split of each).  Both operands
+// are MN-major there and B comes in 64-wide chunks, which makes 64 and 192 columns dearer than above.  The second launch
+// costs 3.8 us and 0.29 us per MB that it moves.
+static PairPlan plan_ordered_width(int M, int N, int K, int pairs, int bn, bool may_split) {
+  static const double step_us[5] = {0, 0.206, 0.225, 0.298, 0.341}, fixed_us[5] = {0, 0.15, 1.0, 1.85, 2.5};
+  const int nk = (K + GEMM_BK - 1) / GEMM_BK;
+  const double step = step_us[bn / 64], fixed = fixed_us[bn / 64];
+  const long tiles = (long)((M + 255) / 256) * ((N + bn - 1) / bn);
+  const long full_waves = tiles / pairs, rest = tiles - full_waves * pairs;
+  const double base = full_waves * (nk * step + fixed);
+  PairPlan best{bn, 1, 0, base + (rest ? nk * step + fixed : 0.0), true};
+  if (may_split && rest)
+    for (int ks = 2; ks <= 8 && nk / ks >= 8; ++ks) {
+      const long waves = (rest * ks + pairs - 1) / pairs;
+      const double mb = rest * 256e-6 * bn * 4 * (ks + 1);
+      const double t = base + waves * ((nk + ks - 1) / ks * step + fixed) + 3.8 + 0.29 * mb;
+      if (t < best.cost * 0.97) best = PairPlan{bn, ks, (int)rest, t, true};
     }
   return best;
 }
@@ -434,23 +456,58 @@ static int split_single(int M, int N, int K, int num_sms, bool narrow) {
 // Narrow outputs waste less of the last wave with the 128-wide tile of the one-SM kernel.
 static bool narrow_single(int N) { return N <= 128 || (N % 256 != 0 && N % 256 <= 128); }
 
-static PairPlan plan_pair(int M, int N, int K, int pairs, bool accumulate) {
-  PairPlan best = plan_pair_width(M, N, K, pairs, 256, accumulate);
-  for (int bn = 192; bn >= 64; bn -= 64) {
-    const PairPlan p = plan_pair_width(M, N, K, pairs, bn, accumulate);
+template <typename F>
+static PairPlan best_width(F plan) {
+  PairPlan best = plan(g_force_bn ? g_force_bn : 256);
+  for (int bn = 192; bn >= 64 && !g_force_bn; bn -= 64) {
+    const PairPlan p = plan(bn);
     if (p.cost < best.cost) best = p;
+  }
+  return best;
+}
+
+static PairPlan plan_pair(int M, int N, int K, int pairs) {
+  return best_width([&](int bn) { return plan_pair_width(M, N, K, pairs, bn, false); });
+}
+
+// `C +=`.  Where 128-row tiles would not fill the chip once and be split even so, the parts add in L2 as they come: the
+// second launch of an ordered sum costs such calls up to a third (1024 x 128 over 4096 rows: 8.4 us, ordered 11.3; 640 x 3072
+// over 16384 rows: 55 and 60).  Everything larger repeats bit for bit: parts that add as they come save 3 % at most there
+// (16384 x 3072 over 16384 rows).  Without a workspace an ordered sum is not split.
+static PairPlan plan_accumulate(int M, int N, int K, int num_sms, bool workspace) {
+  const bool narrow = narrow_single(N);
+  const long tiles = (long)((M + GEMM_BM - 1) / GEMM_BM) * ((N + (narrow ? 127 : 255)) / (narrow ? 128 : 256));
+  const bool few = tiles <= num_sms && split_single(M, N, K, num_sms, narrow) > 1;
+  const int pairs = num_sms / 2;
+  PairPlan best = best_width([&](int bn) {
+    return few ? plan_pair_width(M, N, K, pairs, bn, true)
+               : plan_ordered_width(M, N, K, pairs, bn, workspace && split_allowed());
+  });
+  if (g_force_ks > 0 && (few || workspace)) {
+    const int nk = (K + GEMM_BK - 1) / GEMM_BK;
+    best.ks = g_force_ks <= nk ? g_force_ks : nk;
+    best.split_tiles = ((M + 255) / 256) * ((N + best.bn - 1) / best.bn);
   }
   return best;
 }
 
 }  // namespace kb
 
-// Tile rows (256: the two-SM kernel) and K split of the tiles after the last full wave that kb_gemm_bf16 uses for
-// an accumulating fp32 output of this shape.
-extern "C" void kb_gemm_accum_plan(int M, int N, int K, int num_sms, int* tile_rows, int* ks) {
-  const kb::PairPlan pl = kb::plan_pair(M, N, K, num_sms / 2, true);
-  *tile_rows = 256;
+// Tile width, K split and number of split tiles (those after the last full wave) of the two-SM kernel for an
+// accumulating fp32 output of this shape.
+extern "C" void kb_gemm_accum_plan(int M, int N, int K, int num_sms, int* bn, int* ks, int* split_tiles) {
+  const kb::PairPlan pl = kb::plan_accumulate(M, N, K, num_sms, true);
+  *bn = pl.bn;
   *ks = pl.ks;
+  *split_tiles = pl.split_tiles;
+}
+
+// Floats of workspace that kb_gemm_accum_bf16 needs for an output of this shape (0: it splits nothing).
+extern "C" long kb_gemm_accum_scratch_floats(int M, int N, int K, int num_sms) {
+  using namespace kb;
+  if (num_sms <= 0) num_sms = device_sm_count();
+  if (M <= 0 || N <= 0 || K <= 0 || num_sms < 2 || g_force_single) return 0;
+  return plan_accumulate(M, N, K, num_sms, true).scratch_floats();
 }
 
 // Measurement aid: force the tile rows (128 / 256) and K split of accumulating GEMMs; ks = 0 returns to the model.
@@ -472,11 +529,12 @@ extern "C" void kb_gemm_force_width(int bn) {
 //   out_f32: C is fp32 (else bf16); accumulate: C += (fp32 only).  num_sms limits the grid.
 // Strides must be multiples of 8 elements and base pointers 16-byte aligned (TMA rules).
 // kb_gemm_bias_act_bf16 adds the epilogue: bias (bf16 [N], may be null) and act (0 none, 1 GELU); it is not
-// available together with accumulate.
-extern "C" int kb_gemm_bias_act_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda,
-                                     int b_mn, int ldb, int ldc, int out_f32, int accumulate, int num_sms,
-                                     const void* bias, int act, int* status, cudaStream_t stream) {
-  using namespace kb;
+// available together with accumulate.  kb_gemm_accum_bf16 is C += with a workspace of kb_gemm_accum_scratch_floats()
+// floats (16-byte aligned, may be null if that is 0) for the parts of K; kb_gemm_bf16 has none and splits K less often.
+namespace kb {
+static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda, int b_mn, int ldb, int ldc,
+                    int out_f32, int accumulate, int num_sms, const void* bias, int act, float* work, int* status,
+                    cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return ST_BAD_ARG;
   if ((bias != nullptr || act != 0) && accumulate) return ST_BAD_ARG;
   if (act < 0 || act > 1) return ST_BAD_ARG;
@@ -489,14 +547,9 @@ extern "C" int kb_gemm_bias_act_bf16(const void* A, const void* B, void* C, int 
   // The two-SM kernel stores through TMA: 16-byte aligned output rows.
   if (plain && aligned_rows(C, ldc, out_f32) && num_sms >= 2 && !g_force_single) {
     const int pairs = num_sms / 2;
-    PairPlan pl = g_force_bn ? plan_pair_width(M, N, K, pairs, g_force_bn, accumulate != 0)
-                             : plan_pair(M, N, K, pairs, accumulate != 0);
-    if (g_force_ks > 0 && accumulate) {
-      const int nk = (K + GEMM_BK - 1) / GEMM_BK;
-      pl.ks = g_force_ks <= nk ? g_force_ks : nk;
-      pl.split_tiles = ((M + 255) / 256) * ((N + pl.bn - 1) / pl.bn);
-    }
-    return gemm_pair_dispatch(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, pl, pairs, status, stream);
+    const PairPlan pl = accumulate ? plan_accumulate(M, N, K, num_sms, work != nullptr) : plan_pair(M, N, K, pairs);
+    return gemm_pair_dispatch(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, pl, pairs, work, status,
+                              stream);
   }
   const bool narrow = g_force_single ? g_force_single == 128 : narrow_single(N);
   int ks = accumulate ? split_single(M, N, K, num_sms, narrow) : 1;
@@ -512,10 +565,23 @@ extern "C" int kb_gemm_bias_act_bf16(const void* A, const void* B, void* C, int 
   KB_GO(256);
 #undef KB_GO
 }
+}  // namespace kb
+
+extern "C" int kb_gemm_bias_act_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda,
+                                     int b_mn, int ldb, int ldc, int out_f32, int accumulate, int num_sms,
+                                     const void* bias, int act, int* status, cudaStream_t stream) {
+  return kb::gemm_run(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, num_sms, bias, act, nullptr, status,
+                      stream);
+}
+
+extern "C" int kb_gemm_accum_bf16(const void* A, const void* B, float* C, int M, int N, int K, int a_mn, int lda, int b_mn,
+                                  int ldb, int ldc, int num_sms, float* work, int* status, cudaStream_t stream) {
+  return kb::gemm_run(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, 1, 1, num_sms, nullptr, 0, work, status, stream);
+}
 
 extern "C" int kb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda,
                             int b_mn, int ldb, int ldc, int out_f32, int accumulate, int num_sms, int* status,
                             cudaStream_t stream) {
-  return kb_gemm_bias_act_bf16(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, num_sms, nullptr, 0,
-                               status, stream);
+  return kb::gemm_run(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, num_sms, nullptr, 0, nullptr, status,
+                      stream);
 }

@@ -51,6 +51,7 @@ def _declare(L) -> None:
     P, I, LNG, F, U = c_void_p, c_int, c_long, c_float, c_uint
     sig = {
         "kb_gemm_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P],
+        "kb_gemm_accum_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, P, P, P],
         "kb_gemm_bias_act_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, I, P, P],
         "kb_rmsnorm_fwd": [P, P, P, P, I, I, F, P],
         "kb_rmsnorm_fwd_heads": [P, LNG, I, LNG, LNG, P, P, P, I, F, P],
@@ -77,6 +78,8 @@ def _declare(L) -> None:
         fn.restype = c_int
     L.kb_rmsnorm_bwd_scratch_elems.argtypes = [I, I]
     L.kb_rmsnorm_bwd_scratch_elems.restype = c_long
+    L.kb_gemm_accum_scratch_floats.argtypes = [I, I, I, I]
+    L.kb_gemm_accum_scratch_floats.restype = c_long
     for name, args in _OPTIONAL_SIGS.items():
         if hasattr(L, name):
             fn = getattr(L, name)
@@ -401,14 +404,14 @@ def gemm(a, b, trans_a=False, trans_b=True, out_dtype=None, accumulate=None, out
     if accumulate is not None:
         if accumulate.dtype != torch.float32 or not accumulate.is_contiguous() or tuple(accumulate.shape) != (M, N):
             raise KernelError("accumulate must be a contiguous fp32 [M,N] tensor")
-        c, f32, acc = accumulate, 1, 1
+        c, f32 = accumulate, 1
     else:
         dt = out_dtype or torch.bfloat16
         if out is None:
             out = torch.empty(M, N, dtype=dt, device=a.device)
         elif not (out.dim() == 2 and out.stride(1) == 1):
             raise KernelError("gemm out must have a contiguous last dim")
-        c, f32, acc = out, 1 if out.dtype == torch.float32 else 0, 0
+        c, f32 = out, 1 if out.dtype == torch.float32 else 0
     st = status_word(a.device)
     if bias is not None or activation:
         if accumulate is not None:
@@ -429,12 +432,20 @@ def gemm(a, b, trans_a=False, trans_b=True, out_dtype=None, accumulate=None, out
             _check(rc, f"gemm+epilogue M={M} N={N} K={K}")
         _count()
         return c
-    rc = lib().kb_gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, 1 if trans_a else 0, a.stride(0),
-                            0 if trans_b else 1, b.stride(0), c.stride(0), f32, acc,
-                            int(num_sms) if num_sms else 0, st.data_ptr(), _stream())
+    L, sms = lib(), int(num_sms) if num_sms else 0
+    if accumulate is not None:
+        n = L.kb_gemm_accum_scratch_floats(M, N, K, sms)      # partial sums of a K split, added in order by a second kernel
+        work = torch.empty(n, dtype=torch.float32, device=a.device) if n else None
+        rc = L.kb_gemm_accum_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, 1 if trans_a else 0, a.stride(0),
+                                  0 if trans_b else 1, b.stride(0), c.stride(0), sms, work.data_ptr() if n else 0,
+                                  st.data_ptr(), _stream())
+    else:
+        n = 0
+        rc = L.kb_gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, 1 if trans_a else 0, a.stride(0),
+                            0 if trans_b else 1, b.stride(0), c.stride(0), f32, 0, sms, st.data_ptr(), _stream())
     if rc != 0:
         _check(rc, f"gemm M={M} N={N} K={K}")
-    _count()
+    _count(2 if n else 1)
     return c
 
 

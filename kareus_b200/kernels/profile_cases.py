@@ -81,7 +81,7 @@ def wgrad_sweep() -> None:
     L = KC.lib()
     L.kb_gemm_accum_force.argtypes = [ctypes.c_int, ctypes.c_int]
     L.kb_gemm_accum_force.restype = None
-    L.kb_gemm_accum_plan.argtypes = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)] * 2
+    L.kb_gemm_accum_plan.argtypes = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)] * 3
     L.kb_gemm_accum_plan.restype = None
     dev = "cuda"
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
@@ -107,9 +107,9 @@ def wgrad_sweep() -> None:
             L.kb_gemm_accum_force(0, 0)
             t_auto = _timed(run, flush)
             t_lib = _timed(lambda: torch.matmul(dy.t(), x), flush)
-            tile_c, ks_c = ctypes.c_int(), ctypes.c_int()
+            tile_c, ks_c, split_c = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
             L.kb_gemm_accum_plan(n_out, n_in, tokens, KC.sm_count(),
-                                 ctypes.byref(tile_c), ctypes.byref(ks_c))
+                                 ctypes.byref(tile_c), ctypes.byref(ks_c), ctypes.byref(split_c))
             print(f"| tp{tp} {name} | {n_out} x {n_in} | " + " | ".join(f"{c:.0f}" for c in cells)
                   + f" | {tile_c.value}/ks{ks_c.value} | {flops / t_auto / 1e9:.0f} | {flops / t_lib / 1e9:.0f} |")
             del dy, x, acc

@@ -11,15 +11,26 @@ def _lib():
     if not build.LIB.exists():
         pytest.skip("native library not built")
     L = ctypes.CDLL(str(build.LIB))
-    L.kb_gemm_accum_plan.argtypes = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)] * 2
+    L.kb_gemm_accum_plan.argtypes = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)] * 3
     L.kb_gemm_accum_plan.restype = None
+    L.kb_gemm_accum_scratch_floats.argtypes = [ctypes.c_int] * 4
+    L.kb_gemm_accum_scratch_floats.restype = ctypes.c_long
     return L
 
 
 def _plan(L, n_out, n_in, tokens, sms=148):
-    tile, ks = ctypes.c_int(), ctypes.c_int()
-    L.kb_gemm_accum_plan(n_out, n_in, tokens, sms, ctypes.byref(tile), ctypes.byref(ks))
-    return tile.value, ks.value
+    """(tile width, K split), checked against the number of split tiles and the workspace of an ordered sum."""
+    bn, ks, split = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+    L.kb_gemm_accum_plan(n_out, n_in, tokens, sms, ctypes.byref(bn), ctypes.byref(ks), ctypes.byref(split))
+    bn, ks, split = bn.value, ks.value, split.value
+    assert bn in (64, 128, 192, 256)
+    tiles = -(-n_out // 256) * -(-n_in // bn)
+    assert split == (tiles % (sms // 2) if ks > 1 else 0)      # the tiles after the last full wave
+    # outputs that 128-row tiles do not fill the chip with once may add their parts as they come: no workspace
+    tiles128 = -(-n_out // 128) * -(-n_in // (128 if n_in <= 128 or 0 < n_in % 256 <= 128 else 256))
+    scratch = L.kb_gemm_accum_scratch_floats(n_out, n_in, tokens, sms)
+    assert scratch == split * (ks - 1) * 256 * bn or (scratch == 0 and tiles128 <= sms)
+    return bn, ks
 
 
 def test_weight_gradients_with_few_tiles_split_k():
@@ -28,13 +39,17 @@ def test_weight_gradients_with_few_tiles_split_k():
     # TP8 shards of a 3B Llama layer: 36-96 tiles for 148 SMs → more than one CTA per tile
     for n_out, n_in in [(640, 3072), (3072, 384), (2048, 3072), (3072, 1024)]:
         tile, ks = _plan(L, n_out, n_in, tokens)
-        assert tile in (128, 256) and 2 <= ks <= 8, (n_out, n_in, tile, ks)
+        assert 2 <= ks <= 8, (n_out, n_in, tile, ks)
     # the LM head has thousands of tiles: no split
     assert _plan(L, 128256, 3072, tokens) == (256, 1)
     # a split never leaves fewer than eight 64-deep K steps per part
     for k in (512, 1024, 2048):
         _, ks = _plan(L, 640, 3072, k)
         assert ks == 1 or (k // 64) // ks >= 8
+    # more tiles than SM pairs: what is left over after the full waves is split, in order
+    for n_out, n_in in [(16384, 3072), (5120, 3072), (3072, 8192)]:
+        bn, ks = _plan(L, n_out, n_in, tokens)
+        assert ks > 1 and L.kb_gemm_accum_scratch_floats(n_out, n_in, tokens, 148) > 0, (n_out, n_in, bn, ks)
     # the choice follows the number of SMs given to the GEMM
     assert _plan(L, 2048, 3072, tokens, sms=32)[1] <= _plan(L, 2048, 3072, tokens, sms=148)[1]
 

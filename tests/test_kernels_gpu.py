@@ -123,6 +123,32 @@ def test_weight_gradient_odd_rows(n_out, n_in, tokens):
     assert (buf[n_out * n_in:] == 2).all()
 
 
+# full waves of tiles and some left over; forced splits of all tiles with ragged edges and uneven parts
+@pytest.mark.parametrize("n_out,n_in,tokens,ks", [(5120, 3072, 8192, 0), (2048, 3072, 8192, 0), (3072, 8192, 4096, 0),
+                                                  (2304, 2056, 1104, 2), (2304, 2056, 1104, 5), (3000, 2060, 520, 3)])
+def test_weight_gradient_repeats_bitwise(n_out, n_in, tokens, ks):
+    """Outputs of more tiles than SMs: the parts of a K split are added in order, the same operands give the same bits."""
+    import ctypes
+    KC = _K()
+    L = KC.lib()
+    L.kb_gemm_accum_force.argtypes = [ctypes.c_int, ctypes.c_int]
+    L.kb_gemm_accum_force.restype = None
+    g = torch.Generator(device="cuda").manual_seed(n_out)
+    dy = torch.randn(tokens, n_out, device="cuda", generator=g).bfloat16()
+    x = torch.randn(tokens, (n_in + 7) // 8 * 8, device="cuda", generator=g).bfloat16()[:, :n_in]
+    start = torch.randn(n_out, n_in, device="cuda", generator=g)
+    try:
+        L.kb_gemm_accum_force(256, ks)
+        assert L.kb_gemm_accum_scratch_floats(n_out, n_in, tokens, 0) > 0          # the tiles are split
+        runs = [KC.gemm(dy, x, trans_a=True, trans_b=False, accumulate=start.clone()) for _ in range(8)]
+        KC.check_status()
+    finally:
+        L.kb_gemm_accum_force(0, 0)
+    # fp32 sums of exact bf16 products
+    assert _rel(runs[0], (start.double() + dy.double().t() @ x.double()).float()) < 1e-5
+    assert all(torch.equal(r, runs[0]) for r in runs[1:])
+
+
 def test_gemm_sm_limit_and_views():
     KC = _K()
     a = torch.randn(512, 1024, device="cuda").bfloat16()
