@@ -472,17 +472,20 @@ static PairPlan plan_pair(int M, int N, int K, int pairs) {
 
 // `C +=`.  Where 128-row tiles would not fill the chip once and be split even so, the parts add in L2 as they come: the
 // second launch of an ordered sum costs such calls up to a third (1024 x 128 over 4096 rows: 8.4 us, ordered 11.3; 640 x 3072
-// over 16384 rows: 55 and 60).  Everything larger repeats bit for bit: parts that add as they come save 3 % at most there
-// (16384 x 3072 over 16384 rows).  Without a workspace an ordered sum is not split.
+// over 16384 rows: 55 and 60).  Everything larger repeats bit for bit, which costs 0 to 17 % of a call (16384 x 3072 over
+// 16384 rows: 0; 5120 x 3072 over 2048 rows: 9; 2120 x 584 over 5912 rows: 17).  Without a workspace an ordered sum is not
+// split, and over fewer than 16 steps nothing is: widths are then picked as for other outputs (3072 x 8192 over 64 rows:
+// 27 us, 38 with the fit to long sums).
 static PairPlan plan_accumulate(int M, int N, int K, int num_sms, bool workspace) {
   const bool narrow = narrow_single(N);
   const long tiles = (long)((M + GEMM_BM - 1) / GEMM_BM) * ((N + (narrow ? 127 : 255)) / (narrow ? 128 : 256));
   const bool few = tiles <= num_sms && split_single(M, N, K, num_sms, narrow) > 1;
   const int pairs = num_sms / 2;
   PairPlan best = best_width([&](int bn) {
-    return few ? plan_pair_width(M, N, K, pairs, bn, true)
+    return few || K <= 15 * GEMM_BK ? plan_pair_width(M, N, K, pairs, bn, few)
                : plan_ordered_width(M, N, K, pairs, bn, workspace && split_allowed());
   });
+  best.ordered = !few;
   if (g_force_ks > 0 && (few || workspace)) {
     const int nk = (K + GEMM_BK - 1) / GEMM_BK;
     best.ks = g_force_ks <= nk ? g_force_ks : nk;

@@ -434,7 +434,8 @@ def gemm(a, b, trans_a=False, trans_b=True, out_dtype=None, accumulate=None, out
         return c
     L, sms = lib(), int(num_sms) if num_sms else 0
     if accumulate is not None:
-        n = L.kb_gemm_accum_scratch_floats(M, N, K, sms)      # partial sums of a K split, added in order by a second kernel
+        # partial sums of a K split, added in order by a second kernel; nothing is split over fewer than 16 steps of 64
+        n = L.kb_gemm_accum_scratch_floats(M, N, K, sms) if K > 960 else 0
         work = torch.empty(n, dtype=torch.float32, device=a.device) if n else None
         rc = L.kb_gemm_accum_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, 1 if trans_a else 0, a.stride(0),
                                   0 if trans_b else 1, b.stride(0), c.stride(0), sms, work.data_ptr() if n else 0,
