@@ -254,7 +254,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tmem_ld_wait();
         const int col = n0 + c * 32;
         if constexpr (!ACCUM) apply_epilogue(v, ep, col, N);
-        if (OUT_F32 && !(col + 32 <= N && vec_out)) {
+        if (!(col + 32 <= N && vec_out)) {
           // rows that are not 16-byte aligned, or the edge: through the staging buffer (columns XOR-swizzled by row), so
           // that an access takes 32 neighbouring columns of a row and not one column of 32 rows (4096 x 50257 x 3072: fp32
           // 2.03 -> 1.23 ms, with accumulation 5.46 -> 1.54 ms)
@@ -263,7 +263,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           for (int j = 0; j < 32; ++j) st[lane * 32 + (j ^ lane)] = __uint_as_float(v[j]);
           __syncwarp();
           const int rows = min(32, M - (m0 + q * 32));
-          if (col + lane < N) {
+          if (!OUT_F32 && col + lane < N) {
+            __nv_bfloat16* cc = reinterpret_cast<__nv_bfloat16*>(Cout) + static_cast<size_t>(m0 + q * 32) * ldc + col + lane;
+#pragma unroll 4
+            for (int r = 0; r < rows; ++r) cc[static_cast<long>(r) * ldc] = __float2bfloat16(st[r * 32 + (lane ^ r)]);
+          } else if (col + lane < N) {
             float* cc = reinterpret_cast<float*>(Cout) + static_cast<size_t>(m0 + q * 32) * ldc + col + lane;
 #pragma unroll 1
             for (int r0 = 0; r0 < rows; r0 += 8, cc += 8L * ldc) {
@@ -301,18 +305,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
           } else {
             __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + static_cast<size_t>(row) * ldc + col;
-            if (col + 32 <= N && vec_out) {
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                uint4 o;
-                o.x = pack_bf16x2(__uint_as_float(v[8 * j + 0]), __uint_as_float(v[8 * j + 1]));
-                o.y = pack_bf16x2(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3]));
-                o.z = pack_bf16x2(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5]));
-                o.w = pack_bf16x2(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7]));
-                reinterpret_cast<uint4*>(crow)[j] = o;
-              }
-            } else {
-              for (int j = 0; j < 32 && col + j < N; ++j) crow[j] = __float2bfloat16(__uint_as_float(v[j]));
+            for (int j = 0; j < 4; ++j) {
+              uint4 o;
+              o.x = pack_bf16x2(__uint_as_float(v[8 * j + 0]), __uint_as_float(v[8 * j + 1]));
+              o.y = pack_bf16x2(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3]));
+              o.z = pack_bf16x2(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5]));
+              o.w = pack_bf16x2(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7]));
+              reinterpret_cast<uint4*>(crow)[j] = o;
             }
           }
         }
