@@ -394,13 +394,14 @@ static bool split_allowed() {
 }
 
 // Modelled time of the two-SM kernel at tile width `bn`, in 64-deep K steps of a 256 x 256 tile.
-static PairPlan plan_pair_width(int M, int N, int K, int pairs, int bn, bool may_split) {
+static PairPlan plan_pair_width(int M, int N, int K, int pairs, int bn, bool may_split, bool b_mn = false) {
   // Measured per step: a step moves 16 KB of A and bn / 256 x 16 KB of B into each SM, so narrow tiles are bound by the
   // bytes in flight and not by the tensor pipe (16384 x 6144 x 3072, us per step: 0.41 at 256 columns, 0.30 at 192, 0.23 at
-  // 128, 0.17 at 64; with six stages at every width 0.32, 0.24 and 0.175).
-  static const double step_cost[5] = {0, 0.45, 0.57, 0.75, 1.0};
+  // 128, 0.17 at 64; with six stages at every width 0.32, 0.24 and 0.175).  MN-major B comes in 64-wide chunks, 192 columns
+  // move as much of it as 256 (2048 x 8192 x 3072: 76.6 us at 192 columns, 70.9 at 256).
+  static const double step_cost[2][5] = {{0, 0.45, 0.57, 0.75, 1.0}, {0, 0.55, 0.61, 0.83, 1.0}};
   const int nk = (K + GEMM_BK - 1) / GEMM_BK;
-  const double step = step_cost[bn / 64], fixed = 3.0;
+  const double step = step_cost[b_mn][bn / 64], fixed = 3.0;
   const long tiles = (long)((M + 255) / 256) * ((N + bn - 1) / bn);
   const long full_waves = tiles / pairs, rest = tiles - full_waves * pairs;
   const double base = full_waves * (nk * step + fixed);
@@ -466,8 +467,28 @@ static PairPlan best_width(F plan) {
   return best;
 }
 
-static PairPlan plan_pair(int M, int N, int K, int pairs) {
-  return best_width([&](int bn) { return plan_pair_width(M, N, K, pairs, bn, false); });
+static PairPlan plan_pair(int M, int N, int K, int pairs, bool b_mn) {
+  return best_width([&](int bn) { return plan_pair_width(M, N, K, pairs, bn, false, b_mn); });
+}
+
+// Tile width of the one-SM kernel for a plain bf16 output where that is the faster one (0: it is not), from the modelled
+// us of both kernels (fitted to 284 forward and input-gradient calls of 64..20000 rows; rms error 8 to 15 %).  Without a
+// cluster to start it is 1 us quicker to its first product, and 128-row tiles waste less of a short last wave; per step it
+// takes 10 % longer.  776 x 5120 x 3072: 27.7 us on pairs (two waves), 20.7 here (one); 4096 x 1024 x 128: 7.4 and 6.0.  Up to
+// two steps of K it was the faster one whatever the number of waves (15720 x 4344 x 128: 52.3 and 44.1).
+static int single_width(int M, int N, int K, bool b_mn, int num_sms, int pair_bn) {
+  static const double pair_us[5][3] = {{}, {0.16, 1.0, 4.4}, {0.179, 1.4, 4.3}, {0.245, 1.85, 4.0}, {0.304, 1.95, 4.6}};
+  const int nk = (K + GEMM_BK - 1) / GEMM_BK;
+  auto waves = [](int M_, int N_, int bm, int bn, int slots) {
+    return (long)(((long)((M_ + bm - 1) / bm) * ((N_ + bn - 1) / bn) + slots - 1) / slots);
+  };
+  const double* c = pair_us[pair_bn / 64];
+  // an MN-major B comes in 64-wide chunks, of which 64-wide tiles use half
+  const double pair = c[2] + (b_mn && pair_bn == 64 ? 0.4 : 0.0) + waves(M, N, 256, pair_bn, num_sms / 2) * (nk * c[0] + c[1]);
+  const double w128 = 3.5 + waves(M, N, 128, 128, num_sms) * (nk * 0.275 + 0.95);
+  const double w256 = 3.2 + waves(M, N, 128, 256, num_sms) * (nk * 0.337 + 2.2);
+  if (nk > 2 && (w128 < w256 ? w128 : w256) >= (b_mn ? 1.0 : 0.97) * pair) return 0;
+  return w128 < w256 ? 128 : 256;
 }
 
 // `C +=`.  Where 128-row tiles would not fill the chip once and be split even so, the parts add in L2 as they come: the
@@ -503,6 +524,13 @@ extern "C" void kb_gemm_accum_plan(int M, int N, int K, int num_sms, int* bn, in
   *bn = pl.bn;
   *ks = pl.ks;
   *split_tiles = pl.split_tiles;
+}
+
+// Tile width that kb_gemm_bf16 uses for a bf16 output of this shape (rows 16-byte aligned): positive on the two-SM kernel,
+// negative on the one-SM kernel.
+extern "C" int kb_gemm_plan(int M, int N, int K, int b_mn, int num_sms) {
+  const int bn = kb::plan_pair(M, N, K, num_sms / 2, b_mn != 0).bn, one = N % 8 ? 0 : kb::single_width(M, N, K, b_mn != 0, num_sms, bn);
+  return one ? -one : bn;
 }
 
 // Floats of workspace that kb_gemm_accum_bf16 needs for an output of this shape (0: it splits nothing).
@@ -548,13 +576,17 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
   if (num_sms <= 0) num_sms = device_sm_count();
   if (accumulate && !out_f32) return ST_BAD_ARG;
   // The two-SM kernel stores through TMA: 16-byte aligned output rows.
-  if (plain && aligned_rows(C, ldc, out_f32) && num_sms >= 2 && !g_force_single) {
+  int single = g_force_single;
+  if (plain && aligned_rows(C, ldc, out_f32) && num_sms >= 2 && !single) {
     const int pairs = num_sms / 2;
-    const PairPlan pl = accumulate ? plan_accumulate(M, N, K, num_sms, work != nullptr) : plan_pair(M, N, K, pairs);
-    return gemm_pair_dispatch(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, pl, pairs, work, status,
-                              stream);
+    const PairPlan pl = accumulate ? plan_accumulate(M, N, K, num_sms, work != nullptr)
+                                   : plan_pair(M, N, K, pairs, b_mn != 0);
+    if (!out_f32 && N % 8 == 0 && !g_force_bn) single = single_width(M, N, K, b_mn != 0, num_sms, pl.bn);
+    if (!single)
+      return gemm_pair_dispatch(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, pl, pairs, work, status,
+                                stream);
   }
-  const bool narrow = g_force_single ? g_force_single == 128 : narrow_single(N);
+  const bool narrow = single ? single == 128 : narrow_single(N);
   int ks = accumulate ? split_single(M, N, K, num_sms, narrow) : 1;
   if (g_force_ks > 0 && accumulate) ks = g_force_ks <= (K + GEMM_BK - 1) / GEMM_BK ? g_force_ks : (K + GEMM_BK - 1) / GEMM_BK;
 #define KB_GO(BN_)                                                                                         \

@@ -54,6 +54,22 @@ def test_weight_gradients_with_few_tiles_split_k():
     assert _plan(L, 2048, 3072, tokens, sms=32)[1] <= _plan(L, 2048, 3072, tokens, sms=148)[1]
 
 
+def test_kernel_choice_for_plain_outputs():
+    L = _lib()
+    L.kb_gemm_plan.argtypes = [ctypes.c_int] * 5
+    plan = lambda m, n, k, b_mn=0: L.kb_gemm_plan(m, n, k, b_mn, 148)
+    # one wave of 128-row tiles instead of two of pairs; latency-bound calls; K of up to two steps
+    assert plan(776, 5120, 3072) == -256
+    for m, n, k in [(104, 13760, 512), (1024, 4096, 512), (4096, 1024, 256), (2048, 1024, 128), (64, 1024, 128), (15720, 4344, 128)]:
+        assert plan(m, n, k) < 0, (m, n, k)
+    # long or wide problems stay on pairs of SMs, as do rows whose length is no multiple of 16 bytes
+    for m, n, k in [(16384, 16384, 3072), (16384, 3072, 8192), (16384, 640, 3072), (4096, 6144, 4096), (8192, 8192, 8192)]:
+        assert plan(m, n, k) > 0, (m, n, k)
+    assert plan(776, 5124, 3072) > 0
+    # an MN-major B of 192 columns comes in as many bytes as one of 256
+    assert plan(2048, 8192, 3072, 1) == 256
+
+
 def test_copy_driver_count_scales_with_output_width_and_budget():
     from kareus_b200.ops.fused import FusedAGGemm as F
     assert F.auto_drivers(12, 640) == 36 and F.auto_drivers(12, 1024) == 24 and F.auto_drivers(12, 2048) == 12
