@@ -547,9 +547,9 @@ static int launch_fwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     if (rc) return rc;
   }
   // Pairs of query tiles halve the K/V traffic; where single tiles already fit the chip in one wave, they halve the
-  // work of the longest CTA instead.
+  // work of the longest CTA instead.  One key tile cannot be shared, and the meeting of the warpgroups costs 0.5 us.
   const int n_q = (sq + FA_BM - 1) / FA_BM, bh = g * rep * b;
-  if ((long)n_q * bh <= device_sm_count()) return launch_variant<true>(tmQ, kv, tmO, p, bh * n_q, stream);
+  if (skv > FA_BN && (long)n_q * bh <= device_sm_count()) return launch_variant<true>(tmQ, kv, tmO, p, bh * n_q, stream);
   return launch_variant<false>(tmQ, kv, tmO, p, bh * ((n_q + 1) / 2), stream);
 }
 
