@@ -7,7 +7,8 @@
 // shape, a private copy of its argument values (tensor maps included) and the stream it ran on.
 // kb_replay() then re-issues the whole list from C++ with no interpreter in the loop, on the same
 // streams and with the same event edges, so the order in which kernels that wait on peer GPUs are
-// started stays exactly what it was when the list was recorded.
+// started stays exactly what it was when the list was recorded.  A list that stays on one stream and
+// carries no epochs has no such order to keep: it is re-issued as one CUDA graph.
 //
 // Per-call values: kernels of the peer-memory token protocol take a channel epoch that must grow
 // by one on every call.  The host keeps that counter in memory it names with
@@ -15,9 +16,9 @@
 // the kernel's arguments (EpochLoc), and a replay increments the counter and patches the copy of
 // the arguments before launching.
 //
-// This is the role CUDA graphs play elsewhere; an own list keeps explicit control of stream
-// assignment (two peer-waiting kernels must be started in the same order on every rank) and lets
-// the epochs be patched without per-node update calls.
+// For lists with side streams an own list does what a graph cannot: explicit control of stream
+// assignment (two peer-waiting kernels must be started in the same order on every rank), and epochs
+// that are patched without per-node update calls.
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>

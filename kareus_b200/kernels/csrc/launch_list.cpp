@@ -18,6 +18,7 @@
 //                                       Lists with side streams keep explicit stream order: kernels that wait on peer
 //                                       GPUs must start in the same order on every rank.
 //   kb_rec_launches(list)               kernels in the list (for launch accounting).
+//   kb_rec_is_graph(list)               1 once the list replays as a CUDA graph, 0 while it is issued op by op.
 //   kb_rec_free(list)
 #include "launch.h"
 
@@ -337,6 +338,11 @@ extern "C" long kb_rec_launches(int list) {
 extern "C" long kb_rec_ops(int list) {
   if (list < 1 || list > static_cast<int>(g_lists.size()) || !g_lists[list - 1]) return -1;
   return static_cast<long>(g_lists[list - 1]->ops.size());
+}
+
+extern "C" int kb_rec_is_graph(int list) {
+  if (list < 1 || list > static_cast<int>(g_lists.size()) || !g_lists[list - 1]) return -1;
+  return g_lists[list - 1]->graph != nullptr ? 1 : 0;
 }
 
 extern "C" int kb_rec_free(int list) {

@@ -5,7 +5,8 @@ ctypes; at eight GPUs the kernels are short enough that the interpreter, not the
 pace.  The arguments of those launches repeat from microbatch to microbatch, so the block engine
 records them once (``csrc/launch_list.cpp``: every launch, copy, memset, event record and stream
 wait issued by this library while a recording is open) and afterwards re-issues the list with one
-call: same kernels, same streams, same event edges, no interpreter in the loop.  The reference has
+call: same kernels, same streams, same event edges, no interpreter in the loop.  A list that stays
+on one stream is re-issued as a CUDA graph, any other op by op.  The reference has
 no counterpart: it pays the per-operator Python cost on every step
 (``kareus/megatron/core/partitions/partition_base.py:186-299``).
 
@@ -53,11 +54,12 @@ def _lib():
         L.kb_rec_launches.restype = c_long
         L.kb_rec_ops.argtypes = [I]
         L.kb_rec_ops.restype = c_long
+        L.kb_rec_is_graph.argtypes = [I]
         L.kb_rec_free.argtypes = [I]
         L.kb_memcpy_d2d.argtypes = [P, P, c_size_t, P]
         L.kb_memset.argtypes = [P, I, c_size_t, P]
         for n in ("kb_rec_begin", "kb_rec_abort", "kb_rec_new_event", "kb_rec_event_record", "kb_rec_stream_wait",
-                  "kb_rec_next_epoch", "kb_replay", "kb_rec_free", "kb_memcpy_d2d", "kb_memset"):
+                  "kb_rec_next_epoch", "kb_replay", "kb_rec_is_graph", "kb_rec_free", "kb_memcpy_d2d", "kb_memset"):
             getattr(L, n).restype = c_int
         _DECLARED = True
     return L
@@ -84,6 +86,11 @@ class LaunchList:
         rc = _lib().kb_replay(self.id, KC._stream())
         KC._check(rc, "launch-list replay")
         KC._count(self.launches)
+
+    @property
+    def is_graph(self) -> bool:
+        """True once a replay has turned the list into a CUDA graph."""
+        return _lib().kb_rec_is_graph(self.id) == 1
 
     def free(self) -> None:
         if self.id:

@@ -43,6 +43,89 @@ def test_replayed_steps_match_interpreted_steps():
     assert l_re[-1] < l_re[0]
 
 
+def _small_region(side=None):
+    """A GEMM, a device copy and a memset into given buffers, the copy on a side stream if there is one."""
+    from kareus_b200.kernels import cuda as KC, replay
+    a = torch.randn(64, 128, device="cuda").bfloat16()
+    w = torch.randn(72, 128, device="cuda").bfloat16()
+    c, d = torch.zeros(2, 64, 72, device="cuda").bfloat16()
+    e = torch.zeros(100, dtype=torch.uint8, device="cuda")
+    # the same event handles on both streams, as the engine records them
+    here, there = torch.cuda.Event(), torch.cuda.Event()
+
+    def body():
+        stream = torch.cuda.current_stream()
+        KC.gemm(a, w, out=c)
+        if side is None:
+            replay.memcpy(d, c)
+        else:
+            here.record(stream)
+            replay.note_event_record(here, stream)
+            side.wait_event(here)
+            replay.note_stream_wait(side, here)
+            with torch.cuda.stream(side):
+                replay.memcpy(d, c)
+            there.record(side)
+            replay.note_event_record(there, side)
+            stream.wait_event(there)
+            replay.note_stream_wait(stream, there)
+        KC._check(replay._lib().kb_memset(e.data_ptr(), 7, 100, KC._stream()), "memset")
+
+    def check(lst):
+        for _ in range(2):
+            a.normal_()
+            d.zero_()
+            e.zero_()
+            lst.replay()
+            torch.cuda.synchronize()
+            KC.check_status()
+            assert torch.equal(c, d) and (e == 7).all()
+            assert ((c.float() - a.float() @ w.float().t()).norm() / c.float().norm()).item() < 1e-2
+
+    with replay.Recording() as rec:
+        body()
+    torch.cuda.synchronize()
+    assert rec.result.launches == 1 and rec.result.ops >= 3 and not rec.result.is_graph
+    return rec.result, check
+
+
+def test_list_on_one_stream_replays_as_a_graph():
+    lst, check = _small_region()
+    check(lst)
+    assert lst.is_graph
+    lst.free()
+
+
+def test_training_regions_replay_as_graphs():
+    tr, batches = _trainer(True, layers=2, chunk=2)
+    tr.train_step(batches[0])
+    torch.cuda.synchronize()
+    lists = [r.lst for r in tr.model.decoder.engine._recorded.values()]
+    assert lists and all(lst.is_graph for lst in lists)
+
+
+def test_list_with_a_side_stream_is_issued_op_by_op():
+    lst, check = _small_region(torch.cuda.Stream())
+    check(lst)
+    assert not lst.is_graph
+    lst.free()
+
+
+def test_replay_inside_a_capture_of_the_callers():
+    """Both kinds of list put their operations into the caller's graph; the list's own graph is not launched there."""
+    for side in (None, torch.cuda.Stream()):
+        lst, check = _small_region(side)
+        check(lst)                                  # a list on one stream is a graph by now
+        s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.graph(g, stream=s):
+            lst.replay()
+        check(g)
+        check(lst)                                  # and outside again
+        del g
+        lst.free()
+
+
 def test_regions_with_per_call_state_stay_interpreted():
     """Dropout draws a new seed per call: such a block is never recorded."""
     tr, batches = _trainer(True, layers=2, chunk=2)
