@@ -249,26 +249,6 @@ __device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t taddr, const uint32_
                "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
 }
-// One 32-bit column / four columns of this warp's 32 lanes (lane i of the quarter ↔ thread i).
-__device__ __forceinline__ void tmem_st_32x32_x1(uint32_t taddr, uint32_t v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(v) : "memory");
-}
-__device__ __forceinline__ void tmem_ld_32x32_x4(uint32_t taddr, uint32_t (&r)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(taddr)
-               : "memory");
-}
-// Named barrier `id` over 128 threads that also tells every thread whether `ok` held on all of them.
-__device__ __forceinline__ bool bar128_all(int id, bool ok) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred P, Q;\n\tsetp.ne.u32 P, %2, 0;\n\tbar.red.and.pred Q, %1, 128, P;\n\tselp.u32 %0, 1, 0, Q;\n\t}"
-      : "=r"(r)
-      : "r"(id), "r"(static_cast<uint32_t>(ok))
-      : "memory");
-  return r != 0;
-}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
