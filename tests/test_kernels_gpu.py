@@ -18,7 +18,7 @@ def _rel(a, b):
 
 @pytest.mark.parametrize("M,N,K", [(128, 256, 64), (256, 512, 512), (384, 640, 3072), (1000, 328, 200),
                                    (4096, 3072, 1024), (130, 72, 136),
-                                   # long-K problems with at least one 256x256 tile per SM: the 256x256 kernel
+                                   # long-K problems with more than one wave of 256x256 tiles
                                    (4096, 4096, 4096), (4500, 4096, 2304)])
 @pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, False), (True, True)])
 def test_gemm_layouts(M, N, K, ta, tb):
@@ -310,6 +310,18 @@ def test_adamw_and_sumsq():
     assert abs(KC.sumsq(p).item() / p.double().pow(2).sum().item() - 1) < 1e-3
 
 
+@pytest.mark.parametrize("total", [0.0, 1e-14, 0.81, 1.0, 6.25, 1e30, float("inf"), float("nan")])
+@pytest.mark.parametrize("clip", [1.0, 0.3])
+def test_clip_scale_matches_torch_statements(total, clip):
+    """Norm and clipping factor in one launch against the statements it replaces; one rounding each in fp32."""
+    KC = _K()
+    t = torch.tensor(total, device="cuda")
+    norm, scale = KC.clip_scale(t, clip)
+    want = t.sqrt()
+    torch.testing.assert_close(norm, want, rtol=2e-7, atol=0, equal_nan=True)
+    torch.testing.assert_close(scale, torch.clamp(clip / (want + 1e-6), max=1.0).reshape(1), rtol=5e-7, atol=0, equal_nan=True)
+
+
 def test_bounded_wait_reports_timeout_status():
     """A status word records an expired wait and the context stays usable (host-side check of the
     status plumbing; no kernel is made to hang)."""
@@ -596,6 +608,13 @@ def test_chunked_attention_matches_reference(cp, c, b=2):
                 wv[j * c:(j + 1) * c].abs().max() == 0, ("dv", rank, j)
             if wk[j * c:(j + 1) * c].abs().max() == 0:      # chunk no local query can see: exact zeros
                 assert dkv[dk_base[j]:dk_base[j] + c].abs().max() == 0
+
+
+# more than 148 query tiles, so that they go in pairs: both chunks in one pair, and a middle pair of three tiles per chunk
+@pytest.mark.parametrize("cp,c,b", [(2, 128, 13), (2, 384, 6)])
+def test_chunked_attention_tile_pairs(cp, c, b):
+    assert 2 * c // 128 * 6 * b > _K().sm_count()
+    test_chunked_attention_matches_reference(cp, c, b)
 
 
 # enough (batch, group) pairs that the backward gives all query heads of a group to one CTA, which writes dK/dV itself
