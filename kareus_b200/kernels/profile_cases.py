@@ -11,6 +11,7 @@ Timing tables (CUDA events, no profiler; L2 flushed between launches):
 
     python -m kareus_b200.kernels.profile_cases gemm_table      # model GEMM shapes at TP 1 and TP 8, vs cuBLAS
     python -m kareus_b200.kernels.profile_cases attn_table      # flash attention forward/backward, vs the wheel
+    python -m kareus_b200.kernels.profile_cases small_table     # small calls: device and host time
     python -m torch.distributed.run --nproc-per-node N --master-addr 127.0.0.1 \
         -m kareus_b200.kernels.profile_cases fused                # the eight fused GEMM+collective kernels at TP N
 """
@@ -74,22 +75,29 @@ def gemm_table() -> None:
 
 
 def wgrad_sweep() -> None:
-    """Weight-gradient GEMMs (fp32 accumulate, K = 16384 tokens) of the 3B layer at TP 1/2/8 with every
-    tile (128 / 256 rows) and K split forced in turn; the last column is what the library picks by itself."""
+    """Weight-gradient GEMMs (fp32 accumulate, K = 16384 tokens) of the 3B layer at TP 1/2/8 with every tile width forced
+    in turn, each with the K split that the library picks for it; then what it picks by itself."""
     import ctypes
     from . import cuda as KC
     L = KC.lib()
-    L.kb_gemm_accum_force.argtypes = [ctypes.c_int, ctypes.c_int]
-    L.kb_gemm_accum_force.restype = None
+    L.kb_gemm_force_width.argtypes = [ctypes.c_int]
+    L.kb_gemm_force_width.restype = None
     L.kb_gemm_accum_plan.argtypes = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)] * 3
     L.kb_gemm_accum_plan.restype = None
     dev = "cuda"
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     tokens = 16384
-    splits = (1, 2, 3, 4, 6, 8)
-    print("| wgrad | out x in | " + " | ".join(f"{t}/ks{k}" for t in (128, 256) for k in splits)
-          + " | picked | picked TFLOP/s | cuBLAS TFLOP/s |")
-    print("|---|---|" + "---|" * (2 * len(splits) + 3))
+    widths = (64, 128, 192, 256)
+
+    def plan(n_out, n_in):
+        v = [ctypes.c_int() for _ in range(3)]
+        L.kb_gemm_accum_plan(n_out, n_in, tokens, KC.sm_count(), *[ctypes.byref(x) for x in v])
+        ordered = L.kb_gemm_accum_scratch_floats(n_out, n_in, tokens, 0) > 0
+        return v[0].value, v[1].value, "" if v[1].value == 1 else " in order" if ordered else " as they come"
+
+    print("| wgrad | out x in | " + " | ".join(f"{w} wide" for w in widths)
+          + " | picked (width, parts) | picked TFLOP/s | cuBLAS TFLOP/s |")
+    print("|---|---|" + "---|" * (len(widths) + 3))
     for tp in (1, 2, 8):
         shapes = {"qkv": (5120 // tp, 3072), "proj": (3072, 3072 // tp), "fc1": (16384 // tp, 3072),
                   "fc2": (3072, 8192 // tp)}
@@ -100,18 +108,15 @@ def wgrad_sweep() -> None:
             flops = 2.0 * tokens * n_out * n_in
             run = lambda: KC.gemm(dy, x, trans_a=True, trans_b=False, accumulate=acc)
             cells = []
-            for tile in (128, 256):
-                for ks in splits:
-                    L.kb_gemm_accum_force(tile, ks)
-                    cells.append(flops / _timed(run, flush, iters=5, skip=2) / 1e9)
-            L.kb_gemm_accum_force(0, 0)
+            for w in widths:
+                L.kb_gemm_force_width(w)
+                cells.append(f"{flops / _timed(run, flush, iters=5, skip=2) / 1e9:.0f}/{plan(n_out, n_in)[1]}")
+            L.kb_gemm_force_width(0)
             t_auto = _timed(run, flush)
             t_lib = _timed(lambda: torch.matmul(dy.t(), x), flush)
-            tile_c, ks_c, split_c = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
-            L.kb_gemm_accum_plan(n_out, n_in, tokens, KC.sm_count(),
-                                 ctypes.byref(tile_c), ctypes.byref(ks_c), ctypes.byref(split_c))
-            print(f"| tp{tp} {name} | {n_out} x {n_in} | " + " | ".join(f"{c:.0f}" for c in cells)
-                  + f" | {tile_c.value}/ks{ks_c.value} | {flops / t_auto / 1e9:.0f} | {flops / t_lib / 1e9:.0f} |")
+            bn, ks, how = plan(n_out, n_in)
+            print(f"| tp{tp} {name} | {n_out} x {n_in} | " + " | ".join(cells)
+                  + f" | {bn}, {ks}{how} | {flops / t_auto / 1e9:.0f} | {flops / t_lib / 1e9:.0f} |")
             del dy, x, acc
     KC.check_status()
 
@@ -169,6 +174,70 @@ def memory_table() -> None:
         t = _timed(fn, flush)
         gbs = nbytes / t / 1e6
         print(f"| {name} | {t * 1e3:.0f} | {nbytes / 1e6:.0f} | {gbs:.0f} | {gbs / hbm:.2f} |")
+    KC.check_status()
+
+
+def small_table() -> None:
+    """Small calls: device time (a CUDA graph of 20 calls) and host time per call (300 calls, nothing waited for), and the
+    smoke model's training step with and without launch lists."""
+    import time
+    from . import attention_cuda, cuda as KC
+    dev = "cuda"
+    rnd = lambda *shape: torch.randn(*shape, device=dev).bfloat16()
+    x, w, dy, acc = rnd(328, 1032), rnd(776, 1032), rnd(328, 776), torch.zeros(776, 1032, device=dev)
+    packed = rnd(459, 2, 2, 4 * 128)
+    q, k, v = packed[..., :256].unflatten(-1, (2, 128)), packed[..., 256:384], packed[..., 384:]
+    out, lse = attention_cuda.forward(q, k, v, 128 ** -0.5)
+    do = torch.randn_like(out)
+    xn, wn, gu = rnd(459, 2048), rnd(2048), rnd(459, 2 * 2048)
+    cases = [("gemm 328 x 776 x 1032", lambda: KC.gemm(x, w)),
+             ("its input gradient", lambda: KC.gemm(dy, w, trans_b=False)),
+             ("its weight gradient", lambda: KC.gemm(dy, x, trans_a=True, trans_b=False, accumulate=acc)),
+             ("attention forward, 2 x 459 tokens, 4/2 heads", lambda: attention_cuda.forward(q, k, v, 128 ** -0.5)),
+             ("attention backward", lambda: attention_cuda.backward(do, q, k, v, out, lse, 128 ** -0.5)),
+             ("rmsnorm forward 459 x 2048", lambda: KC.rmsnorm_fwd(xn, wn, 1e-5)),
+             ("swiglu forward 459 x 2048", lambda: KC.swiglu_fwd(gu))]
+    print("| call | device us | host us |\n|---|---|---|")
+    side = torch.cuda.Stream()
+    for name, fn in cases:
+        with torch.cuda.stream(side):
+            fn()
+            side.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=side):
+                for _ in range(20):
+                    fn()
+            best = []
+            for _ in range(9):
+                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                a.record()
+                graph.replay()
+                b.record()
+                b.synchronize()
+                best.append(a.elapsed_time(b) * 50)
+            t0 = time.perf_counter()
+            for _ in range(300):
+                fn()
+            host = (time.perf_counter() - t0) / 300 * 1e6
+            side.synchronize()
+        print(f"| {name} | {sorted(best)[4]:.1f} | {host:.1f} |")
+        del graph
+    from ..config import ParallelConfig, TrainConfig, get_model_config
+    from ..train.trainer import Trainer, synthetic_batch
+    cfg = get_model_config("tiny128")
+    tc = TrainConfig(micro_batch_size=2, global_batch_size=4, seq_len=256, warmup_steps=0)
+    for lists in (False, True):
+        tr = Trainer(cfg, ParallelConfig(num_nanobatches=2, recompute=True), tc, device=dev)
+        tr.model.decoder.engine.replay = lists
+        batch = synthetic_batch(cfg, tc, tr.num_microbatches, seed=0)
+        for _ in range(5):
+            tr.train_step(batch)
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        for _ in range(30):
+            tr.train_step(batch)
+        torch.cuda.synchronize()
+        print(f"| training step of tiny128, launch lists {'on' if lists else 'off'} | | {(time.perf_counter() - t0) / 30 * 1e6:.0f} |")
     KC.check_status()
 
 
@@ -364,8 +433,8 @@ def collectives_table() -> None:
 
 
 # every command of this module: tables (CUDA events) and single-kernel cases (for a profiler capture)
-CASES = ("collectives", "memory_table", "wgrad_sweep", "gemm_table", "attn_table", "fused", "gemm", "gemm_wgrad",
-         "attn_fwd", "attn_bwd", "norm", "swiglu", "rope", "ce", "adamw", "step")
+CASES = ("collectives", "memory_table", "small_table", "wgrad_sweep", "gemm_table", "attn_table", "fused", "gemm",
+         "gemm_one_sm", "gemm_wgrad", "attn_fwd", "attn_bwd", "norm", "swiglu", "rope", "ce", "adamw", "step")
 
 
 def main(case: str, reps: int = 3) -> None:
@@ -383,6 +452,8 @@ def main(case: str, reps: int = 3) -> None:
         return gemm_table()
     if case == "attn_table":
         return attn_table()
+    if case == "small_table":
+        return small_table()
     if case == "fused":
         return fused_table()
     if case == "gemm":
@@ -390,6 +461,12 @@ def main(case: str, reps: int = 3) -> None:
         b = torch.randn(8192, 8192, device=dev).bfloat16()
         for _ in range(reps):
             KC.gemm(a, b)
+    elif case == "gemm_one_sm":
+        a = torch.randn(8192, 8192, device=dev).bfloat16()
+        b = torch.randn(8192, 8192, device=dev).bfloat16()
+        bias = torch.randn(8192, device=dev).bfloat16()
+        for _ in range(reps):
+            KC.gemm(a, b, bias=bias)               # the bias epilogue runs on the one-SM kernel
     elif case == "gemm_wgrad":
         dy = torch.randn(16384, 3072, device=dev).bfloat16()
         x = torch.randn(16384, 8192, device=dev).bfloat16()
