@@ -484,10 +484,10 @@ static int single_width(int M, int N, int K, bool b_mn, int num_sms, int pair_bn
   };
   const double* c = pair_us[pair_bn / 64];
   // an MN-major B comes in 64-wide chunks, of which 64-wide tiles use half
-  const double pair = c[2] + (b_mn && pair_bn == 64 ? 0.4 : 0.0) + waves(M, N, 256, pair_bn, num_sms / 2) * (nk * c[0] + c[1]);
+  const double pair = c[2] + (b_mn && pair_bn == 64 ? 0.6 : 0.0) + waves(M, N, 256, pair_bn, num_sms / 2) * (nk * c[0] + c[1]);
   const double w128 = 3.5 + waves(M, N, 128, 128, num_sms) * (nk * 0.275 + 0.95);
   const double w256 = 3.2 + waves(M, N, 128, 256, num_sms) * (nk * 0.337 + 2.2);
-  if (nk > 2 && (w128 < w256 ? w128 : w256) >= (b_mn ? 1.0 : 0.97) * pair) return 0;
+  if (nk > 2 && (w128 < w256 ? w128 : w256) >= 0.97 * pair) return 0;
   return w128 < w256 ? 128 : 256;
 }
 
