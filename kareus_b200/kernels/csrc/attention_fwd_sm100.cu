@@ -9,7 +9,8 @@
 //   warp 9      MMA issuer (warps 10 and 11 fill its warpgroup): S = Q·Kᵀ (both operands from shared memory) and O += P·V (P from TMEM)
 // The two query tiles alternate: while one is in its softmax the tensor cores work on the other.
 // Where single query tiles already fit the chip in one wave, a CTA has one (its share is half as long) and the two softmax
-// warpgroups take its even and odd key tiles, each with its own scores, O, maximum and sum; they meet in the epilogue.
+// warpgroups take its even and odd key tiles, each with its own scores, O, maximum and sum; they meet in the epilogue
+// (616 queries against 9448 keys, 2 x 8 heads: 121 us with one warpgroup, 78 with both; 4096 tokens, one head: 53 and 34).
 // TMEM: S|P and O of both tiles, 4 x 128 columns.  S of the next key tile is issued behind the P·V that
 // read P, so its arrival also says that O may be touched; O is rescaled only when the running maximum
 // moves by more than 2^8 ("lazy rescale"), which happens on the first tiles only.
