@@ -3,6 +3,7 @@
 // other activation operators (kareus/megatron/core/extensions/ops/bias_gelu.py, bias_geglu.py).
 #include <cuda_bf16.h>
 #include "launch.h"
+#include "pdl.cuh"
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -19,6 +20,7 @@ __device__ __forceinline__ float gelu_df(float x) {
 // mode 0: y = gelu(x) over n elements.  mode 1: x = [gate | up] rows of 2F, y = gelu(gate) * up.
 __global__ void gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long rows, int F,
                                 int gated) {
+  pdl_begin();
   const long total = rows * F;
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
@@ -34,6 +36,7 @@ __global__ void gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat
 }
 __global__ void gelu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                 __nv_bfloat16* __restrict__ dx, long rows, int F, int gated) {
+  pdl_begin();
   const long total = rows * F;
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
@@ -56,7 +59,7 @@ extern "C" int kb_gelu_fwd(const void* x, void* y, long rows, int F, int gated, 
   long b = (rows * F + 255) / 256;
   if (b > 148 * 16) b = 148 * 16;
   if (b < 1) b = 1;
-  KB_LAUNCH(kb::gelu_fwd_kernel, (int)b, 256, 0, st, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, rows, F, gated);
+  KB_LAUNCH_PDL(kb::gelu_fwd_kernel, (int)b, 256, 0, st, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, rows, F, gated);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + (int)e;
 }
@@ -64,7 +67,7 @@ extern "C" int kb_gelu_bwd(const void* dy, const void* x, void* dx, long rows, i
   long b = (rows * F + 255) / 256;
   if (b > 148 * 16) b = 148 * 16;
   if (b < 1) b = 1;
-  KB_LAUNCH(kb::gelu_bwd_kernel, (int)b, 256, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (__nv_bfloat16*)dx, rows,
+  KB_LAUNCH_PDL(kb::gelu_bwd_kernel, (int)b, 256, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (__nv_bfloat16*)dx, rows,
                                               F, gated);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + (int)e;

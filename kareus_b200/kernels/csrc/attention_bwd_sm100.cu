@@ -35,6 +35,7 @@
 // (kareus/flash_attn/flash_attn_interface.py:147-199).
 #include "sm100.cuh"
 #include "launch.h"
+#include "pdl.cuh"
 #include "host_utils.h"
 #include "attention_chunks.h"
 #include <string.h>
@@ -141,6 +142,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   if (smem - smem_raw + FbSmem::USED > FbSmem::TOTAL) {   // the same for all threads
+    pdl_wait();
     if (threadIdx.x == 0) atomicCAS(p.status, 0, ST_BAD_ARG);
     return;
   }
@@ -184,6 +186,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_begin();
   // Pᵀ of query chunk c goes into the first 16 of the 32 columns of its scores.  dQ of a tile goes where its dPᵀ
   // was: that has been read by then.
   const uint32_t t_s = tmem_base, t_dp = tmem_base + 128, t_dv = tmem_base + 256, t_dk = tmem_base + 384;
@@ -515,6 +518,7 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __r
                   const float* __restrict__ lse, float* __restrict__ stats, float4* __restrict__ dq_acc,
                   float4* __restrict__ zero, long n_zero, unsigned S, unsigned S_pad, unsigned B, unsigned H, float scale,
                   bool wide) {
+  pdl_begin();
   const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_zero;
        i += static_cast<long>(gridDim.x) * blockDim.x)
@@ -575,6 +579,7 @@ struct Convert {
 __global__ void __launch_bounds__(256)
 attn_convert_kernel(const __grid_constant__ Convert dq, const __grid_constant__ Convert dk, const __grid_constant__ Convert dv,
                     unsigned B) {
+  pdl_begin();
   const int l = threadIdx.x & 15;
   const unsigned step = (gridDim.x * blockDim.x) >> 4, total = dq.rows + dk.rows + dv.rows;
   auto convert = [&](const Convert& c, unsigned w) {
@@ -662,7 +667,7 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     const long rows = (long)s_pad * b * hq;
     long blocks = (rows * 16 + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    KB_LAUNCH(attn_stats_kernel, (int)blocks, 256, 0, stream, (const __nv_bfloat16*)dO, (const __nv_bfloat16*)o, lse, stats,
+    KB_LAUNCH_PDL(attn_stats_kernel, (int)blocks, 256, 0, stream, (const __nv_bfloat16*)dO, (const __nv_bfloat16*)o, lse, stats,
               reinterpret_cast<float4*>(dq_acc), reinterpret_cast<float4*>(dk_acc), merged ? 0L : 2 * n_dkv / 4, sq, s_pad, b, hq, scale,
               (reinterpret_cast<uintptr_t>(o) & 15) == 0);
   }
@@ -697,7 +702,7 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
   }
   if (n_kv > 0) {
     const dim3 grid((unsigned)(hq / p.heads * b) * n_kv);
-    KB_LAUNCH(flash_attn_bwd_kernel, grid, FB_THREADS, FbSmem::TOTAL, stream, tmQ, kv, tmDO, tmDQ, p);
+    KB_LAUNCH_PDL(flash_attn_bwd_kernel, grid, FB_THREADS, FbSmem::TOTAL, stream, tmQ, kv, tmDO, tmDQ, p);
   }
   {
     auto segment = [&](const float* acc, void* dst, long rows, int r, long st_s, long st_b, long st_g, long st_r,
@@ -712,7 +717,7 @@ static int launch_bwd(const CUtensorMap& tmQ, const KvMaps& kv, const ChunkGeom&
     const Convert ck = segment(dk_acc, out.dk, kv_rows, 1, out.dks_s, out.dks_b, out.dks_g, 0, out.dk_rows);
     const Convert cv = segment(dv_acc, out.dv, kv_rows, 1, out.dvs_s, out.dvs_b, out.dvs_g, 0, out.dv_rows);
     const long blocks = (((long)sq * b * hq + 2 * kv_rows) * 16 + 255) / 256;
-    KB_LAUNCH(attn_convert_kernel, (int)blocks, 256, 0, stream, cq, ck, cv, (unsigned)b);
+    KB_LAUNCH_PDL(attn_convert_kernel, (int)blocks, 256, 0, stream, cq, ck, cv, (unsigned)b);
   }
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + (int)e;

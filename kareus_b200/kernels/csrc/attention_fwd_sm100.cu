@@ -36,6 +36,7 @@
 // kareus/transformer_engine/pytorch/attention/dot_product_attention/backends.py:179-186,328-333).
 #include "sm100.cuh"
 #include "launch.h"
+#include "pdl.cuh"
 #include "host_utils.h"
 #include <string.h>
 
@@ -148,6 +149,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_begin();
   const uint32_t tmem_base = *tmem_slot;     // S|P of tile t at 128 t, O of tile t at 256 + 128 t
 
   if (warp >= 8) {
@@ -520,7 +522,7 @@ static int launch_variant(const CUtensorMap& tmQ, const KvMaps& kv, const CUtens
     if (attr.numRegs * FA_THREADS < FA_REGS_TOTAL) return ST_BAD_ARG;   // the register split would wait forever
     configured = true;
   }
-  KB_LAUNCH(kern, (unsigned)ctas, FA_THREADS, FaSmem::TOTAL, stream, tmQ, kv, tmO, p);
+  KB_LAUNCH_PDL(kern, (unsigned)ctas, FA_THREADS, FaSmem::TOTAL, stream, tmQ, kv, tmO, p);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + (int)e;
 }

@@ -7,6 +7,7 @@
 //   fused AdamW over flat buffers, sum of squares (reference: TE/Apex multi_tensor kernels)
 #include <cuda_bf16.h>
 #include "launch.h"
+#include "pdl.cuh"
 #include "host_utils.h"
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -93,6 +94,7 @@ template <int THREADS, int VPT>
 __global__ void __launch_bounds__(THREADS)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int rows, int H, float eps) {
+  pdl_begin();
   constexpr int NORM_THREADS = THREADS;
   constexpr int NORM_VPT = VPT;
   __shared__ float red[64];
@@ -174,6 +176,7 @@ template <int VPL>
 __global__ void __launch_bounds__(256)
 rmsnorm_fwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                         __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int rows, int H, float eps) {
+  pdl_begin();
   const int lane = threadIdx.x & 31, nvec = H >> 3;
   const uint4* wr = reinterpret_cast<const uint4*>(w);
   for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += gridDim.x * 8) {
@@ -212,6 +215,7 @@ __global__ void __launch_bounds__(256)
 rmsnorm_fwd_heads_kernel(const __nv_bfloat16* __restrict__ x, unsigned inner, long st_outer, long st_inner,
                          const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, float* __restrict__ rstd,
                          unsigned rows, int H, float eps) {
+  pdl_begin();
   const unsigned lanes = H >> 3, per_warp = 32 / lanes, lane = threadIdx.x & 31;
   const unsigned sub = lane / lanes, l = lane - sub * lanes;
   const unsigned step = gridDim.x * 8 * per_warp;
@@ -242,6 +246,7 @@ rmsnorm_fwd_heads_kernel(const __nv_bfloat16* __restrict__ x, unsigned inner, lo
 __global__ void rmsnorm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                         __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int rows, int H,
                                         float eps) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < rows; row += gridDim.x * wpb) {
@@ -266,6 +271,7 @@ __global__ void __launch_bounds__(THREADS)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ w,
                    __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows, int H) {
+  pdl_begin();
   constexpr int NORM_THREADS = THREADS;
   constexpr int NORM_VPT = VPT;
   __shared__ float red[64];
@@ -357,6 +363,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 // `accumulate`: add the sums to dw (the fp32 main gradient of the weight) instead of storing them.
 __global__ void __launch_bounds__(1024)
 rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int nparts, int H, int accumulate) {
+  pdl_begin();
   __shared__ float sum[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
@@ -376,6 +383,7 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ 
 __global__ void rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                         const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ w,
                                         __nv_bfloat16* __restrict__ dx, float* __restrict__ dw, int rows, int H) {
+  pdl_begin();
   extern __shared__ float sdw[];
   for (int c = threadIdx.x; c < H; c += blockDim.x) sdw[c] = 0.f;
   __syncthreads();
@@ -409,6 +417,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ q, long qs_s, long qs_b,
                             __nv_bfloat16* __restrict__ k, long ks_s, long ks_b, long ks_g, int KG,
                             const float* __restrict__ cosb, const float* __restrict__ sinb, int S, int B, int D,
                             float sign) {
+  pdl_begin();
   const int heads = G * R + KG;
   const long total = static_cast<long>(S) * B * heads;
   const int lane = threadIdx.x & 31;
@@ -446,6 +455,7 @@ __global__ void __launch_bounds__(256)
 rope_vec_kernel(__nv_bfloat16* __restrict__ q, long qs_s, long qs_b, long qs_g, long qs_r, int G, int R,
                 __nv_bfloat16* __restrict__ k, long ks_s, long ks_b, long ks_g, int KG,
                 const float* __restrict__ cosb, const float* __restrict__ sinb, int S, int B, int D, float sign) {
+  pdl_begin();
   const int lanes_per_head = D >> 4;                 // 8 for D = 128
   const int groups = 32 / lanes_per_head;
   const int lane = threadIdx.x & 31;
@@ -495,6 +505,7 @@ rope_vec_kernel(__nv_bfloat16* __restrict__ q, long qs_s, long qs_b, long qs_g, 
 template <typename Index>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, Index total, Index fv) {
+  pdl_begin();
   const uint4* xv = reinterpret_cast<const uint4*>(x);
   for (Index i = static_cast<Index>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<Index>(gridDim.x) * blockDim.x) {
@@ -512,6 +523,7 @@ template <typename Index>
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                   __nv_bfloat16* __restrict__ dx, Index total, Index fv) {
+  pdl_begin();
   const uint4* xv = reinterpret_cast<const uint4*>(x);
   for (Index i = static_cast<Index>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<Index>(gridDim.x) * blockDim.x) {
@@ -545,6 +557,7 @@ __device__ __forceinline__ uint32_t hash32(uint64_t idx, uint32_t seed) {
 // function of (seed, e), so backward regenerates it.
 __global__ void dropout_add_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                                        __nv_bfloat16* __restrict__ y, long nvec, float p, uint32_t seed) {
+  pdl_begin();
   const float scale = p > 0.f ? 1.f / (1.f - p) : 1.f;
   const uint32_t thr = static_cast<uint32_t>(p * 4294967296.0);
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec;
@@ -563,6 +576,7 @@ __global__ void dropout_add_fwd_kernel(const __nv_bfloat16* __restrict__ x, cons
 }
 __global__ void dropout_bwd_kernel(const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx, long nvec,
                                    float p, uint32_t seed) {
+  pdl_begin();
   const float scale = 1.f / (1.f - p);
   const uint32_t thr = static_cast<uint32_t>(p * 4294967296.0);
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec;
@@ -576,6 +590,7 @@ __global__ void dropout_bwd_kernel(const __nv_bfloat16* __restrict__ dy, __nv_bf
 }
 __global__ void add_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                            __nv_bfloat16* __restrict__ y, long nvec) {
+  pdl_begin();
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
     float x[8], z[8];
@@ -590,6 +605,7 @@ __global__ void add_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloa
 // ----------------------------------------------------------------------------- embedding
 __global__ void embedding_fwd_kernel(const long* __restrict__ tokens, const __nv_bfloat16* __restrict__ w,
                                      __nv_bfloat16* __restrict__ out, long ntok, int H, long vocab_start, long vlocal) {
+  pdl_begin();
   const int hv = H >> 3;
   for (long t = blockIdx.x; t < ntok; t += gridDim.x) {
     const long id = tokens[t] - vocab_start;
@@ -604,6 +620,7 @@ __global__ void embedding_fwd_kernel(const long* __restrict__ tokens, const __nv
 __global__ void __launch_bounds__(256)
 embedding_bwd_kernel(const long* __restrict__ tokens, const __nv_bfloat16* __restrict__ dout, float* __restrict__ gw,
                      long ntok, int H, long vocab_start, long vlocal, bool wide) {
+  pdl_begin();
   for (long t = blockIdx.x; t < ntok; t += gridDim.x) {
     const long id = tokens[t] - vocab_start;
     if (id < 0 || id >= vlocal) continue;
@@ -643,6 +660,7 @@ __device__ __forceinline__ void exp_pairs(const uint4& u, float base, float2 (&e
 __global__ void __launch_bounds__(CE_THREADS)
 ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restrict__ targets, float* __restrict__ omax,
                 float* __restrict__ osum, float* __restrict__ otgt, long rows, int V, long vocab_start) {
+  pdl_begin();
   __shared__ float red[32];
   for (long row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* lr = logits + row * V;
@@ -698,6 +716,7 @@ ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restrict
 __global__ void __launch_bounds__(CE_THREADS)
 ce_grad_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ targets, const float* __restrict__ gmax,
                const float* __restrict__ gsum, const float* __restrict__ scale, long rows, int V, long vocab_start) {
+  pdl_begin();
   for (long row = blockIdx.x; row < rows; row += gridDim.x) {
     __nv_bfloat16* lr = logits + row * V;
     const int vv = reinterpret_cast<uintptr_t>(lr) & 15 ? 0 : V >> 3;
@@ -749,6 +768,7 @@ __global__ void adamw_kernel(__nv_bfloat16* __restrict__ p, const float* __restr
                              float* __restrict__ v, float* __restrict__ master, long n, float lr, float b1, float b2,
                              float eps, float wd, float bc1, float bc2, const float* __restrict__ grad_scale_ptr,
                              float grad_scale) {
+  pdl_begin();
   const float gs = grad_scale_ptr ? grad_scale * (*grad_scale_ptr) : grad_scale;
   const long n4 = n >> 2;
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
@@ -790,6 +810,7 @@ __global__ void adamw_kernel(__nv_bfloat16* __restrict__ p, const float* __restr
 
 // out[0] += sum(x^2)  (fp32 input); out must be zeroed by the caller.
 __global__ void sumsq_f32_kernel(const float* __restrict__ x, long n, float* __restrict__ out) {
+  pdl_begin();
   __shared__ float red[32];
   float s = 0.f;
   const long n4 = n >> 2;
@@ -813,6 +834,7 @@ __global__ void sumsq_f32_kernel(const float* __restrict__ x, long n, float* __r
   if (threadIdx.x == 0) atomicAdd(out, tot);
 }
 __global__ void sumsq_bf16_kernel(const __nv_bfloat16* __restrict__ x, long n, float* __restrict__ out) {
+  pdl_begin();
   __shared__ float red[32];
   float s = 0.f;
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
@@ -903,7 +925,7 @@ extern "C" int kb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd
     const int grid = grid_for(rows, 8, 148 * 8);
     const int vpl = (H / 8 + 31) / 32;
 #define KB_ROWS(V_)                                                                                               \
-    KB_LAUNCH((rmsnorm_fwd_rows_kernel<V_>), grid, 256, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,    \
+    KB_LAUNCH_PDL((rmsnorm_fwd_rows_kernel<V_>), grid, 256, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,    \
               (__nv_bfloat16*)y, rstd, rows, H, eps)
     if (vpl <= 4) KB_ROWS(4);
     else if (vpl <= 8) KB_ROWS(8);
@@ -913,12 +935,12 @@ extern "C" int kb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd
     const NormVariant nv = norm_variant(H);
     const int grid = grid_for(rows, 1, norm_fwd_ctas(H));          // one resident wave: rows are dealt evenly
 #define KB_FWD(T_, V_)                                                                                            \
-    KB_LAUNCH((rmsnorm_fwd_kernel<T_, V_>), grid, T_, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,      \
+    KB_LAUNCH_PDL((rmsnorm_fwd_kernel<T_, V_>), grid, T_, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,      \
               (__nv_bfloat16*)y, rstd, rows, H, eps)
     KB_NORM_DISPATCH(nv, KB_FWD)
 #undef KB_FWD
   } else {
-    KB_LAUNCH(rmsnorm_fwd_warp_kernel, grid_for(rows, 8, 148 * 8), 256, 0, st, 
+    KB_LAUNCH_PDL(rmsnorm_fwd_warp_kernel, grid_for(rows, 8, 148 * 8), 256, 0, st, 
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rstd, rows, H, eps);
   }
   KB_CHECK_LAUNCH();
@@ -934,7 +956,7 @@ extern "C" int kb_rmsnorm_fwd_heads(const void* x, long outer, int inner, long s
   if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) ||
       ((st_outer | st_inner) & 7))
     return 7;
-  KB_LAUNCH(rmsnorm_fwd_heads_kernel, grid_for(rows * lanes, 256, 148 * 8), 256, 0, st, (const __nv_bfloat16*)x, inner,
+  KB_LAUNCH_PDL(rmsnorm_fwd_heads_kernel, grid_for(rows * lanes, 256, 148 * 8), 256, 0, st, (const __nv_bfloat16*)x, inner,
             st_outer, st_inner, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rstd, (unsigned)rows, H, eps);
   KB_CHECK_LAUNCH();
 }
@@ -943,6 +965,7 @@ extern "C" int kb_rmsnorm_fwd_heads(const void* x, long outer, int inner, long s
 namespace kb {
 __global__ void __launch_bounds__(256)
 scale_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ s, __nv_bfloat16* __restrict__ y, long nvec) {
+  pdl_begin();
   const float f = __bfloat162float(__float2bfloat16(*s));
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
@@ -956,7 +979,7 @@ scale_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ s, _
 }  // namespace kb
 extern "C" int kb_scale(const void* x, const float* s, void* y, long n, cudaStream_t st) {
   if (n % 8) return 7;
-  KB_LAUNCH(scale_kernel, grid_for(n / 8, 256, 148 * 16), 256, 0, st, (const __nv_bfloat16*)x, s, (__nv_bfloat16*)y, n / 8);
+  KB_LAUNCH_PDL(scale_kernel, grid_for(n / 8, 256, 148 * 16), 256, 0, st, (const __nv_bfloat16*)x, s, (__nv_bfloat16*)y, n / 8);
   KB_CHECK_LAUNCH();
 }
 
@@ -975,14 +998,14 @@ extern "C" int kb_rmsnorm_bwd_acc(const void* dy, const void* x, const float* rs
     const int grid = grid_for(rows, 1, norm_bwd_ctas(H));          // must match kb_rmsnorm_bwd_scratch_elems
     if (!scratch) return 7;
 #define KB_BWD(T_, V_)                                                                                              \
-    KB_LAUNCH((rmsnorm_bwd_kernel<T_, V_>), grid, T_, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, rstd, \
+    KB_LAUNCH_PDL((rmsnorm_bwd_kernel<T_, V_>), grid, T_, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, rstd, \
               (const __nv_bfloat16*)w, (__nv_bfloat16*)dx, scratch, rows, H)
     KB_NORM_DISPATCH(nv, KB_BWD)
 #undef KB_BWD
-    KB_LAUNCH(rmsnorm_dw_reduce_kernel, (H + 31) / 32, 1024, 0, st, scratch, dw, grid, H, accumulate);
+    KB_LAUNCH_PDL(rmsnorm_dw_reduce_kernel, (H + 31) / 32, 1024, 0, st, scratch, dw, grid, H, accumulate);
   } else {
     if (!accumulate) kb::memset_async(dw, 0, sizeof(float) * H, st);    // the kernel adds with atomics
-    KB_LAUNCH(rmsnorm_bwd_warp_kernel, grid_for(rows, 8, 148 * 4), 256, sizeof(float) * H, st, 
+    KB_LAUNCH_PDL(rmsnorm_bwd_warp_kernel, grid_for(rows, 8, 148 * 4), 256, sizeof(float) * H, st, 
         (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, rstd, (const __nv_bfloat16*)w, (__nv_bfloat16*)dx, dw,
         rows, H);
   }
@@ -1004,14 +1027,14 @@ extern "C" int kb_rope(void* q, long qs_s, long qs_b, long qs_g, long qs_r, int 
                     (reinterpret_cast<uintptr_t>(q) & 15) == 0 && (k == nullptr || (reinterpret_cast<uintptr_t>(k) & 15) == 0);
     if (al && D % 16 == 0 && D >= 16 && D <= 512 && (32 % (D / 16)) == 0) {
       const long tokens = (long)S * B;
-      KB_LAUNCH(rope_vec_kernel, grid_for(tokens * 32, 256, 148 * 8), 256, 0, st,
+      KB_LAUNCH_PDL(rope_vec_kernel, grid_for(tokens * 32, 256, 148 * 8), 256, 0, st,
           (__nv_bfloat16*)q, qs_s, qs_b, qs_g, qs_r, G, R, (__nv_bfloat16*)k, ks_s, ks_b, ks_g, KG, cosb, sinb, S, B, D,
           inverse ? -1.f : 1.f);
       KB_CHECK_LAUNCH();
     }
   }
   const long warps = (long)S * B * (G * R + KG);
-  KB_LAUNCH(rope_kernel, grid_for(warps * 32, 256, 148 * 16), 256, 0, st, 
+  KB_LAUNCH_PDL(rope_kernel, grid_for(warps * 32, 256, 148 * 16), 256, 0, st, 
       (__nv_bfloat16*)q, qs_s, qs_b, qs_g, qs_r, G, R, (__nv_bfloat16*)k, ks_s, ks_b, ks_g, KG, cosb, sinb, S, B, D,
       inverse ? -1.f : 1.f);
   KB_CHECK_LAUNCH();
@@ -1022,8 +1045,8 @@ extern "C" int kb_swiglu_fwd(const void* x, void* y, long rows, int F, cudaStrea
   const long total = rows * (F / 8);
   const int grid = grid_for(total, 256, 148 * 16);
   const __nv_bfloat16* xb = (const __nv_bfloat16*)x;
-  if (total < (1L << 31)) KB_LAUNCH(swiglu_fwd_kernel<unsigned>, grid, 256, 0, st, xb, (__nv_bfloat16*)y, (unsigned)total, F / 8);
-  else KB_LAUNCH(swiglu_fwd_kernel<long>, grid, 256, 0, st, xb, (__nv_bfloat16*)y, total, F / 8);
+  if (total < (1L << 31)) KB_LAUNCH_PDL(swiglu_fwd_kernel<unsigned>, grid, 256, 0, st, xb, (__nv_bfloat16*)y, (unsigned)total, F / 8);
+  else KB_LAUNCH_PDL(swiglu_fwd_kernel<long>, grid, 256, 0, st, xb, (__nv_bfloat16*)y, total, F / 8);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_swiglu_bwd(const void* dy, const void* x, void* dx, long rows, int F, cudaStream_t st) {
@@ -1031,65 +1054,65 @@ extern "C" int kb_swiglu_bwd(const void* dy, const void* x, void* dx, long rows,
   const long total = rows * (F / 8);
   const int grid = grid_for(total, 256, 148 * 16);
   const __nv_bfloat16 *g = (const __nv_bfloat16*)dy, *xb = (const __nv_bfloat16*)x;
-  if (total < (1L << 31)) KB_LAUNCH(swiglu_bwd_kernel<unsigned>, grid, 256, 0, st, g, xb, (__nv_bfloat16*)dx, (unsigned)total, F / 8);
-  else KB_LAUNCH(swiglu_bwd_kernel<long>, grid, 256, 0, st, g, xb, (__nv_bfloat16*)dx, total, F / 8);
+  if (total < (1L << 31)) KB_LAUNCH_PDL(swiglu_bwd_kernel<unsigned>, grid, 256, 0, st, g, xb, (__nv_bfloat16*)dx, (unsigned)total, F / 8);
+  else KB_LAUNCH_PDL(swiglu_bwd_kernel<long>, grid, 256, 0, st, g, xb, (__nv_bfloat16*)dx, total, F / 8);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_dropout_add_fwd(const void* x, const void* res, void* y, long n, float p, unsigned seed,
                                   cudaStream_t st) {
   if (n % 8) return 7;
-  KB_LAUNCH(dropout_add_fwd_kernel, grid_for(n / 8, 256, 148 * 16), 256, 0, st, 
+  KB_LAUNCH_PDL(dropout_add_fwd_kernel, grid_for(n / 8, 256, 148 * 16), 256, 0, st, 
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (__nv_bfloat16*)y, n / 8, p, seed);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_dropout_bwd(const void* dy, void* dx, long n, float p, unsigned seed, cudaStream_t st) {
   if (n % 8) return 7;
-  KB_LAUNCH(dropout_bwd_kernel, grid_for(n / 8, 256, 148 * 16), 256, 0, st, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx,
+  KB_LAUNCH_PDL(dropout_bwd_kernel, grid_for(n / 8, 256, 148 * 16), 256, 0, st, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx,
                                                                       n / 8, p, seed);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_add(const void* a, const void* b, void* y, long n, cudaStream_t st) {
   if (n % 8) return 7;
-  KB_LAUNCH(add_kernel, grid_for(n / 8, 256, 148 * 16), 256, 0, st, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
+  KB_LAUNCH_PDL(add_kernel, grid_for(n / 8, 256, 148 * 16), 256, 0, st, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
                                                               (__nv_bfloat16*)y, n / 8);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_embedding_fwd(const long* tokens, const void* w, void* out, long ntok, int H, long vocab_start,
                                 long vlocal, cudaStream_t st) {
   if (H % 8) return 7;
-  KB_LAUNCH(embedding_fwd_kernel, grid_for(ntok, 1, 148 * 16), 128, 0, st, tokens, (const __nv_bfloat16*)w,
+  KB_LAUNCH_PDL(embedding_fwd_kernel, grid_for(ntok, 1, 148 * 16), 128, 0, st, tokens, (const __nv_bfloat16*)w,
                                                                      (__nv_bfloat16*)out, ntok, H, vocab_start, vlocal);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_embedding_bwd(const long* tokens, const void* dout, float* gw, long ntok, int H, long vocab_start,
                                 long vlocal, cudaStream_t st) {
   const bool wide = H % 4 == 0 && (reinterpret_cast<uintptr_t>(gw) & 15) == 0 && (reinterpret_cast<uintptr_t>(dout) & 7) == 0;
-  KB_LAUNCH(embedding_bwd_kernel, grid_for(ntok, 1, 148 * 16), 256, 0, st, tokens, (const __nv_bfloat16*)dout, gw, ntok, H,
+  KB_LAUNCH_PDL(embedding_bwd_kernel, grid_for(ntok, 1, 148 * 16), 256, 0, st, tokens, (const __nv_bfloat16*)dout, gw, ntok, H,
                                                                      vocab_start, vlocal, wide);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_ce_stats(const void* logits, const long* targets, float* omax, float* osum, float* otgt, long rows,
                            int V, long vocab_start, cudaStream_t st) {
-  KB_LAUNCH(ce_stats_kernel, grid_for(rows, 1, 148 * 4), CE_THREADS, 0, st, (const __nv_bfloat16*)logits, targets, omax, osum,
+  KB_LAUNCH_PDL(ce_stats_kernel, grid_for(rows, 1, 148 * 4), CE_THREADS, 0, st, (const __nv_bfloat16*)logits, targets, omax, osum,
                                                                       otgt, rows, V, vocab_start);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_ce_grad(void* logits, const long* targets, const float* gmax, const float* gsum, const float* scale,
                           long rows, int V, long vocab_start, cudaStream_t st) {
-  KB_LAUNCH(ce_grad_kernel, grid_for(rows, 1, 148 * 4), CE_THREADS, 0, st, (__nv_bfloat16*)logits, targets, gmax, gsum, scale,
+  KB_LAUNCH_PDL(ce_grad_kernel, grid_for(rows, 1, 148 * 4), CE_THREADS, 0, st, (__nv_bfloat16*)logits, targets, gmax, gsum, scale,
                                                                      rows, V, vocab_start);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_adamw(void* p, const float* g, float* m, float* v, float* master, long n, float lr, float b1,
                         float b2, float eps, float wd, float bc1, float bc2, const float* grad_scale_ptr,
                         float grad_scale, cudaStream_t st) {
-  KB_LAUNCH(adamw_kernel, grid_once(n / 4 + 1, 256), 256, 0, st, (__nv_bfloat16*)p, g, m, v, master, n, lr, b1, b2,
+  KB_LAUNCH_PDL(adamw_kernel, grid_once(n / 4 + 1, 256), 256, 0, st, (__nv_bfloat16*)p, g, m, v, master, n, lr, b1, b2,
                                                                     eps, wd, bc1, bc2, grad_scale_ptr, grad_scale);
   KB_CHECK_LAUNCH();
 }
 extern "C" int kb_sumsq(const void* x, long n, int is_f32, float* out, cudaStream_t st) {
-  if (is_f32) KB_LAUNCH(sumsq_f32_kernel, grid_for(n / 4 + 1, 256, 148 * 8), 256, 0, st, (const float*)x, n, out);
-  else KB_LAUNCH(sumsq_bf16_kernel, grid_for(n, 256, 148 * 8), 256, 0, st, (const __nv_bfloat16*)x, n, out);
+  if (is_f32) KB_LAUNCH_PDL(sumsq_f32_kernel, grid_for(n / 4 + 1, 256, 148 * 8), 256, 0, st, (const float*)x, n, out);
+  else KB_LAUNCH_PDL(sumsq_bf16_kernel, grid_for(n, 256, 148 * 8), 256, 0, st, (const __nv_bfloat16*)x, n, out);
   KB_CHECK_LAUNCH();
 }
 
@@ -1097,6 +1120,7 @@ extern "C" int kb_sumsq(const void* x, long n, int is_f32, float* out, cudaStrea
 // out[0] = sqrt(sumsq), out[1] = min(1, clip / (norm + 1e-6)).
 namespace kb {
 __global__ void clip_scale_kernel(const float* __restrict__ sumsq, float clip, float* __restrict__ out) {
+  pdl_begin();
   const float norm = sqrtf(*sumsq);
   const float f = clip / (norm + 1e-6f);
   out[0] = norm;
@@ -1104,7 +1128,7 @@ __global__ void clip_scale_kernel(const float* __restrict__ sumsq, float clip, f
 }
 }  // namespace kb
 extern "C" int kb_clip_scale(const float* sumsq, float clip, float* out, cudaStream_t st) {
-  KB_LAUNCH(clip_scale_kernel, 1, 1, 0, st, sumsq, clip, out);
+  KB_LAUNCH_PDL(clip_scale_kernel, 1, 1, 0, st, sumsq, clip, out);
   KB_CHECK_LAUNCH();
 }
 
@@ -1133,8 +1157,8 @@ extern "C" int kb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const float
   }
   float* partial = g_rmsnorm_bwd_partial_addr[dev];
   const int grid = rows < NOALLOC_MAX_CTAS ? rows : NOALLOC_MAX_CTAS;
-  KB_LAUNCH((rmsnorm_bwd_kernel<256, 4>), grid, 256, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, rstd,
+  KB_LAUNCH_PDL((rmsnorm_bwd_kernel<256, 4>), grid, 256, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, rstd,
                                                     (const __nv_bfloat16*)w, (__nv_bfloat16*)dx, partial, rows, H);
-  KB_LAUNCH(rmsnorm_dw_reduce_kernel, (H + 31) / 32, 1024, 0, st, partial, dw, grid, H, 0);
+  KB_LAUNCH_PDL(rmsnorm_dw_reduce_kernel, (H + 31) / 32, 1024, 0, st, partial, dw, grid, H, 0);
   KB_CHECK_LAUNCH();
 }

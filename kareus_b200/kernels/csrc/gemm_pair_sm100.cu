@@ -28,6 +28,7 @@
 // 128256 x 3072 (4096 tokens) 4479 / 2335; 640-wide QKV shard 117 / 68 forward.
 #include "sm100.cuh"
 #include "launch.h"
+#include "pdl.cuh"
 #include "host_utils.h"
 #include "gemm_plan.h"
 
@@ -126,6 +127,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   cluster_sync_all();                       // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_begin();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (each CTA: its own halves)
@@ -286,6 +288,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // C += the sums that K parts 1 .. ks - 1 of the split tiles left in the workspace, part by part: four columns a thread.
 __global__ void __launch_bounds__(256)
 gemm_add_parts_kernel(float* __restrict__ C, int ldc, int M, int N, const float* __restrict__ work, const PairWork w, int bn) {
+  pdl_begin();
   const int vecs = bn >> 2, per_tile = GP_BM * vecs, total = w.split_tiles * per_tile;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const int tile = i / per_tile, rest = i - tile * per_tile, r = rest / vecs, c = (rest - r * vecs) * 4;
@@ -363,10 +366,10 @@ static int launch_pair(const void* A, const void* B, void* C, int M, int N, int 
   w.group_m = gm < w.tiles_m ? (int)gm : w.tiles_m;
   const int units = w.whole + w.split_tiles * w.ks;
   const int grid = 2 * (units < pairs ? units : pairs);
-  KB_LAUNCH(kern, grid, GP_THREADS, GP_SMEM, stream, tmA, tmB, tmC, tmW, w, M, N, pl.bn, status);
+  KB_LAUNCH_PDL(kern, grid, GP_THREADS, GP_SMEM, stream, tmA, tmB, tmC, tmW, w, M, N, pl.bn, status);
   if (ordered) {
     const int blocks = w.split_tiles * (GP_BM * pl.bn / 4 / 256);
-    KB_LAUNCH(gemm_add_parts_kernel, blocks, 256, 0, stream, static_cast<float*>(C), ldc, M, N, (const float*)work, w, pl.bn);
+    KB_LAUNCH_PDL(gemm_add_parts_kernel, blocks, 256, 0, stream, static_cast<float*>(C), ldc, M, N, (const float*)work, w, pl.bn);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + static_cast<int>(e);

@@ -13,6 +13,7 @@
 // at kareus/transformer_engine/pytorch/ops/basic/basic_linear.py:572-582,848-859,899-909).
 #include "sm100.cuh"
 #include "launch.h"
+#include "pdl.cuh"
 #include "host_utils.h"
 #include "gemm_plan.h"
 #include <stdlib.h>
@@ -111,6 +112,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_begin();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
@@ -367,7 +369,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   int group_m = (int)((40L << 20) / (panel > 0 ? panel : 1));
   if (group_m < 4) group_m = 4;
   if (group_m > tiles_m) group_m = tiles_m;
-  KB_LAUNCH(kern, grid, GEMM_THREADS, smem, stream, tmA, tmB, C, M, N, K, ldc, aligned_rows(C, ldc, OUT_F32), group_m, ks,
+  KB_LAUNCH_PDL(kern, grid, GEMM_THREADS, smem, stream, tmA, tmB, C, M, N, K, ldc, aligned_rows(C, ldc, OUT_F32), group_m, ks,
             status, ep);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + static_cast<int>(e);

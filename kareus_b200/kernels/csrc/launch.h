@@ -39,30 +39,32 @@ constexpr EpochLoc NO_EPOCH{-1, 0, 0};
 extern bool g_recording;   // set between kb_rec_begin and kb_rec_end
 
 void record_launch(const void* func, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, void* const* args,
-                   const size_t* sizes, const size_t* aligns, int nargs, EpochLoc epoch);
+                   const size_t* sizes, const size_t* aligns, int nargs, EpochLoc epoch, bool pdl);
+// A launch that may overlap the end of the kernel before it on the stream (`pdl`, see pdl.cuh), or a plain one.
+cudaError_t launch_kernel(const void* func, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t stream, bool pdl);
 void record_memcpy(void* dst, const void* src, size_t bytes, cudaStream_t stream);
 void record_memset(void* dst, int value, size_t bytes, cudaStream_t stream);
 
 template <typename... KArgs, typename... Args, size_t... I>
 inline cudaError_t launch_impl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                               EpochLoc epoch, std::index_sequence<I...>, Args&&... args) {
+                               EpochLoc epoch, bool pdl, std::index_sequence<I...>, Args&&... args) {
   std::tuple<std::decay_t<KArgs>...> vals(static_cast<std::decay_t<KArgs>>(std::forward<Args>(args))...);
   void* ptrs[sizeof...(KArgs) > 0 ? sizeof...(KArgs) : 1] = {static_cast<void*>(&std::get<I>(vals))...};
   if (g_recording) {
     static const size_t sizes[] = {sizeof(std::decay_t<KArgs>)..., 0};
     static const size_t aligns[] = {alignof(std::decay_t<KArgs>)..., 0};
     record_launch(reinterpret_cast<const void*>(kernel), grid, block, smem, stream, ptrs, sizes, aligns,
-                  static_cast<int>(sizeof...(KArgs)), epoch);
+                  static_cast<int>(sizeof...(KArgs)), epoch, pdl);
   }
-  return cudaLaunchKernel(reinterpret_cast<const void*>(kernel), grid, block, ptrs, smem, stream);
+  return launch_kernel(reinterpret_cast<const void*>(kernel), grid, block, ptrs, smem, stream, pdl);
 }
 
 // kernel<<<grid, block, smem, stream>>>(args...) that is also recordable.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                          EpochLoc epoch, Args&&... args) {
+                          EpochLoc epoch, bool pdl, Args&&... args) {
   static_assert(sizeof...(KArgs) == sizeof...(Args), "argument count differs from the kernel's parameter list");
-  return launch_impl(kernel, grid, block, smem, stream, epoch, std::index_sequence_for<KArgs...>{},
+  return launch_impl(kernel, grid, block, smem, stream, epoch, pdl, std::index_sequence_for<KArgs...>{},
                      std::forward<Args>(args)...);
 }
 
@@ -79,6 +81,9 @@ inline cudaError_t memset_async(void* dst, int value, size_t bytes, cudaStream_t
 }  // namespace kb
 
 #define KB_LAUNCH(kernel, grid, block, smem, stream, ...) \
-  kb::launch(kernel, dim3(grid), dim3(block), smem, stream, kb::NO_EPOCH, __VA_ARGS__)
+  kb::launch(kernel, dim3(grid), dim3(block), smem, stream, kb::NO_EPOCH, false, __VA_ARGS__)
+// For kernels that follow the rules of pdl.cuh.
+#define KB_LAUNCH_PDL(kernel, grid, block, smem, stream, ...) \
+  kb::launch(kernel, dim3(grid), dim3(block), smem, stream, kb::NO_EPOCH, true, __VA_ARGS__)
 #define KB_LAUNCH_EPOCH(kernel, grid, block, smem, stream, epoch_loc, ...) \
-  kb::launch(kernel, dim3(grid), dim3(block), smem, stream, epoch_loc, __VA_ARGS__)
+  kb::launch(kernel, dim3(grid), dim3(block), smem, stream, epoch_loc, false, __VA_ARGS__)

@@ -14,7 +14,8 @@
 //                                       its epoch from this host counter (incremented on every replay).
 //   kb_replay(list, compute_stream)     enqueue the whole list.  A list that stays on the compute stream and patches no
 //                                       epochs becomes a CUDA graph on its first replay: one launch instead of one per
-//                                       kernel (3.4 us each, which is what a step of a small model consisted of).
+//                                       kernel (3.4 us each, which is what a step of a small model consisted of), with
+//                                       programmatic edges between kernels that may overlap (pdl.cuh).
 //                                       Lists with side streams keep explicit stream order: kernels that wait on peer
 //                                       GPUs must start in the same order on every rank.
 //   kb_rec_launches(list)               kernels in the list (for launch accounting).
@@ -42,6 +43,7 @@ struct Op {
   const void* func = nullptr;
   dim3 grid, block;
   size_t smem = 0;
+  bool pdl = false;           // may overlap the end of the kernel before it (pdl.cuh)
   size_t args_off = 0;        // first argument pointer in LaunchList::argptrs
   int nargs = 0;
   // epoch patch
@@ -88,11 +90,14 @@ struct LaunchList {
       return;
     }
     cudaGraphNode_t last = nullptr;
+    bool last_is_kernel = false;
     bool ok = true;
     for (const Op& op : ops) {
       cudaGraphNode_t node = nullptr;
-      const cudaGraphNode_t* deps = last ? &last : nullptr;
-      const size_t ndeps = last ? 1 : 0;
+      // a kernel that may overlap the one before it gets its edge below
+      const bool overlaps = op.kind == OP_LAUNCH && op.pdl && last_is_kernel;
+      const cudaGraphNode_t* deps = last && !overlaps ? &last : nullptr;
+      const size_t ndeps = deps ? 1 : 0;
       cudaError_t e = cudaSuccess;
       if (op.kind == OP_LAUNCH) {
         cudaKernelNodeParams p{};
@@ -102,6 +107,12 @@ struct LaunchList {
         p.sharedMemBytes = static_cast<unsigned>(op.smem);
         p.kernelParams = argptrs.data() + op.args_off;
         e = cudaGraphAddKernelNode(&node, g, deps, ndeps, &p);
+        if (e == cudaSuccess && overlaps) {
+          cudaGraphEdgeData edge{};
+          edge.from_port = cudaGraphKernelNodePortProgrammatic;
+          edge.type = cudaGraphDependencyTypeProgrammatic;
+          e = cudaGraphAddDependencies_v2(g, &last, &node, &edge, 1);
+        }
       } else if (op.kind == OP_MEMCPY) {
         e = cudaGraphAddMemcpyNode1D(&node, g, deps, ndeps, op.dst, op.src, op.bytes, cudaMemcpyDeviceToDevice);
       } else if (op.kind == OP_MEMSET) {
@@ -120,6 +131,7 @@ struct LaunchList {
         break;
       }
       last = node;
+      last_is_kernel = op.kind == OP_LAUNCH;
     }
     if (ok && cudaGraphInstantiate(&graph, g, 0) != cudaSuccess) graph = nullptr;
     cudaGraphDestroy(g);
@@ -138,8 +150,23 @@ uint64_t* g_next_epoch = nullptr;
 
 }  // namespace
 
+cudaError_t launch_kernel(const void* func, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t stream, bool pdl) {
+  if (!pdl) return cudaLaunchKernel(func, grid, block, args, smem, stream);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, func, args);
+}
+
 void record_launch(const void* func, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, void* const* args,
-                   const size_t* sizes, const size_t* aligns, int nargs, EpochLoc epoch) {
+                   const size_t* sizes, const size_t* aligns, int nargs, EpochLoc epoch, bool pdl) {
   LaunchList* L = g_open;
   if (!L) return;
   Op op;
@@ -149,6 +176,7 @@ void record_launch(const void* func, dim3 grid, dim3 block, size_t smem, cudaStr
   op.grid = grid;
   op.block = block;
   op.smem = smem;
+  op.pdl = pdl;
   op.args_off = L->arg_offsets.size();
   op.nargs = nargs;
   for (int i = 0; i < nargs; ++i) {
@@ -309,7 +337,7 @@ extern "C" int kb_replay(int list, cudaStream_t compute_stream) {
             memcpy(at, &v32, 4);
           }
         }
-        e = cudaLaunchKernel(op.func, op.grid, op.block, L->argptrs.data() + op.args_off, op.smem, st);
+        e = launch_kernel(op.func, op.grid, op.block, L->argptrs.data() + op.args_off, op.smem, st, op.pdl);
         break;
       }
       case OP_MEMCPY:

@@ -4,6 +4,7 @@
 // (kareus/megatron/core/extensions/ops/te_norm.py, kareus/transformer_engine/pytorch/ops/basic/bias.py).
 #include <cuda_bf16.h>
 #include "launch.h"
+#include "pdl.cuh"
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -34,6 +35,7 @@ __global__ void __launch_bounds__(LN_THREADS)
 layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                      const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y, float* __restrict__ mean,
                      float* __restrict__ rstd, int rows, int H, float eps) {
+  pdl_begin();
   __shared__ float red[32];
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* xr = x + static_cast<size_t>(row) * H;
@@ -63,6 +65,7 @@ __global__ void __launch_bounds__(LN_THREADS)
 layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                      const float* __restrict__ mean, const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ w,
                      __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows, int H) {
+  pdl_begin();
   __shared__ float red[32];
   float* pw = partial + static_cast<size_t>(blockIdx.x) * 2 * H;
   float* pb = pw + H;
@@ -95,6 +98,7 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
 
 __global__ void ln_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, float* __restrict__ db,
                                  int nparts, int H) {
+  pdl_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= H) return;
   float a = 0.f, b = 0.f;
@@ -108,6 +112,7 @@ __global__ void ln_reduce_kernel(const float* __restrict__ partial, float* __res
 
 __global__ void bias_add_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ b,
                                 __nv_bfloat16* __restrict__ y, long rows, int H) {
+  pdl_begin();
   const long total = rows * H;
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<long>(gridDim.x) * blockDim.x)
@@ -117,6 +122,7 @@ __global__ void bias_add_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
 // db[c] += sum over rows of dy[r][c]  (fp32 atomics; db zeroed or accumulated by the caller)
 __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ db, long rows, int H,
                               int rows_per_block) {
+  pdl_begin();
   const long r0 = static_cast<long>(blockIdx.y) * rows_per_block;
   const long r1 = min(rows, r0 + rows_per_block);
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < H; c += gridDim.x * blockDim.x) {
@@ -134,7 +140,7 @@ using namespace kb;
 extern "C" int kb_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, int rows,
                                 int H, float eps, cudaStream_t st) {
   const int grid = rows < 148 * 8 ? rows : 148 * 8;
-  KB_LAUNCH(layernorm_fwd_kernel, grid, LN_THREADS, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+  KB_LAUNCH_PDL(layernorm_fwd_kernel, grid, LN_THREADS, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
                                                     (const __nv_bfloat16*)b, (__nv_bfloat16*)y, mean, rstd, rows, H, eps);
   LN_RET();
 }
@@ -145,20 +151,20 @@ extern "C" long kb_layernorm_bwd_scratch_elems(int rows, int H) {
 extern "C" int kb_layernorm_bwd(const void* dy, const void* x, const float* mean, const float* rstd, const void* w,
                                 void* dx, float* dw, float* db, float* scratch, int rows, int H, cudaStream_t st) {
   const int grid = rows < 148 * 2 ? rows : 148 * 2;
-  KB_LAUNCH(layernorm_bwd_kernel, grid, LN_THREADS, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, mean, rstd,
+  KB_LAUNCH_PDL(layernorm_bwd_kernel, grid, LN_THREADS, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, mean, rstd,
                                                     (const __nv_bfloat16*)w, (__nv_bfloat16*)dx, scratch, rows, H);
-  KB_LAUNCH(ln_reduce_kernel, (H + 255) / 256, 256, 0, st, scratch, dw, db, grid, H);
+  KB_LAUNCH_PDL(ln_reduce_kernel, (H + 255) / 256, 256, 0, st, scratch, dw, db, grid, H);
   LN_RET();
 }
 extern "C" int kb_bias_add(const void* x, const void* b, void* y, long rows, int H, cudaStream_t st) {
   long blocks = (rows * H + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  KB_LAUNCH(bias_add_kernel, (int)blocks, 256, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)b, (__nv_bfloat16*)y, rows, H);
+  KB_LAUNCH_PDL(bias_add_kernel, (int)blocks, 256, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)b, (__nv_bfloat16*)y, rows, H);
   LN_RET();
 }
 extern "C" int kb_colsum_accumulate(const void* dy, float* db, long rows, int H, cudaStream_t st) {
   const int rpb = 256;
   dim3 grid((H + 255) / 256, (unsigned)((rows + rpb - 1) / rpb));
-  KB_LAUNCH(colsum_kernel, grid, 256, 0, st, (const __nv_bfloat16*)dy, db, rows, H, rpb);
+  KB_LAUNCH_PDL(colsum_kernel, grid, 256, 0, st, (const __nv_bfloat16*)dy, db, rows, H, rpb);
   LN_RET();
 }
