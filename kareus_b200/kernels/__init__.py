@@ -24,6 +24,9 @@ import torch
 from . import ref
 
 _LAUNCHES = [0]
+# The native calls of csrc/torch/fastcall.cpp, once the library is loaded.  Each returns None for a call that it leaves to
+# the statements below it.
+_FAST = None
 
 
 def launch_count() -> int:
@@ -125,6 +128,10 @@ def add(a, b):
 def gemm(a, b, trans_a=False, trans_b=True, out_dtype=None, accumulate=None, out=None, bias=None, activation=None):
     """``op(a) @ op(b)``.  ``accumulate`` is an fp32 tensor that receives ``+=``.  ``bias`` (per output
     feature) and ``activation`` (``"gelu"``) run in the GEMM's epilogue."""
+    if _FAST is not None and out_dtype is None and out is None and bias is None and not activation:
+        r = _FAST.gemm(a, b, trans_a, trans_b, accumulate)
+        if r is not None:
+            return r
     if is_cuda(a):
         if library_baseline():
             return _cuda().gemm_library(a, b, trans_a, trans_b, out_dtype, accumulate, out, bias, activation)
@@ -154,6 +161,10 @@ def attention_fwd(q, k, v, scale, causal=True, q_offset=0, kv_len=None, peer=Fal
     if peer:
         _peer_guard(q, "attention_fwd")
         return _cuda().attention_fwd(q, k, v, scale, causal, q_offset, kv_len, strict=True)
+    if _FAST is not None and kv_len is None:
+        r = _FAST.attention_fwd(q, k, v, scale, causal, q_offset)
+        if r is not None:
+            return r
     if is_cuda(q):
         if library_baseline():
             return _cuda().attention_fwd_library(q, k, v, scale, causal, q_offset, kv_len)
@@ -167,6 +178,10 @@ def attention_bwd(do, q, k, v, o, lse, scale, causal=True, q_offset=0, kv_len=No
     if peer:
         _peer_guard(q, "attention_bwd")
         return _cuda().attention_bwd(do, q, k, v, o, lse, scale, causal, q_offset, kv_len, out, strict=True)
+    if _FAST is not None and kv_len is None and out is None:
+        r = _FAST.attention_bwd(q, k, v, scale, causal, q_offset, do, o, lse)
+        if r is not None:
+            return r
     if is_cuda(q):
         if library_baseline():
             return _cuda().attention_bwd_library(do, q, k, v, o, lse, scale, causal, q_offset, kv_len, out)

@@ -3,6 +3,8 @@
 All kernels are compiled in-tree (no runtime JIT: the reference compiles its collective kernels to
 PTX at run time, ``3rdparty/mscclpp/python/mscclpp/utils.py:85-127``).  The library exposes a
 plain C ABI, so it has no dependency on PyTorch headers and builds in seconds without a GPU.
+``_fastcall.so`` (``csrc/torch/fastcall.cpp``) is the extension module between PyTorch tensors and that ABI
+for the calls whose host time counts.
 
     python -m kareus_b200.kernels.build          # build if sources are newer than the library
     python -m kareus_b200.kernels.build --force
@@ -14,6 +16,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 from typing import List
@@ -22,6 +25,8 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OBJ = HERE / "build"
 LIB = HERE / "libkareus_b200.so"
+FASTCALL_SRC = CSRC / "torch" / "fastcall.cpp"
+FASTCALL = HERE / "_fastcall.so"
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC"
@@ -54,6 +59,35 @@ def is_current() -> bool:
     return LIB.exists() and stamp.exists() and stamp.read_text() == _digest()
 
 
+def _fastcall_digest() -> str:
+    import torch
+    h = hashlib.sha256(FASTCALL_SRC.read_bytes())
+    h.update(f"{torch.__version__} {sysconfig.get_config_var('SOABI')}".encode())
+    return h.hexdigest()
+
+
+def build_fastcall(force: bool = False) -> Path:
+    """The extension module; needs the library to link against."""
+    stamp = OBJ / "fastcall.digest"
+    digest = _fastcall_digest()
+    if not force and FASTCALL.exists() and stamp.exists() and stamp.read_text() == digest:
+        return FASTCALL
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda_inc = Path(nvcc()).resolve().parent.parent / "include"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wno-attributes",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", str(root / "include"), "-I", str(root / "include/torch/csrc/api/include"),
+           "-I", sysconfig.get_paths()["include"], "-I", str(cuda_inc), str(FASTCALL_SRC), "-o", str(FASTCALL),
+           "-L", str(root / "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+           "-L", str(HERE), "-l:" + LIB.name, "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {FASTCALL_SRC.name}:\n{r.stdout}\n{r.stderr}")
+    stamp.write_text(digest)
+    return FASTCALL
+
+
 def _compile(src: Path, verbose: bool) -> Path:
     obj = OBJ / (src.stem + ".o")
     cmd = [nvcc(), *ARCH_FLAGS, *NVCC_FLAGS, "-I", str(CSRC), "-c", str(src), "-o", str(obj)]
@@ -73,6 +107,7 @@ def _compile(src: Path, verbose: bool) -> Path:
 
 def build(force: bool = False, verbose: bool = False) -> Path:
     if not force and is_current():
+        build_fastcall()
         return LIB
     OBJ.mkdir(exist_ok=True)
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 2)) as ex:
@@ -82,6 +117,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
     (OBJ / "digest").write_text(_digest())
+    build_fastcall(force)
     return LIB
 
 

@@ -38,9 +38,25 @@ def lib() -> ctypes.CDLL:
             raise KernelError(
                 f"{LIB_PATH} is missing: build it with `python -m kareus_b200.kernels.build` "
                 "(bf16 CUDA tensors have no PyTorch fallback)")
-        _LIB = ctypes.CDLL(str(LIB_PATH), mode=ctypes.RTLD_GLOBAL)
-        _declare(_LIB)
+        L = ctypes.CDLL(str(LIB_PATH), mode=ctypes.RTLD_GLOBAL)
+        _declare(L)
+        _load_fastcall()
+        _LIB = L
     return _LIB
+
+
+def _load_fastcall() -> None:
+    """The extension module that takes plain GEMM and attention calls without the statements of this file."""
+    import kareus_b200.kernels as K
+    try:
+        from . import _fastcall
+    except ImportError as e:
+        raise KernelError(f"{_HERE / '_fastcall.so'} cannot be loaded ({e}): build it with "
+                          "`python -m kareus_b200.kernels.build`") from e
+    _fastcall.init(K._LAUNCHES, _check)
+    for idx, t in _STATUS.items():
+        _fastcall.set_status(idx, t.data_ptr())
+    K._FAST = _fastcall
 
 
 def is_loaded() -> bool:
@@ -138,6 +154,9 @@ def status_word(device) -> torch.Tensor:
     if t is None:
         t = torch.zeros(1, dtype=torch.int32, device=f"cuda:{idx}")
         _STATUS[idx] = t
+        from . import _FAST
+        if _FAST is not None:
+            _FAST.set_status(idx, t.data_ptr())
     return t
 
 

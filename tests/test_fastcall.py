@@ -1,0 +1,139 @@
+"""The native GEMM and attention calls take what they can launch as it lies, and leave everything else to the Python statements."""
+import math
+
+import pytest
+import torch
+
+import kareus_b200.kernels as K
+
+
+class _Sub(torch.Tensor):
+    pass
+
+
+def test_calls_without_a_launch_are_left_alone():
+    KC = pytest.importorskip("kareus_b200.kernels.cuda")
+    KC.lib()
+    a = torch.randn(8, 16, dtype=torch.bfloat16)
+    for x in (a, a.float(), a.as_subclass(_Sub), a.to_sparse(), torch.empty(8, 16, device="meta"), None, 3):
+        assert K._FAST.gemm(x, a, False, True, None) is None
+        assert K._FAST.attention_fwd(x, a, a, 1.0, True, 0) is None
+    assert torch.equal(K.gemm(a, a), K.ref.gemm(a, a))
+
+
+def _outcome(fn):
+    """Result of a call, or the type of its error."""
+    try:
+        r = fn()
+    except Exception as e:
+        return type(e)
+    torch.cuda.synchronize()
+    return r if isinstance(r, tuple) else (r,)
+
+
+def _same_as_python(monkeypatch, fn):
+    from kareus_b200.kernels import launch_count
+    n0 = launch_count()
+    fast = _outcome(fn)
+    n1 = launch_count()
+    with monkeypatch.context() as m:
+        m.setattr(K, "_FAST", None)
+        slow = _outcome(fn)
+    assert launch_count() - n1 == n1 - n0
+    assert isinstance(fast, type) == isinstance(slow, type), (fast, slow)
+    if isinstance(fast, type):
+        assert fast is slow
+        return
+    for a, b in zip(fast, slow, strict=True):
+        assert type(a) is type(b) and a.shape == b.shape and a.stride() == b.stride() and a.dtype == b.dtype
+        assert a.requires_grad == b.requires_grad and torch.equal(a, b)
+
+
+def _bf16(*shape):
+    return torch.randn(*shape, device="cuda").bfloat16()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["plain", "rows", "param", "odd_rows", "offset", "cols", "subclass", "fp32", "three", "one_row",
+                                  "no_rows", "mismatch"])
+@pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, False), (True, True)])
+def test_gemm_forms(monkeypatch, form, ta, tb):
+    torch.manual_seed(0)
+    M, N, Kd = 72, 136, 200
+    a, b = _bf16(*((Kd, M) if ta else (M, Kd))), _bf16(*((N, Kd) if tb else (Kd, N)))
+    wide = lambda t, pad, off: torch.cat([torch.zeros(t.shape[0], off, device="cuda").bfloat16(), t,
+                                          torch.zeros(t.shape[0], pad, device="cuda").bfloat16()], 1)[:, off:off + t.shape[1]]
+    a, b = {
+        "plain": lambda: (a, b), "rows": lambda: (wide(a, 24, 8), wide(b, 8, 16)),
+        "param": lambda: (a, torch.nn.Parameter(b)), "odd_rows": lambda: (wide(a, 3, 0), b), "offset": lambda: (wide(a, 7, 1), b),
+        "cols": lambda: (a.t().contiguous().t(), b), "subclass": lambda: (a.as_subclass(_Sub), b), "fp32": lambda: (a.float(), b.float()),
+        "three": lambda: (a[None], b), "one_row": lambda: (a[:, :1] if ta else a[:1], b),
+        "no_rows": lambda: (a[:, :0] if ta else a[:0], b), "mismatch": lambda: (a[8:] if ta else a[:, 8:], b),
+    }[form]()
+    _same_as_python(monkeypatch, lambda: K.gemm(a, b, trans_a=ta, trans_b=tb))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens", [64, 4096])
+@pytest.mark.parametrize("form", ["plain", "view", "transposed", "bf16", "shape"])
+def test_accumulating_gemm_forms(monkeypatch, tokens, form):
+    torch.manual_seed(0)
+    dy, x = _bf16(tokens, 3072), _bf16(tokens, 2048)      # more tiles than SMs: parts of a K split add in order
+    base = torch.randn(3072, 2048, device="cuda")
+
+    def call():
+        c = {"plain": lambda: base.clone(), "view": lambda: torch.cat([base, base])[3072:], "transposed": lambda: base.t().clone().t(),
+             "bf16": lambda: base.bfloat16(), "shape": lambda: base[:8].clone()}[form]()
+        r = K.gemm(dy, x, trans_a=True, trans_b=False, accumulate=c)
+        assert r is c
+        return r
+    _same_as_python(monkeypatch, call)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["packed", "four_dims", "off_keys", "batch_major", "int_scale", "float_offset", "kv_len", "wide_head",
+                                  "groups", "no_queries"])
+def test_attention_forms(monkeypatch, form):
+    torch.manual_seed(0)
+    s, b, g, rep, d = 70, 2, 2, 2, 128
+    packed = _bf16(s, b, g, (rep + 2) * d)
+    q, k, v = packed[..., :rep * d].unflatten(-1, (rep, d)), packed[..., rep * d:-d], packed[..., -d:]
+    scale, off, kw = 1 / math.sqrt(d), 0, {}
+    if form == "four_dims":
+        q = q.reshape(s, b, g * rep, d)
+    elif form == "off_keys":
+        k, v, off = _bf16(s + 128, b, g, d), _bf16(s + 128, b, g, d), 128
+    elif form == "batch_major":
+        k, v = (t.transpose(0, 1).contiguous().transpose(0, 1) for t in (k, v))
+    elif form == "int_scale":
+        scale = 1
+    elif form == "float_offset":
+        off = 0.0
+    elif form == "kv_len":
+        kw = {"kv_len": 33}
+    elif form == "wide_head":
+        q, k, v = _bf16(s, b, g, rep, 64), _bf16(s, b, g, 64), _bf16(s, b, g, 64)
+    elif form == "groups":
+        k, v = k[:, :, :1], v[:, :, :1]
+    elif form == "no_queries":
+        q = q[:0]
+    fwd = lambda: K.attention_fwd(q, k, v, scale, causal=True, q_offset=off, **kw)
+    _same_as_python(monkeypatch, fwd)
+    r = _outcome(fwd)
+    if isinstance(r, type):
+        return
+    out, lse = r
+    do = _bf16(*out.shape)
+    # every dK and dV has one sum of its own, and dQ the contributions of at most two key tiles: bitwise the same each time
+    _same_as_python(monkeypatch, lambda: K.attention_bwd(do, q, k, v, out, lse, scale, causal=True, q_offset=off, **kw))
+
+@pytest.mark.gpu
+def test_transforms_and_switches(monkeypatch):
+    a, b = _bf16(4, 64, 64), _bf16(64, 64)
+    K.gemm(a[0], b)
+    with pytest.raises(Exception):
+        torch.vmap(lambda x: K.gemm(x, b))(a)
+    monkeypatch.setenv("KAREUS_B200_LIBRARY_BASELINE", "1")
+    n = K.launch_count()
+    K.gemm(a[0], b)
+    assert K.launch_count() == n
