@@ -236,6 +236,20 @@ def cross_entropy_local_stats(logits, targets, vocab_start):
     return ref.cross_entropy_local_stats(logits, targets, vocab_start)
 
 
+def linear_cross_entropy_stats(x, w, targets, vocab_start, store=True, weight=None):
+    """Logits of a vocabulary shard and what a cross entropy needs of their rows: ``(logits, max, sum of exponentials, target
+    logit, loss)``.  ``store=False``: the logits are not wanted (``None``).  ``weight`` (one value per row): the loss is
+    ``sum(weight * (max + log(sum) - target))``, for a shard that is the whole vocabulary; without it ``None``."""
+    if is_cuda(x) and not library_baseline():
+        r = _cuda().linear_cross_entropy_stats(x, w, targets, vocab_start, store, weight)
+        if r is not None:
+            return r
+    logits = gemm(x, w, trans_b=True)
+    m, se, tl = cross_entropy_local_stats(logits, targets, vocab_start)
+    loss = None if weight is None else ((m + torch.log(se) - tl) * weight.to(m.dtype)).sum()
+    return logits, m, se, tl, loss
+
+
 def cross_entropy_finish(logits, targets, vocab_start, gmax, gsum, grad_scale):
     if is_cuda(logits):
         return _cuda().cross_entropy_finish(logits, targets, vocab_start, gmax, gsum, grad_scale)

@@ -19,4 +19,12 @@ int gemm_pair_dispatch(const void* A, const void* B, void* C, int M, int N, int 
                        int ldc, int out_f32, int accumulate, const PairPlan& pl, int pairs, float* work, int* status,
                        cudaStream_t stream);
 
+// bf16 C = A * B^T (both K-major; null: the product is not stored) and the softmax statistics of its rows, see RowStats in
+// gemm_pair_sm100.cu.  `part`: row_stats_floats() floats, 16-byte aligned.  With `weight` ([M]) *loss becomes the
+// sum of weight * (max + log(sum) - target).
+inline long row_stats_floats(int M, int N, int bn) { return 4L * ((N + bn - 1) / bn) * M + (M + 31) / 32; }
+int gemm_pair_row_stats(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, const PairPlan& pl,
+                        int pairs, const long* targets, long first_col, float* part, float* omax, float* osum, float* otgt,
+                        const float* weight, float* loss, int* status, cudaStream_t stream);
+
 }  // namespace kb

@@ -622,3 +622,24 @@ extern "C" int kb_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
   return kb::gemm_run(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, num_sms, nullptr, 0, nullptr, status,
                       stream);
 }
+
+// Logits of a vocabulary shard and the statistics of their rows that a cross entropy needs: maximum, sum of exponentials and
+// target logit, in the epilogue of the product (see RowStats in gemm_pair_sm100.cu).  A [M, K], B [N, K], C [M, N] contiguous
+// (N a multiple of 8) or null; targets are columns plus vocab_start.  With `weight` *loss is the weighted sum of the rows'
+// losses (statistics of the whole vocabulary only).  `part` holds kb_gemm_row_stats_floats() floats.
+extern "C" long kb_gemm_row_stats_floats(int M, int N, int K) {
+  using namespace kb;
+  return M <= 0 || N <= 0 || K <= 0 ? 0 : row_stats_floats(M, N, plan_pair(M, N, K, device_sm_count() / 2, false).bn);
+}
+extern "C" int kb_gemm_row_stats(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
+                                 const long* targets, long vocab_start, float* part, float* omax, float* osum, float* otgt,
+                                 const float* weight, float* loss, int* status, cudaStream_t stream) {
+  using namespace kb;
+  if (M <= 0 || N <= 0 || K <= 0 || (N & 7) || (lda & 7) || (ldb & 7)) return ST_BAD_ARG;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C) |
+       reinterpret_cast<uintptr_t>(part)) & 15)
+    return ST_BAD_ARG;
+  const int pairs = device_sm_count() / 2;
+  return gemm_pair_row_stats(A, B, C, M, N, K, lda, ldb, plan_pair(M, N, K, pairs, false), pairs, targets, vocab_start, part, omax,
+                             osum, otgt, weight, loss, status, stream);
+}

@@ -68,6 +68,7 @@ def _declare(L) -> None:
     sig = {
         "kb_gemm_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P],
         "kb_gemm_accum_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, P, P, P],
+        "kb_gemm_row_stats": [P, P, P, I, I, I, I, I, P, LNG, P, P, P, P, P, P, P, P],
         "kb_gemm_bias_act_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, I, P, P],
         "kb_rmsnorm_fwd": [P, P, P, P, I, I, F, P],
         "kb_rmsnorm_fwd_heads": [P, LNG, I, LNG, LNG, P, P, P, I, F, P],
@@ -94,6 +95,8 @@ def _declare(L) -> None:
         fn.restype = c_int
     L.kb_rmsnorm_bwd_scratch_elems.argtypes = [I, I]
     L.kb_rmsnorm_bwd_scratch_elems.restype = c_long
+    L.kb_gemm_row_stats_floats.argtypes = [I, I, I]
+    L.kb_gemm_row_stats_floats.restype = c_long
     L.kb_gemm_accum_scratch_floats.argtypes = [I, I, I, I]
     L.kb_gemm_accum_scratch_floats.restype = c_long
     for name, args in _OPTIONAL_SIGS.items():
@@ -600,6 +603,31 @@ def cross_entropy_local_stats(logits, targets, vocab_start):
                              st[2].data_ptr(), rows, V, int(vocab_start), _stream()), "ce_stats")
     _count()
     return st[0], st[1], st[2]
+
+
+def linear_cross_entropy_stats(x, w, targets, vocab_start, store=True, weight=None):
+    """See :func:`kareus_b200.kernels.linear_cross_entropy_stats`; ``None`` for operands that the kernel does not take."""
+    if not (_bf16(x) and _bf16(w) and x.dim() == 2 and _rowmajor_ok(x) and _rowmajor_ok(w) and x.shape[1] == w.shape[1]
+            and x.numel() and w.shape[0] and w.shape[0] % 8 == 0 and targets.dtype == torch.int64 and w.device == x.device
+            and targets.device == x.device and targets.numel() == x.shape[0]):
+        return None
+    if weight is not None and (weight.dtype != torch.float32 or weight.device != x.device or weight.numel() != x.shape[0]):
+        return None
+    (M, Kd), N, L = x.shape, w.shape[0], lib()
+    targets = targets.contiguous()
+    logits = torch.empty(M, N, dtype=x.dtype, device=x.device) if store else None
+    st = torch.empty(3, M, dtype=torch.float32, device=x.device)
+    part = torch.empty(L.kb_gemm_row_stats_floats(M, N, Kd), dtype=torch.float32, device=x.device)
+    loss = None
+    if weight is not None:
+        weight, loss = weight.contiguous(), torch.empty((), dtype=torch.float32, device=x.device)
+    m, se, tl = st.unbind()
+    _check(L.kb_gemm_row_stats(x.data_ptr(), w.data_ptr(), logits.data_ptr() if store else 0, M, N, Kd, x.stride(0), w.stride(0),
+                               targets.data_ptr(), int(vocab_start), part.data_ptr(), m.data_ptr(), se.data_ptr(), tl.data_ptr(),
+                               weight.data_ptr() if weight is not None else 0, loss.data_ptr() if loss is not None else 0,
+                               status_word(x.device).data_ptr(), _stream()), f"gemm+row statistics M={M} N={N} K={Kd}")
+    _count(2 if weight is None else 3)
+    return logits, m, se, tl, loss
 
 
 def cross_entropy_finish(logits, targets, vocab_start, gmax, gsum, grad_scale):

@@ -182,9 +182,9 @@ class _HeadLossFn(torch.autograd.Function):
             (x,) = module.fwd_gather.run((x.contiguous(),))
         s, b, h = x.shape
         x2 = x.reshape(-1, h)
-        logits = K.gemm(x2, w, trans_b=True)                            # [T, V_local]
-        tgt = labels.reshape(-1)
-        m, se, tl = K.cross_entropy_local_stats(logits, tgt, module.vocab_start)
+        tgt, lw = labels.reshape(-1), loss_weight.reshape(-1)
+        logits, m, se, tl, loss = K.linear_cross_entropy_stats(x2, w, tgt, module.vocab_start, store=want_grad,   # [T, V_local]
+                                                               weight=lw if module.tp == 1 else None)
         if module.tp > 1:
             stats = torch.stack([m, se, tl], dim=0)                        # [3, T]
             flat = torch.empty((module.tp * 3, stats.shape[1]), dtype=stats.dtype, device=stats.device)
@@ -193,11 +193,10 @@ class _HeadLossFn(torch.autograd.Function):
             gm = gathered[:, 0].max(dim=0).values
             gs = (gathered[:, 1] * torch.exp(gathered[:, 0] - gm)).sum(0)
             gt = gathered[:, 2].sum(0)
+            loss = ((gm + torch.log(gs) - gt) * lw.to(gm.dtype)).sum()     # over the whole vocabulary
         else:
-            gm, gs, gt = m, se, tl
-        per_token = (gm + torch.log(gs) - gt)                              # [T] fp32
-        lw = loss_weight.reshape(-1).to(per_token.dtype)
-        loss = (per_token * lw).sum()
+            gm, gs = m, se
+        lw = lw.to(gm.dtype)
         if want_grad:
             K.cross_entropy_finish(logits, tgt, module.vocab_start, gm, gs, lw)   # logits := dlogits
             dx = K.gemm(logits, w, trans_b=False)                          # [T, h] partial over TP

@@ -688,6 +688,33 @@ def test_cross_entropy_vector_groups(rows, V):
     assert _rel(logits, want) < 4e-3
 
 
+@pytest.mark.parametrize("M,N,Kd", [(1, 8, 64), (130, 1000, 72), (300, 2048, 520), (257, 16392, 128), (513, 4104, 1032), (128, 64, 8)])
+def test_logits_with_row_statistics(M, N, Kd):
+    """Statistics from the epilogue of the product against those of the product, with and without storing it."""
+    import kareus_b200.kernels as KK
+    KC = _K()
+    x, w = torch.randn(M, Kd, device="cuda").bfloat16(), (torch.randn(N, Kd, device="cuda") / Kd ** 0.5).bfloat16()
+    start = 40
+    tgt = torch.randint(0, N + 2 * start, (M,), device="cuda")
+    tgt[0], tgt[-1] = start, start + N - 1
+    weight = torch.rand(M, device="cuda")
+    logits, m, se, tl, loss = KK.linear_cross_entropy_stats(x, w, tgt, start, weight=weight)
+    torch.cuda.synchronize()
+    KC.check_status()
+    assert _rel(logits, KC.gemm(x, w)) < 2e-3              # another order of summation moves some bf16 roundings
+    mr, sr, tr = KC.cross_entropy_local_stats(logits, tgt, start)
+    assert torch.equal(m, mr) and torch.equal(tl, tr)
+    assert _rel(se.double(), (logits.double() - m.double()[:, None]).exp().sum(-1)) < 2e-6
+    want = ((m.double() + se.double().log() - tl.double()) * weight.double()).sum()
+    assert abs(loss.double() - want) < 1e-5 * ((m.double() + se.double().log() - tl.double()).abs() * weight.double()).sum()
+    none, m2, se2, tl2, no_loss = KK.linear_cross_entropy_stats(x, w, tgt, start, store=False)
+    assert none is None and no_loss is None
+    assert torch.equal(m, m2) and torch.equal(se, se2) and torch.equal(tl, tl2)
+    x[0] = float("nan")
+    _, m, se, _, _ = KK.linear_cross_entropy_stats(x, w, tgt, start, store=False)
+    assert se[0].isnan() and (M == 1 or not se[1:].isnan().any())
+
+
 @pytest.mark.parametrize("H", [8, 1032, 3072])
 def test_embedding_backward_vectors(H):
     KC = _K()
