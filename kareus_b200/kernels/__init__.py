@@ -105,6 +105,22 @@ def swiglu_bwd(dy, x):
     return ref.swiglu_bwd(dy, x)
 
 
+def linear_swiglu(x, w, store=True):
+    """``(y, swiglu(y))`` of the ``[gate | up]`` projection ``y = x @ w.T`` in one launch, or ``None`` where two are the way to
+    go (:func:`gemm`, :func:`swiglu_fwd`).  ``store=False``: ``y`` is not wanted and ``None``."""
+    if is_cuda(x) and not library_baseline():
+        return _cuda().linear_swiglu(x, w, store)
+    return None
+
+
+def linear_swiglu_dgrad(dy, w, x):
+    """Gradient of ``x = [gate | up]`` for the gradient ``dy`` of ``swiglu(x) @ w.T``, in one launch, or ``None`` where two are the
+    way to go (:func:`gemm`, :func:`swiglu_bwd`)."""
+    if is_cuda(dy) and not library_baseline():
+        return _cuda().linear_swiglu_dgrad(dy, w, x)
+    return None
+
+
 # ----------------------------------------------------------------------------- dropout-add
 def dropout_add_fwd(x, residual, p, seed):
     if is_cuda(x):

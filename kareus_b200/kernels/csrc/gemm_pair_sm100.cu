@@ -90,6 +90,8 @@ struct PairWork {
 enum PairEpilogue : int {
   EPI_NONE = 0,
   EPI_ROW_STATS = 1,    // maximum and sum of exponentials of the row pieces that it stores (see RowStats)
+  EPI_SWIGLU = 2,       // silu(gate) * up of a [gate | up] product (see SwigluOut)
+  EPI_SWIGLU_BWD = 3,   // from the gradient of silu(gate) * up, which is the product, that of [gate | up]
 };
 
 // Row statistics of the bf16 product for a softmax over its columns.  A thread of the epilogue has a row of its tile in
@@ -106,10 +108,96 @@ struct RowStats {
   bool store;            // false: the product itself is not wanted
 };
 
+// EPI_SWIGLU: a tile has 128 gate columns (B rows that CTA 0 loads) and the up columns of the same features (CTA 1), so
+// a thread of the epilogue holds both and stores their activation; the product itself leaves only if it is wanted
+// for a backward pass (as halves of a [M, 2 * features] matrix).
+// EPI_SWIGLU_BWD: the epilogue fetches gate and up of its columns and stores both gradients; the gradient of the
+// activation never reaches memory.
+// Everything is rounded to bf16 where the separate kernels store it.  One B200, us with kernels of their own / in the epilogue:
+// forward 16384 x 3072 → 2 x 8192 1176 / 1059 (1002 without the product), 3800 x 2048 → 2 x 6144 146 / 123 (117); backward
+// 16384 x 3072 → 8192 741 / 604, 3800 x 2048 → 6144 111 / 91.
+struct SwigluOut {
+  CUtensorMap gate, up;     // boxes of 32 rows x 64 columns
+  int features;
+  bool store;               // the product is wanted
+};
+struct SwigluGrad {
+  const __nv_bfloat16* x;   // [gate | up] of the forward pass, [M, 2 * features]
+  __nv_bfloat16* dx;        // its gradient
+};
+template <int EPI> struct EpiArgs { struct type {}; };
+template <> struct EpiArgs<EPI_ROW_STATS> { using type = RowStats; };
+template <> struct EpiArgs<EPI_SWIGLU> { using type = SwigluOut; };
+template <> struct EpiArgs<EPI_SWIGLU_BWD> { using type = SwigluGrad; };
+
+__device__ __forceinline__ float2 bf16_pair(uint32_t v) {
+  return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// 64 accumulator columns of a thread's row as packed bf16 pairs.
+__device__ __forceinline__ void pack_row(const uint32_t (&v0)[32], const uint32_t (&v1)[32], uint32_t (&o)[32]) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    o[j] = pack_bf16x2(__uint_as_float(v0[2 * j]), __uint_as_float(v0[2 * j + 1]));
+    o[16 + j] = pack_bf16x2(__uint_as_float(v1[2 * j]), __uint_as_float(v1[2 * j + 1]));
+  }
+}
+
+// A warp's slab (32 rows x 128 bytes, a row per thread) into its staging buffer, 16-byte units swizzled by row as the tensor maps
+// expect, once the store before it has read the buffer.
+__device__ __forceinline__ void put_slab(const uint32_t (&o)[32], uint32_t stg_row, int lane) {
+  if (lane == 0) tma_store_wait_read<0>();
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) st_shared_v4(stg_row + ((j ^ (lane & 7)) << 4), o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+  fence_proxy_async_smem();
+  __syncwarp();
+}
+
+// 32 rows x 64 columns of a matrix, whole 128-byte row segments per access; rows past M and columns past N (a multiple of 8) read
+// as zero.
+__device__ __forceinline__ void load_slab(const __nv_bfloat16* x, int ld, int row0, int M, int col, int N, int lane, uint4 (&v)[8]) {
+  const int unit = lane & 7;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = row0 + i * 4 + (lane >> 3);
+    v[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (r < M && col + unit * 8 < N) v[i] = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(r) * ld + col + unit * 8);
+  }
+}
+// What load_slab returned into a (free) 4 KB buffer, 16-byte units swizzled by row, and such a buffer out to a matrix.
+__device__ __forceinline__ void slab_to_smem(const uint4 (&v)[8], uint8_t* buf, int lane) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = i * 4 + (lane >> 3);
+    *reinterpret_cast<uint4*>(buf + r * 128 + (((lane & 7) ^ (r & 7)) << 4)) = v[i];
+  }
+}
+__device__ __forceinline__ void slab_from_smem(const uint8_t* buf, __nv_bfloat16* x, int ld, int row0, int M, int col, int N, int lane) {
+  const int unit = lane & 7;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = i * 4 + (lane >> 3);
+    const uint4 v = *reinterpret_cast<const uint4*>(buf + r * 128 + ((unit ^ (r & 7)) << 4));
+    if (row0 + r < M && col + unit * 8 < N) *reinterpret_cast<uint4*>(x + static_cast<size_t>(row0 + r) * ld + col + unit * 8) = v;
+  }
+}
+
+// 1 / (1 + e^-a) of two values.
+__device__ __forceinline__ float2 sigmoid2(float2 a) {
+  constexpr float L2E = 1.4426950408889634f;
+  float2 e = __fmul2_rn(a, make_float2(-L2E, -L2E));
+  e = __fadd2_rn(make_float2(ex2_approx(e.x), ex2_approx(e.y)), make_float2(1.f, 1.f));
+  float2 r;                                          // keeps subnormal results, unlike a quick division
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r.x) : "f"(e.x));
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r.y) : "f"(e.y));
+  return r;
 }
 
 // Adds 64 columns of a row (packed bf16 pairs, the first `valid` of them count) to a running maximum and sum.
@@ -149,7 +237,7 @@ template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmW, const PairWork w,
-                 const int M, const int N, const int bn, int* status, const RowStats stats) {
+                 const int M, const int N, const int bn, int* status, const __grid_constant__ typename EpiArgs<EPI>::type epi) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + GP_TILE_BYTES + GP_STG_BYTES);   // used in the leader
@@ -166,7 +254,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int half_n = bn >> 1;
   // What a narrow tile waits for is latency times bytes in flight, so it gets all the stages that fit
   const int b_bytes = gp_b_bytes(bn, B_MN), stage_bytes = GP_A_BYTES + b_bytes;
-  const int stages = min(GP_MAX_STAGES, GP_TILE_BYTES / stage_bytes);
+  // one stage less where the epilogue works on two slabs a warp
+  constexpr int RING = GP_TILE_BYTES - (EPI == EPI_SWIGLU_BWD ? GP_EPI_WARPS * 4096 : 0);
+  const int stages = min(GP_MAX_STAGES, RING / stage_bytes);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < GP_MAX_STAGES; ++i) {
@@ -203,7 +293,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         int tm, tn, kb0, kb1;
         w.decode(u, tm, tn, kb0, kb1);
         const int m0 = tm * GP_BM + rank * 128;
-        const int n0 = tn * bn + rank * half_n;
+        int n0 = tn * bn + rank * half_n;
+        if constexpr (EPI == EPI_SWIGLU) n0 = tn * 128 + rank * epi.features;
         for (int kb_ = kb0; kb_ < kb1; ++kb_) {
           if (!mbar_wait(&empty[s], ph, abort_flag, status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
           uint8_t* a_dst = smem + s * stage_bytes;
@@ -275,24 +366,129 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // ------------------------------------------------------------------ epilogue
     const int q = warp & 3;                   // TMEM lane quarter
     const int h = (warp - 2) >> 2;            // this warp takes the column slabs h, h + 2, ...
-    uint8_t* stg = smem + GP_TILE_BYTES + (warp - 2) * 4096;
+    uint8_t* stg = smem + RING + (warp - 2) * (EPI == EPI_SWIGLU_BWD ? 8192 : 4096);
     constexpr int SLAB = OUT_F32 ? 32 : 64;   // output columns of one 128-byte wide slab
     const int slabs = bn / SLAB;
     const uint32_t stg_row = smem_u32(stg) + lane * 128;
     uint32_t tile_i = 0;
+    if constexpr (EPI == EPI_SWIGLU_BWD) {
+      // Gate and up of the next slab, of this tile or the next, are on their way while one is worked on and while the
+      // accumulator is waited for; the gradients take their place in shared memory, a row per thread.
+      uint4 vg[8], vu[8];
+      auto fetch = [&](int u, int c) {
+        int tm, tn, kb0, kb1;
+        w.decode(u, tm, tn, kb0, kb1);
+        const int row0 = tm * GP_BM + rank * 128 + q * 32, col = tn * bn + c * SLAB;
+        load_slab(epi.x, 2 * N, row0, M, col, N, lane, vg);
+        load_slab(epi.x + N, 2 * N, row0, M, col, N, lane, vu);
+      };
+      if (first < num_units && h < slabs) fetch(first, h);
+      for (int u = first; u < num_units; u += step, ++tile_i) {
+        int tm, tn, kb0, kb1;
+        w.decode(u, tm, tn, kb0, kb1);
+        const uint32_t buf = tile_i & 1u;
+        const int row0 = tm * GP_BM + rank * 128 + q * 32;
+        if (!mbar_wait_warp(&tfull[buf], (tile_i >> 1) & 1u, abort_flag, status, ST_TIMEOUT_TMEM_FULL)) break;
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + buf * 256 + (static_cast<uint32_t>(q * 32) << 16);
+#pragma unroll 1
+        for (int c = h; c < slabs; c += 2) {
+          slab_to_smem(vg, stg, lane);
+          slab_to_smem(vu, stg + 4096, lane);
+          __syncwarp();
+          if (c + 2 < slabs) fetch(u, c + 2);
+          else if (u + step < num_units) fetch(u + step, h);
+          const float2 one = make_float2(1.f, 1.f);
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t v[32];
+            tmem_ld_32x32(taddr + c * 64 + half * 32, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              uint4* pg = reinterpret_cast<uint4*>(stg + lane * 128 + (((half * 4 + j) ^ (lane & 7)) << 4));
+              uint4* pu = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(pg) + 4096);
+              uint4 g4 = *pg, u4 = *pu;
+              uint32_t* g = reinterpret_cast<uint32_t*>(&g4);
+              uint32_t* up = reinterpret_cast<uint32_t*>(&u4);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float2 d = bf16_pair(pack_bf16x2(__uint_as_float(v[8 * j + 2 * i]), __uint_as_float(v[8 * j + 2 * i + 1])));
+                const float2 a = bf16_pair(g[i]), sg = sigmoid2(a), ds = __fmul2_rn(d, sg);
+                const float2 t = __ffma2_rn(a, __fadd2_rn(one, make_float2(-sg.x, -sg.y)), one);      // 1 + a (1 - sigmoid)
+                const float2 da = __fmul2_rn(__fmul2_rn(ds, bf16_pair(up[i])), t), db = __fmul2_rn(ds, a);
+                g[i] = pack_bf16x2(da.x, da.y);
+                up[i] = pack_bf16x2(db.x, db.y);
+              }
+              *pg = g4;
+              *pu = u4;
+            }
+          }
+          if (c + 2 >= slabs) tc_fence_before();
+          __syncwarp();
+          if (c + 2 >= slabs && lane == 0) mbar_arrive_cluster(cluster_addr(&tempty[buf], 0));
+          const int col = tn * bn + c * SLAB;
+          slab_from_smem(stg, epi.dx, 2 * N, row0, M, col, N, lane);
+          slab_from_smem(stg + 4096, epi.dx + N, 2 * N, row0, M, col, N, lane);
+          __syncwarp();
+        }
+        if (slabs <= h) {                             // no slab for this warp (narrow tile): release all the same
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(cluster_addr(&tempty[buf], 0));
+        }
+      }
+    } else
     for (int u = first; u < num_units; u += step, ++tile_i) {
       int tm, tn, kb0, kb1;
       w.decode(u, tm, tn, kb0, kb1);
       const uint32_t buf = tile_i & 1u;
+      const int row0 = tm * GP_BM + rank * 128 + q * 32;
       if (!mbar_wait_warp(&tfull[buf], (tile_i >> 1) & 1u, abort_flag, status, ST_TIMEOUT_TMEM_FULL)) break;
       tc_fence_after();
-      const int row0 = tm * GP_BM + rank * 128 + q * 32;
       const uint32_t taddr = tmem_base + buf * 256 + (static_cast<uint32_t>(q * 32) << 16);
+      if constexpr (EPI == EPI_SWIGLU) {
+        // this warp's 64 features: gate at column 64 h of the accumulator, up at 128 + 64 h
+        uint32_t g[32], u[32];
+        {
+          uint32_t v0[32], v1[32];
+          tmem_ld_32x32(taddr + h * 64, v0);
+          tmem_ld_32x32(taddr + h * 64 + 32, v1);
+          tmem_ld_wait();
+          pack_row(v0, v1, g);
+          tmem_ld_32x32(taddr + 128 + h * 64, v0);
+          tmem_ld_32x32(taddr + 128 + h * 64 + 32, v1);
+          tmem_ld_wait();
+          pack_row(v0, v1, u);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(cluster_addr(&tempty[buf], 0));
+        const int col = tn * 128 + h * 64;
+        const bool here = row0 < M && col < N;
+        if (epi.store) {
+          put_slab(g, stg_row, lane);
+          if (lane == 0 && here) tma_store_2d(&epi.gate, stg, col, row0);
+          if (lane == 0) tma_store_commit();
+          put_slab(u, stg_row, lane);
+          if (lane == 0 && here) tma_store_2d(&epi.up, stg, col, row0);
+          if (lane == 0) tma_store_commit();
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float2 a = bf16_pair(g[j]), y = __fmul2_rn(__fmul2_rn(a, sigmoid2(a)), bf16_pair(u[j]));
+          g[j] = pack_bf16x2(y.x, y.y);
+        }
+        put_slab(g, stg_row, lane);
+        if (lane == 0 && here) tma_store_2d(&tmC, stg, col, row0);
+        if (lane == 0) tma_store_commit();
+        continue;
+      }
       const int row = row0 + lane;
       float row_max = -INFINITY, row_sum = 0.f;
       long target = -1;                               // column of this tile that holds the row's target
       if constexpr (EPI == EPI_ROW_STATS) {
-        if (row < M) target = stats.targets[row] - stats.first_col;
+        if (row < M) target = epi.targets[row] - epi.first_col;
         target = target >= 0 && target < N ? target - tn * bn : -1;
       }
 #pragma unroll 1
@@ -306,11 +502,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           tmem_ld_32x32(taddr + c * 64, v0);
           tmem_ld_32x32(taddr + c * 64 + 32, v1);
           tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            o[j] = pack_bf16x2(__uint_as_float(v0[2 * j]), __uint_as_float(v0[2 * j + 1]));
-            o[16 + j] = pack_bf16x2(__uint_as_float(v1[2 * j]), __uint_as_float(v1[2 * j + 1]));
-          }
+          pack_row(v0, v1, o);
         }
         if (c + 2 >= slabs) {
           // this warp's last read of the accumulator: hand it back before the stores go out
@@ -331,9 +523,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
               for (int j = 0; j < n; ++j) pick[j] = t & (2 * n) ? pick[n + j] : pick[j];
             const uint32_t pair = pick[0];
-            stats.target[row] = __uint_as_float(t & 1 ? pair & 0xffff0000u : pair << 16);
+            epi.target[row] = __uint_as_float(t & 1 ? pair & 0xffff0000u : pair << 16);
           }
-          if (!stats.store) continue;
+          if (!epi.store) continue;
         }
         if (lane == 0) tma_store_wait_read<0>();      // the previous slab has left the staging buffer
         __syncwarp();
@@ -351,7 +543,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       }
       if constexpr (EPI == EPI_ROW_STATS) {
-        if (row < M) stats.part[static_cast<size_t>(2 * tn + h) * M + row] = make_float2(row_max, row_sum);
+        if (row < M) epi.part[static_cast<size_t>(2 * tn + h) * M + row] = make_float2(row_max, row_sum);
       }
       if (slabs <= h) {                               // no slab for this warp (narrow tile): release all the same
         tc_fence_before();
@@ -462,13 +654,13 @@ gemm_add_parts_kernel(float* __restrict__ C, int ldc, int M, int N, const float*
 template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int EPI = EPI_NONE>
 static int launch_pair(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                        const PairPlan& pl, int pairs, float* work, int* status, cudaStream_t stream,
-                       const RowStats& stats = RowStats{}) {
+                       const typename EpiArgs<EPI>::type& epi = {}) {
   CUtensorMap tmA, tmB, tmC, tmW;
   int rc;
   if (!A_MN) rc = make_tmap_2d_bf16(&tmA, A, K, M, lda, GP_BK, 128);
   else       rc = make_tmap_2d_bf16(&tmA, A, M, K, lda, 64, GP_BK);
   if (rc) return rc;
-  if (!B_MN) rc = make_tmap_2d_bf16(&tmB, B, K, N, ldb, GP_BK, pl.bn / 2);
+  if (!B_MN) rc = make_tmap_2d_bf16(&tmB, B, K, EPI == EPI_SWIGLU ? 2 * N : N, ldb, GP_BK, pl.bn / 2);
   else       rc = make_tmap_2d_bf16(&tmB, B, N, K, ldb, 64, GP_BK);
   if (rc) return rc;
   {
@@ -496,7 +688,7 @@ static int launch_pair(const void* A, const void* B, void* C, int M, int N, int 
   }
   PairWork w;
   w.tiles_m = (M + GP_BM - 1) / GP_BM;
-  w.tiles_n = (N + pl.bn - 1) / pl.bn;
+  w.tiles_n = EPI == EPI_SWIGLU ? (N + 127) / 128 : (N + pl.bn - 1) / pl.bn;
   w.nk = (K + GP_BK - 1) / GP_BK;
   w.ks = split ? pl.ks : 1;
   w.ordered = ordered;
@@ -510,7 +702,7 @@ static int launch_pair(const void* A, const void* B, void* C, int M, int N, int 
   w.group_m = gm < w.tiles_m ? (int)gm : w.tiles_m;
   const int units = w.whole + w.split_tiles * w.ks;
   const int grid = 2 * (units < pairs ? units : pairs);
-  KB_LAUNCH_PDL(kern, grid, GP_THREADS, GP_SMEM, stream, tmA, tmB, tmC, tmW, w, M, N, pl.bn, status, stats);
+  KB_LAUNCH_PDL(kern, grid, GP_THREADS, GP_SMEM, stream, tmA, tmB, tmC, tmW, w, M, N, pl.bn, status, epi);
   if (ordered) {
     const int blocks = w.split_tiles * (GP_BM * pl.bn / 4 / 256);
     KB_LAUNCH_PDL(gemm_add_parts_kernel, blocks, 256, 0, stream, static_cast<float*>(C), ldc, M, N, (const float*)work, w, pl.bn);
@@ -549,6 +741,33 @@ int gemm_pair_row_stats(const void* A, const void* B, void* C, int M, int N, int
   if (weight) KB_LAUNCH_PDL(sum_kernel, 1, 256, 0, stream, (const float*)block_loss, blocks, loss);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 2000 + static_cast<int>(e);
+}
+
+static int swiglu_maps(SwigluOut* e, const void* x, int M, int features) {
+  const uint64_t dims[2] = {(uint64_t)features, (uint64_t)M};
+  const uint64_t str[1] = {(uint64_t)features * 4};
+  const uint32_t box[2] = {64u, 32u};
+  const int rc = make_tmap(&e->gate, x, 2, 2, dims, str, box, 3);
+  return rc ? rc : make_tmap(&e->up, reinterpret_cast<const __nv_bfloat16*>(x) + features, 2, 2, dims, str, box, 3);
+}
+
+int gemm_pair_swiglu(const void* A, const void* B, void* X, void* H, int M, int features, int K, int lda, int ldb, int pairs,
+                     int* status, cudaStream_t stream) {
+  SwigluOut e;
+  e.features = features;
+  e.store = X != nullptr;
+  // without a product to store its tensor maps are never used; they still need an address
+  const int rc = swiglu_maps(&e, X ? X : H, M, features);
+  if (rc) return rc;
+  return launch_pair<false, false, false, false, EPI_SWIGLU>(A, B, H, M, features, K, lda, ldb, features, PairPlan{256, 1, 0, 0.0, false},
+                                                             pairs, nullptr, status, stream, e);
+}
+
+int gemm_pair_swiglu_bwd(const void* A, const void* B, const void* X, void* dX, int M, int features, int K, int lda, int ldb,
+                         const PairPlan& pl, int pairs, int* status, cudaStream_t stream) {
+  const SwigluGrad e{reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<__nv_bfloat16*>(dX)};
+  return launch_pair<false, true, false, false, EPI_SWIGLU_BWD>(A, B, dX, M, features, K, lda, ldb, 2 * features, pl, pairs, nullptr,
+                                                                status, stream, e);
 }
 
 }  // namespace kb

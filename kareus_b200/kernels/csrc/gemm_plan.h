@@ -27,4 +27,12 @@ int gemm_pair_row_stats(const void* A, const void* B, void* C, int M, int N, int
                         int pairs, const long* targets, long first_col, float* part, float* omax, float* osum, float* otgt,
                         const float* weight, float* loss, int* status, cudaStream_t stream);
 
+// H [M, features] = silu(gate) * up of [gate | up] = A [M, K] * B [2 * features, K]^T, which goes to X ([M, 2 * features]) unless X
+// is null.
+int gemm_pair_swiglu(const void* A, const void* B, void* X, void* H, int M, int features, int K, int lda, int ldb, int pairs,
+                     int* status, cudaStream_t stream);
+// dX [M, 2 * features] = gradient of X = [gate | up] when that of silu(gate) * up is A [M, K] * B [K, features].
+int gemm_pair_swiglu_bwd(const void* A, const void* B, const void* X, void* dX, int M, int features, int K, int lda, int ldb,
+                         const PairPlan& pl, int pairs, int* status, cudaStream_t stream);
+
 }  // namespace kb

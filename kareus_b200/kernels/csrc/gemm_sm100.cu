@@ -478,19 +478,47 @@ static PairPlan plan_pair(int M, int N, int K, int pairs, bool b_mn) {
 // cluster to start it is 1 us quicker to its first product, and 128-row tiles waste less of a short last wave; per step it
 // takes 10 % longer.  776 x 5120 x 3072: 27.7 us on pairs (two waves), 20.7 here (one); 4096 x 1024 x 128: 7.4 and 6.0.  Up to
 // two steps of K it was the faster one whatever the number of waves (15720 x 4344 x 128: 52.3 and 44.1).
-static int single_width(int M, int N, int K, bool b_mn, int num_sms, int pair_bn) {
-  static const double pair_us[5][3] = {{}, {0.16, 1.0, 4.4}, {0.179, 1.4, 4.3}, {0.245, 1.85, 4.0}, {0.304, 1.95, 4.6}};
+static const double pair_us[5][3] = {{}, {0.16, 1.0, 4.4}, {0.179, 1.4, 4.3}, {0.245, 1.85, 4.0}, {0.304, 1.95, 4.6}};   // step, wave, call
+struct PlainTimes { double pair, w128, w256; };
+static PlainTimes plain_times(int M, int N, int K, bool b_mn, int num_sms, int pair_bn) {
   const int nk = (K + GEMM_BK - 1) / GEMM_BK;
   auto waves = [](int M_, int N_, int bm, int bn, int slots) {
     return (long)(((long)((M_ + bm - 1) / bm) * ((N_ + bn - 1) / bn) + slots - 1) / slots);
   };
   const double* c = pair_us[pair_bn / 64];
   // an MN-major B comes in 64-wide chunks, of which 64-wide tiles use half
-  const double pair = c[2] + (b_mn && pair_bn == 64 ? 0.6 : 0.0) + waves(M, N, 256, pair_bn, num_sms / 2) * (nk * c[0] + c[1]);
-  const double w128 = 3.5 + waves(M, N, 128, 128, num_sms) * (nk * 0.275 + 0.95);
-  const double w256 = 3.2 + waves(M, N, 128, 256, num_sms) * (nk * 0.337 + 2.2);
-  if (nk > 2 && (w128 < w256 ? w128 : w256) >= 0.97 * pair) return 0;
-  return w128 < w256 ? 128 : 256;
+  return {c[2] + (b_mn && pair_bn == 64 ? 0.6 : 0.0) + waves(M, N, 256, pair_bn, num_sms / 2) * (nk * c[0] + c[1]),
+          3.5 + waves(M, N, 128, 128, num_sms) * (nk * 0.275 + 0.95), 3.2 + waves(M, N, 128, 256, num_sms) * (nk * 0.337 + 2.2)};
+}
+static int single_width(int M, int N, int K, bool b_mn, int num_sms, int pair_bn) {
+  const PlainTimes t = plain_times(M, N, K, b_mn, num_sms, pair_bn);
+  if ((K + GEMM_BK - 1) / GEMM_BK > 2 && (t.w128 < t.w256 ? t.w128 : t.w256) >= 0.97 * t.pair) return 0;
+  return t.w128 < t.w256 ? 128 : 256;
+}
+
+static bool g_force_swiglu = false;
+enum SwigluKind : int { SWIGLU_STORE = 0, SWIGLU_BACKWARD = 1, SWIGLU_NO_STORE = 2 };
+// Is the activation in the epilogue faster than the product followed by a kernel of its own (2.5 us, and 6 bytes an element
+// forward, 10 backward, at 5.5 TB/s)?  The epilogue of a 256-column tile takes about 5 us where it stores the product too, 3.5
+// where it does not, and 12 to 14.5 backward (memory latency; it has eight warps); it runs under the main loop of the next
+// tile, the last one alone.  Measured, us of two kernels / one: forward 512 x 512 → 2 x 1024 13.5 / 14.1 (12.4 without the
+// product), 300 x 2048 → 2 x 6144 24.4 / 32.6, 3800 x 2048 → 2 x 6144 145 / 122; backward 20000 x 128 → 1024 54.7 / 68.4, 4096 x 3072
+// → 1024 34.5 / 35.8, 1900 x 3072 → 8192 102 / 89, 8997 x 2048 → 6144 245 / 195.
+static bool swiglu_pays(int M, int features, int K, int kind, int num_sms) {
+  if (g_force_swiglu) return true;
+  const bool backward = kind == SWIGLU_BACKWARD;
+  const int nk = (K + GEMM_BK - 1) / GEMM_BK, N = backward ? features : 2 * features, pairs = num_sms / 2;
+  const int bn = plan_pair(M, N, K, pairs, backward).bn;
+  const PlainTimes t = plain_times(M, N, K, backward, num_sms, bn);
+  const double plain = t.pair < t.w128 ? (t.pair < t.w256 ? t.pair : t.w256) : (t.w128 < t.w256 ? t.w128 : t.w256);
+  const int fbn = backward ? bn : 256;
+  const double* c = pair_us[fbn / 64];
+  const long waves = ((long)((M + 255) / 256) * ((N + fbn - 1) / fbn) + pairs - 1) / pairs;
+  const double last = (backward ? 12.0 : kind == SWIGLU_STORE ? 5.0 : 3.5) * fbn / 256;
+  const double main_loop = (nk * c[0] + c[1]) * (backward ? 1.15 : 1.0);
+  const double epilogue = (backward ? 14.5 : kind == SWIGLU_STORE ? 4.2 : 3.1) * fbn / 256;
+  const double fused = c[2] + waves * (main_loop > epilogue ? main_loop : epilogue) + last;
+  return fused < plain + 2.5 + (backward ? 10.0 : 6.0) * M * features / 5.5e6;
 }
 
 // `C +=`.  Where 128-row tiles would not fill the chip once and be split even so, the parts add in L2 as they come: the
@@ -642,4 +670,35 @@ extern "C" int kb_gemm_row_stats(const void* A, const void* B, void* C, int M, i
   const int pairs = device_sm_count() / 2;
   return gemm_pair_row_stats(A, B, C, M, N, K, lda, ldb, plan_pair(M, N, K, pairs, false), pairs, targets, vocab_start, part, omax,
                              osum, otgt, weight, loss, status, stream);
+}
+
+// SwiGLU in the epilogue of the GEMM beside it (see SwigluOut in gemm_pair_sm100.cu).  A [M, K], B [2 * features, K], X [M, 2 *
+// features] (or null), H [M, features]; backward: A [M, K], B [K, features], X and dX [M, 2 * features].  X, H and dX are
+// contiguous, features a multiple of 8.  kb_gemm_swiglu_pays: is that the faster way (kind: 0 forward with X, 1 backward, 2 forward
+// without X)?
+extern "C" int kb_gemm_swiglu_pays(int M, int features, int K, int kind) {
+  using namespace kb;
+  if (M <= 0 || features <= 0 || K <= 0 || (features & 7) || features > (1 << 29)) return 0;
+  return swiglu_pays(M, features, K, kind, device_sm_count()) ? 1 : 0;
+}
+// Measurement and test aid: take the epilogue for every shape.
+extern "C" void kb_gemm_swiglu_force(int on) { kb::g_force_swiglu = on != 0; }
+
+static bool swiglu_args_ok(int M, int features, int K, int lda, int ldb, const void* A, const void* B, const void* X, const void* Y) {
+  return M > 0 && features > 0 && K > 0 && features <= (1 << 29) && !((features | lda | ldb) & 7) &&
+         !((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(X) |
+            reinterpret_cast<uintptr_t>(Y)) & 15);
+}
+extern "C" int kb_gemm_swiglu(const void* A, const void* B, void* X, void* H, int M, int features, int K, int lda, int ldb, int* status,
+                              cudaStream_t stream) {
+  using namespace kb;
+  if (!swiglu_args_ok(M, features, K, lda, ldb, A, B, X, H) || !H) return ST_BAD_ARG;
+  return gemm_pair_swiglu(A, B, X, H, M, features, K, lda, ldb, device_sm_count() / 2, status, stream);
+}
+extern "C" int kb_gemm_swiglu_bwd(const void* A, const void* B, const void* X, void* dX, int M, int features, int K, int lda, int ldb,
+                                  int* status, cudaStream_t stream) {
+  using namespace kb;
+  if (!swiglu_args_ok(M, features, K, lda, ldb, A, B, X, dX) || !X || !dX) return ST_BAD_ARG;
+  const int pairs = device_sm_count() / 2;
+  return gemm_pair_swiglu_bwd(A, B, X, dX, M, features, K, lda, ldb, plan_pair(M, features, K, pairs, true), pairs, status, stream);
 }

@@ -69,6 +69,9 @@ def _declare(L) -> None:
         "kb_gemm_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P],
         "kb_gemm_accum_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, P, P, P],
         "kb_gemm_row_stats": [P, P, P, I, I, I, I, I, P, LNG, P, P, P, P, P, P, P, P],
+        "kb_gemm_swiglu_pays": [I, I, I, I],
+        "kb_gemm_swiglu": [P, P, P, P, I, I, I, I, I, P, P],
+        "kb_gemm_swiglu_bwd": [P, P, P, P, I, I, I, I, I, P, P],
         "kb_gemm_bias_act_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, I, P, P],
         "kb_rmsnorm_fwd": [P, P, P, P, I, I, F, P],
         "kb_rmsnorm_fwd_heads": [P, LNG, I, LNG, LNG, P, P, P, I, F, P],
@@ -333,6 +336,38 @@ def swiglu_bwd(dy, x):
     rows, F2 = x.shape
     dx = torch.empty_like(x)
     _check(lib().kb_swiglu_bwd(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), rows, F2 // 2, _stream()), "swiglu_bwd")
+    _count()
+    return dx
+
+
+def linear_swiglu(x, w, store):
+    """See :func:`kareus_b200.kernels.linear_swiglu`; ``None`` where the two kernels of its own are the way to go."""
+    if not (_bf16(x) and _bf16(w) and x.dim() == 2 and w.dim() == 2 and x.numel() and w.numel() and w.shape[0] % 16 == 0
+            and x.shape[1] == w.shape[1] and _rowmajor_ok(x) and _rowmajor_ok(w)):
+        return None
+    (M, Kd), F, L = x.shape, w.shape[0] // 2, lib()
+    if not L.kb_gemm_swiglu_pays(M, F, Kd, 0 if store else 2):
+        return None
+    y = torch.empty(M, 2 * F, dtype=x.dtype, device=x.device) if store else None
+    h = torch.empty(M, F, dtype=x.dtype, device=x.device)
+    _check(L.kb_gemm_swiglu(x.data_ptr(), w.data_ptr(), y.data_ptr() if store else 0, h.data_ptr(), M, F, Kd, x.stride(0),
+                            w.stride(0), status_word(x.device).data_ptr(), _stream()), f"gemm+swiglu M={M} F={F} K={Kd}")
+    _count()
+    return y, h
+
+
+def linear_swiglu_dgrad(dy, w, x):
+    """See :func:`kareus_b200.kernels.linear_swiglu_dgrad`; ``None`` as above."""
+    if not (_bf16(dy) and _bf16(w) and _bf16(x) and dy.dim() == 2 and w.dim() == 2 and x.dim() == 2 and dy.numel() and w.numel()
+            and dy.shape[1] == w.shape[0] and tuple(x.shape) == (dy.shape[0], 2 * w.shape[1]) and w.shape[1] % 8 == 0
+            and x.is_contiguous() and x.data_ptr() % 16 == 0 and _rowmajor_ok(dy) and _rowmajor_ok(w)):
+        return None
+    (M, Kd), F, L = dy.shape, w.shape[1], lib()
+    if not L.kb_gemm_swiglu_pays(M, F, Kd, 1):
+        return None
+    dx = torch.empty_like(x)
+    _check(L.kb_gemm_swiglu_bwd(dy.data_ptr(), w.data_ptr(), x.data_ptr(), dx.data_ptr(), M, F, Kd, dy.stride(0), w.stride(0),
+                                status_word(x.device).data_ptr(), _stream()), f"gemm+swiglu backward M={M} F={F} K={Kd}")
     _count()
     return dx
 

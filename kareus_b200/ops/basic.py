@@ -96,9 +96,13 @@ class SwiGLUOp(GraphOperator):
 
     def __init__(self, name: str = "swiglu"):
         self.name = name
+        self.fused_features = 0             # width of an activation that the linear layer before it has computed already
 
     def forward(self, ctx, x):
         shp = x.shape
+        if shp[-1] == self.fused_features:
+            ctx.save_for_backward()
+            return (x,)
         x2 = x.reshape(-1, shp[-1])
         y = K.swiglu_fwd(x2)
         if ctx.requires_grad:
@@ -106,6 +110,8 @@ class SwiGLUOp(GraphOperator):
         return (y.reshape(shp[:-1] + (shp[-1] // 2,)),)
 
     def backward(self, ctx, dy):
+        if not ctx.saved_tensors:
+            return (dy,)
         (x2,) = ctx.saved_tensors
         dx = K.swiglu_bwd(dy.reshape(-1, dy.shape[-1]), x2)
         return (dx.reshape(dy.shape[:-1] + (x2.shape[-1],)),)

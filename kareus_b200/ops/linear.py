@@ -56,6 +56,11 @@ class _LinearBase(nn.Module, GraphOperator):
     def _bwd_staging(self, shape, dtype, nb, device):
         return None
 
+    # The SwiGLU between fc1 and fc2 can run in the epilogues of the GEMMs beside it: fc1 then returns the activation, which
+    # :class:`SwiGLUOp` passes on, and fc2 returns the gradient of fc1's output.  Shapes say which of the two a tensor is.
+    # `_swiglu_in` on the activation is fc1's output (kept where there will be a backward pass).
+    fuse_swiglu = False                     # set on fc1 and fc2 of a layer whose activation it is
+
     def forward(self, ctx, x):
         shp = x.shape
         x2 = x.reshape(-1, shp[-1])
@@ -66,7 +71,7 @@ class _LinearBase(nn.Module, GraphOperator):
         return (y.reshape(shp[:-1] + (self.out_features,)),)
 
     def backward(self, ctx, dy):
-        (x2,) = ctx.saved_tensors
+        x2 = ctx.saved_tensors[0]
         shp = dy.shape
         dy2 = dy.reshape(-1, shp[-1])
         out = self._bwd_staging((dy2.shape[0], self.in_features), dy2.dtype, ctx.nb_index, dy2.device)
@@ -94,6 +99,27 @@ class ColumnParallelLinear(_LinearBase):
             return None
         op = self.bwd_allreduce if self.tp_comm == "allreduce" else self.bwd_reducescatter
         return op.staging(shape, dtype, nb, device)
+
+    def forward(self, ctx, x):
+        if not self.fuse_swiglu:
+            return super().forward(ctx, x)
+        shp = x.shape
+        x2 = x.reshape(-1, shp[-1])
+        r = K.linear_swiglu(x2, self.weight, store=ctx.requires_grad)
+        if r is None:
+            return super().forward(ctx, x)
+        y, h = r
+        h = h.reshape(shp[:-1] + (self.out_features // 2,))
+        if ctx.requires_grad:
+            ctx.save_for_backward(x2, y)
+            h._swiglu_in = y
+        return (h,)
+
+    def backward(self, ctx, dy):
+        if len(ctx.saved_tensors) == 2 and dy.shape[-1] != self.out_features:      # gradient of the activation
+            y = ctx.saved_tensors[1]
+            dy = K.swiglu_bwd(dy.reshape(-1, dy.shape[-1]), y).reshape(dy.shape[:-1] + (self.out_features,))
+        return super().backward(ctx, dy)
 
     def forward_specs(self) -> List[object]:
         compute = ComputeSpec(self, ("main",), ("main",))
@@ -138,6 +164,23 @@ class RowParallelLinear(_LinearBase):
             return None
         op = self.fwd_allreduce if self.tp_comm == "allreduce" else self.fwd_reducescatter
         return op.staging(shape, dtype, nb, device)
+
+    def forward(self, ctx, x):
+        out = super().forward(ctx, x)
+        y = getattr(x, "_swiglu_in", None) if self.fuse_swiglu else None
+        if y is not None and ctx.requires_grad:
+            ctx.save_for_backward(*ctx.saved_tensors, y)
+        return out
+
+    def backward(self, ctx, dy):
+        if len(ctx.saved_tensors) == 2:
+            h2, y = ctx.saved_tensors
+            dy2 = dy.reshape(-1, dy.shape[-1])
+            dx = K.linear_swiglu_dgrad(dy2, self.weight, y)
+            if dx is not None:
+                K.gemm(dy2, h2, trans_a=True, trans_b=False, accumulate=ensure_main_grad(self.weight))
+                return (dx.reshape(dy.shape[:-1] + (y.shape[-1],)),)
+        return super().backward(ctx, dy)
 
     def forward_specs(self) -> List[object]:
         compute = ComputeSpec(self, ("main",), ("main",))

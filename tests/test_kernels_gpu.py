@@ -715,6 +715,33 @@ def test_logits_with_row_statistics(M, N, Kd):
     assert se[0].isnan() and (M == 1 or not se[1:].isnan().any())
 
 
+@pytest.mark.parametrize("M,F,Kd", [(1, 8, 8), (130, 72, 64), (257, 200, 520), (513, 1000, 1032), (128, 128, 64), (300, 328, 72)])
+def test_swiglu_in_gemm_epilogues(M, F, Kd):
+    """Against the two kernels of its own: the same roundings, so errors against 64 bits as large as theirs."""
+    import kareus_b200.kernels as KK
+    from kareus_b200.kernels import ref
+    KC = _K()
+    x, w1 = torch.randn(M, Kd, device="cuda").bfloat16(), (3 * torch.randn(2 * F, Kd, device="cuda") / Kd ** 0.5).bfloat16()
+    dy, w2 = torch.randn(M, Kd, device="cuda").bfloat16(), (torch.randn(Kd, F, device="cuda") / Kd ** 0.5).bfloat16()
+    x[-1] *= 40                                           # activations far out on both sides
+    try:
+        KC.lib().kb_gemm_swiglu_force(1)
+        y, h = KK.linear_swiglu(x, w1)
+        none, h2 = KK.linear_swiglu(x, w1, store=False)
+        dx = KK.linear_swiglu_dgrad(dy, w2, y)
+    finally:
+        KC.lib().kb_gemm_swiglu_force(0)
+    torch.cuda.synchronize()
+    KC.check_status()
+    assert none is None and torch.equal(h, h2)
+    assert _rel(y, KC.gemm(x, w1)) < 2e-3                 # another order of summation moves some bf16 roundings
+    want = ref.swiglu_fwd(y.double())
+    assert _rel(h, want) < 1.01 * _rel(KC.swiglu_fwd(y), want) + 1e-7
+    dh = KC.gemm(dy, w2, trans_b=False)
+    sep, want = KC.swiglu_bwd(dh, y), ref.swiglu_bwd((dy.double() @ w2.double()), y.double())
+    assert _rel(dx, want) < 1.02 * _rel(sep, want) + 1e-7
+
+
 @pytest.mark.parametrize("H", [8, 1032, 3072])
 def test_embedding_backward_vectors(H):
     KC = _K()
