@@ -237,7 +237,8 @@ template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmW, const PairWork w,
-                 const int M, const int N, const int bn, int* status, const __grid_constant__ typename EpiArgs<EPI>::type epi) {
+                 const int M, const int N, const int bn, void* const C, const int ldc, int* status,
+                 const __grid_constant__ typename EpiArgs<EPI>::type epi) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + GP_TILE_BYTES + GP_STG_BYTES);   // used in the leader
@@ -535,7 +536,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         fence_proxy_async_smem();
         __syncwarp();
         const int col = tn * bn + c * SLAB;
-        if (lane == 0 && row0 < M && col < N) {       // the tensor map clips what crosses the edge
+        // A TMA store ends on a 16-byte boundary: the map of a plain output holds whole units, and the columns after the last
+        // one are stored one by one from the staging buffer (what lies behind them may be someone else's).
+        const int whole = ACCUM ? N : N & ~(OUT_F32 ? 3 : 7);
+        if (!ACCUM && whole < N && whole >= col && whole < col + SLAB && row0 + lane < M) {
+          const int unit = (whole - col) / (OUT_F32 ? 4 : 8);
+          const uint8_t* src = stg + lane * 128 + ((unit ^ (lane & 7)) << 4);
+          for (int j = 0; whole + j < N; ++j) {
+            const size_t at = static_cast<size_t>(row0 + lane) * ldc + whole + j;
+            if constexpr (OUT_F32) static_cast<float*>(C)[at] = reinterpret_cast<const float*>(src)[j];
+            else static_cast<__nv_bfloat16*>(C)[at] = reinterpret_cast<const __nv_bfloat16*>(src)[j];
+          }
+        }
+        if (lane == 0 && row0 < M && col < whole) {   // the tensor map clips what crosses the edge
           if (ACCUM && w.slab(u) >= 0) tma_store_2d(&tmW, stg, c * SLAB, w.slab(u) * GP_BM + rank * 128 + q * 32);
           else if constexpr (ACCUM) tma_reduce_add_2d(&tmC, stg, col, row0);
           else tma_store_2d(&tmC, stg, col, row0);
@@ -664,7 +677,7 @@ static int launch_pair(const void* A, const void* B, void* C, int M, int N, int 
   else       rc = make_tmap_2d_bf16(&tmB, B, N, K, ldb, 64, GP_BK);
   if (rc) return rc;
   {
-    const uint64_t dims[2] = {(uint64_t)N, (uint64_t)M};
+    const uint64_t dims[2] = {(uint64_t)(ACCUM ? N : N & ~(OUT_F32 ? 3 : 7)), (uint64_t)M};
     const uint64_t str[1] = {(uint64_t)ldc * (OUT_F32 ? 4 : 2)};
     const uint32_t box[2] = {OUT_F32 ? 32u : 64u, 32u};
     rc = make_tmap(&tmC, C, OUT_F32 ? 4 : 2, 2, dims, str, box, 3);
@@ -702,7 +715,7 @@ static int launch_pair(const void* A, const void* B, void* C, int M, int N, int 
   w.group_m = gm < w.tiles_m ? (int)gm : w.tiles_m;
   const int units = w.whole + w.split_tiles * w.ks;
   const int grid = 2 * (units < pairs ? units : pairs);
-  KB_LAUNCH_PDL(kern, grid, GP_THREADS, GP_SMEM, stream, tmA, tmB, tmC, tmW, w, M, N, pl.bn, status, epi);
+  KB_LAUNCH_PDL(kern, grid, GP_THREADS, GP_SMEM, stream, tmA, tmB, tmC, tmW, w, M, N, pl.bn, C, ldc, status, epi);
   if (ordered) {
     const int blocks = w.split_tiles * (GP_BM * pl.bn / 4 / 256);
     KB_LAUNCH_PDL(gemm_add_parts_kernel, blocks, 256, 0, stream, static_cast<float*>(C), ldc, M, N, (const float*)work, w, pl.bn);

@@ -607,7 +607,7 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
   if (accumulate && !out_f32) return ST_BAD_ARG;
   // The two-SM kernel stores through TMA: 16-byte aligned output rows.
   int single = g_force_single;
-  if (plain && aligned_rows(C, ldc, out_f32) && num_sms >= 2 && !single) {
+  if (plain && aligned_rows(C, ldc, out_f32) && N >= 8 && num_sms >= 2 && !single) {
     const int pairs = num_sms / 2;
     const PairPlan pl = accumulate ? plan_accumulate(M, N, K, num_sms, work != nullptr)
                                    : plan_pair(M, N, K, pairs, b_mn != 0);

@@ -688,6 +688,17 @@ def test_cross_entropy_vector_groups(rows, V):
     assert _rel(logits, want) < 4e-3
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,Kd", [(300, 1093, 64), (5000, 1093, 1040), (300, 9, 136), (129, 65, 64), (300, 3, 64), (257, 1030, 520)])
+def test_gemm_leaves_the_columns_behind_its_output_alone(M, N, Kd, dtype):
+    KC = _K()
+    a, b = torch.randn(M, Kd, device="cuda").bfloat16(), torch.randn(N, Kd, device="cuda").bfloat16()
+    wide = torch.full((M, (N + 7) // 8 * 8 + 8), 7.0, device="cuda", dtype=dtype)
+    KC.gemm(a, b, out=wide[:, :N])
+    assert bool((wide[:, N:] == 7.0).all())
+    assert _rel(wide[:, :N], a.double() @ b.double().t()) < (2e-3 if dtype == torch.bfloat16 else 1e-5)
+
+
 @pytest.mark.parametrize("M,N,Kd", [(1, 8, 64), (130, 1000, 72), (300, 2048, 520), (257, 16392, 128), (513, 4104, 1032), (128, 64, 8)])
 def test_logits_with_row_statistics(M, N, Kd):
     """Statistics from the epilogue of the product against those of the product, with and without storing it."""
