@@ -14,7 +14,7 @@
 //               (bf16 / fp32 output) or TMA reduce-add (fp32 `C +=`: the addition happens in L2, so
 //               nobody waits for the old value)
 //
-// K parts of a tile (`C +=` only).  Ordered: the first part adds to C, the others store their sums to a workspace, which a
+// K parts of a tile.  A bf16 output sums them from a workspace in a second small kernel, in order (EPI_PARTS).  `C +=`, ordered: the first part adds to C, the others store their sums to a workspace, which a
 // second small kernel adds part by part, so that every run gives the same bits.  Not ordered: all parts add in L2 as they
 // come; this is for outputs of few tiles, where the second launch would cost a third of the time (see gemm_sm100.cu).
 //
@@ -92,6 +92,7 @@ enum PairEpilogue : int {
   EPI_ROW_STATS = 1,    // maximum and sum of exponentials of the row pieces that it stores (see RowStats)
   EPI_SWIGLU = 2,       // silu(gate) * up of a [gate | up] product (see SwigluOut)
   EPI_SWIGLU_BWD = 3,   // from the gradient of silu(gate) * up, which is the product, that of [gate | up]
+  EPI_PARTS = 4,        // the tiles after the last full wave are split in K: their parts go to a workspace as fp32 sums
 };
 
 // Row statistics of the bf16 product for a softmax over its columns.  A thread of the epilogue has a row of its tile in
@@ -448,6 +449,27 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!mbar_wait_warp(&tfull[buf], (tile_i >> 1) & 1u, abort_flag, status, ST_TIMEOUT_TMEM_FULL)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + buf * 256 + (static_cast<uint32_t>(q * 32) << 16);
+      if constexpr (EPI == EPI_PARTS) {
+        if (u >= w.whole) {                           // a K part: 32-column slabs of the workspace
+#pragma unroll 1
+          for (int c = h; c < bn / 32; c += 2) {
+            uint32_t v[32];
+            tmem_ld_32x32(taddr + c * 32, v);
+            tmem_ld_wait();
+            if (c + 2 >= bn / 32) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster(cluster_addr(&tempty[buf], 0));
+            }
+            put_slab(v, stg_row, lane);
+            if (lane == 0) {
+              tma_store_2d(&tmW, stg, c * 32, (u - w.whole) * GP_BM + rank * 128 + q * 32);
+              tma_store_commit();
+            }
+          }
+          continue;
+        }
+      }
       if constexpr (EPI == EPI_SWIGLU) {
         // this warp's 64 features: gate at column 64 h of the accumulator, up at 128 + 64 h
         uint32_t g[32], u[32];
@@ -664,6 +686,40 @@ gemm_add_parts_kernel(float* __restrict__ C, int ldc, int M, int N, const float*
   }
 }
 
+// C (bf16) = the sum of the K parts of the split tiles, in order: eight columns a thread.
+__global__ void __launch_bounds__(256)
+gemm_sum_parts_kernel(__nv_bfloat16* __restrict__ C, int ldc, int M, int N, const float* __restrict__ work, const PairWork w, int bn) {
+  pdl_begin();
+  const int vecs = bn >> 3, per_tile = GP_BM * vecs, total = w.split_tiles * per_tile;
+  const size_t part = static_cast<size_t>(w.split_tiles) * GP_BM * bn;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int tile = i / per_tile, rest = i - tile * per_tile, r = rest / vecs, c = (rest - r * vecs) * 8;
+    int tm, tn;
+    w.coords(w.whole + tile, tm, tn);
+    const int row = tm * GP_BM + r, col = tn * bn + c;
+    if (row >= M || col >= N) continue;
+    const float4* src = reinterpret_cast<const float4*>(work + (static_cast<size_t>(tile) * GP_BM + r) * bn + c);
+    float4 a = src[0], b = src[1];
+#pragma unroll 4
+    for (int p = 1; p < w.ks; ++p) {
+      src += part / 4;
+      const float4 x = src[0], y = src[1];
+      a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+      b.x += y.x; b.y += y.y; b.z += y.z; b.w += y.w;
+    }
+    const uint4 o = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
+    __nv_bfloat16* dst = C + static_cast<size_t>(row) * ldc + col;
+    if (col + 8 <= N) {
+      *reinterpret_cast<uint4*>(dst) = o;
+    } else {
+      const uint32_t v[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (col + j < N) dst[j] = __ushort_as_bfloat16(static_cast<unsigned short>(v[j >> 1] >> (j & 1 ? 16 : 0)));
+    }
+  }
+}
+
 template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int EPI = EPI_NONE>
 static int launch_pair(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                        const PairPlan& pl, int pairs, float* work, int* status, cudaStream_t stream,
@@ -683,10 +739,10 @@ static int launch_pair(const void* A, const void* B, void* C, int M, int N, int 
     rc = make_tmap(&tmC, C, OUT_F32 ? 4 : 2, 2, dims, str, box, 3);
     if (rc) return rc;
   }
-  const bool split = ACCUM && pl.ks > 1 && pl.split_tiles > 0, ordered = split && pl.ordered;
+  const bool split = (ACCUM || EPI == EPI_PARTS) && pl.ks > 1 && pl.split_tiles > 0, ordered = split && pl.ordered;
   tmW = tmC;
   if (ordered) {
-    const uint64_t dims[2] = {(uint64_t)pl.bn, (uint64_t)pl.split_tiles * (pl.ks - 1) * GP_BM};
+    const uint64_t dims[2] = {(uint64_t)pl.bn, (uint64_t)pl.split_tiles * (EPI == EPI_PARTS ? pl.ks : pl.ks - 1) * GP_BM};
     const uint64_t str[1] = {(uint64_t)pl.bn * 4};
     const uint32_t box[2] = {32u, 32u};
     rc = make_tmap(&tmW, work, 4, 2, dims, str, box, 3);
@@ -716,7 +772,11 @@ static int launch_pair(const void* A, const void* B, void* C, int M, int N, int 
   const int units = w.whole + w.split_tiles * w.ks;
   const int grid = 2 * (units < pairs ? units : pairs);
   KB_LAUNCH_PDL(kern, grid, GP_THREADS, GP_SMEM, stream, tmA, tmB, tmC, tmW, w, M, N, pl.bn, C, ldc, status, epi);
-  if (ordered) {
+  if constexpr (EPI == EPI_PARTS) {
+    const int blocks = w.split_tiles * (GP_BM * pl.bn / 8 / 256);
+    KB_LAUNCH_PDL(gemm_sum_parts_kernel, blocks, 256, 0, stream, static_cast<__nv_bfloat16*>(C), ldc, M, N, (const float*)work, w,
+                  pl.bn);
+  } else if (ordered) {
     const int blocks = w.split_tiles * (GP_BM * pl.bn / 4 / 256);
     KB_LAUNCH_PDL(gemm_add_parts_kernel, blocks, 256, 0, stream, static_cast<float*>(C), ldc, M, N, (const float*)work, w, pl.bn);
   }
@@ -731,6 +791,8 @@ int gemm_pair_dispatch(const void* A, const void* B, void* C, int M, int N, int 
   do {                                                                                                         \
     if (out_f32 && accumulate) return launch_pair<AM, BM_, true, true>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, work, status, stream);\
     if (out_f32) return launch_pair<AM, BM_, true, false>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, work, status, stream);             \
+    if (pl.ks > 1 && pl.split_tiles > 0)                                                                                                 \
+      return launch_pair<AM, BM_, false, false, EPI_PARTS>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, work, status, stream);            \
     return launch_pair<AM, BM_, false, false>(A, B, C, M, N, K, lda, ldb, ldc, pl, pairs, work, status, stream);                         \
   } while (0)
   if (!a_mn && !b_mn) GP_GO(false, false);

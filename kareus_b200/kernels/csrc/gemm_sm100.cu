@@ -497,6 +497,42 @@ static int single_width(int M, int N, int K, bool b_mn, int num_sms, int pair_bn
 }
 
 static bool g_force_swiglu = false;
+static int g_force_parts = 0, g_force_parts_bn = 0;   // measurement and test aid, see kb_gemm_parts_force
+// Plan of a bf16 output with a workspace: the tiles after the last full wave in K parts that a second kernel adds in order, where
+// the model says that this is faster than the best unsplit plan.  Two kinds of shapes gain: long sums over few tiles (203 x 504 x
+// 15384 85 → 24 us, 128 x 1024 x 8192 28 → 18) and long sums whose last wave is short (3800 x 2048 x 12288 154 → 136; the
+// 4096 x 3072 input gradient of a 128256-word vocabulary 2233 → 2062).  Us per step, wave and MB of partial sums (written once, read
+// once) fitted to 3400 calls of 160 shapes (64..20000 rows, 1024..96000 deep; rms 8 to 13 %); the unsplit times of the table above
+// are 10 % too short there.  Over those shapes the picks take 0.82 of the unsplit time, the best ones 0.79, the worst 1.04 of it.
+static PairPlan plan_parts(int M, int N, int K, bool b_mn, int num_sms) {
+  static const double cost[2][5][3] = {{{}, {0.187, 1.39, 0.11}, {0.22, 2.6, 0.05}, {0.288, 2.1, 0.14}, {0.361, 2.06, 0.164}},
+                                       {{}, {0.222, 0.0, 0.45}, {0.227, 0.44, 0.32}, {0.31, 1.16, 0.28}, {0.344, 1.6, 0.21}}};
+  const int nk = (K + GEMM_BK - 1) / GEMM_BK, pairs = num_sms / 2;
+  PairPlan best = plan_pair(M, N, K, pairs, b_mn);
+  const PlainTimes t = plain_times(M, N, K, b_mn, num_sms, best.bn);
+  const double plain = t.pair < t.w128 ? (t.pair < t.w256 ? t.pair : t.w256) : (t.w128 < t.w256 ? t.w128 : t.w256);
+  double best_us = 0.95 * 1.1 * plain;
+  if (!split_allowed() || g_force_parts == 1 || g_force_bn || g_force_single) return best;
+  for (int bn = 256; bn >= 64; bn -= 64) {
+    if (g_force_parts_bn && bn != g_force_parts_bn) continue;
+    const double* c = cost[b_mn][bn / 64];
+    const long tiles = (long)((M + 255) / 256) * ((N + bn - 1) / bn), full = tiles / pairs, rest = tiles - full * pairs;
+    for (int ks = 2; rest && ks <= 16 && nk / ks >= 4; ++ks) {
+      const PairPlan plan{bn, ks, (int)rest, 0.0, true};
+      if (g_force_parts > 1 && ks == g_force_parts) return plan;
+      const double mb = plan.bf16_scratch_floats() * 4e-6;
+      if (mb > 64.0) break;
+      const long waves = (rest * ks + pairs - 1) / pairs;
+      const double us = 7.0 + full * (nk * c[0] + c[1]) + waves * ((nk + ks - 1) / ks * c[0] + c[1]) + c[2] * mb;
+      if (us < best_us) {
+        best_us = us;
+        best = plan;
+      }
+    }
+  }
+  return best;
+}
+
 enum SwigluKind : int { SWIGLU_STORE = 0, SWIGLU_BACKWARD = 1, SWIGLU_NO_STORE = 2 };
 // Is the activation in the epilogue faster than the product followed by a kernel of its own (2.5 us, and 6 bytes an element
 // forward, 10 backward, at 5.5 TB/s)?  The epilogue of a 256-column tile takes about 5 us where it stores the product too, 3.5
@@ -595,7 +631,7 @@ extern "C" void kb_gemm_force_width(int bn) {
 namespace kb {
 static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda, int b_mn, int ldb, int ldc,
                     int out_f32, int accumulate, int num_sms, const void* bias, int act, float* work, int* status,
-                    cudaStream_t stream) {
+                    cudaStream_t stream, bool parts = false) {
   if (M <= 0 || N <= 0 || K <= 0) return ST_BAD_ARG;
   if ((bias != nullptr || act != 0) && accumulate) return ST_BAD_ARG;
   if (act < 0 || act > 1) return ST_BAD_ARG;
@@ -610,8 +646,9 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
   if (plain && aligned_rows(C, ldc, out_f32) && N >= 8 && num_sms >= 2 && !single) {
     const int pairs = num_sms / 2;
     const PairPlan pl = accumulate ? plan_accumulate(M, N, K, num_sms, work != nullptr)
+                        : parts    ? plan_parts(M, N, K, b_mn != 0, num_sms)
                                    : plan_pair(M, N, K, pairs, b_mn != 0);
-    if (!out_f32 && N % 8 == 0 && !g_force_bn) single = single_width(M, N, K, b_mn != 0, num_sms, pl.bn);
+    if (!out_f32 && N % 8 == 0 && !g_force_bn && !(parts && pl.ks > 1)) single = single_width(M, N, K, b_mn != 0, num_sms, pl.bn);
     if (!single)
       return gemm_pair_dispatch(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, pl, pairs, work, status,
                                 stream);
@@ -642,6 +679,24 @@ extern "C" int kb_gemm_bias_act_bf16(const void* A, const void* B, void* C, int 
 extern "C" int kb_gemm_accum_bf16(const void* A, const void* B, float* C, int M, int N, int K, int a_mn, int lda, int b_mn,
                                   int ldb, int ldc, int num_sms, float* work, int* status, cudaStream_t stream) {
   return kb::gemm_run(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, 1, 1, num_sms, nullptr, 0, work, status, stream);
+}
+
+// bf16 output with a workspace of kb_gemm_scratch_floats() floats (16-byte aligned; none where that is 0) for the K parts of its
+// last tiles.
+extern "C" long kb_gemm_scratch_floats(int M, int N, int K, int b_mn, int num_sms) {
+  using namespace kb;
+  if (num_sms <= 0) num_sms = device_sm_count();
+  if (M <= 0 || N <= 0 || K <= 0 || num_sms < 2) return 0;
+  return plan_parts(M, N, K, b_mn != 0, num_sms).bf16_scratch_floats();
+}
+extern "C" int kb_gemm_work_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda, int b_mn, int ldb,
+                                 int ldc, int num_sms, float* work, int* status, cudaStream_t stream) {
+  return kb::gemm_run(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, 0, 0, num_sms, nullptr, 0, work, status, stream, work != nullptr);
+}
+// Measurement and test aid: K parts of the last tiles of bf16 outputs (1: none, 0: by the model) and their width (0: any).
+extern "C" void kb_gemm_parts_force(int ks, int bn) {
+  kb::g_force_parts = ks;
+  kb::g_force_parts_bn = bn;
 }
 
 extern "C" int kb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda,

@@ -19,8 +19,9 @@
 #include <cstdlib>
 
 extern "C" {
-int kb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda, int b_mn, int ldb, int ldc,
-                 int out_f32, int accumulate, int num_sms, int* status, cudaStream_t stream);
+int kb_gemm_work_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int lda, int b_mn, int ldb, int ldc,
+                      int num_sms, float* work, int* status, cudaStream_t stream);
+long kb_gemm_scratch_floats(int M, int N, int K, int b_mn, int num_sms);
 int kb_gemm_accum_bf16(const void* A, const void* B, float* C, int M, int N, int K, int a_mn, int lda, int b_mn, int ldb,
                        int ldc, int num_sms, float* work, int* status, cudaStream_t stream);
 long kb_gemm_accum_scratch_floats(int M, int N, int K, int num_sms);
@@ -128,10 +129,15 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   }
   at::Tensor out = at::empty({M, N}, a->options().requires_grad(false));
   void* pc = out.data_ptr();
+  // partial sums of the last tiles' K parts, in rows that TMA can store; nothing is split over fewer than 16 steps of 64
+  const long n = K >= 1024 && N % 8 == 0 ? kb_gemm_scratch_floats(M, N, K, !tb, 0) : 0;
+  at::Tensor work;
+  if (n) work = at::empty({n}, a->options().dtype(at::kFloat).requires_grad(false));
+  float* pw = n ? work.data_ptr<float>() : nullptr;
   const int rc = without_gil([&] {
-    return kb_gemm_bf16(pa, pb, pc, M, N, K, ta, lda, !tb, ldb, static_cast<int>(N), 0, 0, 0, status, stream);
+    return kb_gemm_work_bf16(pa, pb, pc, M, N, K, ta, lda, !tb, ldb, static_cast<int>(N), 0, pw, status, stream);
   });
-  if (!finish(rc, "gemm", 1)) return nullptr;
+  if (!finish(rc, "gemm", n ? 2 : 1)) return nullptr;
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }

@@ -67,6 +67,7 @@ def _declare(L) -> None:
     P, I, LNG, F, U = c_void_p, c_int, c_long, c_float, c_uint
     sig = {
         "kb_gemm_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P],
+        "kb_gemm_work_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, P, P, P],
         "kb_gemm_accum_bf16": [P, P, P, I, I, I, I, I, I, I, I, I, P, P, P],
         "kb_gemm_row_stats": [P, P, P, I, I, I, I, I, P, LNG, P, P, P, P, P, P, P, P],
         "kb_gemm_swiglu_pays": [I, I, I, I],
@@ -100,6 +101,10 @@ def _declare(L) -> None:
     L.kb_rmsnorm_bwd_scratch_elems.restype = c_long
     L.kb_gemm_row_stats_floats.argtypes = [I, I, I]
     L.kb_gemm_row_stats_floats.restype = c_long
+    L.kb_gemm_scratch_floats.argtypes = [I, I, I, I, I]
+    L.kb_gemm_scratch_floats.restype = c_long
+    L.kb_gemm_parts_force.argtypes = [I, I]
+    L.kb_gemm_parts_force.restype = None
     L.kb_gemm_accum_scratch_floats.argtypes = [I, I, I, I]
     L.kb_gemm_accum_scratch_floats.restype = c_long
     for name, args in _OPTIONAL_SIGS.items():
@@ -423,6 +428,8 @@ def _aligned_rows(t: torch.Tensor) -> torch.Tensor:
     return c
 
 
+SPLIT_MIN_K = 1024      # bf16 outputs are not split over fewer than 16 steps of 64 (csrc/torch/fastcall.cpp has the same line)
+
 ACTIVATIONS = {None: 0, "none": 0, "gelu": 1}
 
 
@@ -497,6 +504,12 @@ def gemm(a, b, trans_a=False, trans_b=True, out_dtype=None, accumulate=None, out
         rc = L.kb_gemm_accum_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, 1 if trans_a else 0, a.stride(0),
                                   0 if trans_b else 1, b.stride(0), c.stride(0), sms, work.data_ptr() if n else 0,
                                   st.data_ptr(), _stream())
+    elif not f32 and K >= SPLIT_MIN_K and c.stride(0) % 8 == 0 and c.data_ptr() % 16 == 0:
+        n = L.kb_gemm_scratch_floats(M, N, K, 0 if trans_b else 1, sms)
+        work = torch.empty(n, dtype=torch.float32, device=a.device) if n else None
+        rc = L.kb_gemm_work_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, 1 if trans_a else 0, a.stride(0),
+                                 0 if trans_b else 1, b.stride(0), c.stride(0), sms, work.data_ptr() if n else 0, st.data_ptr(),
+                                 _stream())
     else:
         n = 0
         rc = L.kb_gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, 1 if trans_a else 0, a.stride(0),

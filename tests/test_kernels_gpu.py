@@ -699,6 +699,38 @@ def test_gemm_leaves_the_columns_behind_its_output_alone(M, N, Kd, dtype):
     assert _rel(wide[:, :N], a.double() @ b.double().t()) < (2e-3 if dtype == torch.bfloat16 else 1e-5)
 
 
+@pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, False)])
+@pytest.mark.parametrize("M,N,Kd,ks,bn", [(1, 8, 1024, 4, 64), (130, 200, 1032, 2, 128), (300, 1000, 1344, 5, 256), (72, 328, 4104, 7, 192),
+                                          (5000, 1096, 1040, 3, 256)])
+def test_bf16_outputs_in_parts_of_k(M, N, Kd, ks, bn, ta, tb):
+    """Rows, columns and steps that fill no tile and no part; whole tiles before split ones in the last shape."""
+    import kareus_b200.kernels as KK
+    KC = _K()
+    a, b = torch.randn(*((Kd, M) if ta else (M, Kd)), device="cuda").bfloat16(), torch.randn(*((N, Kd) if tb else (Kd, N)), device="cuda").bfloat16()
+    if ta and M % 8:
+        a = torch.cat([a, a.new_zeros(Kd, 8 - M % 8)], 1)[:, :M]
+    want = (a.double().t() if ta else a.double()) @ (b.double().t() if tb else b.double())
+    try:
+        KC.lib().kb_gemm_parts_force(1, 0)
+        one = _rel(KK.gemm(a, b, trans_a=ta, trans_b=tb), want)
+        KC.lib().kb_gemm_parts_force(ks, bn)
+        assert KC.lib().kb_gemm_scratch_floats(M, N, Kd, 0 if tb else 1, 0) > 0
+        got = [KK.gemm(a, b, trans_a=ta, trans_b=tb) for _ in range(3)]
+        odd = torch.zeros(M, N + 8, device="cuda", dtype=torch.bfloat16)          # rows of a wider output
+        got.append(KC.gemm(a, b, trans_a=ta, trans_b=tb, out=odd[:, :N]))
+        if tb:                                                                    # a length that is no multiple of a vector
+            got.append(KC.gemm(a, b, out=torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)))
+            KC.gemm(a, b[:N - 3], out=odd[:, :N - 3])
+    finally:
+        KC.lib().kb_gemm_parts_force(0, 0)
+    torch.cuda.synchronize()
+    KC.check_status()
+    assert not odd[:, N:].any() and torch.equal(odd[:, :N], got[0])
+    for g in got:
+        assert torch.equal(g, got[0]) and _rel(g, want) < 1.01 * one
+    assert KC.lib().kb_gemm_scratch_floats(M, N, 64, 0, 0) == 0
+
+
 @pytest.mark.parametrize("M,N,Kd", [(1, 8, 64), (130, 1000, 72), (300, 2048, 520), (257, 16392, 128), (513, 4104, 1032), (128, 64, 8)])
 def test_logits_with_row_statistics(M, N, Kd):
     """Statistics from the epilogue of the product against those of the product, with and without storing it."""
