@@ -497,21 +497,49 @@ static int single_width(int M, int N, int K, bool b_mn, int num_sms, int pair_bn
 }
 
 static bool g_force_swiglu = false;
+// Kernel and width of a plain bf16 output: the width (64..256) of pairs, or negative that (128, 256) of the one-SM kernel; `us`:
+// modelled time.  The table above was fitted to calls of up to about 50 us; longer ones run at lower clocks, and wide tiles,
+// which move fewer bytes for a product, lose less: fitted again to 133 calls of 45 to 700 us (rms 9 to 20 %) the picks take
+// 1.1 % longer than the best kernel and width of each, by the first table 3.6 % (3934 x 14264 x 5640: one-SM 668, pairs of 256
+// columns 521; 11384 x 2072 x 2584: 192 columns 137, 256 columns 120).
+static int plain_choice(int M, int N, int K, bool b_mn, int num_sms, double* us) {
+  static const double long_us[2][6][3] = {   // step, wave, call of 64, 128, 192, 256 columns on pairs, 128 and 256 on one SM
+      {{0.186, 0.6, 11.8}, {0.242, 0.99, 3.4}, {0.309, 1.33, 3.0}, {0.385, 1.62, 1.9}, {0.331, 0.53, 14.0}, {0.471, 1.29, 7.5}},
+      {{0.215, 1.0, 13.6}, {0.232, 1.26, 9.7}, {0.33, 1.61, 8.3}, {0.368, 1.93, 5.6}, {0.339, 0.69, 12.1}, {0.478, 1.66, 9.0}}};
+  const int pairs = num_sms / 2, bn = plan_pair(M, N, K, pairs, b_mn).bn, nk = (K + GEMM_BK - 1) / GEMM_BK;
+  const PlainTimes t = plain_times(M, N, K, b_mn, num_sms, bn);
+  const int one = N % 8 ? 0 : single_width(M, N, K, b_mn, num_sms, bn);
+  *us = one == 128 ? t.w128 : one ? t.w256 : t.pair;
+  if (*us < 50.0 || nk <= 2 || g_force_bn) return one ? -one : bn;
+  int best = 0;
+  for (int i = 0; i < (N % 8 ? 4 : 6); ++i) {
+    const int width = i < 4 ? 64 * (i + 1) : 128 * (i - 3), rows = i < 4 ? 256 : 128, slots = i < 4 ? pairs : num_sms;
+    const long waves = ((long)((M + rows - 1) / rows) * ((N + width - 1) / width) + slots - 1) / slots;
+    const double* c = long_us[b_mn][i];
+    const double x = waves * (nk * c[0] + c[1]) + c[2];
+    if (!best || x < *us) {
+      *us = x;
+      best = i < 4 ? width : -width;
+    }
+  }
+  return best;
+}
+
 static int g_force_parts = 0, g_force_parts_bn = 0;   // measurement and test aid, see kb_gemm_parts_force
 // Plan of a bf16 output with a workspace: the tiles after the last full wave in K parts that a second kernel adds in order, where
 // the model says that this is faster than the best unsplit plan.  Two kinds of shapes gain: long sums over few tiles (203 x 504 x
 // 15384 85 → 24 us, 128 x 1024 x 8192 28 → 18) and long sums whose last wave is short (3800 x 2048 x 12288 154 → 136; the
 // 4096 x 3072 input gradient of a 128256-word vocabulary 2233 → 2062).  Us per step, wave and MB of partial sums (written once, read
-// once) fitted to 3400 calls of 160 shapes (64..20000 rows, 1024..96000 deep; rms 8 to 13 %); the unsplit times of the table above
-// are 10 % too short there.  Over those shapes the picks take 0.82 of the unsplit time, the best ones 0.79, the worst 1.04 of it.
+// once) fitted to 3400 calls of 160 shapes (64..20000 rows, 1024..96000 deep; rms 8 to 13 %); unsplit times below 50 us are
+// 10 % too short there.  Over those shapes the picks take 0.82 of the unsplit time, the best ones 0.79, the worst 1.04 of it.
 static PairPlan plan_parts(int M, int N, int K, bool b_mn, int num_sms) {
   static const double cost[2][5][3] = {{{}, {0.187, 1.39, 0.11}, {0.22, 2.6, 0.05}, {0.288, 2.1, 0.14}, {0.361, 2.06, 0.164}},
                                        {{}, {0.222, 0.0, 0.45}, {0.227, 0.44, 0.32}, {0.31, 1.16, 0.28}, {0.344, 1.6, 0.21}}};
   const int nk = (K + GEMM_BK - 1) / GEMM_BK, pairs = num_sms / 2;
-  PairPlan best = plan_pair(M, N, K, pairs, b_mn);
-  const PlainTimes t = plain_times(M, N, K, b_mn, num_sms, best.bn);
-  const double plain = t.pair < t.w128 ? (t.pair < t.w256 ? t.pair : t.w256) : (t.w128 < t.w256 ? t.w128 : t.w256);
-  double best_us = 0.95 * 1.1 * plain;
+  double plain;
+  const int choice = plain_choice(M, N, K, b_mn, num_sms, &plain);
+  PairPlan best{choice > 0 ? choice : 256, 1, 0, 0.0, false};        // unsplit: the caller picks by plain_choice
+  double best_us = 0.95 * (plain < 50.0 ? 1.1 : 1.0) * plain;
   if (!split_allowed() || g_force_parts == 1 || g_force_bn || g_force_single) return best;
   for (int bn = 256; bn >= 64; bn -= 64) {
     if (g_force_parts_bn && bn != g_force_parts_bn) continue;
@@ -595,8 +623,8 @@ extern "C" void kb_gemm_accum_plan(int M, int N, int K, int num_sms, int* bn, in
 // Tile width that kb_gemm_bf16 uses for a bf16 output of this shape (rows 16-byte aligned): positive on the two-SM kernel,
 // negative on the one-SM kernel.
 extern "C" int kb_gemm_plan(int M, int N, int K, int b_mn, int num_sms) {
-  const int bn = kb::plan_pair(M, N, K, num_sms / 2, b_mn != 0).bn, one = N % 8 ? 0 : kb::single_width(M, N, K, b_mn != 0, num_sms, bn);
-  return one ? -one : bn;
+  double us;
+  return kb::plain_choice(M, N, K, b_mn != 0, num_sms, &us);
 }
 
 // Floats of workspace that kb_gemm_accum_bf16 needs for an output of this shape (0: it splits nothing).
@@ -645,10 +673,15 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
   int single = g_force_single;
   if (plain && aligned_rows(C, ldc, out_f32) && N >= 8 && num_sms >= 2 && !single) {
     const int pairs = num_sms / 2;
-    const PairPlan pl = accumulate ? plan_accumulate(M, N, K, num_sms, work != nullptr)
-                        : parts    ? plan_parts(M, N, K, b_mn != 0, num_sms)
-                                   : plan_pair(M, N, K, pairs, b_mn != 0);
-    if (!out_f32 && N % 8 == 0 && !g_force_bn && !(parts && pl.ks > 1)) single = single_width(M, N, K, b_mn != 0, num_sms, pl.bn);
+    PairPlan pl = accumulate ? plan_accumulate(M, N, K, num_sms, work != nullptr)
+                  : parts    ? plan_parts(M, N, K, b_mn != 0, num_sms)
+                             : plan_pair(M, N, K, pairs, b_mn != 0);
+    if (!out_f32 && !g_force_bn && !(parts && pl.ks > 1)) {
+      double us;
+      const int choice = plain_choice(M, N, K, b_mn != 0, num_sms, &us);
+      if (choice < 0) single = -choice;
+      else pl = PairPlan{choice, 1, 0, us, false};
+    }
     if (!single)
       return gemm_pair_dispatch(A, B, C, M, N, K, a_mn, lda, b_mn, ldb, ldc, out_f32, accumulate, pl, pairs, work, status,
                                 stream);
