@@ -400,6 +400,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           __syncwarp();
           if (c + 2 < slabs) fetch(u, c + 2);
           else if (u + step < num_units) fetch(u + step, h);
+          __syncwarp();                               // rows and columns past the edge are left out lane by lane
           const float2 one = make_float2(1.f, 1.f);
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
@@ -454,6 +455,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll 1
           for (int c = h; c < bn / 32; c += 2) {
             uint32_t v[32];
+            __syncwarp();
             tmem_ld_32x32(taddr + c * 32, v);
             tmem_ld_wait();
             if (c + 2 >= bn / 32) {
@@ -517,6 +519,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll 1
       for (int c = h; c < slabs; c += 2) {
         uint32_t o[32];
+        // TMEM is read by whole warps: what lanes did on their own before (a row's target, the stores of the slab before) ends here
+        __syncwarp();
         if constexpr (OUT_F32) {
           tmem_ld_32x32(taddr + c * 32, o);
           tmem_ld_wait();

@@ -252,6 +252,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
         uint32_t v[32];
+        __syncwarp();                       // rows past the edge store nothing: the warp reads TMEM as a whole again
         tmem_ld_32x32(taddr + c * 32, v);
         tmem_ld_wait();
         const int col = n0 + c * 32;

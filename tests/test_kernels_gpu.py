@@ -758,6 +758,24 @@ def test_logits_with_row_statistics(M, N, Kd):
     assert se[0].isnan() and (M == 1 or not se[1:].isnan().any())
 
 
+@pytest.mark.parametrize("M,N,Kd", [(2003, 16392, 64), (5001, 2056, 136)])
+def test_row_statistics_alone_over_many_tiles(M, N, Kd):
+    """Many tiles for each pair of SMs and no product to store: nothing but the statistics stands between two reads of TMEM, and
+    rows, columns and targets inside and outside of a tile part the lanes of a warp."""
+    import kareus_b200.kernels as KK
+    KC = _K()
+    x, w = torch.randn(M, Kd, device="cuda").bfloat16(), (torch.randn(N, Kd, device="cuda") / Kd ** 0.5).bfloat16()
+    tgt = torch.randint(-N // 2, 2 * N, (M,), device="cuda")
+    logits, m, se, tl, _ = KK.linear_cross_entropy_stats(x, w, tgt, 0)
+    for _ in range(5):
+        none, m2, se2, tl2, _ = KK.linear_cross_entropy_stats(x, w, tgt, 0, store=False)
+        assert none is None and torch.equal(m, m2) and torch.equal(se, se2) and torch.equal(tl, tl2)
+    torch.cuda.synchronize()
+    KC.check_status()
+    mr, _, tr = KC.cross_entropy_local_stats(logits, tgt, 0)
+    assert torch.equal(m, mr) and torch.equal(tl, tr)
+
+
 @pytest.mark.parametrize("M,F,Kd", [(1, 8, 8), (130, 72, 64), (257, 200, 520), (513, 1000, 1032), (128, 128, 64), (300, 328, 72)])
 def test_swiglu_in_gemm_epilogues(M, F, Kd):
     """Against the two kernels of its own: the same roundings, so errors against 64 bits as large as theirs."""
