@@ -16,7 +16,7 @@ import torch
 class OpContext:
     """State an operator keeps between its forward and backward."""
 
-    __slots__ = ("saved_tensors", "requires_grad", "needs_input_grad", "extra", "nb_index")
+    __slots__ = ("saved_tensors", "requires_grad", "needs_input_grad", "extra", "nb_index", "chained")
 
     def __init__(self, nb_index: int = 0):
         self.saved_tensors: Tuple[Optional[torch.Tensor], ...] = ()
@@ -24,6 +24,7 @@ class OpContext:
         self.needs_input_grad: Tuple[bool, ...] = ()
         self.extra: Dict[str, Any] = {}
         self.nb_index = nb_index
+        self.chained = False       # the operator runs in a graph that has its whole fusion chain in a row (see graph.py)
 
     def save_for_backward(self, *tensors: Optional[torch.Tensor]) -> None:
         self.saved_tensors = tuple(tensors)

@@ -69,6 +69,7 @@ class Node:
     backward: bool = False
     segment: str = ""      # context-parallel plan vocabulary: segment name (qkv, ao, a, o, mlp) ...
     short: str = ""        # ... and collective type (ar, ag, rs)
+    chained: bool = False  # member of a fusion chain that is complete in this graph
 
     @property
     def name(self) -> str:
@@ -200,6 +201,27 @@ class TensorGraphBuilder:
         return g
 
 
+# Operators that may compute a neighbour's result in their own kernel, by the role that their class itself declares: a subclass
+# that computes something else does not inherit it.  Such an operator asks its context (`chained`) whether the others are there.
+FUSION_CHAINS = (("gate_up_linear", "swiglu", "down_linear"),)
+
+
+def _fusion_roles(op) -> Tuple[str, ...]:
+    return type(op).__dict__.get("fusion_roles", ())
+
+
+def mark_fusion_chains(nodes: Sequence[Node]) -> None:
+    """Mark the compute nodes of every chain whose members follow one another, each reading what the one before it wrote and
+    nothing else.  Another operator or a collective between them (a bias, a gather) keeps them apart."""
+    for chain in FUSION_CHAINS:
+        for i in range(len(nodes) - len(chain) + 1):
+            run = nodes[i:i + len(chain)]
+            if (all(not n.is_comm and role in _fusion_roles(n.operator) for n, role in zip(run, chain))
+                    and all(a.outputs == b.inputs and len(a.outputs) == 1 for a, b in zip(run, run[1:]))):
+                for n in run:
+                    n.chained = True
+
+
 def build_graphs(operators: Sequence[GraphOperator],
                  forward_inputs: Dict[str, str], backward_inputs: Dict[str, str]
                  ) -> Tuple[TensorGraph, TensorGraph]:
@@ -214,6 +236,7 @@ def build_graphs(operators: Sequence[GraphOperator],
     for op in operators:
         for spec in op.forward_specs():
             fb.add(spec)
+    mark_fusion_chains(fb._nodes)
     bb = TensorGraphBuilder()
     bb.add_initial_channels(backward_inputs)
     for op in reversed(list(operators)):

@@ -321,6 +321,7 @@ class PartitionProgram:
         if not self.backward:
             ctx = nbctx.ctx_for(node.op_id)
             ctx.requires_grad = grad_enabled
+            ctx.chained = node.chained
             outs = op.forward(ctx, *ins)
         else:
             ctx = nbctx.ctx_for(node.op_id, create=False)

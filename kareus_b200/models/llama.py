@@ -75,9 +75,6 @@ class TransformerLayer(nn.Module):
                 and dtype == torch.bfloat16 and torch.device(device or "cpu").type == "cuda":
             from ..ops.fused import attach_fused
             attach_fused(self, comm.heap)
-        else:
-            self.fc1.fuse_swiglu = self.fc2.fuse_swiglu = True
-            self.act.fused_features = f
 
     def operators(self):
         return [self.attn_fork, self.input_norm, self.qkv, self.qkv_post, self.rope, self.core_attn,

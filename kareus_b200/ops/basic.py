@@ -93,16 +93,17 @@ class SwiGLUOp(GraphOperator):
     """``silu(gate) * up`` on a ``[gate | up]`` packed last dim (reference ``bias_swiglu.py:18-19``)."""
 
     group = "activation"
+    fusion_roles = ("swiglu",)
 
     def __init__(self, name: str = "swiglu"):
         self.name = name
-        self.fused_features = 0             # width of an activation that the linear layer before it has computed already
 
     def forward(self, ctx, x):
-        shp = x.shape
-        if shp[-1] == self.fused_features:
-            ctx.save_for_backward()
+        if ctx.chained and hasattr(x, "swiglu_input"):      # the linear layer before it has computed the activation
+            if ctx.requires_grad:
+                ctx.save_for_backward(x.swiglu_input)
             return (x,)
+        shp = x.shape
         x2 = x.reshape(-1, shp[-1])
         y = K.swiglu_fwd(x2)
         if ctx.requires_grad:
@@ -110,9 +111,9 @@ class SwiGLUOp(GraphOperator):
         return (y.reshape(shp[:-1] + (shp[-1] // 2,)),)
 
     def backward(self, ctx, dy):
-        if not ctx.saved_tensors:
-            return (dy,)
         (x2,) = ctx.saved_tensors
+        if ctx.chained and dy.shape[-1] == x2.shape[-1]:    # the linear layer behind it has gone through the activation
+            return (dy,)
         dx = K.swiglu_bwd(dy.reshape(-1, dy.shape[-1]), x2)
         return (dx.reshape(dy.shape[:-1] + (x2.shape[-1],)),)
 

@@ -56,11 +56,6 @@ class _LinearBase(nn.Module, GraphOperator):
     def _bwd_staging(self, shape, dtype, nb, device):
         return None
 
-    # The SwiGLU between fc1 and fc2 can run in the epilogues of the GEMMs beside it: fc1 then returns the activation, which
-    # :class:`SwiGLUOp` passes on, and fc2 returns the gradient of fc1's output.  Shapes say which of the two a tensor is.
-    # `_swiglu_in` on the activation is fc1's output (kept where there will be a backward pass).
-    fuse_swiglu = False                     # set on fc1 and fc2 of a layer whose activation it is
-
     def forward(self, ctx, x):
         shp = x.shape
         x2 = x.reshape(-1, shp[-1])
@@ -83,6 +78,8 @@ class _LinearBase(nn.Module, GraphOperator):
 class ColumnParallelLinear(_LinearBase):
     """Output features sharded over TP (QKV, FC1)."""
 
+    fusion_roles = ("gate_up_linear",)
+
     tp_shard_axis = 0
 
     def __init__(self, *a, **kw):
@@ -101,25 +98,20 @@ class ColumnParallelLinear(_LinearBase):
         return op.staging(shape, dtype, nb, device)
 
     def forward(self, ctx, x):
-        if not self.fuse_swiglu:
-            return super().forward(ctx, x)
-        shp = x.shape
-        x2 = x.reshape(-1, shp[-1])
-        r = K.linear_swiglu(x2, self.weight, store=ctx.requires_grad)
-        if r is None:
-            return super().forward(ctx, x)
-        y, h = r
-        h = h.reshape(shp[:-1] + (self.out_features // 2,))
-        if ctx.requires_grad:
-            ctx.save_for_backward(x2, y)
-            h._swiglu_in = y
-        return (h,)
-
-    def backward(self, ctx, dy):
-        if len(ctx.saved_tensors) == 2 and dy.shape[-1] != self.out_features:      # gradient of the activation
-            y = ctx.saved_tensors[1]
-            dy = K.swiglu_bwd(dy.reshape(-1, dy.shape[-1]), y).reshape(dy.shape[:-1] + (self.out_features,))
-        return super().backward(ctx, dy)
+        """Where the SwiGLU and the layer that reads its result come next (``ctx.chained``), the product may leave as the
+        activation, computed in the GEMM's epilogue.  Such a tensor says so: ``swiglu_input`` on it is the product, for
+        the backward passes of the two (``None`` without one)."""
+        if ctx.chained:
+            shp = x.shape
+            x2 = x.reshape(-1, shp[-1])
+            r = K.linear_swiglu(x2, self.weight, store=ctx.requires_grad)
+            if r is not None:
+                if ctx.requires_grad:
+                    ctx.save_for_backward(x2)
+                h = r[1].reshape(shp[:-1] + (self.out_features // 2,))
+                h.swiglu_input = r[0]
+                return (h,)
+        return super().forward(ctx, x)
 
     def forward_specs(self) -> List[object]:
         compute = ComputeSpec(self, ("main",), ("main",))
@@ -148,6 +140,8 @@ class ColumnParallelLinear(_LinearBase):
 class RowParallelLinear(_LinearBase):
     """Input features sharded over TP (attention out-proj, FC2); output is a partial sum."""
 
+    fusion_roles = ("down_linear",)
+
     tp_shard_axis = 1
 
     def __init__(self, *a, **kw):
@@ -167,12 +161,12 @@ class RowParallelLinear(_LinearBase):
 
     def forward(self, ctx, x):
         out = super().forward(ctx, x)
-        y = getattr(x, "_swiglu_in", None) if self.fuse_swiglu else None
-        if y is not None and ctx.requires_grad:
-            ctx.save_for_backward(*ctx.saved_tensors, y)
+        if ctx.chained and ctx.requires_grad and hasattr(x, "swiglu_input"):
+            ctx.save_for_backward(*ctx.saved_tensors, x.swiglu_input)
         return out
 
     def backward(self, ctx, dy):
+        """Behind an activation from an epilogue its gradient may leave as that of the product before it."""
         if len(ctx.saved_tensors) == 2:
             h2, y = ctx.saved_tensors
             dy2 = dy.reshape(-1, dy.shape[-1])

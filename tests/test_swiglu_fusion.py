@@ -1,0 +1,130 @@
+"""fc1, SwiGLU and fc2 of a layer as one fusion chain: the activation in the epilogues of the GEMMs beside it gives what the three
+operators give, in a chain that is whole, and only there."""
+import pytest
+import torch
+
+import kareus_b200.kernels as K
+from kareus_b200.config import ParallelConfig, get_model_config
+from kareus_b200.engine.block import BlockEngine
+from kareus_b200.engine.context import OpContext
+from kareus_b200.engine.graph import GraphOperator
+from kareus_b200.kernels import ref
+from kareus_b200.models.llama import GPTModel, TransformerLayer
+from kareus_b200.ops.basic import SwiGLUOp
+from kareus_b200.ops.extras import BiasOp
+from kareus_b200.parallel.collectives import CommFactory
+
+
+@pytest.fixture
+def stand_in(monkeypatch):
+    """Fused calls on the CPU, stated in PyTorch; returns how often each was taken."""
+    taken = {"forward": 0, "saving": 0, "backward": 0}
+
+    def install(forward=True, backward=True):
+        def fwd(x, w, store=True):
+            if not forward:
+                return None
+            taken["forward"] += 1
+            taken["saving"] += store
+            y = ref.gemm(x, w, False, True, None, None)
+            return (y if store else None), ref.swiglu_fwd(y)
+
+        def bwd(dy, w, x):
+            if not backward:
+                return None
+            taken["backward"] += 1
+            return ref.swiglu_bwd(ref.gemm(dy, w, False, False, None, None), x)
+        monkeypatch.setattr(K, "linear_swiglu", fwd)
+        monkeypatch.setattr(K, "linear_swiglu_dgrad", bwd)
+        return taken
+    return install
+
+
+def _grads(model, batch):
+    model(*batch).backward()
+    return [p.main_grad.clone() for p in model.parameters()]
+
+
+@pytest.mark.parametrize("recompute", [False, True])
+@pytest.mark.parametrize("backward", [False, True])
+def test_whole_chains_fuse(stand_in, recompute, backward):
+    cfg = get_model_config("tiny")
+    g = torch.Generator().manual_seed(0)
+    tokens, labels = (torch.randint(0, cfg.vocab_size, (4, 32), generator=g) for _ in range(2))
+    batch = tokens, labels, torch.ones(4, 32)
+    par = ParallelConfig(num_nanobatches=2, recompute=recompute)
+    want = _grads(GPTModel(cfg, par, dtype="fp64"), batch)
+    taken = stand_in(backward=backward)
+    got = _grads(GPTModel(cfg, par, dtype="fp64"), batch)
+    calls = 2 * cfg.num_layers
+    assert taken == {"forward": calls * (2 if recompute else 1), "saving": calls, "backward": calls if backward else 0}
+    for a, b in zip(got, want, strict=True):
+        torch.testing.assert_close(a, b, rtol=1e-12, atol=1e-15)
+    with torch.no_grad():
+        n = taken["saving"]
+        GPTModel(cfg, par, dtype="fp64")(*batch)
+        assert taken["saving"] == n                       # nothing is kept for a backward pass that does not come
+
+
+class _Doubled(SwiGLUOp):
+    """Another activation in the place of the layer's own."""
+
+    def forward(self, ctx, x):
+        (y,) = super().forward(ctx, x)
+        return (2 * y,)
+
+    def backward(self, ctx, dy):
+        return super().backward(ctx, 2 * dy)
+
+
+class _Square(GraphOperator):
+    group = "activation"
+    name = "square"
+
+    def forward(self, ctx, x):
+        ctx.save_for_backward(x)
+        return (x[..., :x.shape[-1] // 2] * x[..., x.shape[-1] // 2:],)
+
+    def backward(self, ctx, dy):
+        a, b = ctx.saved_tensors[0].chunk(2, -1)
+        return (torch.cat([dy * b, dy * a], -1),)
+
+
+@pytest.mark.parametrize("form", ["bias", "subclass", "replaced"])
+def test_anything_else_in_the_chain_gets_the_product(stand_in, form):
+    cfg = get_model_config("tiny")
+
+    def run():
+        layer = TransformerLayer(cfg, ParallelConfig(), CommFactory(), 0, torch.float64, "cpu", seed=3)
+        ops = layer.operators()
+        i = ops.index(layer.fc1)
+        if form == "bias":
+            b = BiasOp(2 * cfg.ffn_hidden_size, dtype=torch.float64)
+            b.bias.data.normal_(generator=torch.Generator().manual_seed(4))
+            ops.insert(i + 1, b)
+        else:
+            ops[i + 1] = _Doubled() if form == "subclass" else _Square()
+        engine = BlockEngine([ops], 1, recompute=False)
+        x = torch.randn(16, 2, cfg.hidden_size, dtype=torch.float64, generator=torch.Generator().manual_seed(5)).requires_grad_()
+        (y,) = engine([x], ref.rope_table(16, cfg.hd, cfg.rope_theta, device="cpu"))
+        y.square().sum().backward()
+        return [y.detach(), x.grad, layer.fc1.weight.main_grad, layer.fc2.weight.main_grad]
+
+    want = run()
+    taken = stand_in()
+    for a, b in zip(run(), want, strict=True):
+        torch.testing.assert_close(a, b, rtol=1e-12, atol=1e-15)
+    assert taken["forward"] == taken["backward"] == 0
+
+
+def test_an_operator_alone_returns_its_product(stand_in):
+    cfg = get_model_config("tiny")
+    stand_in()
+    layer = TransformerLayer(cfg, ParallelConfig(), CommFactory(), 0, torch.float64, "cpu", seed=3)
+    x = torch.randn(8, cfg.hidden_size, dtype=torch.float64)
+    (y,) = layer.fc1.forward(OpContext(), x)
+    torch.testing.assert_close(y, x @ layer.fc1.weight.t())
+    (h,) = layer.act.forward(OpContext(), y)
+    torch.testing.assert_close(h, ref.swiglu_fwd(y))
+    narrow = layer.act.forward(OpContext(), h)[0]          # a [gate | up] input of any width is one
+    torch.testing.assert_close(narrow, ref.swiglu_fwd(h))
