@@ -351,7 +351,7 @@ def linear_swiglu(x, w, store):
             and x.shape[1] == w.shape[1] and _rowmajor_ok(x) and _rowmajor_ok(w)):
         return None
     (M, Kd), F, L = x.shape, w.shape[0] // 2, lib()
-    if not L.kb_gemm_swiglu_pays(M, F, Kd, 0 if store else 2):
+    if not L.kb_gemm_swiglu_pays(M, F, Kd, 0):
         return None
     y = torch.empty(M, 2 * F, dtype=x.dtype, device=x.device) if store else None
     h = torch.empty(M, F, dtype=x.dtype, device=x.device)

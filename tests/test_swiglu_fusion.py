@@ -128,3 +128,34 @@ def test_an_operator_alone_returns_its_product(stand_in):
     torch.testing.assert_close(h, ref.swiglu_fwd(y))
     narrow = layer.act.forward(OpContext(), h)[0]          # a [gate | up] input of any width is one
     torch.testing.assert_close(narrow, ref.swiglu_fwd(h))
+
+
+# ----------------------------------------------------------------------------- the rule and its callers
+def _library():
+    import ctypes
+    from kareus_b200.kernels import build
+    if not build.LIB.exists():
+        pytest.skip("native library not built")
+    return ctypes.CDLL(str(build.LIB))
+
+
+def test_passes_with_and_without_a_product_take_the_same_kernels(monkeypatch):
+    """A recomputing step runs a layer once without keeping fc1's product and once with it: the second activation has to be the first."""
+    from kareus_b200.kernels import cuda as KC
+    real = _library()
+
+    class Lib:
+        kb_gemm_swiglu_pays = staticmethod(real.kb_gemm_swiglu_pays)
+        kb_gemm_swiglu = staticmethod(lambda *a: 0)
+    monkeypatch.setattr(KC, "lib", lambda: Lib)
+    monkeypatch.setattr(KC, "_stream", lambda: 0)
+    monkeypatch.setattr(KC, "status_word", lambda dev: torch.zeros(1, dtype=torch.int32))
+    answers = set()
+    for h, f in [(512, 1024), (2048, 3072), (3072, 4096), (3072, 8192)]:
+        w = torch.empty(2 * f, h, dtype=torch.bfloat16)
+        for tokens in list(range(64, 1024, 32)) + [1728, 2016, 2560, 4096]:
+            x = torch.empty(tokens, h, dtype=torch.bfloat16)
+            with_, without = (KC.linear_swiglu(x, w, store) is None for store in (True, False))
+            assert with_ == without, (tokens, h, f)
+            answers.add(with_)
+    assert answers == {True, False}
