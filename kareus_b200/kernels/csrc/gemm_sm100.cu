@@ -497,16 +497,16 @@ static int single_width(int M, int N, int K, bool b_mn, int num_sms, int pair_bn
   return t.w128 < t.w256 ? 128 : 256;
 }
 
-static bool g_force_swiglu = false;
+static int g_force_swiglu = 0;      // measurement and test aid, see kb_gemm_swiglu_force
+static const double long_us[2][6][3] = {   // step, wave, call of 64, 128, 192, 256 columns on pairs, 128 and 256 on one SM
+    {{0.186, 0.6, 11.8}, {0.242, 0.99, 3.4}, {0.309, 1.33, 3.0}, {0.385, 1.62, 1.9}, {0.331, 0.53, 14.0}, {0.471, 1.29, 7.5}},
+    {{0.215, 1.0, 13.6}, {0.232, 1.26, 9.7}, {0.33, 1.61, 8.3}, {0.368, 1.93, 5.6}, {0.339, 0.69, 12.1}, {0.478, 1.66, 9.0}}};
 // Kernel and width of a plain bf16 output: the width (64..256) of pairs, or negative that (128, 256) of the one-SM kernel; `us`:
 // modelled time.  The table above was fitted to calls of up to about 50 us; longer ones run at lower clocks, and wide tiles,
 // which move fewer bytes for a product, lose less: fitted again to 133 calls of 45 to 700 us (rms 9 to 20 %) the picks take
 // 1.1 % longer than the best kernel and width of each, by the first table 3.6 % (3934 x 14264 x 5640: one-SM 668, pairs of 256
 // columns 521; 11384 x 2072 x 2584: 192 columns 137, 256 columns 120).
 static int plain_choice(int M, int N, int K, bool b_mn, int num_sms, double* us) {
-  static const double long_us[2][6][3] = {   // step, wave, call of 64, 128, 192, 256 columns on pairs, 128 and 256 on one SM
-      {{0.186, 0.6, 11.8}, {0.242, 0.99, 3.4}, {0.309, 1.33, 3.0}, {0.385, 1.62, 1.9}, {0.331, 0.53, 14.0}, {0.471, 1.29, 7.5}},
-      {{0.215, 1.0, 13.6}, {0.232, 1.26, 9.7}, {0.33, 1.61, 8.3}, {0.368, 1.93, 5.6}, {0.339, 0.69, 12.1}, {0.478, 1.66, 9.0}}};
   const int pairs = num_sms / 2, bn = plan_pair(M, N, K, pairs, b_mn).bn, nk = (K + GEMM_BK - 1) / GEMM_BK;
   const PlainTimes t = plain_times(M, N, K, b_mn, num_sms, bn);
   const int one = N % 8 ? 0 : single_width(M, N, K, b_mn, num_sms, bn);
@@ -539,9 +539,10 @@ static PairPlan plan_parts(int M, int N, int K, bool b_mn, int num_sms) {
   const int nk = (K + GEMM_BK - 1) / GEMM_BK, pairs = num_sms / 2;
   double plain;
   const int choice = plain_choice(M, N, K, b_mn, num_sms, &plain);
-  PairPlan best{choice > 0 ? choice : 256, 1, 0, 0.0, false};        // unsplit: the caller picks by plain_choice
-  double best_us = 0.95 * (plain < 50.0 ? 1.1 : 1.0) * plain;
-  if (!split_allowed() || g_force_parts == 1 || g_force_bn || g_force_single) return best;
+  PairPlan best{choice > 0 ? choice : 256, 1, 0, (plain < 50.0 ? 1.1 : 1.0) * plain, false};        // unsplit: the caller picks by plain_choice
+  double best_us = 0.95 * best.cost;
+  // callers without room for 16 steps of 64 do not ask for a workspace
+  if (K < 1024 || !split_allowed() || g_force_parts == 1 || g_force_bn || g_force_single) return best;
   for (int bn = 256; bn >= 64; bn -= 64) {
     if (g_force_parts_bn && bn != g_force_parts_bn) continue;
     const double* c = cost[b_mn][bn / 64];
@@ -556,34 +557,35 @@ static PairPlan plan_parts(int M, int N, int K, bool b_mn, int num_sms) {
       if (us < best_us) {
         best_us = us;
         best = plan;
+        best.cost = us;
       }
     }
   }
   return best;
 }
 
-enum SwigluKind : int { SWIGLU_STORE = 0, SWIGLU_BACKWARD = 1, SWIGLU_NO_STORE = 2 };
-// Is the activation in the epilogue faster than the product followed by a kernel of its own (2.5 us, and 6 bytes an element
-// forward, 10 backward, at 5.5 TB/s)?  The epilogue of a 256-column tile takes about 5 us where it stores the product too, 3.5
-// where it does not, and 12 to 14.5 backward (memory latency; it has eight warps); it runs under the main loop of the next
-// tile, the last one alone.  Measured, us of two kernels / one: forward 512 x 512 → 2 x 1024 13.5 / 14.1 (12.4 without the
-// product), 300 x 2048 → 2 x 6144 24.4 / 32.6, 3800 x 2048 → 2 x 6144 145 / 122; backward 20000 x 128 → 1024 54.7 / 68.4, 4096 x 3072
-// → 1024 34.5 / 35.8, 1900 x 3072 → 8192 102 / 89, 8997 x 2048 → 6144 245 / 195.
-static bool swiglu_pays(int M, int features, int K, int kind, int num_sms) {
-  if (g_force_swiglu) return true;
-  const bool backward = kind == SWIGLU_BACKWARD;
+// Is the activation in the epilogue faster than the product followed by a kernel of its own?  The product is taken as it would run:
+// plain_choice, or in K parts, which the epilogue cannot have; both sides by the same table.  A 256-column tile's epilogue takes
+// 4.2 us forward and 12 backward (memory latency; it has eight warps) and runs under the main loop of the next tile, the last one
+// alone.  The other constants are fitted to 376 calls of 64..17000 rows of the configured layers and their shards (`swiglu_sweep` of
+// kernels/profile_cases.py): the picks take 0.3 % longer than the faster of the two, 13 of them more than 3 %; by unsplit times of
+// short calls, as this rule was, 1.6 % forward and 0.5 % backward, 42 of them more than 3 % (on 72 layers drawn later the picks
+// take 1.5 and 0.3 % longer; up to 120 rows the forward epilogue would be up to 20 % faster where the rule says no).  Measured, us of two kernels / one: forward 512 x 512 → 2 x 1024 9.2 / 10.1, 427 x
+// 3072 → 2 x 4096 28.5 / 23.4, 3798 x 2048 → 2 x 3072 101 / 73; backward 148 x 2048 → 3072 12.8 / 14.1, 904 x 4096 → 14336 128 / 135
+// (in K parts), 4074 x 2048 → 1536 36.1 / 38.5, 7784 x 2048 → 3072 127 / 114, 16646 x 2048 → 6144 516 / 390.
+// Forward passes with and without storing the product (a recomputing step has both) get one answer: they agree bit for bit.
+static bool swiglu_pays(int M, int features, int K, bool backward, int num_sms) {
+  if (g_force_swiglu) return g_force_swiglu == 1 || (g_force_swiglu == 2 && !backward);
   const int nk = (K + GEMM_BK - 1) / GEMM_BK, N = backward ? features : 2 * features, pairs = num_sms / 2;
-  const int bn = plan_pair(M, N, K, pairs, backward).bn;
-  const PlainTimes t = plain_times(M, N, K, backward, num_sms, bn);
-  const double plain = t.pair < t.w128 ? (t.pair < t.w256 ? t.pair : t.w256) : (t.w128 < t.w256 ? t.w128 : t.w256);
-  const int fbn = backward ? bn : 256;
-  const double* c = pair_us[fbn / 64];
+  const PairPlan two = plan_parts(M, N, K, backward, num_sms);
+  const int fbn = backward ? plan_pair(M, N, K, pairs, true).bn : 256;
+  double us;
+  const bool is_long = plain_choice(M, N, K, backward, num_sms, &us) != 0 && us >= 50.0 && nk > 2;
+  const double* c = is_long ? long_us[backward][fbn / 64 - 1] : pair_us[fbn / 64];
   const long waves = ((long)((M + 255) / 256) * ((N + fbn - 1) / fbn) + pairs - 1) / pairs;
-  const double last = (backward ? 12.0 : kind == SWIGLU_STORE ? 5.0 : 3.5) * fbn / 256;
-  const double main_loop = (nk * c[0] + c[1]) * (backward ? 1.15 : 1.0);
-  const double epilogue = (backward ? 14.5 : kind == SWIGLU_STORE ? 4.2 : 3.1) * fbn / 256;
+  const double main_loop = nk * c[0] + c[1], epilogue = (backward ? 12.0 : 4.2) * fbn / 256, last = (backward ? 18.0 : 2.0) * fbn / 256;
   const double fused = c[2] + waves * (main_loop > epilogue ? main_loop : epilogue) + last;
-  return fused < plain + 2.5 + (backward ? 10.0 : 6.0) * M * features / 5.5e6;
+  return (us < 50.0 ? 1.1 : 1.0) * fused < two.cost + (backward ? 1.0 : 3.5) + (backward ? 12.0 : 9.0) * M * features / 5.5e6;
 }
 
 // `C +=`.  Where 128-row tiles would not fill the chip once and be split even so, the parts add in L2 as they come: the
@@ -763,15 +765,14 @@ extern "C" int kb_gemm_row_stats(const void* A, const void* B, void* C, int M, i
 
 // SwiGLU in the epilogue of the GEMM beside it (see SwigluOut in gemm_pair_sm100.cu).  A [M, K], B [2 * features, K], X [M, 2 *
 // features] (or null), H [M, features]; backward: A [M, K], B [K, features], X and dX [M, 2 * features].  X, H and dX are
-// contiguous, features a multiple of 8.  kb_gemm_swiglu_pays: is that the faster way (kind: 0 forward with X, 1 backward, 2 forward
-// without X)?
-extern "C" int kb_gemm_swiglu_pays(int M, int features, int K, int kind) {
+// contiguous, features a multiple of 8.  kb_gemm_swiglu_pays: is that the faster way?
+extern "C" int kb_gemm_swiglu_pays(int M, int features, int K, int backward) {
   using namespace kb;
   if (M <= 0 || features <= 0 || K <= 0 || (features & 7) || features > (1 << 29)) return 0;
-  return swiglu_pays(M, features, K, kind, device_sm_count()) ? 1 : 0;
+  return swiglu_pays(M, features, K, backward != 0, device_sm_count()) ? 1 : 0;
 }
-// Measurement and test aid: take the epilogue for every shape.
-extern "C" void kb_gemm_swiglu_force(int on) { kb::g_force_swiglu = on != 0; }
+// Measurement and test aid: 0 by the rule, 1 the epilogue for every shape, 2 forward only, 3 never.
+extern "C" void kb_gemm_swiglu_force(int how) { kb::g_force_swiglu = how; }
 
 static bool swiglu_args_ok(int M, int features, int K, int lda, int ldb, const void* A, const void* B, const void* X, const void* Y) {
   return M > 0 && features > 0 && K > 0 && features <= (1 << 29) && !((features | lda | ldb) & 7) &&

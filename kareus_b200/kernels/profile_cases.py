@@ -12,6 +12,8 @@ Timing tables (CUDA events, no profiler; L2 flushed between launches):
     python -m kareus_b200.kernels.profile_cases gemm_table      # model GEMM shapes at TP 1 and TP 8, vs cuBLAS
     python -m kareus_b200.kernels.profile_cases attn_table      # flash attention forward/backward, vs the wheel
     python -m kareus_b200.kernels.profile_cases small_table     # small calls: device and host time
+    python -m kareus_b200.kernels.profile_cases swiglu_sweep    # drawn layers: SwiGLU in the GEMMs' epilogues or on its own
+    python -m kareus_b200.kernels.profile_cases route_sweep     # drawn layers: kernels, widths and K parts of bf16 outputs
     python -m torch.distributed.run --nproc-per-node N --master-addr 127.0.0.1 \
         -m kareus_b200.kernels.profile_cases fused                # the eight fused GEMM+collective kernels at TP N
 """
@@ -241,6 +243,117 @@ def small_table() -> None:
     KC.check_status()
 
 
+def _in_turn(fns, rounds: int = 5, target_ms: float = 4.0) -> dict:
+    """Median us per call of each function through CUDA graphs of 8 calls, in another order each round: calls of 100 us and more
+    take up to a fifth longer after one that draws more power.  ``fn(i)`` is call number i."""
+    import random
+    rng, graphs = random.Random(0), {}
+    for name, fn in fns.items():
+        fn(0)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for i in range(8):
+                fn(i)
+        graphs[name] = g
+    us = {name: [] for name in fns}
+    for r in range(rounds + 1):
+        for name, g in rng.sample(list(graphs.items()), len(graphs)):
+            reps = 1 if r == 0 else max(1, int(target_ms * 1e3 / (8 * us[name][0])))
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            g.replay()
+            a.record()
+            for _ in range(reps):
+                g.replay()
+            b.record()
+            torch.cuda.synchronize()
+            us[name].append(a.elapsed_time(b) * 1e3 / (8 * reps))
+    return {name: sorted(t[1:])[rounds // 2] for name, t in us.items()}
+
+
+def _drawn_layers(n: int, seed: int):
+    """Rows, hidden and feed-forward widths of the configured layers and their tensor-parallel shards."""
+    import math
+    import random
+    rng = random.Random(seed)
+    widths = ((512, 1024), (2048, 6144), (2048, 3072), (2048, 1536), (3072, 8192), (3072, 4096), (3072, 2048), (4096, 14336),
+              (4096, 7168), (4096, 3584), (5120, 13824), (5120, 6912))
+    return [(int(round(math.exp(rng.uniform(math.log(64), math.log(17000))))),) + widths[i % len(widths)] for i in range(n)]
+
+
+def _picks(rows) -> None:
+    """What the picks cost: ``rows`` are (label, us of the pick, us of the best)."""
+    import math
+    over = sorted(((p / b, label, p, b) for label, p, b in rows), reverse=True)
+    print(f"{len(rows)} calls: picks take {math.exp(sum(math.log(r[0]) for r in over) / len(over)) - 1:.1%} longer than the best")
+    for r in over[:10]:
+        print(f"  {r[0]:.3f}  {r[1]}: {r[2]:.1f} us, best {r[3]:.1f}")
+
+
+def swiglu_sweep(n: int = 72, seed: int = 0) -> None:
+    """The rule that puts a SwiGLU into the epilogue of the GEMM beside it against both ways."""
+    import kareus_b200.kernels as K
+    from . import cuda as KC
+    L = KC.lib()
+    rows = {"forward": [], "backward": []}
+    for T, h, f in _drawn_layers(n, seed):
+        R = max(1, min(8, int(3e8 // (2 * (T * h + 2 * f * h + 3 * T * f)))))     # operands that do not stay in L2
+        rnd = lambda *s: [torch.randn(*s, device="cuda").bfloat16() for _ in range(R)]
+        x, w1, w2, y = rnd(T, h), rnd(2 * f, h), rnd(h, f), rnd(T, 2 * f)
+        try:
+            L.kb_gemm_swiglu_force(1)
+            us = _in_turn({"forward one": lambda i: K.linear_swiglu(x[i % R], w1[i % R]),
+                           "forward two": lambda i: K.swiglu_fwd(K.gemm(x[i % R], w1[i % R])),
+                           "backward one": lambda i: K.linear_swiglu_dgrad(x[i % R], w2[i % R], y[i % R]),
+                           "backward two": lambda i: K.swiglu_bwd(K.gemm(x[i % R], w2[i % R], trans_b=False), y[i % R])})
+        finally:
+            L.kb_gemm_swiglu_force(0)
+        for backward, d in enumerate(rows):
+            one, two = us[d + " one"], us[d + " two"]
+            rows[d].append((f"{T} rows, {h} and {f}", one if L.kb_gemm_swiglu_pays(T, f, h, backward) else two, min(one, two)))
+        del x, w1, w2, y
+    for d, r in rows.items():
+        print(d, end=", ")
+        _picks(r)
+    KC.check_status()
+
+
+def route_sweep(n: int = 24, seed: int = 0) -> None:
+    """Kernel, tile width and K parts that plain bf16 outputs get against every kernel and width and a range of K parts."""
+    import kareus_b200.kernels as K
+    from . import cuda as KC
+    L = KC.lib()
+    rows = []
+    for T, h, f in _drawn_layers(n, seed):
+        for N, Kd, tb in ((2 * f, h, True), (h, f, True), (f, h, False), (h, 2 * f, False)):
+            R = max(1, min(8, int(3e8 // (2 * (T * Kd + N * Kd + T * N)))))
+            rnd = lambda *s: [torch.randn(*s, device="cuda").bfloat16() for _ in range(R)]
+            a, b = rnd(T, Kd), rnd(*((N, Kd) if tb else (Kd, N)))
+            call = lambda i: K.gemm(a[i % R], b[i % R], trans_b=tb)
+
+            def forced(width, ks, bn):
+                def fn(i):
+                    L.kb_gemm_force_width(width)
+                    L.kb_gemm_parts_force(ks, bn)
+                    try:
+                        return call(i)
+                    finally:
+                        L.kb_gemm_force_width(0)
+                        L.kb_gemm_parts_force(0, 0)
+                return fn
+            fns = {"pick": call}
+            fns.update({f"width {w}": forced(w, 1, 0) for w in (64, 128, 192, 256, -128, -256)})
+            if Kd >= 1024:
+                fns.update({f"{ks} parts of {bn}": forced(0, ks, bn) for ks in (2, 3, 4, 6, 8, 12, 16) for bn in (128, 192, 256)
+                            if Kd // 64 // ks >= 4})
+            us = _in_turn(fns, rounds=3, target_ms=2.0)
+            best = min(us, key=us.get)
+            rows.append((f"{T} x {N} x {Kd}{'' if tb else ' (input gradient)'}, best with {best}", us["pick"], us[best]))
+            del a, b
+    _picks(rows)
+    KC.check_status()
+
+
 def attn_table() -> None:
     """Causal GQA flash attention at the 3B shapes (per nanobatch of 4 sequences): TP 1 (24/8 heads) and
     TP 8 (3/1 heads), forward and backward, vs the flash-attention wheel when it is installed."""
@@ -433,7 +546,7 @@ def collectives_table() -> None:
 
 
 # every command of this module: tables (CUDA events) and single-kernel cases (for a profiler capture)
-CASES = ("collectives", "memory_table", "small_table", "wgrad_sweep", "gemm_table", "attn_table", "fused", "gemm",
+CASES = ("collectives", "memory_table", "small_table", "wgrad_sweep", "swiglu_sweep", "route_sweep", "gemm_table", "attn_table", "fused", "gemm",
          "gemm_one_sm", "gemm_wgrad", "attn_fwd", "attn_bwd", "norm", "swiglu", "rope", "ce", "adamw", "step")
 
 
@@ -448,6 +561,10 @@ def main(case: str, reps: int = 3) -> None:
         return memory_table()
     if case == "wgrad_sweep":
         return wgrad_sweep()
+    if case == "swiglu_sweep":
+        return swiglu_sweep()
+    if case == "route_sweep":
+        return route_sweep()
     if case == "gemm_table":
         return gemm_table()
     if case == "attn_table":

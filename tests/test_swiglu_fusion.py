@@ -159,3 +159,80 @@ def test_passes_with_and_without_a_product_take_the_same_kernels(monkeypatch):
             assert with_ == without, (tokens, h, f)
             answers.add(with_)
     assert answers == {True, False}
+
+
+@pytest.mark.parametrize("backward,tokens,h,f,fused", [
+    # us of two kernels / one: 13 / 17, 18 / 22, 28 / 23, 21 / 18, 101 / 73, 866 / 590
+    (0, 157, 2048, 1536, 0), (0, 316, 3072, 2048, 0), (0, 427, 3072, 4096, 1), (0, 1237, 2048, 1536, 1), (0, 3798, 2048, 3072, 1),
+    (0, 16646, 2048, 6144, 1),
+    # 13 / 14, 13 / 14, 36 / 38, 52 / 58; a short last wave that the product alone has in K parts 128 / 135, 114 / 120
+    (1, 148, 2048, 3072, 0), (1, 357, 2048, 1536, 0), (1, 4074, 2048, 1536, 0), (1, 16806, 512, 1024, 0), (1, 904, 4096, 14336, 0),
+    (1, 900, 4096, 14336, 0),
+    # 127 / 114, 516 / 390, 216 / 173
+    (1, 7784, 2048, 3072, 1), (1, 16646, 2048, 6144, 1), (1, 6703, 2048, 6144, 1)])
+def test_epilogue_is_taken_where_it_is_faster_than_the_route_beside_it(backward, tokens, h, f, fused):
+    assert _library().kb_gemm_swiglu_pays(tokens, f, h, backward) == fused
+
+
+# ----------------------------------------------------------------------------- the kernels
+@pytest.fixture
+def force():
+    from kareus_b200.kernels import cuda as KC
+    yield lambda how: KC.lib().kb_gemm_swiglu_force(how)       # 1 everywhere, 2 forward only, 3 nowhere
+    KC.lib().kb_gemm_swiglu_force(0)
+
+
+def _steps(recompute, replay, seq=192, steps=3):
+    """Losses of some steps and the gradients of the last, on weights that no step changes."""
+    from kareus_b200.config import TrainConfig
+    from kareus_b200.kernels import cuda as KC
+    from kareus_b200.train.trainer import Trainer, synthetic_batch
+    cfg = get_model_config("tiny128")
+    tc = TrainConfig(micro_batch_size=2, global_batch_size=2, seq_len=seq, warmup_steps=0, lr=0.0, min_lr=0.0, seed=1)
+    tr = Trainer(cfg, ParallelConfig(num_nanobatches=2, recompute=recompute), tc, device="cuda")
+    tr.model.decoder.engine.replay = replay
+    batch = synthetic_batch(cfg, tc, tr.num_microbatches, seed=2)
+    losses = [tr.train_step(batch) for _ in range(steps)]
+    torch.cuda.synchronize()
+    KC.check_status()
+    if recompute and replay:
+        assert tr.model.decoder.engine.replayed_regions > 0
+    return losses, tr.optimizer.grad_flat.double()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("recompute,replay", [(False, False), (True, False), (True, True)])
+@pytest.mark.parametrize("how", [1, 2])
+def test_a_step_with_the_fusion_is_the_step_without(force, monkeypatch, how, recompute, replay):
+    force(3)
+    want_loss, want = _steps(recompute, replay)
+    taken = []
+    real = K.linear_swiglu_dgrad
+    monkeypatch.setattr(K, "linear_swiglu_dgrad", lambda *a: (lambda r: (taken.append(r is not None), r)[1])(real(*a)))
+    force(how)
+    loss, grads = _steps(recompute, replay)
+    # every backward pass of fc2 had fc1's product at hand, and used it or left it to the SwiGLU operator
+    assert taken and all(t == (how == 1) for t in taken)
+    # a different order of sums moves roundings to bf16 (2^-9) of two layers: well under a percent of a gradient's norm
+    assert all(abs(a - b) < 5e-3 for a, b in zip(loss, want_loss, strict=True))
+    assert (grads - want).norm() < 1e-2 * want.norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", [0, 1])
+@pytest.mark.parametrize("tokens,h,f", [(130, 512, 1024), (200, 3072, 8192), (400, 3072, 4096), (600, 2048, 3072), (2016, 512, 1024)])
+def test_recomputed_activation_is_the_one_of_the_forward_pass(force, how, tokens, h, f):
+    force(how)
+    layer = TransformerLayer(get_model_config("tiny128").replace(hidden_size=h, ffn_hidden_size=f), ParallelConfig(), CommFactory(), 0,
+                             torch.bfloat16, "cuda", seed=3)
+    x = torch.randn(tokens, h, device="cuda").bfloat16()
+    outs = []
+    for saving in (False, True):
+        ctxs = [OpContext() for _ in range(3)]
+        y = x
+        for c, op in zip(ctxs, (layer.fc1, layer.act, layer.fc2)):
+            c.requires_grad, c.chained = saving, True
+            (y,) = op.forward(c, y)
+            outs.append(y)
+    torch.cuda.synchronize()
+    assert torch.equal(outs[1], outs[4]) and torch.equal(outs[2], outs[5])
