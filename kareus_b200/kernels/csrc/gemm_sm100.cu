@@ -570,9 +570,10 @@ static PairPlan plan_parts(int M, int N, int K, bool b_mn, int num_sms) {
 // alone.  The other constants are fitted to 376 calls of 64..17000 rows of the configured layers and their shards (`swiglu_sweep` of
 // kernels/profile_cases.py): the picks take 0.3 % longer than the faster of the two, 13 of them more than 3 %; by unsplit times of
 // short calls, as this rule was, 1.6 % forward and 0.5 % backward, 42 of them more than 3 % (on 72 layers drawn later the picks
-// take 1.5 and 0.3 % longer; up to 120 rows the forward epilogue would be up to 20 % faster where the rule says no).  Measured, us of two kernels / one: forward 512 x 512 → 2 x 1024 9.2 / 10.1, 427 x
-// 3072 → 2 x 4096 28.5 / 23.4, 3798 x 2048 → 2 x 3072 101 / 73; backward 148 x 2048 → 3072 12.8 / 14.1, 904 x 4096 → 14336 128 / 135
-// (in K parts), 4074 x 2048 → 1536 36.1 / 38.5, 7784 x 2048 → 3072 127 / 114, 16646 x 2048 → 6144 516 / 390.
+// take 1.5 and 0.3 % longer; up to 120 rows the forward epilogue would be up to 20 % faster where the rule says no).  Measured, us
+// of two kernels / one: forward 324 x 512 → 2 x 1024 7.6 / 9.0, 427 x 3072 → 2 x 4096 28.5 / 23.4, 3798 x 2048 → 2 x 3072 101 / 73;
+// backward 148 x 2048 → 3072 12.8 / 14.1, 904 x 4096 → 14336 128 / 135 (in K parts), 4074 x 2048 → 1536 36.1 / 38.5, 7784 x 2048 →
+// 3072 127 / 114, 16646 x 2048 → 6144 516 / 390.
 // Forward passes with and without storing the product (a recomputing step has both) get one answer: they agree bit for bit.
 static bool swiglu_pays(int M, int features, int K, bool backward, int num_sms) {
   if (g_force_swiglu) return g_force_swiglu == 1 || (g_force_swiglu == 2 && !backward);

@@ -87,7 +87,7 @@ class PartitionExecutor:
         fwd, bwd = self.chunk.fwd, self.chunk.bwd
         self._seed(self.chunk.fwd_graph, self.inputs, "main")
         if not self.backward:
-            fwd.run_steps(self.ctxs, fwd.steps[: self.step.index], streams=self.streams, grad_enabled=False)
+            fwd.run_steps(self.ctxs, fwd.steps[: self.step.index], streams=self.streams, grad_enabled=not self.par.recompute)
             return
         fwd.run(self.ctxs, streams=self.streams, grad_enabled=True)
         final = self.chunk.fwd_graph.final["main"]
@@ -103,7 +103,7 @@ class PartitionExecutor:
                 resource_shape: Tuple[Optional[int], Optional[int]] = (16, 1024)) -> None:
         sched = _OneKeySchedule(self.key, CommConfig(tuple(overlap_window), tuple(resource_shape)))
         self.program.run_steps(self.ctxs, [self.step], schedule=sched, streams=self.streams,
-                               grad_enabled=False, release_saved=False)
+                               grad_enabled=not self.par.recompute, release_saved=False)
 
     def slots(self):
         return dict(self.step.slots)

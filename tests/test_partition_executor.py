@@ -21,6 +21,26 @@ def test_executor_runs_one_partition_repeatedly(key):
         PartitionExecutor(cfg, ParallelConfig(num_nanobatches=2), "fwd_attn", 4, 32, dtype="fp32")  # needs tp > 1
 
 
+@pytest.mark.parametrize("recompute", [False, True])
+def test_forward_partitions_are_those_of_the_run_they_are_timed_for(monkeypatch, recompute):
+    """fc1 leaves its product in memory in a run that keeps its activations, and not in the first pass of one that recomputes them."""
+    import kareus_b200.kernels as K
+    from kareus_b200.kernels import ref
+    stored = []
+
+    def fused(x, w, store=True):
+        stored.append(store)
+        y = ref.gemm(x, w, False, True, None, None)
+        return (y if store else None), ref.swiglu_fwd(y)
+    monkeypatch.setattr(K, "linear_swiglu", fused)
+    ex = PartitionExecutor(get_model_config("tiny"), ParallelConfig(num_nanobatches=2, recompute=recompute), "fwd_trail", 4, 32,
+                           dtype="fp32")
+    stored.clear()
+    for _ in range(3):
+        ex.execute(("linear_0", "none"), (8, 1024))
+    assert stored == [not recompute] * 3
+
+
 def test_evaluator_and_nonpartition(tmp_path):
     class Clock:
         t = 0.0
