@@ -26,6 +26,7 @@ CSRC = HERE / "csrc"
 OBJ = HERE / "build"
 LIB = HERE / "libkareus_b200.so"
 FASTCALL_SRC = CSRC / "torch" / "fastcall.cpp"
+FASTCALL_DEPS = (FASTCALL_SRC, CSRC / "native_calls.h")
 FASTCALL = HERE / "_fastcall.so"
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -61,7 +62,7 @@ def is_current() -> bool:
 
 def _fastcall_digest() -> str:
     import torch
-    h = hashlib.sha256(FASTCALL_SRC.read_bytes())
+    h = hashlib.sha256(b"".join(p.read_bytes() for p in FASTCALL_DEPS))
     h.update(f"{torch.__version__} {sysconfig.get_config_var('SOABI')}".encode())
     return h.hexdigest()
 

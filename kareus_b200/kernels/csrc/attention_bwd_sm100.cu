@@ -37,6 +37,7 @@
 #include "launch.h"
 #include "pdl.cuh"
 #include "host_utils.h"
+#include "native_calls.h"
 #include "attention_chunks.h"
 #include <string.h>
 

@@ -38,6 +38,7 @@
 #include "launch.h"
 #include "pdl.cuh"
 #include "host_utils.h"
+#include "native_calls.h"
 #include <string.h>
 
 namespace kb {

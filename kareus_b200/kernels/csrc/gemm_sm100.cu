@@ -15,6 +15,7 @@
 #include "launch.h"
 #include "pdl.cuh"
 #include "host_utils.h"
+#include "native_calls.h"
 #include "gemm_plan.h"
 #include <stdlib.h>
 

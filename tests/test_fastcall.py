@@ -1,5 +1,6 @@
 """The native GEMM and attention calls take what they can launch as it lies, and leave everything else to the Python statements."""
 import math
+import re
 
 import pytest
 import torch
@@ -21,6 +22,17 @@ def test_calls_without_a_launch_are_left_alone():
         assert K._FAST.gemm(x, a, False, True, None) is None
         assert K._FAST.attention_fwd(x, a, a, 1.0, True, 0) is None
     assert torch.equal(K.gemm(a, a), K.ref.gemm(a, a))
+
+
+def test_both_sides_of_a_native_call_include_its_signature():
+    from kareus_b200.kernels import build
+    header = (build.CSRC / "native_calls.h").read_text()
+    called = set(re.findall(r"\bkb_\w+(?=\()", build.FASTCALL_SRC.read_text()))
+    assert called == set(re.findall(r"\bkb_\w+(?=\()", header)) and len(called) == 7
+    for name in called:
+        sources = [p for p in build.CSRC.glob("*.cu") if re.search(rf'extern "C" \w+ {name}\(', p.read_text())]
+        assert len(sources) == 1 and '#include "native_calls.h"' in sources[0].read_text(), name
+    assert build.CSRC / "native_calls.h" in build.FASTCALL_DEPS
 
 
 def _outcome(fn):
