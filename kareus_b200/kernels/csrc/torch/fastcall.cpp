@@ -279,4 +279,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", nullptr, -1, methods, 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__fastcall() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__fastcall() {
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "torch_version", KB_TORCH_VERSION) != 0) Py_CLEAR(m);
+  return m;
+}

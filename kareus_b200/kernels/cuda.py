@@ -46,13 +46,19 @@ def lib() -> ctypes.CDLL:
 
 
 def _load_fastcall() -> None:
-    """The extension module that takes plain GEMM and attention calls without the statements of this file."""
+    """The extension module that takes plain GEMM and attention calls without the statements of this file.  They run all calls
+    where it is missing or was built for another PyTorch."""
     import kareus_b200.kernels as K
     try:
         from . import _fastcall
+        built_for = getattr(_fastcall, "torch_version", "of another version")
+        if built_for != torch.__version__:
+            raise ImportError(f"built for PyTorch {built_for}, this is {torch.__version__}")
     except ImportError as e:
-        raise KernelError(f"{_HERE / '_fastcall.so'} cannot be loaded ({e}): build it with "
-                          "`python -m kareus_b200.kernels.build`") from e
+        import warnings
+        warnings.warn(f"{_HERE / '_fastcall.so'} cannot be loaded ({e}): GEMM and attention calls take more host time; build it "
+                      "with `python -m kareus_b200.kernels.build`", RuntimeWarning, stacklevel=3)
+        return
     _fastcall.init(K._LAUNCHES, _check)
     for idx, t in _STATUS.items():
         _fastcall.set_status(idx, t.data_ptr())

@@ -1,6 +1,8 @@
 """The native GEMM and attention calls take what they can launch as it lies, and leave everything else to the Python statements."""
 import math
 import re
+import sys
+import types
 
 import pytest
 import torch
@@ -22,6 +24,37 @@ def test_calls_without_a_launch_are_left_alone():
         assert K._FAST.gemm(x, a, False, True, None) is None
         assert K._FAST.attention_fwd(x, a, a, 1.0, True, 0) is None
     assert torch.equal(K.gemm(a, a), K.ref.gemm(a, a))
+
+
+@pytest.mark.parametrize("module", [None, types.SimpleNamespace(torch_version="1.0"), types.SimpleNamespace()])
+def test_library_loads_without_the_module(monkeypatch, module):
+    """Missing, built for another PyTorch, built from older sources: every call takes the Python statements."""
+    from kareus_b200.kernels import build, cuda as KC
+    if not build.LIB.exists():
+        pytest.skip("native library not built")
+    monkeypatch.setattr(KC, "_LIB", None)
+    monkeypatch.setattr(K, "_FAST", None)
+    monkeypatch.delattr(K, "_fastcall", raising=False)
+    monkeypatch.setitem(sys.modules, "kareus_b200.kernels._fastcall", module)
+    with pytest.warns(RuntimeWarning, match="cannot be loaded"):
+        KC.lib()
+    assert KC.is_loaded() and K._FAST is None
+    a = torch.randn(8, 16, dtype=torch.bfloat16)
+    assert torch.equal(K.gemm(a, a), K.ref.gemm(a, a))
+
+
+def test_build_goes_on_without_the_module(monkeypatch, tmp_path):
+    from kareus_b200.kernels import build
+
+    def fails(force=False):
+        raise RuntimeError("no Python.h")
+    monkeypatch.setattr(build, "build_fastcall", fails)
+    monkeypatch.setattr(build, "is_current", lambda: True)
+    monkeypatch.setattr(build, "FASTCALL", tmp_path / "_fastcall.so")
+    build.FASTCALL.write_bytes(b"of other sources")
+    with pytest.warns(RuntimeWarning, match="no Python.h"):
+        assert build.build() == build.LIB
+    assert not build.FASTCALL.exists()
 
 
 def test_both_sides_of_a_native_call_include_its_signature():
