@@ -16,6 +16,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <climits>
+#include <cstdio>
 #include <cstdlib>
 
 #include "../native_calls.h"
@@ -71,6 +72,15 @@ bool finish(int rc, const char* what, long launches) {
   return !PyErr_Occurred() && PyList_SetItem(g_counter, 0, PyLong_FromLong(n + launches)) == 0;
 }
 
+// The same with the shape in the error, as the Python statements have it.
+bool finish_gemm(int rc, int64_t M, int64_t N, int64_t K, long launches) {
+  char what[96] = "gemm";
+  if (rc != 0)
+    std::snprintf(what, sizeof(what), "gemm M=%lld N=%lld K=%lld", static_cast<long long>(M), static_cast<long long>(N),
+                  static_cast<long long>(K));
+  return finish(rc, what, launches);
+}
+
 template <typename F>
 int without_gil(F f) {
   int rc;
@@ -107,7 +117,7 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const int rc = without_gil([&] {
       return kb_gemm_accum_bf16(pa, pb, pc, M, N, K, ta, lda, !tb, ldb, static_cast<int>(N), 0, pw, status, stream);
     });
-    if (!finish(rc, "gemm", n ? 2 : 1)) return nullptr;
+    if (!finish_gemm(rc, M, N, K, n ? 2 : 1)) return nullptr;
     Py_INCREF(args[4]);
     return args[4];
   }
@@ -121,7 +131,7 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int rc = without_gil([&] {
     return kb_gemm_work_bf16(pa, pb, pc, M, N, K, ta, lda, !tb, ldb, static_cast<int>(N), 0, pw, status, stream);
   });
-  if (!finish(rc, "gemm", n ? 2 : 1)) return nullptr;
+  if (!finish_gemm(rc, M, N, K, n ? 2 : 1)) return nullptr;
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }

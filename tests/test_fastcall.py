@@ -174,6 +174,29 @@ def test_attention_forms(monkeypatch, form):
     # every dK and dV has one sum of its own, and dQ the contributions of at most two key tiles: bitwise the same each time
     _same_as_python(monkeypatch, lambda: K.attention_bwd(do, q, k, v, out, lse, scale, causal=True, q_offset=off, **kw))
 
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_errors_name_the_shape(monkeypatch, native, accumulate):
+    """An error of the runtime that nobody has fetched (a device number out of range, refused on the host) is reported by the next call."""
+    import ctypes
+    from kareus_b200.kernels import cuda as KC
+    KC.lib()
+    a, b = _bf16(72, 200), _bf16(136, 200)
+    c = torch.zeros(72, 136, device="cuda") if accumulate else None
+    K.gemm(a, b, accumulate=c)
+    assert (K._FAST.gemm(a, b, False, True, c) is not None)
+    if not native:
+        monkeypatch.setattr(K, "_FAST", None)
+    assert ctypes.CDLL("libcudart.so.12").cudaSetDevice(1 << 20) != 0
+    with pytest.raises(KC.KernelError, match="gemm M=72 N=136 K=200 failed"):
+        K.gemm(a, b, accumulate=c)
+    torch.cuda.synchronize()
+    K.gemm(a, b, accumulate=c)
+
+
 @pytest.mark.gpu
 def test_transforms_and_switches(monkeypatch):
     a, b = _bf16(4, 64, 64), _bf16(64, 64)
