@@ -78,8 +78,13 @@ def _outcome(fn):
     return r if isinstance(r, tuple) else (r,)
 
 
-def _same_as_python(monkeypatch, fn):
-    from kareus_b200.kernels import launch_count
+def _same_as_python(monkeypatch, fn, direct, native):
+    """``fn`` with and without the native calls; ``direct`` is the native call itself, which takes the arguments or (``native``
+    false) leaves them alone."""
+    from kareus_b200.kernels import cuda as KC, launch_count
+    KC.lib()
+    KC.status_word(torch.device("cuda", torch.cuda.current_device()))
+    assert K._FAST is not None and (direct() is not None) == native
     n0 = launch_count()
     fast = _outcome(fn)
     n1 = launch_count()
@@ -117,7 +122,8 @@ def test_gemm_forms(monkeypatch, form, ta, tb):
         "three": lambda: (a[None], b), "one_row": lambda: (a[:, :1] if ta else a[:1], b),
         "no_rows": lambda: (a[:, :0] if ta else a[:0], b), "mismatch": lambda: (a[8:] if ta else a[:, 8:], b),
     }[form]()
-    _same_as_python(monkeypatch, lambda: K.gemm(a, b, trans_a=ta, trans_b=tb))
+    _same_as_python(monkeypatch, lambda: K.gemm(a, b, trans_a=ta, trans_b=tb), lambda: K._FAST.gemm(a, b, ta, tb, None),
+                    form in ("plain", "rows", "param", "one_row"))
 
 
 @pytest.mark.gpu
@@ -125,16 +131,22 @@ def test_gemm_forms(monkeypatch, form, ta, tb):
 @pytest.mark.parametrize("form", ["plain", "view", "transposed", "bf16", "shape"])
 def test_accumulating_gemm_forms(monkeypatch, tokens, form):
     torch.manual_seed(0)
-    dy, x = _bf16(tokens, 3072), _bf16(tokens, 2048)      # more tiles than SMs: parts of a K split add in order
-    base = torch.randn(3072, 2048, device="cuda")
+    from kareus_b200.kernels import cuda as KC
+    dy, x = _bf16(tokens, 5120), _bf16(tokens, 3072)
+    # over 4096 rows the parts of a K split add in order, through a workspace
+    assert (KC.lib().kb_gemm_accum_scratch_floats(5120, 3072, tokens, 0) > 0) == (tokens == 4096)
+    base = torch.randn(5120, 3072, device="cuda")
+
+    def out():
+        return {"plain": lambda: base.clone(), "view": lambda: torch.cat([base, base])[5120:], "transposed": lambda: base.t().contiguous().t(),
+                "bf16": lambda: base.bfloat16(), "shape": lambda: base[:8].clone()}[form]()
 
     def call():
-        c = {"plain": lambda: base.clone(), "view": lambda: torch.cat([base, base])[3072:], "transposed": lambda: base.t().clone().t(),
-             "bf16": lambda: base.bfloat16(), "shape": lambda: base[:8].clone()}[form]()
+        c = out()
         r = K.gemm(dy, x, trans_a=True, trans_b=False, accumulate=c)
         assert r is c
         return r
-    _same_as_python(monkeypatch, call)
+    _same_as_python(monkeypatch, call, lambda: K._FAST.gemm(dy, x, True, False, out()), form in ("plain", "view"))
 
 
 @pytest.mark.gpu
@@ -164,16 +176,17 @@ def test_attention_forms(monkeypatch, form):
         k, v = k[:, :, :1], v[:, :, :1]
     elif form == "no_queries":
         q = q[:0]
+    native = form in ("packed", "four_dims", "off_keys", "batch_major")
     fwd = lambda: K.attention_fwd(q, k, v, scale, causal=True, q_offset=off, **kw)
-    _same_as_python(monkeypatch, fwd)
+    _same_as_python(monkeypatch, fwd, lambda: None if kw else K._FAST.attention_fwd(q, k, v, scale, True, off), native)
     r = _outcome(fwd)
     if isinstance(r, type):
         return
     out, lse = r
     do = _bf16(*out.shape)
     # every dK and dV has one sum of its own, and dQ the contributions of at most two key tiles: bitwise the same each time
-    _same_as_python(monkeypatch, lambda: K.attention_bwd(do, q, k, v, out, lse, scale, causal=True, q_offset=off, **kw))
-
+    _same_as_python(monkeypatch, lambda: K.attention_bwd(do, q, k, v, out, lse, scale, causal=True, q_offset=off, **kw),
+                    lambda: None if kw else K._FAST.attention_bwd(q, k, v, scale, True, off, do, out, lse), native)
 
 
 @pytest.mark.gpu
@@ -201,7 +214,7 @@ def test_errors_name_the_shape(monkeypatch, native, accumulate):
 def test_transforms_and_switches(monkeypatch):
     a, b = _bf16(4, 64, 64), _bf16(64, 64)
     K.gemm(a[0], b)
-    with pytest.raises(Exception):
+    with pytest.raises(RuntimeError, match="storage"):              # no data pointer under vmap: refused, as by the Python statements
         torch.vmap(lambda x: K.gemm(x, b))(a)
     monkeypatch.setenv("KAREUS_B200_LIBRARY_BASELINE", "1")
     n = K.launch_count()
