@@ -14,9 +14,10 @@
 //               (bf16 / fp32 output) or TMA reduce-add (fp32 `C +=`: the addition happens in L2, so
 //               nobody waits for the old value)
 //
-// K parts of a tile.  A bf16 output sums them from a workspace in a second small kernel, in order (EPI_PARTS).  `C +=`, ordered: the first part adds to C, the others store their sums to a workspace, which a
-// second small kernel adds part by part, so that every run gives the same bits.  Not ordered: all parts add in L2 as they
-// come; this is for outputs of few tiles, where the second launch would cost a third of the time (see gemm_sm100.cu).
+// K parts of a tile.  A bf16 output sums them from a workspace in a second small kernel, in order (EPI_PARTS).  `C +=`, ordered: the
+// first part adds to C, the others store their sums to a workspace, which a second small kernel adds part by part, so that every
+// run gives the same bits.  Not ordered: all parts add in L2 as they come; this is for outputs of few tiles, where the second launch
+// would cost a third of the time (see gemm_sm100.cu).
 //
 // BN is a run-time multiple of 64 (64..256): the launcher picks the width whose last wave is fullest.
 // Loads use no multicast: every CTA fetches its own halves.

@@ -506,7 +506,7 @@ static const double long_us[2][6][3] = {   // step, wave, call of 64, 128, 192, 
 // modelled time.  The table above was fitted to calls of up to about 50 us; longer ones run at lower clocks, and wide tiles,
 // which move fewer bytes for a product, lose less: fitted again to 133 calls of 45 to 700 us (rms 9 to 20 %) the picks take
 // 1.1 % longer than the best kernel and width of each, by the first table 3.6 % (3934 x 14264 x 5640: one-SM 668, pairs of 256
-// columns 521; 11384 x 2072 x 2584: 192 columns 137, 256 columns 120).
+// columns 521; input gradient 11384 x 2072 x 2584: 192 columns 137, 256 columns 120).
 static int plain_choice(int M, int N, int K, bool b_mn, int num_sms, double* us) {
   const int pairs = num_sms / 2, bn = plan_pair(M, N, K, pairs, b_mn).bn, nk = (K + GEMM_BK - 1) / GEMM_BK;
   const PlainTimes t = plain_times(M, N, K, b_mn, num_sms, bn);
@@ -533,7 +533,8 @@ static int g_force_parts = 0, g_force_parts_bn = 0;   // measurement and test ai
 // 15384 85 → 24 us, 128 x 1024 x 8192 28 → 18) and long sums whose last wave is short (3800 x 2048 x 12288 154 → 136; the
 // 4096 x 3072 input gradient of a 128256-word vocabulary 2233 → 2062).  Us per step, wave and MB of partial sums (written once, read
 // once) fitted to 3400 calls of 160 shapes (64..20000 rows, 1024..96000 deep; rms 8 to 13 %); unsplit times below 50 us are
-// 10 % too short there.  Over those shapes the picks take 0.82 of the unsplit time, the best ones 0.79, the worst 1.04 of it.
+// 10 % too short there.  Over those shapes the picks take 0.82 of the unsplit time, the best ones 0.79, the worst 1.04 of it
+// (`route_sweep` of kernels/profile_cases.py times every kernel, width and a range of parts for drawn layers).
 static PairPlan plan_parts(int M, int N, int K, bool b_mn, int num_sms) {
   static const double cost[2][5][3] = {{{}, {0.187, 1.39, 0.11}, {0.22, 2.6, 0.05}, {0.288, 2.1, 0.14}, {0.361, 2.06, 0.164}},
                                        {{}, {0.222, 0.0, 0.45}, {0.227, 0.44, 0.32}, {0.31, 1.16, 0.28}, {0.344, 1.6, 0.21}}};

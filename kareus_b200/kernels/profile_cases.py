@@ -3,6 +3,7 @@
     python -m kareus_b200.kernels.profile_cases gemm        # 8192 x 8192 x 8192 bf16, 3 launches
     python -m kareus_b200.kernels.profile_cases attn_fwd    # B4 H3 S4096 d128 causal, 3 launches
     python -m kareus_b200.kernels.profile_cases norm | swiglu | ce | adamw | rope
+    python -m kareus_b200.kernels.profile_cases gemm_epilogues   # what GEMM epilogues do besides storing, 5 GEMMs a repetition
 
 Each case touches more than the 126 MB L2 where DRAM figures matter but holds at most a few GB,
 and launches its kernel a handful of times so a ``--set full`` capture ends within minutes.
@@ -183,22 +184,23 @@ def small_table() -> None:
     """Small calls: device time (a CUDA graph of 20 calls) and host time per call (300 calls, nothing waited for), and the
     smoke model's training step with and without launch lists."""
     import time
-    from . import attention_cuda, cuda as KC
+    import kareus_b200.kernels as K
+    from . import cuda as KC
     dev = "cuda"
     rnd = lambda *shape: torch.randn(*shape, device=dev).bfloat16()
     x, w, dy, acc = rnd(328, 1032), rnd(776, 1032), rnd(328, 776), torch.zeros(776, 1032, device=dev)
     packed = rnd(459, 2, 2, 4 * 128)
     q, k, v = packed[..., :256].unflatten(-1, (2, 128)), packed[..., 256:384], packed[..., 384:]
-    out, lse = attention_cuda.forward(q, k, v, 128 ** -0.5)
+    out, lse = K.attention_fwd(q, k, v, 128 ** -0.5)
     do = torch.randn_like(out)
     xn, wn, gu = rnd(459, 2048), rnd(2048), rnd(459, 2 * 2048)
-    cases = [("gemm 328 x 776 x 1032", lambda: KC.gemm(x, w)),
-             ("its input gradient", lambda: KC.gemm(dy, w, trans_b=False)),
-             ("its weight gradient", lambda: KC.gemm(dy, x, trans_a=True, trans_b=False, accumulate=acc)),
-             ("attention forward, 2 x 459 tokens, 4/2 heads", lambda: attention_cuda.forward(q, k, v, 128 ** -0.5)),
-             ("attention backward", lambda: attention_cuda.backward(do, q, k, v, out, lse, 128 ** -0.5)),
-             ("rmsnorm forward 459 x 2048", lambda: KC.rmsnorm_fwd(xn, wn, 1e-5)),
-             ("swiglu forward 459 x 2048", lambda: KC.swiglu_fwd(gu))]
+    cases = [("gemm 328 x 776 x 1032", lambda: K.gemm(x, w)),
+             ("its input gradient", lambda: K.gemm(dy, w, trans_b=False)),
+             ("its weight gradient", lambda: K.gemm(dy, x, trans_a=True, trans_b=False, accumulate=acc)),
+             ("attention forward, 2 x 459 tokens, 4/2 heads", lambda: K.attention_fwd(q, k, v, 128 ** -0.5)),
+             ("attention backward", lambda: K.attention_bwd(do, q, k, v, out, lse, 128 ** -0.5)),
+             ("rmsnorm forward 459 x 2048", lambda: K.rmsnorm_fwd(xn, wn, 1e-5)),
+             ("swiglu forward 459 x 2048", lambda: K.swiglu_fwd(gu))]
     print("| call | device us | host us |\n|---|---|---|")
     side = torch.cuda.Stream()
     for name, fn in cases:
@@ -319,7 +321,8 @@ def swiglu_sweep(n: int = 72, seed: int = 0) -> None:
 
 
 def route_sweep(n: int = 24, seed: int = 0) -> None:
-    """Kernel, tile width and K parts that plain bf16 outputs get against every kernel and width and a range of K parts."""
+    """Kernel, tile width and K parts that plain bf16 outputs get against every kernel and width and a range of K parts.  The best
+    of about 25 medians is by chance some percent below its true time, for calls of milliseconds at the power limit more."""
     import kareus_b200.kernels as K
     from . import cuda as KC
     L = KC.lib()
@@ -547,7 +550,7 @@ def collectives_table() -> None:
 
 # every command of this module: tables (CUDA events) and single-kernel cases (for a profiler capture)
 CASES = ("collectives", "memory_table", "small_table", "wgrad_sweep", "swiglu_sweep", "route_sweep", "gemm_table", "attn_table", "fused", "gemm",
-         "gemm_one_sm", "gemm_wgrad", "attn_fwd", "attn_bwd", "norm", "swiglu", "rope", "ce", "adamw", "step")
+         "gemm_epilogues", "gemm_one_sm", "gemm_wgrad", "attn_fwd", "attn_bwd", "norm", "swiglu", "rope", "ce", "adamw", "step")
 
 
 def main(case: str, reps: int = 3) -> None:
@@ -578,6 +581,18 @@ def main(case: str, reps: int = 3) -> None:
         b = torch.randn(8192, 8192, device=dev).bfloat16()
         for _ in range(reps):
             KC.gemm(a, b)
+    elif case == "gemm_epilogues":
+        # SwiGLU with and without the product, its gradient, row statistics of logits, and a product in K parts
+        import kareus_b200.kernels as K
+        x, w1, w2 = (torch.randn(*s, device=dev).bfloat16() for s in ((8192, 3072), (16384, 3072), (3072, 8192)))
+        head, tgt = torch.randn(32768, 3072, device=dev).bfloat16(), torch.randint(0, 32768, (4096,), device=dev)
+        a, b = torch.randn(3800, 12288, device=dev).bfloat16(), torch.randn(2048, 12288, device=dev).bfloat16()
+        for _ in range(reps):
+            y, _ = K.linear_swiglu(x, w1)
+            K.linear_swiglu(x, w1, store=False)
+            K.linear_swiglu_dgrad(x, w2, y)
+            K.linear_cross_entropy_stats(x[:4096], head, tgt, 0, weight=torch.ones(4096, device=dev))
+            K.gemm(a, b)
     elif case == "gemm_one_sm":
         a = torch.randn(8192, 8192, device=dev).bfloat16()
         b = torch.randn(8192, 8192, device=dev).bfloat16()

@@ -70,6 +70,22 @@ def test_kernel_choice_for_plain_outputs():
     assert plan(2048, 8192, 3072, 1) == 256
 
 
+def test_long_calls_and_parts_of_k_for_plain_outputs():
+    L = _lib()
+    L.kb_gemm_plan.argtypes = [ctypes.c_int] * 5
+    L.kb_gemm_scratch_floats.argtypes = [ctypes.c_int] * 5
+    L.kb_gemm_scratch_floats.restype = ctypes.c_long
+    # beyond 50 us wide tiles on pairs: one-SM tiles took 668 us here and 521 on pairs, 192 columns 137 and 256 columns 120
+    assert L.kb_gemm_plan(3934, 14264, 5640, 0, 148) == 256 and L.kb_gemm_plan(11384, 2072, 2584, 1, 148) == 256
+    # long sums over few tiles and long sums with a short last wave go in parts, in whole tiles of 256 rows
+    for shape in [(203, 504, 15384, 0), (128, 1024, 8192, 0), (3800, 2048, 12288, 0), (4096, 3072, 128256, 1)]:
+        n = L.kb_gemm_scratch_floats(*shape, 148)
+        assert n > 0 and n % (256 * 64) == 0 and 4 * n <= 64e6, (shape, n)
+    # not full waves, narrow outputs of many rows, or sums too short for a part of four steps and a caller's workspace
+    for shape in [(16384, 16384, 3072, 0), (16384, 640, 3072, 0), (8192, 8192, 8192, 0), (128, 1024, 1016, 0), (128, 1024, 64, 1)]:
+        assert L.kb_gemm_scratch_floats(*shape, 148) == 0, shape
+
+
 def test_copy_driver_count_scales_with_output_width_and_budget():
     from kareus_b200.ops.fused import FusedAGGemm as F
     assert F.auto_drivers(12, 640) == 36 and F.auto_drivers(12, 1024) == 24 and F.auto_drivers(12, 2048) == 12
